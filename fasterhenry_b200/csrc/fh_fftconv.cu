@@ -1,6 +1,6 @@
 // The pFFT convolution K (*) q on the device, without a library FFT: pruned
-// mixed-radix (2, 3, 4, 5) Stockham transforms in shared memory, in FP32 or
-// FP64 (pfft/fft.rs:155-320 of the reference, re-designed for the GPU).
+// mixed-radix transforms, in FP32 or FP64 (pfft/fft.rs:155-320 of the
+// reference, re-designed for the GPU).
 //
 // The sources q live on the n0 x n1 x n2 grid; the aperiodic convolution
 // needs transforms of length m_a >= 2 n_a - 1 per axis (a torus of 2^a 3^b
@@ -15,15 +15,37 @@
 //   4. axis 1 inverse  C[n0][m1][m2]  -> B[n0][n1][m2]
 //   5. axis 2 inverse  B[n0][n1][m2]  -> A[n0][n1][n2]   (the potentials)
 //
-// Each step is one launch of fft_lines_kernel: a CTA loads a tile of lines
-// into shared memory (consecutive lines when they are contiguous, else
-// consecutive columns, so every global access is a run of adjacent
-// elements), zero-pads them to m, runs one Stockham pass per radix between
-// two shared buffers, and writes the first `keep` outputs.  Two real source
-// fields travel in one complex grid (real and imaginary parts), as in the
-// reference's convolver.  The kernel's spectrum is computed at set-up by the
-// same kernels (unpruned, FP64) from the wrapped kernel grid; it is real
-// because the wrapped kernel is even.
+// Each step is one launch.  What bounds a step is the shared-memory traffic
+// and the latency of its butterflies, not the device memory, so:
+//   * a length is cut into as few stages as possible (radices up to 16 in
+//     FP32, 12 in FP64, held in registers: 1200 = 8 x 10 x 15 instead of the
+//     five passes of a radix-4/2/3/5 chain);
+//   * the forward transform is decimated in frequency and the inverse in
+//     time, so every stage reads and writes the same places: one buffer of
+//     `lines` lines (a second one would halve the lines in flight), one
+//     barrier per stage, and the transformed axes stay in the stages' own
+//     order, which nothing but the spectrum's layout has to know;
+//   * strided steps take their first stage from device memory into registers
+//     and their last one back, so a line of k stages crosses shared memory
+//     k - 1 times, and zero padding is never loaded or stored;
+//   * in step 3 the last forward stage, the spectrum and the first inverse
+//     stage stay in registers.
+// Measured on 1200 x 1200 x 15 torus points (590 x 589 x 8 sources, two
+// grids), in us for the steps 1 to 5, against the radix-2/3/4/5 Stockham chain
+// with two buffers that came before:
+//   FP32   45 + 115 + 309 + 104 + 58 =  631   (104 + 284 + 1008 + 290 + 101)
+//   FP64  110 + 182 + 511 + 178 + 129 = 1110
+// FP32 issues instructions in 0.6 of the cycles (packed FP32 arithmetic, see
+// cadd; twiddles in rows of 16-byte loads) at 32 warps per SM; 256 and 384
+// threads per CTA measured within 5 %.
+//
+// The inverse runs on swapped real and imaginary parts: with s(z) the swap,
+// IDFT(z) = s(DFT(s(z))) and s(conj(w) z) = w s(z), so both directions share
+// one set of butterflies and twiddles.  Two real source fields travel in one
+// complex grid (real and imaginary parts), as in the reference's convolver.
+// The kernel's spectrum is computed at set-up by the same kernels (unpruned,
+// FP64) from the wrapped kernel grid; it is real because the wrapped kernel
+// is even.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -37,13 +59,13 @@
 namespace fhb {
 namespace {
 
-// Threads per CTA: 512 for FP32 (two CTAs, 32 warps per SM), 256 for FP64
-// (whose wider lines leave fewer butterflies per tile).
+// Threads per CTA, two CTAs per SM.
 template <class T>
 constexpr int fft_threads() {
     return sizeof(T) == 4 ? 512 : 256;
 }
-constexpr size_t kFftSmemBudget = 100 * 1024;  // two CTAs per SM
+constexpr size_t kFftSmemBudget = 110 * 1024;  // two CTAs per SM
+constexpr int kFftTilePoints = 8192;
 constexpr double kPi = 3.14159265358979323846;
 
 template <class T>
@@ -51,207 +73,431 @@ struct Cplx;
 template <>
 struct Cplx<float> {
     using type = float2;
+    using real = float;
 };
 template <>
 struct Cplx<double> {
     using type = double2;
+    using real = double;
 };
+__device__ __forceinline__ float2 cmake(float x, float y) { return make_float2(x, y); }
+__device__ __forceinline__ double2 cmake(double x, double y) { return make_double2(x, y); }
 
-template <class V>
-__device__ __forceinline__ V cmul(V a, V b) {
-    V r;
-    r.x = a.x * b.x - a.y * b.y;
-    r.y = a.x * b.y + a.y * b.x;
+// a + b, a - b and a + s t of complex numbers.  FP32: the packed two-element
+// instructions, one issue slot instead of two (these kernels are bound by
+// issue: 0.63 instructions per scheduler and cycle without them).
+__device__ __forceinline__ unsigned long long pack2(float2 a) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
     return r;
 }
+__device__ __forceinline__ float2 unpack2(unsigned long long a) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+    return r;
+}
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(a)), "l"(pack2(b)));
+    return unpack2(r);
+}
+__device__ __forceinline__ float2 csub(float2 a, float2 b) {
+    unsigned long long r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(a)), "l"(pack2(b)));
+    return unpack2(r);
+}
+__device__ __forceinline__ float2 caxpy(float s, float2 t, float2 a) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pack2(make_float2(s, s))), "l"(pack2(t)), "l"(pack2(a)));
+    return unpack2(r);
+}
+__device__ __forceinline__ float2 cscale(float s, float2 t) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(make_float2(s, s))), "l"(pack2(t)));
+    return unpack2(r);
+}
+__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ double2 caxpy(double s, double2 t, double2 a) {
+    return make_double2(a.x + s * t.x, a.y + s * t.y);
+}
+__device__ __forceinline__ double2 cscale(double s, double2 t) { return make_double2(s * t.x, s * t.y); }
+template <class V>
+__device__ __forceinline__ V cmul(V a, V b) {
+    return cmake(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+template <class V>
+__device__ __forceinline__ V cswap(V a) {
+    return cmake(a.y, a.x);
+}
 
-// R-point DFT of v in place, W = exp(sign 2 pi i / R).
-template <int R, class V, class T>
-__device__ __forceinline__ void small_dft(V (&v)[R], int sign) {
-    if constexpr (R == 2) {
-        V a = v[0], b = v[1];
-        v[0].x = a.x + b.x;
-        v[0].y = a.y + b.y;
-        v[1].x = a.x - b.x;
-        v[1].y = a.y - b.y;
-    } else if constexpr (R == 4) {
-        const V a = v[0], b = v[1], c = v[2], d = v[3];
-        V s0, s1, d0, d1;
-        s0.x = a.x + c.x, s0.y = a.y + c.y;
-        d0.x = a.x - c.x, d0.y = a.y - c.y;
-        s1.x = b.x + d.x, s1.y = b.y + d.y;
-        d1.x = b.x - d.x, d1.y = b.y - d.y;
-        // (b - d) times sign * i
-        V jd;
-        jd.x = -(T)sign * d1.y;
-        jd.y = (T)sign * d1.x;
-        v[0].x = s0.x + s1.x, v[0].y = s0.y + s1.y;
-        v[2].x = s0.x - s1.x, v[2].y = s0.y - s1.y;
-        v[1].x = d0.x + jd.x, v[1].y = d0.y + jd.y;
-        v[3].x = d0.x - jd.x, v[3].y = d0.y - jd.y;
-    } else {
-        // cos and sin of 2 pi k / R, k = 0 .. R-1
-        constexpr double c3[3] = {1.0, -0.5, -0.5};
-        constexpr double s3[3] = {0.0, 0.86602540378443864676, -0.86602540378443864676};
-        constexpr double c5[5] = {1.0, 0.30901699437494742410, -0.80901699437494742410, -0.80901699437494742410,
-                                  0.30901699437494742410};
-        constexpr double s5[5] = {0.0, 0.95105651629515357212, 0.58778525229247312917, -0.58778525229247312917,
-                                  -0.95105651629515357212};
-        V out[R];
+// ---------------------------------------------------------------------------
+// Register transforms: v <- DFT_R v, W = exp(-2 pi i / R), natural order in
+// and out.  2, 3, 4 and 5 directly; a product of coprime factors by the prime
+// factor map (no twiddles), 8, 9 and 16 by their two equal-base factors.
+// ---------------------------------------------------------------------------
+template <class V>
+__device__ __forceinline__ void dft2(V &a, V &b) {
+    const V t = csub(a, b);
+    a = cadd(a, b);
+    b = t;
+}
+template <class V>
+__device__ __forceinline__ void dft3(V &a, V &b, V &c) {
+    using T = decltype(a.x);
+    const V t = cadd(b, c), d = csub(b, c);
+    const T s = (T)0.86602540378443864676;
+    const V m = caxpy((T)-0.5, t, a);
+    a = cadd(a, t);
+    b = cmake(m.x + s * d.y, m.y - s * d.x);
+    c = cmake(m.x - s * d.y, m.y + s * d.x);
+}
+template <class V>
+__device__ __forceinline__ void dft4(V &a, V &b, V &c, V &d) {
+    const V s0 = cadd(a, c), d0 = csub(a, c), s1 = cadd(b, d), d1 = csub(b, d);
+    a = cadd(s0, s1);
+    c = csub(s0, s1);
+    b = cmake(d0.x + d1.y, d0.y - d1.x);
+    d = cmake(d0.x - d1.y, d0.y + d1.x);
+}
+template <class V>
+__device__ __forceinline__ void dft5(V &a, V &b, V &c, V &d, V &e) {
+    using T = decltype(a.x);
+    const T c1 = (T)0.30901699437494742410, c2 = (T)-0.80901699437494742410;
+    const T s1 = (T)0.95105651629515357212, s2 = (T)0.58778525229247312917;
+    const V t1 = cadd(b, e), t2 = cadd(c, d), t3 = csub(b, e), t4 = csub(c, d);
+    const V m1 = caxpy(c2, t2, caxpy(c1, t1, a)), m2 = caxpy(c1, t2, caxpy(c2, t1, a));
+    const V n1 = caxpy(s2, t4, cscale(s1, t3)), n2 = caxpy(-s1, t4, cscale(s2, t3));
+    a = cadd(a, cadd(t1, t2));
+    b = cmake(m1.x + n1.y, m1.y - n1.x);
+    e = cmake(m1.x - n1.y, m1.y + n1.x);
+    c = cmake(m2.x + n2.y, m2.y - n2.x);
+    d = cmake(m2.x - n2.y, m2.y + n2.x);
+}
+
+template <int R, class V>
+__device__ __forceinline__ void dft(V (&v)[R]);
+
+// N = A B coprime: input (B i + A j) mod N, output (B B' k + A A' l) mod N
+// with B B' = 1 mod A and A A' = 1 mod B.
+constexpr int inverse_mod(int a, int n) {
+    for (int k = 1; k < n; ++k)
+        if (a * k % n == 1) return k;
+    return 1;
+}
+template <int A, int B, class V>
+__device__ __forceinline__ void dft_coprime(V (&v)[A * B]) {
+    constexpr int N = A * B, bi = B * inverse_mod(B % A, A), ai = A * inverse_mod(A % B, B);
+    V t[B][A];
 #pragma unroll
-        for (int b = 0; b < R; ++b) {
-            V acc = v[0];
+    for (int j = 0; j < B; ++j) {
 #pragma unroll
-            for (int a = 1; a < R; ++a) {
-                const int e = (a * b) % R;
-                const T c = (T)(R == 3 ? c3[e] : c5[e]);
-                const T s = (T)sign * (T)(R == 3 ? s3[e] : s5[e]);
-                acc.x += v[a].x * c - v[a].y * s;
-                acc.y += v[a].x * s + v[a].y * c;
-            }
-            out[b] = acc;
-        }
+        for (int i = 0; i < A; ++i) t[j][i] = v[(B * i + A * j) % N];
+        dft<A>(t[j]);
+    }
 #pragma unroll
-        for (int b = 0; b < R; ++b) v[b] = out[b];
+    for (int k = 0; k < A; ++k) {
+        V u[B];
+#pragma unroll
+        for (int j = 0; j < B; ++j) u[j] = t[j][k];
+        dft<B>(u);
+#pragma unroll
+        for (int l = 0; l < B; ++l) v[(bi * k + ai * l) % N] = u[l];
     }
 }
 
-// One Stockham pass of radix R over `lines` interleaved lines of length m
-// (element t of line l at t * lines + l), src -> dst; tw holds
-// exp(-2 pi i t / m) in shared memory.
-template <int R, class V, class T>
-__device__ void stockham_pass(const V *__restrict__ src, V *__restrict__ dst, int m, int lines, int Ns,
-                              const V *__restrict__ tw, int sign) {
-    const int nb = m / R;
-    const int tw_step = m / (Ns * R);
-    for (int idx = threadIdx.x; idx < nb * lines; idx += blockDim.x) {
-        const int line = idx % lines, j = idx / lines;
+// cos and sin of 2 pi k / N for the equal-base products (N = 8, 9, 16).
+template <int N>
+__device__ constexpr double root_cos(int k) {
+    constexpr double c8[4] = {1.0, 0.70710678118654752440, 0.0, -0.70710678118654752440};
+    constexpr double c9[5] = {1.0, 0.76604444311897803520, 0.17364817766693034885, -0.5, -0.93969262078590838405};
+    constexpr double c16[10] = {1.0, 0.92387953251128675613, 0.70710678118654752440, 0.38268343236508977173, 0.0,
+                                -0.38268343236508977173, -0.70710678118654752440, -0.92387953251128675613, -1.0,
+                                -0.92387953251128675613};
+    return N == 8 ? c8[k & 3] : N == 9 ? c9[k % 5] : c16[k % 10];
+}
+template <int N>
+__device__ constexpr double root_sin(int k) {
+    constexpr double s8[4] = {0.0, 0.70710678118654752440, 1.0, 0.70710678118654752440};
+    constexpr double s9[5] = {0.0, 0.64278760968653932632, 0.98480775301220805937, 0.86602540378443864676,
+                              0.34202014332566873304};
+    constexpr double s16[10] = {0.0, 0.38268343236508977173, 0.70710678118654752440, 0.92387953251128675613, 1.0,
+                                0.92387953251128675613, 0.70710678118654752440, 0.38268343236508977173, 0.0,
+                                -0.38268343236508977173};
+    return N == 8 ? s8[k & 3] : N == 9 ? s9[k % 5] : s16[k % 10];
+}
+// N = A B: input i B + j, output k + A l.
+template <int A, int B, class V>
+__device__ __forceinline__ void dft_product(V (&v)[A * B]) {
+    using T = decltype(v[0].x);
+    V t[B][A];
+#pragma unroll
+    for (int j = 0; j < B; ++j) {
+#pragma unroll
+        for (int i = 0; i < A; ++i) t[j][i] = v[i * B + j];
+        dft<A>(t[j]);
+    }
+#pragma unroll
+    for (int k = 0; k < A; ++k) {
+        V u[B];
+#pragma unroll
+        for (int j = 0; j < B; ++j) {
+            if (j * k == 0)
+                u[j] = t[j][k];
+            else if (4 * j * k == A * B)  // -i
+                u[j] = cmake(t[j][k].y, -t[j][k].x);
+            else
+                u[j] = cmul(t[j][k], cmake((T)root_cos<A * B>(j * k), (T)-root_sin<A * B>(j * k)));
+        }
+        dft<B>(u);
+#pragma unroll
+        for (int l = 0; l < B; ++l) v[k + A * l] = u[l];
+    }
+}
+template <int R, class V>
+__device__ __forceinline__ void dft(V (&v)[R]) {
+    if constexpr (R == 2) dft2(v[0], v[1]);
+    else if constexpr (R == 3) dft3(v[0], v[1], v[2]);
+    else if constexpr (R == 4) dft4(v[0], v[1], v[2], v[3]);
+    else if constexpr (R == 5) dft5(v[0], v[1], v[2], v[3], v[4]);
+    else if constexpr (R == 6) dft_coprime<2, 3>(v);
+    else if constexpr (R == 8) dft_product<4, 2>(v);
+    else if constexpr (R == 9) dft_product<3, 3>(v);
+    else if constexpr (R == 10) dft_coprime<2, 5>(v);
+    else if constexpr (R == 12) dft_coprime<4, 3>(v);
+    else if constexpr (R == 15) dft_coprime<3, 5>(v);
+    else if constexpr (R == 16) dft_product<4, 4>(v);
+}
+
+// ---------------------------------------------------------------------------
+// Stages.
+// ---------------------------------------------------------------------------
+// x / d for x < 2^16, d < 2^16, magic = ceil(2^32 / d) (d > 1): the error
+// x (magic d - 2^32) / d stays below 2^32 / d.
+__device__ __forceinline__ int fast_div(int x, unsigned magic) {
+    return magic ? (int)__umulhi((unsigned)x, magic) : x;
+}
+
+// v_r <- v_r w^r from a row of the stage's table (r = 0 included, padded to an
+// even length: 16-byte loads at constant offsets).
+__host__ __device__ constexpr int twiddle_row(int R) { return (R + 1) & ~1; }
+template <int R>
+__device__ __forceinline__ void twiddle(float2 (&v)[R], const float2 *__restrict__ row) {
+    const float4 *__restrict__ q = reinterpret_cast<const float4 *>(row);
+#pragma unroll
+    for (int h = 0; h < twiddle_row(R) / 2; ++h) {
+        const float4 w = __ldg(q + h);
+        if (h > 0) v[2 * h] = cmul(v[2 * h], make_float2(w.x, w.y));
+        if (2 * h + 1 < R) v[2 * h + 1] = cmul(v[2 * h + 1], make_float2(w.z, w.w));
+    }
+}
+template <int R>
+__device__ __forceinline__ void twiddle(double2 (&v)[R], const double2 *__restrict__ row) {
+#pragma unroll
+    for (int r = 1; r < R; ++r) v[r] = cmul(v[r], __ldg(row + r));
+}
+
+// Where a tile's lines lie in device memory.
+template <class V>
+struct Lines {
+    const V *src;   // point 0 of line 0 (input), `inner` between points, 1 between lines
+    V *dst;
+    int inner;
+    int count;      // lines of this tile
+    int n_in, keep; // points read, points written; the rest is zero
+};
+
+// One stage of radix R = ax.R[st] over the tile's lines: point b R S + k + r S
+// of every block b, offset k, by one thread.  Element (point t, line l) of the
+// shared buffer is t * 2^lg + l (kContig: l * pitch + t).
+//   DIT = false: DFT then twiddle (forward); true: twiddle then DFT (inverse).
+//   GIN / GOUT: from / to device memory instead of the buffer.
+//   MID: the forward's last stage, the spectrum and the inverse's first.
+template <int R, class T, bool CONTIG, bool DIT, bool GIN, bool GOUT, bool MID>
+__device__ __forceinline__ void fft_stage(typename Cplx<T>::type *buf, const FftAxis &ax, int st, int lg, int pitch,
+                                          const typename Cplx<T>::type *__restrict__ tw_all,
+                                          const Lines<typename Cplx<T>::type> &g, const T *__restrict__ spectrum) {
+    using V = typename Cplx<T>::type;
+    const int S = ax.S[st], nb = ax.m / R;
+    const V *__restrict__ tw = tw_all + ax.tw[st];
+    const int total = nb << lg;
+    for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
+        int l, j;
+        if (CONTIG) {
+            l = fast_div(idx, ax.magic_nb[st]);
+            j = idx - l * nb;
+        } else {
+            l = idx & ((1 << lg) - 1);
+            j = idx >> lg;
+        }
+        const int b = fast_div(j, ax.magic_S[st]);
+        const int k = j - b * S;
+        const int t0 = b * R * S + k;
         V v[R];
+        const bool live = CONTIG || l < g.count;
 #pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = src[(j + r * nb) * lines + line];
-        const int k = j % Ns;
-#pragma unroll
-        for (int r = 1; r < R; ++r) {
-            V w = tw[k * r * tw_step];
-            if (sign > 0) w.y = -w.y;
-            v[r] = cmul(v[r], w);
+        for (int r = 0; r < R; ++r) {
+            const int t = t0 + r * S;
+            if (GIN) {
+                v[r] = cmake((T)0, (T)0);
+                if (live && t < g.n_in) v[r] = g.src[t * g.inner + l];
+                if (DIT) v[r] = cswap(v[r]);
+            } else {
+                v[r] = buf[CONTIG ? l * pitch + t : (t << lg) + l];
+            }
         }
-        small_dft<R, V, T>(v, sign);
-        const int base = (j / Ns) * Ns * R + k;
+        if (DIT && S > 1) twiddle<R>(v, tw + k * twiddle_row(R));
+        dft<R>(v);
+        if (MID) {
 #pragma unroll
-        for (int r = 0; r < R; ++r) dst[(base + r * Ns) * lines + line] = v[r];
+            for (int r = 0; r < R; ++r) {
+                const T s = live ? spectrum[(t0 + r * S) * g.inner + l] : (T)0;
+                v[r] = cmake(s * v[r].y, s * v[r].x);  // swapped: the inverse begins
+            }
+            dft<R>(v);
+        }
+        if (!DIT && !MID && S > 1) twiddle<R>(v, tw + k * twiddle_row(R));
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int t = t0 + r * S;
+            if (GOUT) {
+                if (live && t < g.keep) g.dst[t * g.inner + l] = DIT || MID ? cswap(v[r]) : v[r];
+            } else {
+                buf[CONTIG ? l * pitch + t : (t << lg) + l] = v[r];
+            }
+        }
     }
 }
 
-// The transform of `lines` lines of length m held in a (interleaved), with b
-// as the second buffer; returns the buffer holding the result.
-template <class V, class T>
-__device__ V *stockham(V *a, V *b, int m, int lines, const FftAxis &ax, const V *__restrict__ tw, int sign) {
-    int Ns = 1;
-    for (int f = 0; f < ax.nfac; ++f) {
-        const int R = ax.fac[f];
-        __syncthreads();
-        if (R == 4)
-            stockham_pass<4, V, T>(a, b, m, lines, Ns, tw, sign);
-        else if (R == 2)
-            stockham_pass<2, V, T>(a, b, m, lines, Ns, tw, sign);
-        else if (R == 3)
-            stockham_pass<3, V, T>(a, b, m, lines, Ns, tw, sign);
-        else
-            stockham_pass<5, V, T>(a, b, m, lines, Ns, tw, sign);
-        Ns *= R;
-        V *t = a;
-        a = b;
-        b = t;
+template <class T, bool CONTIG, bool DIT, bool GIN, bool GOUT, bool MID>
+__device__ __forceinline__ void fft_stage_any(typename Cplx<T>::type *buf, const FftAxis &ax, int st, int lg,
+                                              int pitch, const typename Cplx<T>::type *__restrict__ tw,
+                                              const Lines<typename Cplx<T>::type> &g,
+                                              const T *__restrict__ spectrum) {
+    switch (ax.R[st]) {
+#define FHB_FFT_RADIX(r)                                                                             \
+    case r:                                                                                          \
+        fft_stage<r, T, CONTIG, DIT, GIN, GOUT, MID>(buf, ax, st, lg, pitch, tw, g, spectrum);       \
+        break;
+        FHB_FFT_RADIX(1)
+        FHB_FFT_RADIX(2)
+        FHB_FFT_RADIX(3)
+        FHB_FFT_RADIX(4)
+        FHB_FFT_RADIX(5)
+        FHB_FFT_RADIX(6)
+        FHB_FFT_RADIX(8)
+        FHB_FFT_RADIX(9)
+        FHB_FFT_RADIX(10)
+        FHB_FFT_RADIX(12)
+        default:
+            if constexpr (sizeof(T) == 4) {
+                if (ax.R[st] == 15)
+                    fft_stage<15, T, CONTIG, DIT, GIN, GOUT, MID>(buf, ax, st, lg, pitch, tw, g, spectrum);
+                else
+                    fft_stage<16, T, CONTIG, DIT, GIN, GOUT, MID>(buf, ax, st, lg, pitch, tw, g, spectrum);
+            }
+#undef FHB_FFT_RADIX
     }
-    __syncthreads();
-    return a;
 }
+
+enum FftKind { kForward, kInverse, kFused };
 
 // One pruned axis transform over a batch of arrays.  An array holds
 // `outer` x len x `inner` complex elements (len = n_in for the input, keep
-// for the output); line (o, c) is elements (o len + t) inner + c.  Lines are
-// tiled `tile` at a time: consecutive o when inner == 1 (each line
-// contiguous), else consecutive c.  With `spectrum`, the forward transform is
-// multiplied by spectrum[t inner + c] (real) and transformed back (sign
-// flipped) before the write.  in and out may be the same array (the fused
-// axis-0 step): a CTA reads its whole tile before it writes, and tiles are
-// disjoint.
-template <class T>
-__global__ void __launch_bounds__(fft_threads<T>())
-    fft_lines_kernel(const typename Cplx<T>::type *in, typename Cplx<T>::type *out,
-                     int64_t in_stride, int64_t out_stride, int64_t outer, int64_t inner, int n_in, int keep,
-                     FftAxis ax, const typename Cplx<T>::type *__restrict__ tw_global, int sign, int tile,
-                     const T *__restrict__ spectrum) {
+// for the output); line (o, c) is elements (o len + t) inner + c.  A tile is
+// 2^lg lines of consecutive c (tail tiles: fewer).  kFused: forward, times
+// spectrum[t inner + c] (real), and back; in and out may be the same array,
+// since a CTA reads its whole tile before it writes and tiles are disjoint.
+template <class T, int KIND>
+__global__ void __launch_bounds__(fft_threads<T>(), 2)
+    fft_strided_kernel(const typename Cplx<T>::type *in, typename Cplx<T>::type *out, int64_t in_stride,
+                       int64_t out_stride, int64_t outer, int inner, int n_in, int keep, FftAxis ax, int lg,
+                       const typename Cplx<T>::type *__restrict__ tw, const T *__restrict__ spectrum) {
     using V = typename Cplx<T>::type;
     extern __shared__ __align__(16) unsigned char fft_smem[];
-    V *bufa = reinterpret_cast<V *>(fft_smem);
-    V *bufb = bufa + (size_t)tile * ax.m;
-    V *tw = bufb + (size_t)tile * ax.m;  // the twiddles, read by every pass
-    const int m = ax.m;
-    for (int t = threadIdx.x; t < m; t += blockDim.x) tw[t] = tw_global[t];
-    const V *src = in + (int64_t)blockIdx.y * in_stride;
-    V *dst = out + (int64_t)blockIdx.y * out_stride;
-    const bool contiguous = inner == 1;
-    const int64_t tiles = contiguous ? (outer + tile - 1) / tile : outer * ((inner + tile - 1) / tile);
+    V *buf = reinterpret_cast<V *>(fft_smem);
+    const int per = (inner + (1 << lg) - 1) >> lg;
+    const int64_t tiles = outer * per;
+    const int last = ax.nst - 1;
     for (int64_t tt = blockIdx.x; tt < tiles; tt += gridDim.x) {
-        int64_t o0, c0;
-        int lines;
-        if (contiguous) {
-            o0 = tt * tile;
-            c0 = 0;
-            lines = (int)(outer - o0 < tile ? outer - o0 : (int64_t)tile);
-        } else {
-            const int64_t per = (inner + tile - 1) / tile;
-            o0 = tt / per;
-            c0 = (tt % per) * tile;
-            lines = (int)(inner - c0 < tile ? inner - c0 : (int64_t)tile);
+        const int64_t o = tt / per;
+        const int c0 = (int)(tt - o * per) << lg;
+        Lines<V> g;
+        g.inner = inner;
+        g.count = min(1 << lg, inner - c0);
+        g.n_in = n_in;
+        g.keep = keep;
+        g.src = in + (int64_t)blockIdx.y * in_stride + o * n_in * inner + c0;
+        g.dst = out + (int64_t)blockIdx.y * out_stride + o * keep * inner + c0;
+        const T *spec = KIND == kFused ? spectrum + c0 : nullptr;
+        if (last == 0) {
+            fft_stage_any<T, false, KIND == kInverse, true, true, KIND == kFused>(buf, ax, 0, lg, 0, tw, g, spec);
+            continue;
         }
-        __syncthreads();  // the previous tile's reads of the buffers are done
-        // load (zero-padded to m)
-        for (int idx = threadIdx.x; idx < lines * m; idx += blockDim.x) {
-            int l, t;
-            if (contiguous) {
-                l = idx / m;
-                t = idx % m;
-            } else {
-                t = idx / lines;
-                l = idx % lines;
+        if (KIND != kInverse) {
+            fft_stage_any<T, false, false, true, false, false>(buf, ax, 0, lg, 0, tw, g, spec);
+            for (int st = 1; st < last; ++st) {
+                __syncthreads();
+                fft_stage_any<T, false, false, false, false, false>(buf, ax, st, lg, 0, tw, g, spec);
             }
-            V v;
-            v.x = v.y = (T)0;
-            if (t < n_in)
-                v = contiguous ? src[(o0 + l) * (int64_t)n_in + t] : src[(o0 * n_in + t) * inner + c0 + l];
-            bufa[t * lines + l] = v;
+            __syncthreads();
+            fft_stage_any<T, false, false, false, KIND == kForward, KIND == kFused>(buf, ax, last, lg, 0, tw, g, spec);
         }
-        V *res = stockham<V, T>(bufa, bufb, m, lines, ax, tw, sign);
-        if (spectrum) {
-            for (int idx = threadIdx.x; idx < lines * m; idx += blockDim.x) {
-                const int t = idx / lines, l = idx % lines;
-                const T s = spectrum[(int64_t)t * inner + c0 + l];
-                V v = res[idx];
-                v.x *= s;
-                v.y *= s;
-                res[idx] = v;
+        if (KIND != kForward) {
+            if (KIND == kInverse) fft_stage_any<T, false, true, true, false, false>(buf, ax, last, lg, 0, tw, g, spec);
+            for (int st = last - 1; st > 0; --st) {
+                __syncthreads();
+                fft_stage_any<T, false, true, false, false, false>(buf, ax, st, lg, 0, tw, g, spec);
             }
-            V *other = res == bufa ? bufb : bufa;
-            res = stockham<V, T>(res, other, m, lines, ax, tw, -sign);
+            __syncthreads();
+            fft_stage_any<T, false, true, false, true, false>(buf, ax, 0, lg, 0, tw, g, spec);
         }
-        for (int idx = threadIdx.x; idx < lines * keep; idx += blockDim.x) {
-            int l, t;
-            if (contiguous) {
-                l = idx / keep;
-                t = idx % keep;
-            } else {
-                t = idx / lines;
-                l = idx % lines;
-            }
-            const V v = res[t * lines + l];
-            if (contiguous)
-                dst[(o0 + l) * (int64_t)keep + t] = v;
-            else
-                dst[(o0 * keep + t) * inner + c0 + l] = v;
+        __syncthreads();  // the next tile's first stage writes the buffer
+    }
+}
+
+// The same for contiguous lines (inner = 1, axis 2): a tile of `lines` whole
+// lines is one run of device memory, copied in and out of the buffer in order
+// and transformed there.
+template <class T, int KIND>
+__global__ void __launch_bounds__(fft_threads<T>(), 2)
+    fft_contiguous_kernel(const typename Cplx<T>::type *in, typename Cplx<T>::type *out, int64_t in_stride,
+                          int64_t out_stride, int64_t outer, int n_in, int keep, FftAxis ax, int lg,
+                          unsigned magic_in, unsigned magic_keep, const typename Cplx<T>::type *__restrict__ tw) {
+    using V = typename Cplx<T>::type;
+    extern __shared__ __align__(16) unsigned char fft_smem[];
+    V *buf = reinterpret_cast<V *>(fft_smem);
+    const int lines = 1 << lg, pitch = ax.m | 1;
+    const int64_t tiles = (outer + lines - 1) >> lg;
+    const Lines<V> none = {};
+    for (int64_t tt = blockIdx.x; tt < tiles; tt += gridDim.x) {
+        const int64_t o0 = tt << lg;
+        const int count = (int)min((int64_t)lines, outer - o0);
+        const V *src = in + (int64_t)blockIdx.y * in_stride + o0 * n_in;
+        V *dst = out + (int64_t)blockIdx.y * out_stride + o0 * keep;
+        const int pad = ax.m - n_in;
+        for (int idx = threadIdx.x; idx < count * n_in; idx += blockDim.x) {
+            const int l = fast_div(idx, magic_in);
+            const V v = src[idx];
+            buf[l * pitch + idx - l * n_in] = KIND == kInverse ? cswap(v) : v;
         }
+        for (int idx = threadIdx.x; idx < (pad << lg); idx += blockDim.x)
+            buf[(idx & (lines - 1)) * pitch + n_in + (idx >> lg)] = cmake((T)0, (T)0);
+        if (count < lines)  // a tail tile: the missing lines are transformed too
+            for (int idx = threadIdx.x; idx < (lines - count) * pitch; idx += blockDim.x)
+                buf[count * pitch + idx] = cmake((T)0, (T)0);
+        for (int k = 0; k < ax.nst; ++k) {
+            __syncthreads();
+            fft_stage_any<T, true, KIND == kInverse, false, false, false>(
+                buf, ax, KIND == kInverse ? ax.nst - 1 - k : k, lg, pitch, tw, none, nullptr);
+        }
+        __syncthreads();
+        for (int idx = threadIdx.x; idx < count * keep; idx += blockDim.x) {
+            const int l = fast_div(idx, magic_keep);
+            const V v = buf[l * pitch + idx - l * keep];
+            dst[idx] = KIND == kInverse ? cswap(v) : v;
+        }
+        __syncthreads();  // the next tile's loads write the buffer
     }
 }
 
@@ -283,65 +529,145 @@ __global__ void wrapped_kernel_kernel(double2 *__restrict__ out, int64_t n0, int
     }
 }
 
+// The spectrum, scaled by 1 / P, from the FP64 transform's order to the
+// convolution's: map[a] gives for each place of axis a the place of the same
+// frequency in the FP64 transform.
 template <class T>
-__global__ void spectrum_store_kernel(const double2 *__restrict__ in, T *__restrict__ out, int64_t total) {
+__global__ void spectrum_store_kernel(const double2 *__restrict__ in, T *__restrict__ out, int64_t m0, int64_t m1,
+                                      int64_t m2, const int *__restrict__ map) {
+    const int64_t total = m0 * m1 * m2;
     const double scale = 1.0 / (double)total;
-    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < total; p += (int64_t)gridDim.x * blockDim.x)
-        out[p] = (T)(in[p].x * scale);
+    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < total; p += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t k = p % m2, rest = p / m2, j = rest % m1, i = rest / m1;
+        out[p] = (T)(in[((int64_t)map[i] * m1 + map[m0 + j]) * m2 + map[m0 + m1 + k]].x * scale);
+    }
 }
 
 unsigned blocks_of(int64_t work, int threads, int64_t cap = 148 * 16) {
     return (unsigned)std::max<int64_t>(1, std::min<int64_t>((work + threads - 1) / threads, cap));
 }
 
-// Lines per CTA: as many as two buffers of them and the twiddles fit the
-// shared-memory budget, up to about 8,192 points per tile (short lines come
-// many to a tile).
+unsigned magic_of(int d) { return d > 1 ? (unsigned)(((uint64_t(1) << 32) + (uint64_t)d - 1) / (uint64_t)d) : 0u; }
+
+// log2 of the lines per tile: lines of 64 bytes or more per point (8 FP32, 4
+// FP64) where two CTAs of them fit an SM, else fewer; short lines come up to
+// kFftTilePoints points to a tile.
 template <class T>
-int tile_for(int m) {
+int tile_lg(int m, int64_t inner) {
     const size_t elem = sizeof(typename Cplx<T>::type);
-    const size_t per = 2 * elem * (size_t)m;
-    const size_t want = std::max<size_t>(16, 8192 / (size_t)m);
-    const size_t room = kFftSmemBudget > elem * (size_t)m ? kFftSmemBudget - elem * (size_t)m : 0;
-    return (int)std::max<size_t>(1, std::min<size_t>(want, room / per));
+    int lg = 0;
+    while (lg < 9) {
+        const size_t next = (size_t)2 << lg;
+        if (next * (size_t)(m | 1) * elem > kFftSmemBudget) break;
+        if (next * elem > 64 && next * (size_t)m > (size_t)kFftTilePoints) break;
+        if (inner > 1 && (int64_t)1 << lg >= inner) break;
+        ++lg;
+    }
+    return lg;
 }
 
 // One axis step: outer x n_in x inner -> outer x keep x inner, `batch` arrays.
-template <class T>
+template <class T, int KIND>
 fh_status axis_step(const void *in, void *out, int64_t in_stride, int64_t out_stride, int64_t outer, int64_t inner,
-                    int n_in, int keep, const FftAxis &ax, const void *tw, int sign, const T *spectrum, int batch,
+                    int n_in, int keep, const FftAxis &ax, const void *tw, const T *spectrum, int batch,
                     cudaStream_t s, fh_error_info *err) {
     using V = typename Cplx<T>::type;
-    const int tile = tile_for<T>(ax.m);
-    const size_t smem = sizeof(V) * ((2 * (size_t)tile + 1) * ax.m);
+    const int lg = tile_lg<T>(ax.m, inner);
+    const size_t smem = sizeof(V) * ((size_t)(ax.m | 1) << lg);
     if (smem > 227 * 1024)
         return fail(err, FH_ERR_PFFT, "pFFT convolution: axis length " + std::to_string(ax.m) +
                                           " does not fit the transform kernel's shared memory");
-    const int64_t tiles = inner == 1 ? (outer + tile - 1) / tile : outer * ((inner + tile - 1) / tile);
-    FHB_CUDA(cudaFuncSetAttribute(fft_lines_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int64_t tiles = inner == 1 && KIND != kFused ? (outer + (1 << lg) - 1) >> lg
+                                                       : outer * ((inner + (1 << lg) - 1) >> lg);
     const unsigned gx = (unsigned)std::max<int64_t>(1, std::min<int64_t>(tiles, 148 * 8));
-    fft_lines_kernel<T><<<dim3(gx, (unsigned)batch), fft_threads<T>(), smem, s>>>(
-        static_cast<const V *>(in), static_cast<V *>(out), in_stride, out_stride, outer, inner, n_in, keep, ax,
-        static_cast<const V *>(tw), sign, tile, spectrum);
+    const dim3 grid(gx, (unsigned)batch);
+    // the contiguous form exists for plain transforms; a fused step of a
+    // single line (m1 = m2 = 1) is a strided one with one line per tile
+    if (inner == 1 && KIND != kFused) {
+        constexpr int K = KIND == kFused ? kForward : KIND;
+        FHB_CUDA(cudaFuncSetAttribute(fft_contiguous_kernel<T, K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)smem));
+        fft_contiguous_kernel<T, K><<<grid, fft_threads<T>(), smem, s>>>(
+            static_cast<const V *>(in), static_cast<V *>(out), in_stride, out_stride, outer, n_in, keep, ax, lg,
+            magic_of(n_in), magic_of(keep), static_cast<const V *>(tw));
+    } else {
+        FHB_CUDA(cudaFuncSetAttribute(fft_strided_kernel<T, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)smem));
+        fft_strided_kernel<T, KIND><<<grid, fft_threads<T>(), smem, s>>>(
+            static_cast<const V *>(in), static_cast<V *>(out), in_stride, out_stride, outer, (int)inner, n_in, keep, ax,
+            lg, static_cast<const V *>(tw), spectrum);
+    }
     FHB_CUDA(cudaGetLastError());
     return FH_OK;
 }
 
 }  // namespace
 
-bool fft_axis_plan(int64_t m, FftAxis &ax) {
+// The place of every frequency of an axis after the forward stages: stage s
+// writes residue r of the frequencies of its block to offset r S.
+std::vector<int> fft_places(const FftAxis &ax) {
+    std::vector<int> place((size_t)ax.m);
+    for (int f = 0; f < ax.m; ++f) {
+        int rest = f, at = 0;
+        for (int s = 0; s < ax.nst; ++s) {
+            at += rest % ax.R[s] * ax.S[s];
+            rest /= ax.R[s];
+        }
+        place[(size_t)f] = at;
+    }
+    return place;
+}
+
+// Radices of a length: the fewest stages, then an odd last one (stage S = 1
+// strides the shared buffer by R: an odd R keeps a half-warp's lines off each
+// other's banks), then the smallest largest radix (registers).
+bool fft_axis_plan(int64_t m, bool fp32, FftAxis &ax) {
     ax = FftAxis();
     if (m < 1 || m > kFftMaxLength) return false;
-    ax.m = (int)m;
-    int64_t r = m;
-    // radix 4 first, then 2, 3, 5
-    for (int p : {4, 2, 3, 5})
-        while (r % p == 0) {
-            if (ax.nfac == kFftMaxFactors) return false;
-            ax.fac[ax.nfac++] = p;
-            r /= p;
+    static const int all[] = {2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16};
+    const int count = fp32 ? 11 : 9;
+    int best[kFftMaxStages], trial[kFftMaxStages], best_n = 0, best_cost = 1 << 30;
+    struct Search {
+        const int *radix;
+        int count;
+        int *trial, *best, *best_n, *best_cost;
+        void go(int64_t rest, int depth, int largest) const {
+            if (rest == 1) {
+                const int cost = 100 * depth + (depth > 1 && trial[depth - 1] % 2 == 0 ? 20 : 0) + largest;
+                if (cost < *best_cost) {
+                    *best_cost = cost;
+                    *best_n = depth;
+                    std::copy(trial, trial + depth, best);
+                }
+                return;
+            }
+            if (depth == kFftMaxStages || 100 * (depth + 1) > *best_cost) return;
+            for (int i = count - 1; i >= 0; --i)
+                if (rest % radix[i] == 0) {
+                    trial[depth] = radix[i];
+                    go(rest / radix[i], depth + 1, std::max(largest, radix[i]));
+                }
         }
-    return r == 1;
+    };
+    if (m == 1)
+        best[best_n++] = 1;  // one stage that changes nothing
+    else
+        Search{all, count, trial, best, &best_n, &best_cost}.go(m, 0, 0);
+    if (best_n == 0) return false;
+    ax.m = (int)m;
+    ax.nst = best_n;
+    int len = ax.m, tw = 0;
+    for (int s = 0; s < best_n; ++s) {
+        ax.R[s] = best[s];
+        len /= best[s];
+        ax.S[s] = len;
+        ax.magic_S[s] = magic_of(len);
+        ax.magic_nb[s] = magic_of(ax.m / best[s]);
+        ax.tw[s] = tw;
+        tw += twiddle_row(best[s]) * len;
+    }
+    ax.tw_count = tw;
+    return true;
 }
 
 size_t fftconv_work_elems(const FftConvShape &sh) {
@@ -355,62 +681,86 @@ template <class T>
 fh_status fftconv_setup(const FftConvShape &sh, double spacing, FftConvTables &tab, cudaStream_t s,
                         fh_error_info *err) {
     using V = typename Cplx<T>::type;
+    constexpr bool fp32 = sizeof(T) == 4;
+    FftAxis ax64[3];
     for (int a = 0; a < 3; ++a)
-        if (!fft_axis_plan(sh.m[a], tab.axis[a]))
+        if (!fft_axis_plan(sh.m[a], fp32, tab.axis[a]) || !fft_axis_plan(sh.m[a], false, ax64[a]))
             return fail(err, FH_ERR_PFFT,
                         "pFFT convolution: padded axis length " + std::to_string((long long)sh.m[a]) +
                             " is not a 2^a 3^b 5^c length up to " + std::to_string(kFftMaxLength));
-    // Twiddle tables exp(-2 pi i t / m), computed in FP64 on the host.
+    // Twiddles of every stage, [k][r] = exp(-2 pi i r k / (R S)), computed in
+    // FP64 on the host.
     for (int a = 0; a < 3; ++a) {
-        const int64_t m = sh.m[a];
-        std::vector<double2> h64((size_t)m);
-        for (int64_t t = 0; t < m; ++t) {
-            const double ang = -2.0 * kPi * (double)t / (double)m;
-            h64[(size_t)t] = make_double2(std::cos(ang), std::sin(ang));
+        auto stage_twiddles = [](const FftAxis &ax) {
+            std::vector<double2> h((size_t)std::max(1, ax.tw_count));
+            for (int st = 0; st < ax.nst; ++st)
+                for (int k = 0; k < ax.S[st]; ++k)
+                    for (int r = 0; r < ax.R[st]; ++r) {
+                        const double ang = -2.0 * kPi * (double)r * (double)k / ((double)ax.R[st] * ax.S[st]);
+                        h[(size_t)(ax.tw[st] + k * twiddle_row(ax.R[st]) + r)] =
+                            make_double2(std::cos(ang), std::sin(ang));
+                    }
+            return h;
+        };
+        const std::vector<double2> h64 = stage_twiddles(ax64[a]);
+        const std::vector<double2> hd = stage_twiddles(tab.axis[a]);
+        std::vector<V> h(hd.size());
+        for (size_t t = 0; t < hd.size(); ++t) {
+            h[t].x = (T)hd[t].x;
+            h[t].y = (T)hd[t].y;
         }
-        std::vector<V> h((size_t)m);
-        for (int64_t t = 0; t < m; ++t) {
-            h[(size_t)t].x = (T)h64[(size_t)t].x;
-            h[(size_t)t].y = (T)h64[(size_t)t].y;
-        }
-        FHB_CUDA(cache_alloc(&tab.tw[a], sizeof(V) * (size_t)m, s));
-        FHB_CUDA(cudaMemcpyAsync(tab.tw[a], h.data(), sizeof(V) * (size_t)m, cudaMemcpyHostToDevice, s));
-        if (sizeof(T) == 4) {
-            FHB_CUDA(cache_alloc(&tab.tw64[a], sizeof(double2) * (size_t)m, s));
-            FHB_CUDA(cudaMemcpyAsync(tab.tw64[a], h64.data(), sizeof(double2) * (size_t)m, cudaMemcpyHostToDevice, s));
+        FHB_CUDA(cache_alloc(&tab.tw[a], sizeof(V) * h.size(), s));
+        FHB_CUDA(cudaMemcpyAsync(tab.tw[a], h.data(), sizeof(V) * h.size(), cudaMemcpyHostToDevice, s));
+        if (fp32) {
+            FHB_CUDA(cache_alloc(&tab.tw64[a], sizeof(double2) * h64.size(), s));
+            FHB_CUDA(cudaMemcpyAsync(tab.tw64[a], h64.data(), sizeof(double2) * h64.size(), cudaMemcpyHostToDevice,
+                                     s));
         } else {
             tab.tw64[a] = tab.tw[a];
         }
         FHB_CUDA(cudaStreamSynchronize(s));
+    }
+    // places of the FP64 transform's frequencies in the convolution's order
+    std::vector<int> map;
+    for (int a = 0; a < 3; ++a) {
+        const std::vector<int> here = fft_places(tab.axis[a]), wide = fft_places(ax64[a]);
+        std::vector<int> part((size_t)sh.m[a], 0);
+        for (size_t f = 0; f < here.size(); ++f) part[(size_t)here[f]] = wide[f];
+        map.insert(map.end(), part.begin(), part.end());
     }
     // Spectrum: unpruned FP64 forward transform of the wrapped kernel.
     const int64_t P = sh.m[0] * sh.m[1] * sh.m[2];
     double2 *grid = nullptr, *tmp = nullptr;
     FHB_CUDA(cache_alloc(reinterpret_cast<void **>(&grid), sizeof(double2) * (size_t)P, s));
     FHB_CUDA(cache_alloc(reinterpret_cast<void **>(&tmp), sizeof(double2) * (size_t)P, s));
+    int *d_map = nullptr;
+    FHB_CUDA(cache_alloc(reinterpret_cast<void **>(&d_map), sizeof(int) * map.size(), s));
     struct Release {
-        void *a, *b;
+        void *a, *b, *c;
         cudaStream_t s;
         ~Release() {
             cache_free(a, s);
             cache_free(b, s);
+            cache_free(c, s);
         }
-    } release{grid, tmp, s};
+    } release{grid, tmp, d_map, s};
+    FHB_CUDA(cudaMemcpyAsync(d_map, map.data(), sizeof(int) * map.size(), cudaMemcpyHostToDevice, s));
     wrapped_kernel_kernel<<<blocks_of(P, 256), 256, 0, s>>>(grid, sh.n[0], sh.n[1], sh.n[2], sh.m[0], sh.m[1],
                                                            sh.m[2], spacing);
     FHB_CUDA(cudaGetLastError());
     const int64_t m0 = sh.m[0], m1 = sh.m[1], m2 = sh.m[2];
-    fh_status e = axis_step<double>(grid, tmp, 0, 0, m0 * m1, 1, (int)m2, (int)m2, tab.axis[2], tab.tw64[2], -1,
-                                    nullptr, 1, s, err);
+    fh_status e = axis_step<double, kForward>(grid, tmp, 0, 0, m0 * m1, 1, (int)m2, (int)m2, ax64[2], tab.tw64[2],
+                                              nullptr, 1, s, err);
     if (!e)
-        e = axis_step<double>(tmp, grid, 0, 0, m0, m2, (int)m1, (int)m1, tab.axis[1], tab.tw64[1], -1, nullptr, 1, s,
-                              err);
+        e = axis_step<double, kForward>(tmp, grid, 0, 0, m0, m2, (int)m1, (int)m1, ax64[1], tab.tw64[1], nullptr, 1, s,
+                                        err);
     if (!e)
-        e = axis_step<double>(grid, tmp, 0, 0, 1, m1 * m2, (int)m0, (int)m0, tab.axis[0], tab.tw64[0], -1, nullptr, 1,
-                              s, err);
+        e = axis_step<double, kForward>(grid, tmp, 0, 0, 1, m1 * m2, (int)m0, (int)m0, ax64[0], tab.tw64[0], nullptr,
+                                        1, s, err);
     if (e) return e;
     FHB_CUDA(cache_alloc(&tab.spectrum, sizeof(T) * (size_t)P, s));
-    spectrum_store_kernel<T><<<blocks_of(P, 256), 256, 0, s>>>(tmp, static_cast<T *>(tab.spectrum), P);
+    spectrum_store_kernel<T><<<blocks_of(P, 256), 256, 0, s>>>(tmp, static_cast<T *>(tab.spectrum), m0, m1, m2,
+                                                               d_map);
     FHB_CUDA(cudaGetLastError());
     FHB_CUDA(cudaStreamSynchronize(s));
     tab.shape = sh;
@@ -428,17 +778,20 @@ fh_status fftconv_run(const FftConvTables &tab, void *work, int grids, cudaStrea
     V *B = A + sa * grids;
     V *C = B + sb * grids;
     const T *spec = static_cast<const T *>(tab.spectrum);
-    fh_status e = axis_step<T>(A, B, sa, sb, n0 * n1, 1, (int)n2, (int)m2, tab.axis[2], tab.tw[2], -1, nullptr, grids,
-                               s, err);
+    fh_status e = axis_step<T, kForward>(A, B, sa, sb, n0 * n1, 1, (int)n2, (int)m2, tab.axis[2], tab.tw[2], nullptr,
+                                         grids, s, err);
     if (!e)
-        e = axis_step<T>(B, C, sb, sc, n0, m2, (int)n1, (int)m1, tab.axis[1], tab.tw[1], -1, nullptr, grids, s, err);
+        e = axis_step<T, kForward>(B, C, sb, sc, n0, m2, (int)n1, (int)m1, tab.axis[1], tab.tw[1], nullptr, grids, s,
+                                   err);
     if (!e)
-        e = axis_step<T>(C, C, sc, sc, 1, m1 * m2, (int)n0, (int)n0, tab.axis[0], tab.tw[0], -1, spec, grids, s, err);
+        e = axis_step<T, kFused>(C, C, sc, sc, 1, m1 * m2, (int)n0, (int)n0, tab.axis[0], tab.tw[0], spec, grids, s,
+                                 err);
     if (!e)
-        e = axis_step<T>(C, B, sc, sb, n0, m2, (int)m1, (int)n1, tab.axis[1], tab.tw[1], +1, nullptr, grids, s, err);
+        e = axis_step<T, kInverse>(C, B, sc, sb, n0, m2, (int)m1, (int)n1, tab.axis[1], tab.tw[1], nullptr, grids, s,
+                                   err);
     if (!e)
-        e = axis_step<T>(B, A, sb, sa, n0 * n1, 1, (int)m2, (int)n2, tab.axis[2], tab.tw[2], +1, nullptr, grids, s,
-                         err);
+        e = axis_step<T, kInverse>(B, A, sb, sa, n0 * n1, 1, (int)m2, (int)n2, tab.axis[2], tab.tw[2], nullptr, grids,
+                                   s, err);
     return e;
 }
 

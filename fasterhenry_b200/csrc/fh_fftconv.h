@@ -1,26 +1,35 @@
 // The pFFT convolution without a library FFT (fh_fftconv.cu): pruned
-// mixed-radix Stockham transforms in shared memory, FP32 or FP64.
+// mixed-radix transforms, FP32 or FP64.
 #pragma once
 
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <vector>
 
 #include "fh_internal.h"
 
 namespace fhb {
 
-constexpr int kFftMaxFactors = 24;
-constexpr int64_t kFftMaxLength = 4800;  // longest padded axis: two FP64 lines of it and its twiddles fit a CTA
+constexpr int kFftMaxStages = 8;
+constexpr int64_t kFftMaxLength = 4800;  // longest padded axis
 
-// One axis: its length and its radices (4, then 2, 3, 5), passed by value to
-// the kernels.
+// One axis: its length and its stages (radix R over blocks of R S points),
+// with the constants of the stages' index divisions and the places of their
+// twiddles in the axis' table, passed by value to the kernels. 
 struct FftAxis {
     int m = 1;
-    int nfac = 0;
-    int fac[kFftMaxFactors] = {};
+    int nst = 0;
+    int R[kFftMaxStages] = {};
+    int S[kFftMaxStages] = {};
+    unsigned magic_S[kFftMaxStages] = {};
+    unsigned magic_nb[kFftMaxStages] = {};  // of m / R
+    int tw[kFftMaxStages] = {};
+    int tw_count = 0;
 };
-bool fft_axis_plan(int64_t m, FftAxis &ax);
+bool fft_axis_plan(int64_t m, bool fp32, FftAxis &ax);
+// The place of every frequency of an axis after its forward stages.
+std::vector<int> fft_places(const FftAxis &ax);
 
 // Unpadded grid n (axis 2 fastest) and the padded torus m (m_a >= 2 n_a - 1).
 struct FftConvShape {
@@ -28,9 +37,10 @@ struct FftConvShape {
     int64_t m[3] = {1, 1, 1};
 };
 
-// Per-operator tables: twiddles exp(-2 pi i t / m_a) per axis (in the
-// convolution's precision, and FP64 for the set-up) and the kernel's real
-// spectrum on the padded grid (times 1 / P), laid out [i][j][k].
+// Per-operator tables: the stages' twiddles per axis (in the convolution's
+// precision, and FP64 for the set-up) and the kernel's real spectrum on the
+// padded grid (times 1 / P), laid out [i][j][k], each axis in the order that
+// its forward stages leave the frequencies in.
 struct FftConvTables {
     FftConvShape shape;
     FftAxis axis[3];
@@ -54,6 +64,8 @@ fh_status fftconv_setup(const FftConvShape &sh, double spacing, FftConvTables &t
 // on return the potentials.
 template <class T>
 fh_status fftconv_run(const FftConvTables &tab, void *work, int grids, cudaStream_t s, fh_error_info *err);
+// The same with the FP32 tables for the port columns (fh_fftconv_ports.cu).
+fh_status fftconv_run_ports(const FftConvTables &tab, void *work, int grids, cudaStream_t s, fh_error_info *err);
 void fftconv_free(FftConvTables &tab, cudaStream_t s);
 
 }  // namespace fhb

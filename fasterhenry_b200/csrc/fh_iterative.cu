@@ -193,7 +193,8 @@ fh_status apply_ee(fh_iterative *s, double omega, const double2 *x, double2 *y, 
     if (omega != 0.0) {
         split_kernel<<<grid_n(n), 256, 0, s->stream>>>(s->d_c, s->d_parts, n);
         FHB_CUDA(cudaGetLastError());
-        fh_status st = pfft_apply(s->op, s->d_parts, s->d_flux, 2, err, full_precision);
+        fh_status st = pfft_apply(s->op, s->d_parts, s->d_flux, 2, err,
+                                  full_precision ? PfftProduct::Full : PfftProduct::Plain);
         if (st) return st;
         flux = s->d_flux;
     }
@@ -430,7 +431,7 @@ fh_status fh_iterative_create(const fh_node *nodes, size_t n_nodes, const fh_seg
             std::fill(current.begin(), current.end(), 0.0);
             for (int64_t k = rp[m + q]; k < rp[m + q + 1]; ++k) current[br[k]] += sg[k];
             FHB_CUDA(cudaMemcpyAsync(d_cur, current.data(), sizeof(double) * n, cudaMemcpyHostToDevice, cs));
-            st = pfft_apply(s->op, d_cur, d_fl, 1, err);
+            st = pfft_apply(s->op, d_cur, d_fl, 1, err, PfftProduct::Ports);
             if (st) return st;
             FHB_CUDA(cudaMemcpyAsync(flux.data(), d_fl, sizeof(double) * n, cudaMemcpyDeviceToHost, cs));
             FHB_CUDA(cudaStreamSynchronize(cs));

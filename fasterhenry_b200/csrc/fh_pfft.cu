@@ -169,7 +169,7 @@ inline unsigned blocks_for(int64_t work, int threads, int64_t cap = 148 * 16) {
 }  // namespace
 
 fh_status pfft_apply_impl(PfftDevice &op, const double *d_x, double *d_y, int count, fh_error_info *err,
-                          bool full_precision);
+                          PfftProduct kind);
 
 PfftDevice::~PfftDevice() {
     cudaStream_t s = (cudaStream_t)stream;
@@ -292,10 +292,10 @@ fh_status pfft_build(const fh_filament *fil, int64_t n, const PfftConfig &cfg, v
 // in FP64) the pruned transform chain of fh_fftconv.cu: the sources A written
 // and read, B = n0 n1 m2 and C = n0 m1 m2 written and read twice each, the
 // spectrum (P reals), and the potentials A written and read.
-double pfft_apply_bytes(const PfftDevice &op, int count, bool full_precision) {
+double pfft_apply_bytes(const PfftDevice &op, int count, PfftProduct kind) {
     const int ncomp = (int)op.components.size();
     const double grids = (double)((count * ncomp + 1) / 2);
-    const double E = op.fft_fp32 && !full_precision ? 8.0 : 16.0;
+    const double E = op.fft_fp32 && kind != PfftProduct::Full ? 8.0 : 16.0;
     const FftConvShape &sh = op.conv.shape;
     const double A = (double)sh.n[0] * sh.n[1] * sh.n[2], B = (double)sh.n[0] * sh.n[1] * sh.m[2],
                  C = (double)sh.n[0] * sh.m[1] * sh.m[2], P = (double)op.P;
@@ -305,18 +305,18 @@ double pfft_apply_bytes(const PfftDevice &op, int count, bool full_precision) {
 }
 
 fh_status pfft_apply(PfftDevice &op, const double *d_x, double *d_y, int count, fh_error_info *err,
-                     bool full_precision) {
+                     PfftProduct kind) {
     if (op.n == 0 || count <= 0) return FH_OK;
     prof_begin((cudaStream_t)op.stream, FH_PROF_PFFT_APPLY);
-    fh_status st = pfft_apply_impl(op, d_x, d_y, count, err, full_precision);
-    prof_end((cudaStream_t)op.stream, FH_PROF_PFFT_APPLY, pfft_apply_bytes(op, count, full_precision));
+    fh_status st = pfft_apply_impl(op, d_x, d_y, count, err, kind);
+    prof_end((cudaStream_t)op.stream, FH_PROF_PFFT_APPLY, pfft_apply_bytes(op, count, kind));
     return st;
 }
 
 namespace {
 template <class T>
 fh_status apply_far(PfftDevice &op, const FftConvTables &conv, const double *d_x, double *d_y, int count,
-                    fh_error_info *err) {
+                    PfftProduct kind, fh_error_info *err) {
     cudaStream_t s = (cudaStream_t)op.stream;
     const int ncomp = (int)op.components.size();
     const int grids = (count * ncomp + 1) / 2;
@@ -337,7 +337,8 @@ fh_status apply_far(PfftDevice &op, const FftConvTables &conv, const double *d_x
     spread_kernel<T><<<blocks_for(op.G, 256), 256, 0, s>>>(op.d_spread_off, op.d_spread_fil, op.d_spread_w, op.d_dir,
                                                             d_x, work, a);
     FHB_CUDA(cudaGetLastError());
-    e = fftconv_run<T>(conv, work, grids, s, err);
+    e = sizeof(T) == 4 && kind == PfftProduct::Ports ? fftconv_run_ports(conv, work, grids, s, err)
+                                                     : fftconv_run<T>(conv, work, grids, s, err);
     if (e) return e;
     interp_kernel<T><<<blocks_for(op.n * 32, 256), 256, 0, s>>>(op.d_proj_off, op.d_proj_idx, op.d_proj_w, op.d_dir,
                                                                  work, d_y, a);
@@ -347,14 +348,14 @@ fh_status apply_far(PfftDevice &op, const FftConvTables &conv, const double *d_x
 }  // namespace
 
 fh_status pfft_apply_impl(PfftDevice &op, const double *d_x, double *d_y, int count, fh_error_info *err,
-                          bool full_precision) {
+                          PfftProduct kind) {
     cudaStream_t s = (cudaStream_t)op.stream;
     near_kernel<<<blocks_for(op.n * 32, 256), 256, 0, s>>>(op.d_near_off, op.d_near_col, op.d_near_val, d_x, d_y,
                                                              op.n, count);
     FHB_CUDA(cudaGetLastError());
     if (op.components.empty()) return FH_OK;
-    if (op.fft_fp32 && !full_precision) return apply_far<float>(op, op.conv, d_x, d_y, count, err);
-    return apply_far<double>(op, op.fft_fp32 ? op.conv64 : op.conv, d_x, d_y, count, err);
+    if (op.fft_fp32 && kind != PfftProduct::Full) return apply_far<float>(op, op.conv, d_x, d_y, count, kind, err);
+    return apply_far<double>(op, op.fft_fp32 ? op.conv64 : op.conv, d_x, d_y, count, kind, err);
 }
 
 }  // namespace fhb

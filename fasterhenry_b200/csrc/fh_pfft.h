@@ -147,10 +147,12 @@ struct PfftDevice {
 fh_status pfft_build(const fh_filament *fil, int64_t n, const PfftConfig &cfg, void *stream, PfftDevice &op,
                      fh_error_info *err);
 // y = L x for `count` vectors of length n (device pointers, vector v at
-// x + v n), on op.stream.  With full_precision, an operator built with the
-// FP32 convolution convolves in FP64 (for refinement residuals).
+// x + v n), on op.stream.  An operator built with the FP32 convolution
+// convolves in FP64 for Full (refinement residuals), and by the transform of
+// fh_fftconv_ports.cu for Ports (port columns).
+enum class PfftProduct { Plain, Full, Ports };
 fh_status pfft_apply(PfftDevice &op, const double *d_x, double *d_y, int count, fh_error_info *err,
-                     bool full_precision = false);
+                     PfftProduct kind = PfftProduct::Plain);
 
 }  // namespace fhb
 
