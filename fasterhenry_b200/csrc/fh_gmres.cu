@@ -94,49 +94,77 @@ __global__ void __launch_bounds__(kRT) sum_final_kernel(const double *__restrict
 }
 
 // The projections of w on the cnt basis vectors V_0 .. V_cnt-1 at once
-// (classical Gram-Schmidt): per block and vector k, the partial sum of
-// conj(V_k[i]) w[i] over the block's rows (warp shuffles, then the warps in
-// order) into partial[2 (k kRB + block)].
-__global__ void __launch_bounds__(kRT) multidot_partial_kernel(const double2 *__restrict__ V,
-                                                               const double2 *__restrict__ w, int64_t n, int cnt,
-                                                               double *__restrict__ partial) {
-    __shared__ double2 sh[kRT / 32];
+// (classical Gram-Schmidt): conj(V_k) . w over one of kDotChunks chunks of
+// the rows for kDotVecs vectors per block, into partial[2 (k kDotChunks +
+// chunk)].
+//
+// Bound by reading the basis once: 1.25 MB per vector at 78,307 loops.  A
+// block takes several vectors so that w is read once for them and each
+// thread has kDotVecs loads in flight, and its 2 kDotVecs sums cross the warp
+// in 16 exchanges (each step halves the values a lane keeps).  Over a cycle
+// of 400 vectors of 78,307: 163 us on average with one vector at a time per
+// block and a block-wide reduction for each, 36 us now.  The chunks depend on
+// n alone, so a result does not depend on the device's scheduling.
+constexpr int kDotVecs = 8;
+constexpr int kDotChunks = 64;
+constexpr int kDotThreads = 128;
+__global__ void __launch_bounds__(kDotThreads) multidot_partial_kernel(const double2 *__restrict__ V,
+                                                                       const double2 *__restrict__ w, int64_t n,
+                                                                       int cnt, double *__restrict__ partial) {
+    __shared__ double sh[kDotThreads / 32][2 * kDotVecs];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int k = 0; k < cnt; ++k) {
-        const double2 *vk = V + (size_t)k * n;
-        double2 acc = make_double2(0.0, 0.0);
-        for (int64_t i = (int64_t)blockIdx.x * kRT + threadIdx.x; i < n; i += (int64_t)kRB * kRT) {
-            const double2 a = vk[i], b = w[i];
-            acc = cadd(acc, make_double2(a.x * b.x + a.y * b.y, a.x * b.y - a.y * b.x));
+    const int k0 = blockIdx.y * kDotVecs;
+    const int64_t rows = (n + kDotChunks - 1) / kDotChunks;
+    const int64_t begin = blockIdx.x * rows, end = begin + rows < n ? begin + rows : n;
+    const double2 *vk[kDotVecs];
+#pragma unroll
+    for (int q = 0; q < kDotVecs; ++q) vk[q] = V + (size_t)(k0 + q < cnt ? k0 + q : cnt - 1) * n;
+    double acc[2 * kDotVecs] = {};
+    for (int64_t i = begin + threadIdx.x; i < end; i += kDotThreads) {
+        const double2 b = w[i];
+#pragma unroll
+        for (int q = 0; q < kDotVecs; ++q) {
+            const double2 a = vk[q][i];
+            acc[2 * q] += a.x * b.x + a.y * b.y;
+            acc[2 * q + 1] += a.x * b.y - a.y * b.x;
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            acc.x += __shfl_down_sync(0xffffffffu, acc.x, o);
-            acc.y += __shfl_down_sync(0xffffffffu, acc.y, o);
-        }
-        if (lane == 0) sh[warp] = acc;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double2 t = sh[0];
-            for (int q = 1; q < kRT / 32; ++q) t = cadd(t, sh[q]);
-            partial[2 * ((size_t)k * kRB + blockIdx.x)] = t.x;
-            partial[2 * ((size_t)k * kRB + blockIdx.x) + 1] = t.y;
-        }
-        __syncthreads();
+    }
+    // After the step of distance o a lane holds the sums over its pair of the
+    // half of the values that its bit o selects; value `lane >> 1` at last.
+#pragma unroll
+    for (int o = 16, have = 2 * kDotVecs; o > 1; o >>= 1, have >>= 1) {
+#pragma unroll
+        for (int q = 0; q < kDotVecs; ++q)
+            if (q < have / 2) {
+                const double keep = lane & o ? acc[q + have / 2] : acc[q];
+                const double give = lane & o ? acc[q] : acc[q + have / 2];
+                acc[q] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+            }
+    }
+    acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
+    if (!(lane & 1)) sh[warp][lane >> 1] = acc[0];
+    __syncthreads();
+    if (threadIdx.x < 2 * kDotVecs) {
+        double t = sh[0][threadIdx.x];
+        for (int q = 1; q < kDotThreads / 32; ++q) t += sh[q][threadIdx.x];
+        const int k = k0 + threadIdx.x / 2;
+        if (k < cnt) partial[2 * ((size_t)k * kDotChunks + blockIdx.x) + (threadIdx.x & 1)] = t;
     }
 }
 
-// h[k] = the sum of vector k's kRB partials (block k, fixed tree).
-__global__ void __launch_bounds__(kRT) multidot_final_kernel(const double *__restrict__ partial,
+// h[k] = the sum of vector k's kDotChunks partials (a warp each, fixed tree).
+__global__ void __launch_bounds__(kRT) multidot_final_kernel(const double *__restrict__ partial, int cnt,
                                                              double2 *__restrict__ h) {
-    __shared__ double2 sh[kRT];
-    const size_t base = (size_t)blockIdx.x * kRB;
-    sh[threadIdx.x] = make_double2(partial[2 * (base + threadIdx.x)], partial[2 * (base + threadIdx.x) + 1]);
-    __syncthreads();
-    for (int s = kRT / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) sh[threadIdx.x] = cadd(sh[threadIdx.x], sh[threadIdx.x + s]);
-        __syncthreads();
+    const int lane = threadIdx.x & 31, k = blockIdx.x * (kRT / 32) + (threadIdx.x >> 5);
+    if (k >= cnt) return;
+    const double2 *p = reinterpret_cast<const double2 *>(partial) + (size_t)k * kDotChunks;
+    double2 t = make_double2(0.0, 0.0);
+    for (int c = lane; c < kDotChunks; c += 32) t = cadd(t, p[c]);
+    for (int o = 16; o > 0; o >>= 1) {
+        t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
+        t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
     }
-    if (threadIdx.x == 0) h[blockIdx.x] = sh[0];
+    if (lane == 0) h[k] = t;
 }
 
 // w -= sum_k h[k] V_k, the terms taken in increasing k.
@@ -244,7 +272,7 @@ fh_status GmresWork::ensure(int64_t n_, int restart_, fh_error_info *err) {
         alloc((void **)&t, sizeof(double2) * n) != cudaSuccess || alloc((void **)&u, sizeof(double2) * n) != cudaSuccess ||
         alloc((void **)&h, sizeof(double2) * 2 * (restart + 1)) != cudaSuccess ||
         alloc((void **)&red, sizeof(double) * kRedLen) != cudaSuccess ||
-        alloc((void **)&part, sizeof(double) * 2 * kRB * (size_t)(restart + 1)) != cudaSuccess) {
+        alloc((void **)&part, sizeof(double) * 2 * kDotChunks * (size_t)(restart + 1)) != cudaSuccess) {
         cudaGetLastError();
         return fail(err, FH_ERR_OUT_OF_MEMORY, "device allocation of the GMRES workspace failed");
     }
@@ -331,8 +359,9 @@ fh_status gmres_solve(int64_t n, const DeviceOp &apply, const DeviceOp &precondi
             // basis vector).
             for (int pass = 0; pass < 2; ++pass) {
                 double2 *hp = work.h + pass * (restart + 1);
-                multidot_partial_kernel<<<kRB, kRT, 0, s>>>(work.V, work.w, n, j + 1, work.part);
-                multidot_final_kernel<<<j + 1, kRT, 0, s>>>(work.part, hp);
+                multidot_partial_kernel<<<dim3(kDotChunks, (unsigned)(j / kDotVecs + 1)), kDotThreads, 0, s>>>(
+                    work.V, work.w, n, j + 1, work.part);
+                multidot_final_kernel<<<j / (kRT / 32) + 1, kRT, 0, s>>>(work.part, j + 1, hp);
                 multi_axpy_kernel<<<grid_of(n), 256, sizeof(double2) * (j + 1), s>>>(work.w, work.V, hp, j + 1, n);
             }
             FHB_CUDA(cudaGetLastError());

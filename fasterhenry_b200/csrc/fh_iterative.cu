@@ -41,21 +41,61 @@ double wall_s() {
     return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
 
-// c_b = sum over the internal loops through branch b of sign x_loop, in loop
-// order (transposed loop basis; iterative.rs:403-411).
-__global__ void scatter_kernel(const double2 *__restrict__ x, const int64_t *__restrict__ off,
-                               const int32_t *__restrict__ loop, const double *__restrict__ sign,
-                               double2 *__restrict__ c, int64_t n) {
-    for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < n; b += (int64_t)gridDim.x * blockDim.x) {
-        double2 acc = make_double2(0.0, 0.0);
-        for (int64_t k = off[b]; k < off[b + 1]; ++k) {
-            const double2 v = x[loop[k]];
-            const double s = sign[k];
-            acc.x += v.x * s;
-            acc.y += v.y * s;
-        }
-        c[b] = acc;
+// y_i = sum over row i's entries of sign v_idx (a CSR matrix of signs): the
+// loops' branches (iterative.rs:488-505) and, transposed, the loops through a
+// branch (iterative.rs:403-411).  Most rows hold a few entries, those of a
+// ground plane's spanning tree hundreds, and a thread that walks such a row
+// alone sets the kernel's time.  Rows of up to kShortRow entries take eight
+// lanes, the others (listed in `lng`) a warp each, in the blocks after the
+// first `short_blocks`.  78,307 loops of a meander over a 64 x 64 plane, both
+// products: 85 us with a thread per row, 28 us so.
+constexpr int kShortRow = 64;
+__global__ void __launch_bounds__(256) row_sum_kernel(const double2 *__restrict__ v, const int64_t *__restrict__ off,
+                                                      const int32_t *__restrict__ idx,
+                                                      const double *__restrict__ sign, double2 *__restrict__ y,
+                                                      int64_t rows, const int32_t *__restrict__ lng, int n_long,
+                                                      unsigned short_blocks) {
+    const bool is_long = blockIdx.x >= short_blocks;
+    const int lanes = is_long ? 32 : 8;
+    const int64_t slot = ((int64_t)(is_long ? blockIdx.x - short_blocks : blockIdx.x) * blockDim.x + threadIdx.x) / lanes;
+    const int lane = threadIdx.x & (lanes - 1);
+    int64_t i = -1;
+    if (is_long ? slot < n_long : slot < rows) i = is_long ? lng[slot] : slot;
+    int64_t b = 0, e = 0;
+    if (i >= 0) {
+        b = off[i];
+        e = off[i + 1];
+        if (!is_long && e - b > kShortRow) i = -1, e = b;
     }
+    double2 acc = make_double2(0.0, 0.0);
+#pragma unroll 4
+    for (int64_t k = b + lane; k < e; k += lanes) {
+        const double2 t = v[idx[k]];
+        const double s = sign[k];
+        acc.x += t.x * s;
+        acc.y += t.y * s;
+    }
+    for (int o = lanes / 2; o > 0; o >>= 1) {
+        acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
+        acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
+    }
+    if (lane == 0 && i >= 0) y[i] = acc;
+}
+
+// The rows of more than kShortRow entries.
+std::vector<int32_t> long_rows(const std::vector<int64_t> &off, int64_t rows) {
+    std::vector<int32_t> out;
+    for (int64_t i = 0; i < rows; ++i)
+        if (off[(size_t)i + 1] - off[(size_t)i] > kShortRow) out.push_back((int32_t)i);
+    return out;
+}
+
+void row_sum(const double2 *v, const int64_t *off, const int32_t *idx, const double *sign, double2 *y, int64_t rows,
+             const int32_t *lng, int n_long, cudaStream_t s) {
+    const unsigned short_blocks = (unsigned)((rows + 31) / 32), long_blocks = (unsigned)((n_long + 7) / 8);
+    if (rows > 0)
+        row_sum_kernel<<<short_blocks + long_blocks, 256, 0, s>>>(v, off, idx, sign, y, rows, lng, n_long,
+                                                                  short_blocks);
 }
 
 // Real and imaginary parts as two real vectors (one pFFT product of both).
@@ -75,22 +115,6 @@ __global__ void drop_kernel(const double2 *__restrict__ c, const double *__restr
             drop[b] = make_double2(rb * c[b].x - omega * flux[n + b], rb * c[b].y + omega * flux[b]);
         else
             drop[b] = make_double2(c[b].x * rb, c[b].y * rb);
-    }
-}
-
-// y_i = sum over loop i's branches of sign v_b, in row order (iterative.rs:488-505).
-__global__ void gather_kernel(const double2 *__restrict__ v, const int64_t *__restrict__ row_ptr,
-                              const int32_t *__restrict__ branch, const double *__restrict__ sign,
-                              double2 *__restrict__ y, int64_t loops) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < loops; i += (int64_t)gridDim.x * blockDim.x) {
-        double2 acc = make_double2(0.0, 0.0);
-        for (int64_t k = row_ptr[i]; k < row_ptr[i + 1]; ++k) {
-            const double2 t = v[branch[k]];
-            const double s = sign[k];
-            acc.x += t.x * s;
-            acc.y += t.y * s;
-        }
-        y[i] = acc;
     }
 }
 
@@ -145,6 +169,8 @@ struct fh_iterative {
     // Device: loop basis rows and its transpose over the internal loops.
     int64_t *d_row_ptr = nullptr, *d_t_off = nullptr;
     int32_t *d_branch = nullptr, *d_t_loop = nullptr;
+    int32_t *d_long = nullptr, *d_t_long = nullptr;  // their rows of more than kShortRow entries
+    int n_long = 0, n_t_long = 0;
     double *d_sign = nullptr, *d_t_sign = nullptr, *d_r = nullptr;
     double2 *d_c = nullptr, *d_drop = nullptr, *d_diag = nullptr, *d_b = nullptr, *d_x = nullptr;
     double *d_parts = nullptr, *d_flux = nullptr;
@@ -163,7 +189,7 @@ struct fh_iterative {
         void *ptrs[] = {d_row_ptr, d_t_off, d_branch, d_t_loop, d_sign,  d_t_sign, d_r,    d_c,    d_drop,
                         d_diag,    d_b,     d_x,      d_parts,  d_flux,  d_res,    d_cor,  d_ax,   d_col_ptr,
                         d_first,   d_segi,  d_col_loop, d_col_sign, d_whr, d_ip,   d_ib,   d_dens, d_pow,
-                        d_segc,    d_segp,  d_segpk};
+                        d_segc,    d_segp,  d_segpk, d_long,  d_t_long};
         for (void *q : ptrs)
             if (q) cudaFree(q);
     }
@@ -187,7 +213,7 @@ __global__ void axpy_kernel(double2 *__restrict__ x, const double2 *__restrict__
 fh_status apply_ee(fh_iterative *s, double omega, const double2 *x, double2 *y, fh_error_info *err,
                    bool full_precision = false) {
     const int64_t n = s->n;
-    scatter_kernel<<<grid_n(n), 256, 0, s->stream>>>(x, s->d_t_off, s->d_t_loop, s->d_t_sign, s->d_c, n);
+    row_sum(x, s->d_t_off, s->d_t_loop, s->d_t_sign, s->d_c, n, s->d_t_long, s->n_t_long, s->stream);
     FHB_CUDA(cudaGetLastError());
     const double *flux = nullptr;
     if (omega != 0.0) {
@@ -199,7 +225,7 @@ fh_status apply_ee(fh_iterative *s, double omega, const double2 *x, double2 *y, 
         flux = s->d_flux;
     }
     drop_kernel<<<grid_n(n), 256, 0, s->stream>>>(s->d_c, s->d_r, flux, omega, s->d_drop, n);
-    gather_kernel<<<grid_n(s->m), 256, 0, s->stream>>>(s->d_drop, s->d_row_ptr, s->d_branch, s->d_sign, y, s->m);
+    row_sum(s->d_drop, s->d_row_ptr, s->d_branch, s->d_sign, y, s->m, s->d_long, s->n_long, s->stream);
     FHB_CUDA(cudaGetLastError());
     return FH_OK;
 }
@@ -510,6 +536,11 @@ fh_status fh_iterative_create(const fh_node *nodes, size_t n_nodes, const fh_seg
     FHB_CUDA(put(&s->d_t_loop, internal.loop, cs));
     FHB_CUDA(put(&s->d_t_sign, internal.sign, cs));
     FHB_CUDA(put(&s->d_r, s->resistances, cs));
+    const std::vector<int32_t> lng = long_rows(rp, m), t_lng = long_rows(internal.offset, n);
+    s->n_long = (int)lng.size();
+    s->n_t_long = (int)t_lng.size();
+    FHB_CUDA(put(&s->d_long, lng, cs));
+    FHB_CUDA(put(&s->d_t_long, t_lng, cs));
     auto alloc = [&](void **q, size_t bytes) { return cudaMalloc(q, std::max<size_t>(bytes, 16)); };
     if (alloc((void **)&s->d_c, sizeof(double2) * n) || alloc((void **)&s->d_drop, sizeof(double2) * n) ||
         alloc((void **)&s->d_diag, sizeof(double2) * m) || alloc((void **)&s->d_b, sizeof(double2) * m) ||

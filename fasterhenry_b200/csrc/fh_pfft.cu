@@ -3,20 +3,25 @@
 //
 //   y = C x + mu0/4pi sum_c d_c . W^T (K (*) (W (d_c . x)))
 //
-// per product, for `count` vectors at once:
-//   1. near_kernel        y = C x (CSR rows of precorrected near pairs; warp
-//                         per filament, every vector from one pass over the
-//                         row);
-//   2. spread_kernel      the grid sources q_{v,c}(g) = sum_i W_ig d_ic x_vi,
+// per product, for `count` vectors at once, taken in pairs:
+//   1. sources_kernel     pairs x_v, x_v+1 side by side, and the sources
+//                         d_ic x_vi of every filament likewise, so that the
+//                         gathers below take one 16-byte load per pair;
+//   2. near_kernel        y = C x (CSR rows of precorrected near pairs; warp
+//                         per filament, up to two pairs of vectors from one
+//                         pass over the row);
+//   3. spread_kernel      the grid sources q_{v,c}(g) = sum_i W_ig d_ic x_vi,
 //                         one thread per grid point over the transposed
 //                         projection (no atomics), written to compact complex
 //                         grids (two real sources per grid: real and imaginary
 //                         part) in the convolution's precision;
-//   3. fftconv_run        the aperiodic convolution K (*) q by pruned
+//   4. fftconv_run        the aperiodic convolution K (*) q by pruned
 //                         mixed-radix transforms on the 2N-1 padded torus
 //                         (fh_fftconv.cu; FP64 or FP32);
-//   4. interp_kernel      y_vi += mu0/4pi sum_c d_ic sum_g W_ig phi_{v,c}(g),
+//   5. interp_kernel      y_vi += mu0/4pi sum_c d_ic sum_g W_ig phi_{v,c}(g),
 //                         warp per filament, from the compact grids.
+// Real source r = v ncomp + c is part r % 2 of complex grid r / 2, so a pair
+// of vectors fills ncomp whole grids.
 //
 // The near-field corrections C_ij = L_ij(exact) - mu0/4pi cos_ij G_ij are
 // built at set-up from the device's grid approximations G_ij and the exact
@@ -29,6 +34,7 @@
 #include <algorithm>
 #include <chrono>
 #include <string>
+#include <type_traits>
 
 #include "fh_device.cuh"
 #include "fh_pfft.h"
@@ -55,94 +61,152 @@ cudaError_t upload(T **d, const std::vector<T> &h, cudaStream_t s) {
 // Products.
 // ---------------------------------------------------------------------------
 struct ApplyArgs {
-    int64_t n, G, P;
-    int64_t n1, n2, m1, m2;  // unpadded / padded extents of axes 1 and 2
-    int ncomp;
+    int64_t n, G;
     int comp[3];
-    int count;
+    int count;   // vectors
+    int pairs;   // (count + 1) / 2
+    int grids;   // (count ncomp + 1) / 2
 };
 
-// y_v = C x_v, warp per row; the row is read once for up to kNearVec vectors.
-constexpr int kNearVec = 4;
+// Pair p of the vectors: xp[p n + i] = (x_2p,i, x_2p+1,i) (a missing second
+// vector is zero), and its NC complex sources sp[(p n + i) NC + g].
+template <int NC>
+__global__ void __launch_bounds__(256) sources_kernel(const double *__restrict__ x, const double *__restrict__ dir,
+                                                      double2 *__restrict__ xp, double2 *__restrict__ sp,
+                                                      ApplyArgs a) {
+    const int p = blockIdx.y;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double2 v = make_double2(x[2 * (int64_t)p * a.n + i],
+                                       2 * p + 1 < a.count ? x[(2 * (int64_t)p + 1) * a.n + i] : 0.0);
+        xp[(int64_t)p * a.n + i] = v;
+        double r[2 * (NC > 0 ? NC : 1)];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            const double d = dir[3 * i + a.comp[c]];
+            r[c] = v.x * d;
+            r[NC + c] = v.y * d;
+        }
+#pragma unroll
+        for (int g = 0; g < NC; ++g) sp[((int64_t)p * a.n + i) * NC + g] = make_double2(r[2 * g], r[2 * g + 1]);
+    }
+}
+
+// y_v = C x_v, warp per row; the row is read once for NP pairs of vectors.
+// Bound by the row stream (12 bytes an entry) and the gathers of x: at 15.1 M
+// entries and two vectors 80 us with two separate 8-byte gathers, 52 us with
+// one of 16 bytes.
+template <int NP>
 __global__ void __launch_bounds__(256) near_kernel(const int64_t *__restrict__ off, const uint32_t *__restrict__ col,
-                                                   const double *__restrict__ val, const double *__restrict__ x,
-                                                   double *__restrict__ y, int64_t n, int count) {
+                                                   const double *__restrict__ val, const double2 *__restrict__ xp,
+                                                   double *__restrict__ y, int64_t n, int p0, int count) {
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     for (int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); row < n; row += warps) {
         const int64_t b = off[row], e = off[row + 1];
-        for (int v0 = 0; v0 < count; v0 += kNearVec) {
-            const int nv = count - v0 < kNearVec ? count - v0 : kNearVec;
-            double acc[kNearVec] = {0.0, 0.0, 0.0, 0.0};
-            for (int64_t k = b + lane; k < e; k += 32) {
-                const double a = val[k];
-                const int64_t c = col[k];
+        double2 acc[NP];
 #pragma unroll
-                for (int v = 0; v < kNearVec; ++v)
-                    if (v < nv) acc[v] += a * x[(int64_t)(v0 + v) * n + c];
-            }
+        for (int q = 0; q < NP; ++q) acc[q] = make_double2(0.0, 0.0);
+#pragma unroll 4
+        for (int64_t k = b + lane; k < e; k += 32) {
+            const double a = val[k];
+            const int64_t c = col[k];
 #pragma unroll
-            for (int v = 0; v < kNearVec; ++v) {
-                double t = acc[v];
-                for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-                if (lane == 0 && v < nv) y[(int64_t)(v0 + v) * n + row] = t;
+            for (int q = 0; q < NP; ++q) {
+                const double2 v = xp[(int64_t)(p0 + q) * n + c];
+                acc[q].x += a * v.x;
+                acc[q].y += a * v.y;
             }
+        }
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+            for (int o = 16; o > 0; o >>= 1) {
+                acc[q].x += __shfl_xor_sync(0xffffffffu, acc[q].x, o);
+                acc[q].y += __shfl_xor_sync(0xffffffffu, acc[q].y, o);
+            }
+            const int v = 2 * (p0 + q) + lane;
+            if (lane < 2 && v < count) y[(int64_t)v * n + row] = lane ? acc[q].y : acc[q].x;
         }
     }
 }
 
-// Grid sources into compact complex grids: real source r = v * ncomp + c
-// goes to grid r / 2, part r % 2, at the grid index g.  T: the convolution's
-// precision.
-template <class T>
+// Grid sources into compact complex grids at the grid index g.  T: the
+// convolution's precision.  Bound by latency (a few entries per point, each a
+// gather): at 2.8 M points, 7.1 M entries and two grids 182 us with the
+// entries read once per vector and x and the direction gathered apart, 55 us
+// with one pass and one 16-byte gather per grid.
+template <int NC, class T2>
 __global__ void __launch_bounds__(256) spread_kernel(const int64_t *__restrict__ off,
                                                      const uint32_t *__restrict__ fil,
-                                                     const double *__restrict__ w, const double *__restrict__ dir,
-                                                     const double *__restrict__ x, T *__restrict__ work,
-                                                     ApplyArgs a) {
+                                                     const double *__restrict__ w, const double2 *__restrict__ sp,
+                                                     T2 *__restrict__ work, ApplyArgs a) {
+    const int p = blockIdx.y;
+    const double2 *__restrict__ s = sp + (int64_t)p * a.n * NC;
     for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < a.G; g += (int64_t)gridDim.x * blockDim.x) {
         const int64_t b = off[g], e = off[g + 1];
-        for (int v = 0; v < a.count; ++v) {
-            const double *xv = x + (int64_t)v * a.n;
-            double q[3] = {0.0, 0.0, 0.0};
-            for (int64_t t = b; t < e; ++t) {
-                const uint32_t f = fil[t];
-                const double s = w[t] * xv[f];
-                for (int c = 0; c < a.ncomp; ++c) q[c] += s * dir[3 * (int64_t)f + a.comp[c]];
-            }
-            for (int c = 0; c < a.ncomp; ++c) {
-                const int r = v * a.ncomp + c;
-                work[2 * ((int64_t)(r >> 1) * a.G + g) + (r & 1)] = (T)q[c];
+        double2 q[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) q[c] = make_double2(0.0, 0.0);
+#pragma unroll 4
+        for (int64_t t = b; t < e; ++t) {
+            const int64_t f = fil[t];
+            const double wt = w[t];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const double2 v = s[f * NC + c];
+                q[c].x += wt * v.x;
+                q[c].y += wt * v.y;
             }
         }
-        // the unused imaginary part of an odd number of sources
-        if ((a.count * a.ncomp) & 1) work[2 * ((int64_t)((a.count * a.ncomp) >> 1) * a.G + g) + 1] = (T)0;
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+            if (p * NC + c < a.grids) {
+                T2 o;
+                o.x = q[c].x;
+                o.y = q[c].y;
+                work[(int64_t)(p * NC + c) * a.G + g] = o;
+            }
     }
 }
 
 // y_vi += mu0/4pi sum_c d_ic sum_g W_ig phi_{v,c}(g), warp per filament, from
-// the compact potential grids.
-template <class T>
+// the compact potential grids: the two vectors' sums are formed per lane and
+// reduced together.  At 7.1 M entries and two grids 112 us with a pass and a
+// reduction for each vector and component, 58 us now.
+template <int NC, class T2>
 __global__ void __launch_bounds__(256) interp_kernel(const int64_t *__restrict__ off, const uint32_t *__restrict__ idx,
                                                      const double *__restrict__ w, const double *__restrict__ dir,
-                                                     const T *__restrict__ work, double *__restrict__ y,
+                                                     const T2 *__restrict__ work, double *__restrict__ y,
                                                      ApplyArgs a) {
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, p = blockIdx.y;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < a.n; i += warps) {
         const int64_t b = off[i], e = off[i + 1];
-        for (int v = 0; v < a.count; ++v) {
-            double far = 0.0;
-            for (int c = 0; c < a.ncomp; ++c) {
-                const int r = v * a.ncomp + c;
-                const T *grid = work + 2 * (int64_t)(r >> 1) * a.G + (r & 1);
-                double sum = 0.0;
-                for (int64_t t = b + lane; t < e; t += 32) sum += w[t] * (double)grid[2 * (int64_t)idx[t]];
-                for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
-                far += dir[3 * i + a.comp[c]] * sum;
-            }
-            if (lane == 0) y[(int64_t)v * a.n + i] += kMu0Over4PiP * far;
+        double acc[2 * NC] = {};
+#pragma unroll 2
+        for (int64_t t = b + lane; t < e; t += 32) {
+            const int64_t g = idx[t];
+            const double wt = w[t];
+#pragma unroll
+            for (int c = 0; c < NC; ++c)
+                if (p * NC + c < a.grids) {
+                    const T2 v = work[(int64_t)(p * NC + c) * a.G + g];
+                    acc[2 * c] += wt * (double)v.x;
+                    acc[2 * c + 1] += wt * (double)v.y;
+                }
         }
+        double f0 = 0.0, f1 = 0.0;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            const double d = dir[3 * i + a.comp[c]];
+            f0 += d * acc[c];
+            f1 += d * acc[NC + c];
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            f0 += __shfl_xor_sync(0xffffffffu, f0, o);
+            f1 += __shfl_xor_sync(0xffffffffu, f1, o);
+        }
+        const int v = 2 * p + lane;
+        if (lane < 2 && v < a.count) y[(int64_t)v * a.n + i] += kMu0Over4PiP * (lane ? f1 : f0);
     }
 }
 
@@ -314,48 +378,76 @@ fh_status pfft_apply(PfftDevice &op, const double *d_x, double *d_y, int count, 
 }
 
 namespace {
-template <class T>
-fh_status apply_far(PfftDevice &op, const FftConvTables &conv, const double *d_x, double *d_y, int count,
-                    PfftProduct kind, fh_error_info *err) {
-    cudaStream_t s = (cudaStream_t)op.stream;
+ApplyArgs apply_args(const PfftDevice &op, int count) {
     const int ncomp = (int)op.components.size();
-    const int grids = (count * ncomp + 1) / 2;
-    fh_status e = ensure_work(op, sizeof(T) * 2 * fftconv_work_elems(conv.shape) * (size_t)grids, err);
-    if (e) return e;
     ApplyArgs a;
     a.n = op.n;
     a.G = op.G;
-    a.P = op.P;
-    a.n1 = op.grid.dims[1];
-    a.n2 = op.grid.dims[2];
-    a.m1 = op.padded[1];
-    a.m2 = op.padded[2];
-    a.ncomp = ncomp;
     for (int c = 0; c < 3; ++c) a.comp[c] = c < ncomp ? op.components[c] : 0;
     a.count = count;
-    T *work = static_cast<T *>(op.d_work);
-    spread_kernel<T><<<blocks_for(op.G, 256), 256, 0, s>>>(op.d_spread_off, op.d_spread_fil, op.d_spread_w, op.d_dir,
-                                                            d_x, work, a);
+    a.pairs = (count + 1) / 2;
+    a.grids = (count * ncomp + 1) / 2;
+    return a;
+}
+
+template <int NC, class T>
+fh_status apply_far(PfftDevice &op, const FftConvTables &conv, const double2 *sp, T *work, double *d_y,
+                    const ApplyArgs &a, PfftProduct kind, fh_error_info *err) {
+    using T2 = typename std::conditional<sizeof(T) == 4, float2, double2>::type;
+    cudaStream_t s = (cudaStream_t)op.stream;
+    T2 *grids = reinterpret_cast<T2 *>(work);
+    spread_kernel<NC, T2><<<dim3(blocks_for(op.G, 256), a.pairs), 256, 0, s>>>(op.d_spread_off, op.d_spread_fil,
+                                                                              op.d_spread_w, sp, grids, a);
     FHB_CUDA(cudaGetLastError());
-    e = sizeof(T) == 4 && kind == PfftProduct::Ports ? fftconv_run_ports(conv, work, grids, s, err)
-                                                     : fftconv_run<T>(conv, work, grids, s, err);
+    const fh_status e = sizeof(T) == 4 && kind == PfftProduct::Ports ? fftconv_run_ports(conv, work, a.grids, s, err)
+                                                                     : fftconv_run<T>(conv, work, a.grids, s, err);
     if (e) return e;
-    interp_kernel<T><<<blocks_for(op.n * 32, 256), 256, 0, s>>>(op.d_proj_off, op.d_proj_idx, op.d_proj_w, op.d_dir,
-                                                                 work, d_y, a);
+    interp_kernel<NC, T2><<<dim3(blocks_for(op.n * 32, 256), a.pairs), 256, 0, s>>>(
+        op.d_proj_off, op.d_proj_idx, op.d_proj_w, op.d_dir, grids, d_y, a);
     FHB_CUDA(cudaGetLastError());
+    return FH_OK;
+}
+
+template <int NC>
+fh_status apply_components(PfftDevice &op, const double *d_x, double *d_y, int count, PfftProduct kind,
+                           fh_error_info *err) {
+    cudaStream_t s = (cudaStream_t)op.stream;
+    const ApplyArgs a = apply_args(op, count);
+    const bool fp32 = op.fft_fp32 && kind != PfftProduct::Full;
+    const FftConvTables &conv = op.fft_fp32 && !fp32 ? op.conv64 : op.conv;
+    // workspace: the vectors' pairs, their sources, the convolution's grids
+    const size_t vectors = sizeof(double2) * (size_t)op.n * a.pairs * (1 + NC);
+    const size_t grids = NC ? (fp32 ? 8 : 16) * fftconv_work_elems(conv.shape) * (size_t)a.grids : 0;
+    fh_status e = ensure_work(op, vectors + grids, err);
+    if (e) return e;
+    double2 *xp = static_cast<double2 *>(op.d_work);
+    double2 *sp = xp + op.n * a.pairs;
+    void *work = sp + op.n * a.pairs * NC;
+    sources_kernel<NC><<<dim3(blocks_for(op.n, 256), a.pairs), 256, 0, s>>>(d_x, op.d_dir, xp, sp, a);
+    for (int p = 0; p < a.pairs; p += 2) {
+        const unsigned blocks = blocks_for(op.n * 32, 256);
+        if (p + 1 < a.pairs)
+            near_kernel<2><<<blocks, 256, 0, s>>>(op.d_near_off, op.d_near_col, op.d_near_val, xp, d_y, op.n, p, count);
+        else
+            near_kernel<1><<<blocks, 256, 0, s>>>(op.d_near_off, op.d_near_col, op.d_near_val, xp, d_y, op.n, p, count);
+    }
+    FHB_CUDA(cudaGetLastError());
+    if constexpr (NC > 0) {
+        if (fp32) return apply_far<NC, float>(op, conv, sp, static_cast<float *>(work), d_y, a, kind, err);
+        return apply_far<NC, double>(op, conv, sp, static_cast<double *>(work), d_y, a, kind, err);
+    }
     return FH_OK;
 }
 }  // namespace
 
 fh_status pfft_apply_impl(PfftDevice &op, const double *d_x, double *d_y, int count, fh_error_info *err,
                           PfftProduct kind) {
-    cudaStream_t s = (cudaStream_t)op.stream;
-    near_kernel<<<blocks_for(op.n * 32, 256), 256, 0, s>>>(op.d_near_off, op.d_near_col, op.d_near_val, d_x, d_y,
-                                                             op.n, count);
-    FHB_CUDA(cudaGetLastError());
-    if (op.components.empty()) return FH_OK;
-    if (op.fft_fp32 && kind != PfftProduct::Full) return apply_far<float>(op, op.conv, d_x, d_y, count, kind, err);
-    return apply_far<double>(op, op.fft_fp32 ? op.conv64 : op.conv, d_x, d_y, count, kind, err);
+    switch (op.components.size()) {
+        case 0: return apply_components<0>(op, d_x, d_y, count, kind, err);
+        case 1: return apply_components<1>(op, d_x, d_y, count, kind, err);
+        case 2: return apply_components<2>(op, d_x, d_y, count, kind, err);
+        default: return apply_components<3>(op, d_x, d_y, count, kind, err);
+    }
 }
 
 }  // namespace fhb
