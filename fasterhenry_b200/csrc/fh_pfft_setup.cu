@@ -1,7 +1,7 @@
 // Device part of the precorrected-FFT set-up (pfft/mod.rs:332-460,
 // grid.rs:100-216, near.rs:114-401 of the reference):
 //
-//   * projection: thread per filament.  A composite Gauss-Legendre rule over
+//   * projection: warp per filament.  A composite Gauss-Legendre rule over
 //     the filament's length, width and height (pieces no longer than h, the
 //     order from the 1e-10 / 12 table at the near-field distance) is
 //     interpolated onto the (order+1)^3 Lagrange stencil of every node and
@@ -10,14 +10,15 @@
 //     index, are the filament's row of W.  Its transpose (by grid point, then
 //     filament) comes from a stable radix sort.
 //   * grid approximation of every near pair, sum_g sum_h W_ig W_jh K(g - h):
-//     block per row i, the row's projection staged in shared memory, warp
-//     per partner j, lanes over j's projection, a fixed reduction tree.
-//     K(d) = 1 / (h |d|) (zero at the origin) is tabulated once over the
-//     offsets the pairs reach.
+//     block per row i, which either forms the potential of i's projection on
+//     the grid points that its partners reach, once for all of them, and sums
+//     it over each partner's projection, or sums every pair's products alone
+//     (see precorrect_kernel).  K(d) = 1 / (h |d|) (zero at the origin) is
+//     tabulated once over the offsets the pairs reach.
 //   * the near-field matrix: exact - mu0/4pi cos approximation per pair,
 //     mirrored into full rows ascending in column by one radix sort.
 //
-// Every result is deterministic: each filament's sums run in a fixed order
+// Every result is deterministic: each grid point's sums run in a fixed order
 // on one thread, each pair's on one warp with a fixed shuffle tree.
 #include <cub/cub.cuh>
 
@@ -59,15 +60,13 @@ __host__ __device__ inline int64_t stencil_first(const GridArgs &g, int a, doubl
     return first < last ? first : last;
 }
 
-// The m Lagrange weights of the stencil starting at `first`.
-__device__ inline void stencil_weights(const GridArgs &g, int a, double x, int64_t first, double *w) {
+// Lagrange weight k of the m-point stencil starting at `first`.
+__device__ inline double stencil_weight(const GridArgs &g, int a, double x, int64_t first, int k) {
     const double t = (x - g.origin[a]) / g.spacing - (double)first;
-    for (int k = 0; k < g.m; ++k) {
-        double v = 1.0;
-        for (int l = 0; l < g.m; ++l)
-            if (l != k) v *= (t - (double)l) / ((double)k - (double)l);
-        w[k] = v;
-    }
+    double v = 1.0;
+    for (int l = 0; l < g.m; ++l)
+        if (l != k) v *= (t - (double)l) / ((double)k - (double)l);
+    return v;
 }
 
 // OrderTable(1e-10, 12).order_for (gauss.rs:123-136); 0 when none suffices.
@@ -88,11 +87,20 @@ struct Box {
     int64_t offset;
 };
 
-__global__ void __launch_bounds__(128) project_kernel(const fh_filament *__restrict__ fil, int64_t n, GridArgs g,
-                                                      double far, const Box *__restrict__ boxes,
-                                                      double *__restrict__ scratch, uint8_t *__restrict__ touched,
-                                                      int64_t *__restrict__ counts, int *__restrict__ overflow) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// A warp walks its filament's quadrature nodes in the rule's order; at each,
+// the lanes share the 3 m weights and own the m^3 stencil points (distinct
+// cells of the box), so every cell sums its nodes in that order.  With a
+// thread per filament 10,200 filaments (order 5: 216 points a node) filled a
+// hundred of the SMs' warps: 17.2 ms, 3.6 ms now.
+constexpr int kProjWarps = 4;
+__global__ void __launch_bounds__(32 * kProjWarps)
+    project_kernel(const fh_filament *__restrict__ fil, int64_t n, GridArgs g, double far,
+                   const Box *__restrict__ boxes, double *__restrict__ scratch, uint8_t *__restrict__ touched,
+                   int64_t *__restrict__ counts, int *__restrict__ overflow) {
+    __shared__ double weights[kProjWarps][3][16];
+    const int lane = threadIdx.x & 31;
+    double(*lw)[16] = weights[threadIdx.x >> 5];
+    const int64_t i = (int64_t)blockIdx.x * kProjWarps + (threadIdx.x >> 5);
     if (i >= n) return;
     const fh_filament f = fil[i];
     const Box b = boxes[i];
@@ -114,7 +122,6 @@ __global__ void __launch_bounds__(128) project_kernel(const fh_filament *__restr
     const int m = g.m;
     double *box = scratch + b.offset;
     uint8_t *hit = touched + b.offset;
-    double wx[16], wy[16], wz[16];
     for (int64_t p0 = 0; p0 < pieces[0]; ++p0)
         for (int q0 = 0; q0 < order[0]; ++q0) {
             const double a0 = (double)p0 * piece[0], b0 = (double)(p0 + 1) * piece[0];
@@ -140,28 +147,32 @@ __global__ void __launch_bounds__(128) project_kernel(const fh_filament *__restr
                             const int64_t ox = fx - b.lo[0], oy = fy - b.lo[1], oz = fz - b.lo[2];
                             if (ox < 0 || oy < 0 || oz < 0 || ox + m > b.dims[0] || oy + m > b.dims[1] ||
                                 oz + m > b.dims[2]) {
-                                atomicExch(overflow, 1);  // never writes outside the box
+                                if (lane == 0) atomicExch(overflow, 1);  // never writes outside the box
                                 continue;
                             }
-                            stencil_weights(g, 0, r[0], fx, wx);
-                            stencil_weights(g, 1, r[1], fy, wy);
-                            stencil_weights(g, 2, r[2], fz, wz);
-                            for (int ii = 0; ii < m; ++ii)
-                                for (int jj = 0; jj < m; ++jj) {
-                                    const int64_t row = ((ox + ii) * b.dims[1] + (oy + jj)) * b.dims[2] + oz;
-                                    const double lxy = weight * wx[ii] * wy[jj];
-                                    for (int kk = 0; kk < m; ++kk) {
-                                        box[row + kk] += lxy * wz[kk];
-                                        hit[row + kk] = 1;
-                                    }
-                                }
+                            __syncwarp();  // the previous node's weights are read
+                            for (int t = lane; t < 3 * m; t += 32) {
+                                const int a = t / m, k = t - a * m;
+                                lw[a][k] = stencil_weight(g, a, r[a], a == 0 ? fx : a == 1 ? fy : fz, k);
+                            }
+                            __syncwarp();
+                            for (int t = lane; t < m * m * m; t += 32) {
+                                const int ij = t / m, kk = t - ij * m, ii = ij / m, jj = ij - ii * m;
+                                const int64_t cell = ((ox + ii) * b.dims[1] + (oy + jj)) * b.dims[2] + oz + kk;
+                                const double lxy = weight * lw[0][ii] * lw[1][jj];
+                                box[cell] += lxy * lw[2][kk];
+                                hit[cell] = 1;
+                            }
                         }
                 }
         }
+    // the counting lanes read cells that other lanes wrote
+    __syncwarp();
     const int64_t cells = (int64_t)b.dims[0] * b.dims[1] * b.dims[2];
-    int64_t c = 0;
-    for (int64_t k = 0; k < cells; ++k) c += hit[k];
-    counts[i] = c;
+    int c = 0;
+    for (int64_t k = lane; k < cells; k += 32) c += hit[k];
+    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    if (lane == 0) counts[i] = c;
 }
 
 // Writes the touched points of each box, ascending grid index, with their
@@ -231,42 +242,154 @@ __global__ void reach_kernel(const int2 *__restrict__ pairs, int64_t np, const i
     for (int a = 0; a < 3; ++a) atomicMax(&reach[a], r[a]);
 }
 
-// K(d) = 1 / (h |d|), zero at d = 0, over |d_a| <= reach_a, z fastest (near.rs:114-170).
+// K(d) = 1 / (h |d|), zero at d = 0, over |d_a| <= reach_a (near.rs:114-170),
+// as [x][z][y]: consecutive y of a warp's lanes are then one run of memory,
+// and a thread's consecutive z one stride.  kZTile - 1 more planes in z: a
+// tile of potentials may pass the region's end.
+constexpr int kZTile = 8;
 __global__ void kernel_table_kernel(double *__restrict__ t, int rx, int ry, int rz, double spacing) {
-    const int64_t dy = 2 * ry + 1, dz = 2 * rz + 1, total = (int64_t)(2 * rx + 1) * dy * dz;
+    const int64_t ny = 2 * ry + 1, nz = 2 * rz + kZTile, total = (int64_t)(2 * rx + 1) * ny * nz;
     for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < total; k += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t x = k / (dy * dz) - rx, y = (k / dz) % dy - ry, z = k % dz - rz;
+        const int64_t x = k / (ny * nz) - rx, z = (k / ny) % nz - rz, y = k % ny - ry;
         const double r2 = (double)(x * x + y * y + z * z);
         t[k] = r2 == 0.0 ? 0.0 : 1.0 / (spacing * sqrt(r2));
     }
 }
 
-constexpr int kPreThreads = 128;
+constexpr int kPreThreads = 256;
 constexpr int kPreChunk = 512;
+// Shared memory of a block (two per SM): a row's projection as a dense box,
+// and a slab of potentials.
+constexpr int kPreBox = 2048;
+constexpr int kPrePhi = 11264;
+// A product of the potential path costs about a sixth of one of the pair path
+// (dense FP64 multiply-adds on a window of table values in registers, against
+// a table gather per product); a quarter keeps the margin for its padding.
+constexpr int64_t kPreGain = 4;
 
 // Block per row i: grid[k] = sum over j's entries e of w_e sum over i's
 // entries s of w_s K(e - s), for the row's pairs k.
+//
+// Summed pair by pair that is |W_i| |W_j| products per pair, although the
+// partners of a row lie on the same few thousand grid points.  So the inner
+// sum is formed once per grid point g of the partners' hull,
+// phi_i(g) = sum_s w_s K(g - s), slab by slab in x: a thread takes kZTile
+// consecutive z and slides a window of table values along the box's z.  Then
+// each pair is a dot product of phi_i with W_j.  A row takes this path where
+// hull x box has no more than kPreGain times the products of the pair path
+// and both fit (long filaments with few partners go pair by pair).  10,200
+// filaments of a square meander, order 5, radius 8: 46.5 ms pair by pair,
+// 7.7 ms so; 2 blocks of 256 threads per SM, bound by the FP64 pipe.
 __global__ void __launch_bounds__(kPreThreads) precorrect_kernel(
     int64_t n, GridArgs g, const int64_t *__restrict__ pair_off, const int2 *__restrict__ pairs,
     const int64_t *__restrict__ proj_off, const uint32_t *__restrict__ proj_idx, const double *__restrict__ proj_w,
-    const double *__restrict__ table, int rx, int ry, int rz, double *__restrict__ grid) {
-    __shared__ int32_t sx[kPreChunk], sy[kPreChunk], sz[kPreChunk];
-    __shared__ double sw[kPreChunk];
-    const int64_t dyz = (int64_t)(2 * ry + 1) * (2 * rz + 1), dz = 2 * rz + 1;
+    const int32_t *__restrict__ lohi, const double *__restrict__ table, int rx, int ry, int rz,
+    double *__restrict__ grid) {
+    extern __shared__ __align__(16) double pre_smem[];
+    double *sw = pre_smem, *phi = pre_smem + kPreBox;
+    int32_t *soff = reinterpret_cast<int32_t *>(phi);  // pair path: table offsets of a chunk's points
+    __shared__ int hull[6];
+    __shared__ unsigned long long partner_entries;
+    const int ny = 2 * ry + 1, nz = 2 * rz + kZTile;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = kPreThreads / 32;
+    const unsigned d1 = (unsigned)g.dims[1], d2 = (unsigned)g.dims[2];
     for (int64_t i = blockIdx.x; i < n; i += gridDim.x) {
         const int64_t k0 = pair_off[i], k1 = pair_off[i + 1];
         if (k0 == k1) continue;
         const int64_t s0 = proj_off[i], s1 = proj_off[i + 1];
+        // the partners' hull and how many entries they have
+        __syncthreads();  // the previous row is done with the shared memory
+        if (threadIdx.x < 6) hull[threadIdx.x] = threadIdx.x < 3 ? INT32_MAX : 0;
+        if (threadIdx.x == 6) partner_entries = 0;
+        __syncthreads();
+        for (int64_t k = k0 + threadIdx.x; k < k1; k += kPreThreads) {
+            const int j = pairs[k].y;
+            for (int a = 0; a < 3; ++a) {
+                atomicMin(&hull[a], lohi[6 * (int64_t)j + a]);
+                atomicMax(&hull[3 + a], lohi[6 * (int64_t)j + 3 + a]);
+            }
+            atomicAdd(&partner_entries, (unsigned long long)(proj_off[j + 1] - proj_off[j]));
+        }
+        __syncthreads();
+        int blo[3], bd[3], hd[3];
+        for (int a = 0; a < 3; ++a) {
+            blo[a] = lohi[6 * i + a];
+            bd[a] = lohi[6 * i + 3 + a] - blo[a] + 1;
+            hd[a] = hull[3 + a] - hull[a] + 1;
+        }
+        const int64_t box = (int64_t)bd[0] * bd[1] * bd[2], cells = (int64_t)hd[0] * hd[1] * hd[2];
+        const int64_t plane = (int64_t)hd[1] * hd[2];
+        if (box <= kPreBox && plane <= kPrePhi &&
+            cells * box <= kPreGain * (int64_t)partner_entries * (s1 - s0)) {
+            for (int t = threadIdx.x; t < (int)box; t += kPreThreads) sw[t] = 0.0;
+            __syncthreads();
+            for (int64_t t = s0 + threadIdx.x; t < s1; t += kPreThreads) {
+                const unsigned gi = proj_idx[t], rest = gi / d2, z = gi - rest * d2, x = rest / d1, y = rest - x * d1;
+                sw[(((int)x - blo[0]) * bd[1] + (int)y - blo[1]) * bd[2] + (int)z - blo[2]] = proj_w[t];
+            }
+            const int slab = (int)(kPrePhi / plane), zt = (hd[2] + kZTile - 1) / kZTile;
+            for (int x0 = 0; x0 < hd[0]; x0 += slab) {
+                const int nx = hd[0] - x0 < slab ? hd[0] - x0 : slab;
+                __syncthreads();  // the box is staged; the previous slab's pairs are summed
+                const unsigned tasks = (unsigned)nx * zt * hd[1];
+                for (unsigned task = threadIdx.x; task < tasks; task += kPreThreads) {
+                    const unsigned q = task / (unsigned)hd[1], gy = task - q * hd[1];
+                    const unsigned gx = q / (unsigned)zt, z8 = (q - gx * zt) * kZTile;
+                    // table place of (g - box corner); box point (x, y, z) is at -(x nz + z) ny - y
+                    const int64_t at = ((int64_t)(hull[0] + x0 + (int)gx - blo[0] + rx) * nz +
+                                        (hull[2] + (int)z8 - blo[2] + rz)) *
+                                           ny +
+                                       (hull[1] + (int)gy - blo[1] + ry);
+                    double acc[kZTile] = {};
+                    const double *w = sw;
+                    for (int x = 0; x < bd[0]; ++x)
+                        for (int y = 0; y < bd[1]; ++y, w += bd[2]) {
+                            const double *kp = table + at - (int64_t)x * nz * ny - y;
+                            double win[kZTile];
+#pragma unroll
+                            for (int t = 0; t < kZTile; ++t) win[t] = kp[t * ny];
+                            // at z the window holds K of z8 + t - z in place (t - z) mod kZTile
+                            for (int zb = 0; zb < bd[2]; zb += kZTile) {
+#pragma unroll
+                                for (int zz = 0; zz < kZTile; ++zz) {
+                                    const int z = zb + zz;
+                                    if (z >= bd[2]) break;
+                                    const double wz = w[z];
+#pragma unroll
+                                    for (int t = 0; t < kZTile; ++t)
+                                        acc[t] += wz * win[(t - zz + kZTile) % kZTile];
+                                    if (z + 1 < bd[2]) win[kZTile - 1 - zz] = kp[-(int64_t)(z + 1) * ny];
+                                }
+                            }
+                        }
+#pragma unroll
+                    for (int t = 0; t < kZTile; ++t)
+                        if ((int)z8 + t < hd[2]) phi[((int64_t)gx * hd[2] + z8 + t) * hd[1] + gy] = acc[t];
+                }
+                __syncthreads();
+                for (int64_t k = k0 + warp; k < k1; k += warps) {
+                    const int j = pairs[k].y;
+                    double acc = 0.0;
+                    for (int64_t e = proj_off[j] + lane; e < proj_off[j + 1]; e += 32) {
+                        const unsigned ge = proj_idx[e], rest = ge / d2, z = ge - rest * d2, x = rest / d1,
+                                       y = rest - x * d1;
+                        const int px = (int)x - hull[0] - x0;
+                        if (px >= 0 && px < nx)
+                            acc += proj_w[e] * phi[((int64_t)px * hd[2] + (int)z - hull[2]) * hd[1] + (int)y - hull[1]];
+                    }
+                    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+                    if (lane == 0) grid[k] = (x0 == 0 ? 0.0 : grid[k]) + acc;
+                }
+            }
+            continue;
+        }
         for (int64_t c0 = s0; c0 < s1; c0 += kPreChunk) {
             const int cn = (int)(s1 - c0 < kPreChunk ? s1 - c0 : kPreChunk);
             __syncthreads();
             for (int t = threadIdx.x; t < cn; t += kPreThreads) {
-                const int64_t gi = proj_idx[c0 + t];
-                sz[t] = (int32_t)(gi % g.dims[2]);
-                const int64_t rest = gi / g.dims[2];
-                sy[t] = (int32_t)(rest % g.dims[1]);
-                sx[t] = (int32_t)(rest / g.dims[1]);
+                const unsigned gi = proj_idx[c0 + t], rest = gi / d2, z = gi - rest * d2, x = rest / d1,
+                               y = rest - x * d1;
+                soff[3 * t] = (int)x, soff[3 * t + 1] = (int)y, soff[3 * t + 2] = (int)z;
                 sw[t] = proj_w[c0 + t];
             }
             __syncthreads();
@@ -274,14 +397,13 @@ __global__ void __launch_bounds__(kPreThreads) precorrect_kernel(
                 const int j = pairs[k].y;
                 double acc = 0.0;
                 for (int64_t e = proj_off[j] + lane; e < proj_off[j + 1]; e += 32) {
-                    const int64_t ge = proj_idx[e];
-                    const int32_t ez = (int32_t)(ge % g.dims[2]);
-                    const int64_t rest = ge / g.dims[2];
-                    const int32_t ey = (int32_t)(rest % g.dims[1]), ex = (int32_t)(rest / g.dims[1]);
-                    const double *base = table + (int64_t)(ex + rx) * dyz + (int64_t)(ey + ry) * dz + (ez + rz);
+                    const unsigned ge = proj_idx[e], rest = ge / d2, ez = ge - rest * d2, ex = rest / d1,
+                                   ey = rest - ex * d1;
+                    const double *base =
+                        table + ((int64_t)((int)ex + rx) * nz + ((int)ez + rz)) * ny + ((int)ey + ry);
                     double potential = 0.0;
                     for (int t = 0; t < cn; ++t)
-                        potential += sw[t] * base[-((int64_t)sx[t] * dyz + (int64_t)sy[t] * dz + sz[t])];
+                        potential += sw[t] * base[-(((int64_t)soff[3 * t] * nz + soff[3 * t + 2]) * ny + soff[3 * t + 1])];
                     acc += proj_w[e] * potential;
                 }
                 for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
@@ -425,7 +547,7 @@ fh_status pfft_device_setup(const PfftSetup &st, const fh_filament *fil, const N
     FHB_CUDA(cudaMemsetAsync(d_touched, 0, scratch_cells, s));
     FHB_CUDA(cudaMemsetAsync(d_flag, 0, 16, s));
     FHB_CUDA(cudaMemsetAsync(d_counts + n, 0, 8, s));
-    project_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(d_fil, n, g, st.radius, d_boxes, d_scratch, d_touched,
+    project_kernel<<<(unsigned)((n + kProjWarps - 1) / kProjWarps), 32 * kProjWarps, 0, s>>>(d_fil, n, g, st.radius, d_boxes, d_scratch, d_touched,
                                                                d_counts, d_flag);
     FHB_CUDA(cudaGetLastError());
     // Row offsets of the projection: exclusive sum of the counts.
@@ -498,14 +620,18 @@ fh_status pfft_device_setup(const PfftSetup &st, const fh_filament *fil, const N
         int reach[4] = {0, 0, 0, 0};
         FHB_CUDA(cudaMemcpyAsync(reach, d_reach, 16, cudaMemcpyDeviceToHost, s));
         FHB_CUDA(cudaStreamSynchronize(s));
-        const int64_t tsize = (int64_t)(2 * reach[0] + 1) * (2 * reach[1] + 1) * (2 * reach[2] + 1);
+        const int64_t tsize = (int64_t)(2 * reach[0] + 1) * (2 * reach[1] + 1) * (2 * reach[2] + kZTile);
         double *d_table;
         FHB_CUDA(tmp.get(&d_table, (size_t)tsize));
         kernel_table_kernel<<<blocks(tsize, 256), 256, 0, s>>>(d_table, reach[0], reach[1], reach[2], g.spacing);
         FHB_CUDA(cudaGetLastError());
         const unsigned rows = (unsigned)std::min<int64_t>(n, 148 * 16);
-        precorrect_kernel<<<rows, kPreThreads, 0, s>>>(n, g, d_poff, d_pairs, out.proj_off, out.proj_idx, out.proj_w,
-                                                       d_table, reach[0], reach[1], reach[2], out.pair_grid);
+        constexpr int pre_smem = (kPreBox + kPrePhi) * (int)sizeof(double);
+        static_assert(3 * kPreChunk * sizeof(int32_t) <= kPrePhi * sizeof(double) && kPreChunk <= kPreBox, "chunk");
+        FHB_CUDA(cudaFuncSetAttribute(precorrect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pre_smem));
+        precorrect_kernel<<<rows, kPreThreads, pre_smem, s>>>(n, g, d_poff, d_pairs, out.proj_off, out.proj_idx,
+                                                              out.proj_w, d_lohi, d_table, reach[0], reach[1],
+                                                              reach[2], out.pair_grid);
         FHB_CUDA(cudaGetLastError());
     }
     FHB_CUDA(cudaStreamSynchronize(s));
