@@ -201,7 +201,7 @@ enum PoolSlot {
     kSlotA, kSlotD32, kSlotR, kSlotRnorm, kSlotBnorm, kSlotDnorm, kSlotXnorm, kSlotPiv, kSlotSing, kSlotPv,
     kSlotPi, kSlotTk, kSlotCoop, kSlotLinv, kSlotUinv, kSlotSolve, kSlotPackA, kSlotPackB, kSlotOmega, kSlotX,
     kSlotZ, kSlotXinv, kSlotXpack, kSlotTbuf, kSlotDvec, kSlotFlow, kSlotResPart, kSlotSparseT, kSlotSparseY,
-    kSlotTileCounter,
+    kSlotTileCounter, kSlotLdlt,
     // the persistent batched solve (fh_batch_sweep, mixed), in the first system's pool
     kSlotBatchSys, kSlotBatchOne, kSlotBatchItems, kSlotBatchZ, kSlotBatchStatus, kSlotBatchCounter, kSlotBatchWork
 };
@@ -254,9 +254,10 @@ int outer_for(int64_t m, TrailingUpdate mode) {
     return mode == TrailingUpdate::TensorBf16x3 && m > kOuterFp32 ? kOuterFp32 : 0;
 }
 
-// Factor + solve + Schur for `count` frequencies in FP64.  x_out (count x m x
-// p complex) receives the FP64 solutions; z (count x p x p) the impedances.
-fh_status sweep_chunk_fp64(fh_system *s, const double *d_omega, int count, double *d_x, double *d_z, int *h_singular,
+// Factor + solve + Schur for `count` frequencies in FP64 with partial
+// pivoting.  d_x (count x m x p complex) receives the solutions; z (count x p
+// x p) the impedances.
+fh_status sweep_chunk_pivoted(fh_system *s, const double *d_omega, int count, double *d_x, double *d_z, int *h_singular,
                            float *ms_factor, fh_error_info *err) {
     const int64_t m = s->m, p = s->p, ld = s->nloops;
     cudaStream_t st = s->stream;
@@ -316,6 +317,64 @@ fh_status sweep_chunk_fp64(fh_system *s, const double *d_omega, int count, doubl
         std::fill(h_singular, h_singular + count, 0);
     }
     return schur(s->d_Rm, s->d_Lm, ld, m, p, d_omega, count, d_x, d_z, st, err);
+}
+
+// The FP64 form of `count` frequencies: L D L^T without interchanges
+// (fh_ldlt.cu), and the frequencies whose matrix that does not suit (an
+// inductance matrix made indefinite, for instance by a truncated coupling, or
+// a singular system) again with partial pivoting, which decides whether they
+// are singular.  d_x may be null where only Z is wanted.
+fh_status sweep_chunk_fp64(fh_system *s, const double *d_omega, int count, double *d_x, double *d_z, int *h_singular,
+                           float *ms_factor, fh_error_info *err) {
+    const int64_t m = s->m, p = s->p, M = s->nloops;
+    cudaStream_t st = s->stream;
+    std::fill(h_singular, h_singular + count, 0);
+    if (m == 0) return schur(s->d_Rm, s->d_Lm, M, m, p, d_omega, count, d_x, d_z, st, err);
+    std::vector<int> failed((size_t)count, 0);
+    {
+        PBuf<double> a;
+        PBuf<unsigned char> work;
+        PBuf<int> bad;
+        FHB_PALLOC(s->pool, a, kSlotA, (size_t)count * M * M * 2);
+        FHB_PALLOC(s->pool, work, kSlotLdlt, ldlt_bytes(m, p, count));
+        FHB_PALLOC(s->pool, bad, kSlotSing, (size_t)count);
+        ScopedEvents<2> ev;
+        cudaEventRecord(ev.e[0], st);
+        const fh_status e =
+            ldlt_factor(s->d_Rm, s->d_Lm, m, p, d_omega, count, a.p, work.p, d_z, d_x, bad.p, st, err);
+        cudaEventRecord(ev.e[1], st);
+        if (e) return e;
+        FHB_CUDA(cudaMemcpyAsync(failed.data(), bad.p, sizeof(int) * count, cudaMemcpyDeviceToHost, st));
+        FHB_CUDA(cudaStreamSynchronize(st));
+        float ms = 0;
+        cudaEventElapsedTime(&ms, ev.e[0], ev.e[1]);
+        if (ms_factor) *ms_factor += ms;
+    }
+    std::vector<int> redo;
+    for (int f = 0; f < count; ++f)
+        if (failed[(size_t)f]) redo.push_back(f);
+    if (redo.empty()) return FH_OK;
+    const int again = (int)redo.size();
+    DBuf<double> om(st), x(st), z(st);
+    FHB_ALLOC(om, (size_t)again);
+    FHB_ALLOC(x, (size_t)std::max<int64_t>(1, 2 * again * m * p));
+    FHB_ALLOC(z, (size_t)std::max<int64_t>(1, 2 * again * p * p));
+    for (int k = 0; k < again; ++k)
+        FHB_CUDA(cudaMemcpyAsync(om.p + k, d_omega + redo[(size_t)k], 8, cudaMemcpyDeviceToDevice, st));
+    std::vector<int> singular((size_t)again, 0);
+    const fh_status e = sweep_chunk_pivoted(s, om.p, again, x.p, z.p, singular.data(), ms_factor, err);
+    if (e) return e;
+    for (int k = 0; k < again; ++k) {
+        const int64_t f = redo[(size_t)k];
+        h_singular[f] = singular[(size_t)k];
+        if (p)
+            FHB_CUDA(cudaMemcpyAsync(d_z + 2 * f * p * p, z.p + 2 * (int64_t)k * p * p, 16 * (size_t)(p * p),
+                                     cudaMemcpyDeviceToDevice, st));
+        if (d_x && p)
+            FHB_CUDA(cudaMemcpyAsync(d_x + 2 * f * m * p, x.p + 2 * (int64_t)k * m * p, 16 * (size_t)(m * p),
+                                     cudaMemcpyDeviceToDevice, st));
+    }
+    return FH_OK;
 }
 
 // Mixed form: FP32 factors (trailing updates on the tensor cores when
@@ -1083,7 +1142,9 @@ fh_status fh_sweep(fh_system *sys, const double *freqs, size_t nf, fh_precision 
     // form its two packed operands (8 bytes per entry of an m x 512 block
     // each), the inverses of the diagonal blocks of L and U, and a
     // super-panel's U^-1 in FP32 and packed.
-    const double per = (mixed ? 8.0 : 16.0) * (double)m * (double)m + 64.0 * (double)(m * p + 64) +
+    const double per = (mixed ? 8.0 * (double)m * (double)m
+                              : 16.0 * (double)(m + p) * (double)(m + p) + (double)ldlt_bytes(m, p, 1)) +
+                       64.0 * (double)(m * p + 64) +
                        (outer_for(m, update) ? 16.0 * (double)m * kOuterFp32 + 16.0 * (double)(m + kNbFp32) * kNbFp32 +
                                                    16.0 * kOuterFp32 * kOuterFp32 + 8.0 * kNbFp32 * kOuterFp32
                                              : 0.0);
@@ -1109,7 +1170,7 @@ fh_status fh_sweep(fh_system *sys, const double *freqs, size_t nf, fh_precision 
                                   report && report->residual ? report->residual + c0 : nullptr, &ms_factor, &ms_refine,
                                   update, err);
         } else {
-            e = sweep_chunk_fp64(sys, d_omega.p, count, d_x.p, d_z.p, singular.data() + c0, &ms_factor, err);
+            e = sweep_chunk_fp64(sys, d_omega.p, count, nullptr, d_z.p, singular.data() + c0, &ms_factor, err);
         }
         if (e) return e;
         FHB_CUDA(cudaMemcpyAsync(z_out + 2 * c0 * p * p, d_z.p, 16 * (size_t)count * p * p, cudaMemcpyDeviceToHost, st));
@@ -1121,13 +1182,12 @@ fh_status fh_sweep(fh_system *sys, const double *freqs, size_t nf, fh_precision 
         if (!redo.empty()) {
             std::vector<double> om2;
             for (int f : redo) om2.push_back(omega[f]);
-            DBuf<double> d_om2, d_x2, d_z2;
+            DBuf<double> d_om2, d_z2;
             FHB_ALLOC(d_om2, om2.size());
-            FHB_ALLOC(d_x2, om2.size() * m * p * 2);
             FHB_ALLOC(d_z2, om2.size() * p * p * 2);
             FHB_CUDA(cudaMemcpyAsync(d_om2.p, om2.data(), 8 * om2.size(), cudaMemcpyHostToDevice, st));
             std::vector<int> sing2(om2.size(), 0);
-            e = sweep_chunk_fp64(sys, d_om2.p, (int)om2.size(), d_x2.p, d_z2.p, sing2.data(), &ms_factor, err);
+            e = sweep_chunk_fp64(sys, d_om2.p, (int)om2.size(), nullptr, d_z2.p, sing2.data(), &ms_factor, err);
             if (e) return e;
             std::vector<double> z2(om2.size() * p * p * 2);
             FHB_CUDA(cudaMemcpyAsync(z2.data(), d_z2.p, 8 * z2.size(), cudaMemcpyDeviceToHost, st));
@@ -1343,7 +1403,10 @@ fh_status fh_currents(fh_system *sys, const double *freqs, size_t nf, const doub
             for (int f = 0; f < count; ++f) redo = redo || failed[(size_t)f];
         }
         if (!mixed || redo) {  // refinement that did not converge: the whole batch in FP64
-            e = sweep_chunk_fp64(sys, d_omega.p, count, d_x.p, d_z.p, singular.data(), &ms_factor, err);
+            // With partial pivoting: the filament of largest |J| is a tie
+            // wherever a bundle is symmetric, which the last bits decide, and
+            // the reference decides it by this elimination.
+            e = sweep_chunk_pivoted(sys, d_omega.p, count, d_x.p, d_z.p, singular.data(), &ms_factor, err);
             if (e) return e;
         }
         e = launch_currents(d_x.p, d_ip.p, m, (int)p, false, n, count, sys->d_col_ptr, sys->d_col_loop, sys->d_col_sign,

@@ -1,0 +1,577 @@
+// Batched FP64 factorization of the mesh system without interchanges,
+// A = L D L^T with a unit lower triangular L (no conjugation), for the FP64
+// sweep, the filament currents and the gradient.
+//
+// Z_ee = R_ee + j w L_ee is complex symmetric, and with both parts positive
+// definite elimination without pivoting is stable (N. J. Higham, Math. Comp.
+// 67, 1998).  Against the pivoted LU this leaves out half of the arithmetic
+// (only the lower triangle is updated) and the pivot search, whose exchange
+// among a matrix's CTAs in every column was most of the time of small orders
+// and a quarter of large ones.
+//
+// The matrix is the whole mesh system, the port rows last (order M = m + p);
+// the first m columns are eliminated.  The rows of L below them then hold
+// (D^-1 L^-1 Z_ep)^T, and the trailing p x p block is the Schur complement
+// Z_pp - Z_ep^T Z_ee^-1 Z_ep = Z(w) itself, so a sweep needs no triangular
+// solve; X = Z_ee^-1 Z_ep, where it is wanted, is one backward substitution.
+//
+// Nothing is assumed of the matrix: the factors' backward error is bounded by
+// u |L| |D| |L|^T, whose diagonal sum_k |l_ik|^2 |d_k| is accumulated row by
+// row as the panels go.  A matrix with a row above kGrowthLimit |a_ii| (it is about
+// |a_ii| for the class above), or with a zero or non-finite pivot, is
+// reported as failed, and the caller factors it with partial pivoting.
+//
+// Per panel of 64 columns, three launches over all matrices:
+//   ldlt_diag_kernel    the 64 x 64 diagonal block's L and D, and L^-1;
+//   ldlt_panel_kernel   B = A21 L11^-T, L21 = B D^-1 for the rows below;
+//   ldlt_update_kernel  A22 -= L21 B^T on the tiles on and below the diagonal.
+// The products run on the FP64 tensor cores (mma.sync f64: tcgen05 has no FP64
+// kind), as four real products of split real and imaginary parts.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "fh_device.cuh"
+#include "fh_lu.cuh"
+
+namespace fhb {
+namespace {
+
+constexpr int kLd = kLdltPanel;       // panel width and tile edge
+constexpr int kLdPad = kLd + 2;       // row of a staged chunk: four k and two rows of a fragment load hit all banks once
+constexpr int kLdK = 16;              // k per stage of the update
+constexpr int kLdThreads = 256;
+constexpr int kDiagThreads64 = 512;
+constexpr double kGrowthLimit = 128.0;  // on 1-norms of complex numbers, at most twice the moduli's product
+
+// m16n8k4: two stacked m8n8k4 fragments of A and C.
+__device__ __forceinline__ void dmma(double (&lo)[2], double (&hi)[2], double a0, double a1, double b) {
+    asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
+                 : "+d"(lo[0]), "+d"(lo[1]), "+d"(hi[0]), "+d"(hi[1])
+                 : "d"(a0), "d"(a1), "d"(b));
+}
+// base[at] to shared memory, or zeros when !live (the address is then base's).
+__device__ __forceinline__ void copy16(double2 *dst, const double2 *base, int64_t at, bool live) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(live ? base + at : base),
+                 "r"(live ? 16 : 0));
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;"); }
+template <int N>
+__device__ __forceinline__ void copy_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N));
+}
+
+// A = R + j w L on the tiles on and below the diagonal, order M, and the
+// diagonal's 1-norms.
+__global__ void __launch_bounds__(256) ldlt_form_kernel(const double *__restrict__ R, const double *__restrict__ L,
+                                                        int64_t M, const double *__restrict__ omega, int count,
+                                                        double2 *__restrict__ a, double *__restrict__ diag) {
+    const int64_t col = blockIdx.x, first = col / kLd * kLd;
+    for (int64_t row = first + (int64_t)blockIdx.y * blockDim.x + threadIdx.x; row < M;
+         row += (int64_t)gridDim.y * blockDim.x) {
+        const double r = R[row + col * M], l = L[row + col * M];
+        for (int f = 0; f < count; ++f) {
+            const double x = omega[f] * l;
+            a[(int64_t)f * M * M + row + col * M] = make_double2(r, x);
+            if (row == col) diag[(int64_t)f * M + row] = fabs(r) + fabs(x);
+        }
+    }
+}
+
+// y -= l t
+__device__ __forceinline__ void sub_mul(double2 &y, double2 l, double2 t) {
+    y.x -= l.x * t.x - l.y * t.y;
+    y.y -= l.x * t.y + l.y * t.x;
+}
+
+// The diagonal block [k0, k0 + nb)^2 of every matrix (one CTA each): L below
+// its diagonal and D on it, in place; L^-1 (unit lower, zeros above and
+// beyond nb) and D^-1.  Gauss-Jordan in one array: until step k place (i, k)
+// holds the Schur complement's entry, after it the entry of L^-1, which
+// starts as -l_ik; step j takes l_ij times v from row i, where v is row j of
+// L^-1 left of the pivot and column j of the complement beyond it.
+//
+// A warp owns the columns w + 16 c and its lanes the rows lane and lane + 32,
+// in registers (columns from 32 on only the lower rows); v goes through a
+// double buffer with one barrier per step, and rows at or above the pivot take
+// part with l = 0.  The steps run in four segments of 16, so that which of a
+// warp's columns lie left or right of the pivot is known at compile time.
+//
+// Bound by its chain of 64 steps of one barrier, one division and some forty
+// dependent instructions, at most one CTA per matrix: 38 us (88 us with a row
+// per thread, whose columns' cases diverge in every step).
+struct DiagBlock {
+    double2 lo[2], hi[4];  // rows lane and lane + 32 of column w + 16 c
+    double sum0, sum1;     // the rows' |l|^2 |d| over the block (warp 0)
+};
+template <int JC>
+__device__ __forceinline__ void diag_segment(DiagBlock &b, double2 (&v)[2][kLd], double2 *__restrict__ A, int64_t M,
+                                             int nb, int w, int lane, double2 *__restrict__ dinv,
+                                             int *__restrict__ failed) {
+    constexpr bool upper = JC < 2;  // pivots among the rows `lane`
+    const int r0 = lane, r1 = lane + 32;
+    for (int jw = 0; jw < 16; ++jw) {
+        const int j = 16 * JC + jw;
+        if (j >= nb) return;
+        double2 *vj = v[jw & 1];
+        // row j of L^-1 and column j of the complement
+        if (lane == (j & 31)) {
+#pragma unroll
+            for (int c = 0; c < JC; ++c) vj[w + 16 * c] = upper ? b.lo[c < 2 ? c : 0] : b.hi[c];
+            if (w < jw) vj[w + 16 * JC] = upper ? b.lo[upper ? JC : 0] : b.hi[JC];
+        }
+        if (w == jw) {
+            if (upper && r0 >= j) vj[r0] = b.lo[upper ? JC : 0];
+            if (r1 >= j) vj[r1] = b.hi[JC];
+        }
+        __syncthreads();
+        const double2 d = vj[j], q1 = vj[r1];
+        double2 q0 = make_double2(0.0, 0.0);
+        if (upper) q0 = vj[r0];
+        const double n = 1.0 / (d.x * d.x + d.y * d.y);
+        const double2 inv = make_double2(d.x * n, -d.y * n);
+        double2 l0 = make_double2(q0.x * inv.x - q0.y * inv.y, q0.x * inv.y + q0.y * inv.x);
+        double2 l1 = make_double2(q1.x * inv.x - q1.y * inv.y, q1.x * inv.y + q1.y * inv.x);
+        if (!upper || r0 <= j) l0 = make_double2(0.0, 0.0);
+        if (r1 <= j) l1 = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (c == JC && w == jw) {  // L's column, and the start of L^-1's
+                if (upper && r0 > j) {
+                    if (r0 < nb) A[r0 + (int64_t)j * M] = l0;
+                    b.lo[upper ? JC : 0] = make_double2(-l0.x, -l0.y);
+                }
+                if (r1 > j) {
+                    if (r1 < nb) A[r1 + (int64_t)j * M] = l1;
+                    b.hi[JC] = make_double2(-l1.x, -l1.y);
+                }
+            } else {
+                const double2 t = vj[w + 16 * c];
+                if (c < 2 && upper) sub_mul(b.lo[c < 2 ? c : 0], l0, t);
+                sub_mul(b.hi[c], l1, t);
+            }
+        }
+        if (w == 0) {
+            if (upper) b.sum0 += (fabs(q0.x) + fabs(q0.y)) * (fabs(l0.x) + fabs(l0.y));
+            b.sum1 += (fabs(q1.x) + fabs(q1.y)) * (fabs(l1.x) + fabs(l1.y));
+            if (r0 == j) b.sum0 += fabs(d.x) + fabs(d.y);
+            if (r1 == j) b.sum1 += fabs(d.x) + fabs(d.y);
+        }
+        if (w == 15 && lane == 0) {
+            A[j + (int64_t)j * M] = d;
+            dinv[j] = inv;
+            if (!isfinite(inv.x) || !isfinite(inv.y) || !isfinite(d.x) || !isfinite(d.y)) *failed = 1;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kDiagThreads64) ldlt_diag_kernel(double2 *__restrict__ a, int64_t M, int64_t k0,
+                                                                   int nb, double2 *__restrict__ xinv,
+                                                                   int64_t xinv_stride, double2 *__restrict__ dinv,
+                                                                   double *__restrict__ growth,
+                                                                   int *__restrict__ failed) {
+    static_assert(kLd == 64 && kDiagThreads64 == 512, "16 warps of four columns, two rows per lane");
+    __shared__ double2 v[2][kLd];
+    double2 *A = a + (int64_t)blockIdx.x * M * M + k0 + k0 * M;
+    double2 *X = xinv + (int64_t)blockIdx.x * xinv_stride, *D = dinv + (int64_t)blockIdx.x * kLd;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r0 = lane, r1 = lane + 32;
+    const double2 zero = make_double2(0.0, 0.0);
+    if (threadIdx.x < 2 * kLd) v[threadIdx.x / kLd][threadIdx.x % kLd] = zero;  // rows that no step publishes
+    DiagBlock b;
+    b.sum0 = b.sum1 = 0.0;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const int k = w + 16 * c;
+        if (c < 2) b.lo[c < 2 ? c : 0] = r0 >= k && r0 < nb ? A[r0 + k * M] : zero;
+        b.hi[c] = r1 >= k && r1 < nb ? A[r1 + k * M] : zero;
+    }
+    __syncthreads();
+    diag_segment<0>(b, v, A, M, nb, w, lane, D, failed + blockIdx.x);
+    diag_segment<1>(b, v, A, M, nb, w, lane, D, failed + blockIdx.x);
+    diag_segment<2>(b, v, A, M, nb, w, lane, D, failed + blockIdx.x);
+    diag_segment<3>(b, v, A, M, nb, w, lane, D, failed + blockIdx.x);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const int k = w + 16 * c;
+        X[r0 + k * kLd] = c < 2 && k < r0 && r0 < nb ? b.lo[c < 2 ? c : 0]
+                                                     : make_double2(r0 == k && r0 < nb ? 1.0 : 0.0, 0.0);
+        X[r1 + k * kLd] = k < r1 && r1 < nb ? b.hi[c] : make_double2(r1 == k && r1 < nb ? 1.0 : 0.0, 0.0);
+    }
+    if (w == 0) {
+        double *G = growth + (int64_t)blockIdx.x * M + k0;
+        if (r0 < nb) G[r0] += b.sum0;
+        if (r1 < nb) G[r1] += b.sum1;
+    }
+}
+
+// The fragments of one k4 step of a 64 x 64 tile: warp (wr, wc) owns rows
+// 32 wr .. +32 and columns 16 wc .. +16.  Fragment layout of m16n8k4 f64: A at
+// (rows g and g + 8, k t), B at (k t, column g), C at (rows g and g + 8,
+// columns 2 t, 2 t + 1), with g = lane / 4, t = lane % 4.  SIGN: +1 adds, -1 subtracts.
+template <int SIGN>
+__device__ __forceinline__ void tile_step(const double2 *__restrict__ l, const double2 *__restrict__ u, int wr, int wc,
+                                          int g, int t, double (&re)[4][2][2], double (&im)[4][2][2]) {
+    double2 lf[4], uf[2];
+#pragma unroll
+    for (int fm = 0; fm < 4; ++fm) {
+        lf[fm] = l[t * kLdPad + 32 * wr + 8 * fm + g];
+        if (SIGN < 0) lf[fm].x = -lf[fm].x;
+        else lf[fm].y = -lf[fm].y;
+    }
+#pragma unroll
+    for (int fn = 0; fn < 2; ++fn) uf[fn] = u[t * kLdPad + 16 * wc + 8 * fn + g];
+    // SIGN < 0: lf = (-l_re, l_im); SIGN > 0: lf = (l_re, -l_im)
+    // eight independent products between two on the same accumulator
+#pragma unroll
+    for (int fm = 0; fm < 4; fm += 2)
+#pragma unroll
+        for (int fn = 0; fn < 2; ++fn) {
+            dmma(re[fm][fn], re[fm + 1][fn], lf[fm].x, lf[fm + 1].x, uf[fn].x);
+            dmma(im[fm][fn], im[fm + 1][fn], lf[fm].x, lf[fm + 1].x, uf[fn].y);
+        }
+#pragma unroll
+    for (int fm = 0; fm < 4; fm += 2)
+#pragma unroll
+        for (int fn = 0; fn < 2; ++fn) {
+            dmma(re[fm][fn], re[fm + 1][fn], lf[fm].y, lf[fm + 1].y, uf[fn].y);
+            dmma(im[fm][fn], im[fm + 1][fn], -lf[fm].y, -lf[fm + 1].y, uf[fn].x);
+        }
+}
+
+// Rows [c0, M) of the panel [k0, k0 + nb): B = A21 L11^-T into `panel`
+// (column-major, ld M, by absolute row), L21 = B D^-1 in place, and the rows'
+// growth.  A CTA takes 64 rows; it has read them all before it writes.
+__global__ void __launch_bounds__(kLdThreads, 2)
+    ldlt_panel_kernel(double2 *__restrict__ a, int64_t M, int64_t k0, int nb, const double2 *__restrict__ xinv,
+                      int64_t xinv_stride, const double2 *__restrict__ dinv, double2 *__restrict__ panel,
+                      double *__restrict__ growth) {
+    extern __shared__ __align__(16) unsigned char ld_smem[];
+    double2 *Ls = reinterpret_cast<double2 *>(ld_smem), *Us = Ls + 32 * kLdPad;
+    __shared__ double rowsum[kLd];
+    double2 *A = a + (int64_t)blockIdx.y * M * M;
+    const double2 *X = xinv + (int64_t)blockIdx.y * xinv_stride, *D = dinv + (int64_t)blockIdx.y * kLd;
+    double2 *P = panel + (int64_t)blockIdx.y * M * kLd;
+    const int64_t r0 = k0 + nb + (int64_t)blockIdx.x * kLd;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, t = lane & 3, wr = warp >> 2, wc = warp & 3;
+    double re[4][2][2] = {}, im[4][2][2] = {};
+    if (tid < kLd) rowsum[tid] = 0.0;
+    for (int kc = 0; kc < kLd; kc += 32) {
+        __syncthreads();
+        for (int idx = tid; idx < 32 * kLd; idx += kLdThreads) {
+            const int r = idx & (kLd - 1), k = idx / kLd;
+            copy16(&Ls[k * kLdPad + r], A, r0 + r + (k0 + kc + k) * M, r0 + r < M && kc + k < nb);
+            Us[k * kLdPad + r] = X[r + (kc + k) * kLd];  // L^-1 at (column r of B, k)
+        }
+        copy_commit();
+        copy_wait<0>();
+        __syncthreads();
+        // L^-1 is lower triangular: its columns k >= 32 reach only B's columns >= 32
+        if (kc == 0 || wc >= 2) {
+#pragma unroll 2
+            for (int k4 = 0; k4 < 32; k4 += 4)
+                tile_step<1>(Ls + k4 * kLdPad, Us + k4 * kLdPad, wr, wc, g, t, re, im);
+        }
+    }
+#pragma unroll
+    for (int fm = 0; fm < 4; ++fm) {
+        const int r = 32 * wr + 8 * fm + g;
+        double sum = 0.0;
+#pragma unroll
+        for (int fn = 0; fn < 2; ++fn)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int c = 16 * wc + 8 * fn + 2 * t + e;
+                if (r0 + r >= M || c >= nb) continue;
+                const double2 b = make_double2(re[fm][fn][e], im[fm][fn][e]), d = D[c];
+                const double2 l = make_double2(b.x * d.x - b.y * d.y, b.x * d.y + b.y * d.x);
+                P[r0 + r + (int64_t)c * M] = b;
+                A[r0 + r + (k0 + c) * M] = l;
+                sum += (fabs(b.x) + fabs(b.y)) * (fabs(l.x) + fabs(l.y));  // |l|^2 |d|
+            }
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        if (t == 0) atomicAdd(&rowsum[r], sum);
+    }
+    __syncthreads();
+    if (tid < kLd && r0 + tid < M) growth[(int64_t)blockIdx.y * M + r0 + tid] += rowsum[tid];
+}
+
+// A22 -= L21 B^T: one 64 x 64 tile on or below the diagonal per CTA, k in
+// stages of 16 through two buffers of asynchronous copies, both operands
+// [k][row] with re and im side by side (one 16-byte load per fragment).
+//
+// Bound by the FP64 tensor pipe: 8 x 64 operations per complex entry against
+// 32 bytes of C.  Order 2,321 x 32 matrices: 19.0 ms for the 37 panels, 29
+// TFLOP/s of the 37 that the instruction reaches alone (33.5 with the
+// kernel's memory traffic taken out; a third buffer, a fixed or random start
+// delay per CTA against lockstep, and m8n8k4 fragments measured the same or
+// slower); the full update of the pivoted form takes 38.4 ms.
+__global__ void __launch_bounds__(kLdThreads, 2)
+    ldlt_update_kernel(double2 *__restrict__ a, int64_t M, int64_t k0, int nb, const double2 *__restrict__ panel) {
+    extern __shared__ __align__(16) unsigned char ld_smem[];
+    double2 *smem = reinterpret_cast<double2 *>(ld_smem);  // stage s: L at 2 s kLdK kLdPad, B after it
+    double2 *A = a + (int64_t)blockIdx.y * M * M;
+    const double2 *P = panel + (int64_t)blockIdx.y * M * kLd;
+    // tile index to (ti >= tj)
+    const int tile = blockIdx.x;
+    int ti = (int)((sqrt(8.0 * (double)tile + 1.0) - 1.0) * 0.5);
+    while ((int64_t)ti * (ti + 1) / 2 > tile) --ti;
+    while ((int64_t)(ti + 1) * (ti + 2) / 2 <= tile) ++ti;
+    const int tj = tile - (int)((int64_t)ti * (ti + 1) / 2);
+    const int64_t base = k0 + nb, i0 = base + (int64_t)ti * kLd, j0 = base + (int64_t)tj * kLd;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, t = lane & 3, wr = warp >> 2, wc = warp & 3;
+    const int stages = (nb + kLdK - 1) / kLdK;
+    auto load = [&](int st) {
+        double2 *L = smem + (st & 1) * 2 * kLdK * kLdPad, *U = L + kLdK * kLdPad;
+#pragma unroll
+        for (int idx = tid; idx < kLdK * kLd; idx += kLdThreads) {
+            const int r = idx & (kLd - 1), k = idx / kLd, kk = st * kLdK + k;
+            const bool live = kk < nb;
+            copy16(&L[k * kLdPad + r], A, i0 + r + (k0 + kk) * M, live && i0 + r < M);
+            copy16(&U[k * kLdPad + r], P, j0 + r + (int64_t)kk * M, live && j0 + r < M);
+        }
+        copy_commit();
+    };
+    load(0);
+    double re[4][2][2], im[4][2][2];
+#pragma unroll
+    for (int fm = 0; fm < 4; ++fm)
+#pragma unroll
+        for (int fn = 0; fn < 2; ++fn)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int64_t row = i0 + 32 * wr + 8 * fm + g, col = j0 + 16 * wc + 8 * fn + 2 * t + e;
+                double2 c = make_double2(0.0, 0.0);
+                if (row < M && col < M) c = A[row + col * M];
+                re[fm][fn][e] = c.x;
+                im[fm][fn][e] = c.y;
+            }
+    for (int st = 0; st < stages; ++st) {
+        if (st + 1 < stages) {
+            load(st + 1);
+            copy_wait<1>();
+        } else {
+            copy_wait<0>();
+        }
+        __syncthreads();
+        const double2 *L = smem + (st & 1) * 2 * kLdK * kLdPad, *U = L + kLdK * kLdPad;
+#pragma unroll
+        for (int k4 = 0; k4 < kLdK; k4 += 4)
+            tile_step<-1>(L + k4 * kLdPad, U + k4 * kLdPad, wr, wc, g, t, re, im);
+        __syncthreads();  // before the stage after next overwrites this buffer
+    }
+#pragma unroll
+    for (int fm = 0; fm < 4; ++fm)
+#pragma unroll
+        for (int fn = 0; fn < 2; ++fn)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int64_t row = i0 + 32 * wr + 8 * fm + g, col = j0 + 16 * wc + 8 * fn + 2 * t + e;
+                if (row < M && col < M) A[row + col * M] = make_double2(re[fm][fn][e], im[fm][fn][e]);
+            }
+}
+
+// failed[f] = 1 for a row whose growth is above the limit (or not a number).
+__global__ void __launch_bounds__(256) ldlt_growth_kernel(const double *__restrict__ growth,
+                                                          const double *__restrict__ diag, int64_t M, int64_t m,
+                                                          int *__restrict__ failed) {
+    bool bad = false;
+    for (int64_t i = threadIdx.x; i < m; i += blockDim.x)
+        bad = bad || !(growth[blockIdx.x * M + i] <= kGrowthLimit * diag[blockIdx.x * M + i]);
+    if (__syncthreads_or(bad) && threadIdx.x == 0) failed[blockIdx.x] = 1;
+}
+
+// Z from the trailing block: [f][i][j], symmetric; real at zero frequency
+// (solve.rs:811-815).
+__global__ void ldlt_z_kernel(const double2 *__restrict__ a, int64_t M, int64_t m, int p,
+                              const double *__restrict__ omega, int count, double2 *__restrict__ z) {
+    const int64_t total = (int64_t)count * p * p;
+    for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
+         idx += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t f = idx / (p * p), ij = idx % (p * p);
+        const int64_t i = max(ij / p, ij % p), j = min(ij / p, ij % p);
+        double2 v = a[f * M * M + (m + i) + (m + j) * M];
+        if (omega[f] == 0.0) v.y = 0.0;
+        z[idx] = v;
+    }
+}
+
+// x (f, q) <- row m + q of L: the right-hand side of L^T x = .
+__global__ void ldlt_rows_kernel(const double2 *__restrict__ a, int64_t M, int64_t m, int p, int count,
+                                 double2 *__restrict__ x) {
+    const int64_t total = (int64_t)count * p * m;
+    for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
+         idx += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t fq = idx / m, k = idx % m, f = fq / p, q = fq % p;
+        x[idx] = a[f * M * M + (m + q) + k * M];
+    }
+}
+
+__device__ __forceinline__ double2 warp_sum(double2 v) {
+    for (int o = 16; o > 0; o >>= 1) {
+        v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+        v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+    }
+    return v;
+}
+
+// x[k0 .. k0 + nb) <- (L11^-1)^T x, a warp per entry.
+__global__ void __launch_bounds__(256) ldlt_back_block_kernel(const double2 *__restrict__ xinv, int64_t xinv_stride,
+                                                              int64_t m, int p, int64_t k0, int nb,
+                                                              double2 *__restrict__ x) {
+    __shared__ double2 s[kLd];
+    const int64_t f = blockIdx.x / p;
+    const double2 *X = xinv + f * xinv_stride;
+    double2 *xs = x + (int64_t)blockIdx.x * m + k0;
+    const int lane = threadIdx.x & 31;
+    for (int r = threadIdx.x; r < kLd; r += blockDim.x) s[r] = r < nb ? xs[r] : make_double2(0.0, 0.0);
+    __syncthreads();
+    for (int c = threadIdx.x >> 5; c < nb; c += blockDim.x >> 5) {
+        double2 acc = make_double2(0.0, 0.0);
+        for (int r = lane; r < kLd; r += 32) {
+            const double2 l = X[r + c * kLd], v = s[r];
+            acc.x += l.x * v.x - l.y * v.y;
+            acc.y += l.x * v.y + l.y * v.x;
+        }
+        acc = warp_sum(acc);
+        if (lane == 0) xs[c] = acc;
+    }
+}
+
+// x_j -= sum_r L[k0 + r][j] x[k0 + r] for the columns j < k0, a warp per
+// column (its nb rows are one run of memory), all right-hand sides of a
+// matrix from one read.
+__global__ void __launch_bounds__(256) ldlt_back_update_kernel(const double2 *__restrict__ a, int64_t M, int64_t m,
+                                                               int p, int64_t k0, int nb, double2 *__restrict__ x) {
+    const int64_t f = blockIdx.y, j = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (j >= k0) return;
+    const int lane = threadIdx.x & 31;
+    const double2 *L = a + f * M * M + k0 + j * M;
+    double2 l[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) l[h] = lane + 32 * h < nb ? L[lane + 32 * h] : make_double2(0.0, 0.0);
+    for (int q = 0; q < p; ++q) {
+        double2 *xq = x + (f * p + q) * m;
+        double2 acc = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            if (lane + 32 * h < nb) {
+                const double2 v = xq[k0 + lane + 32 * h];
+                acc.x += l[h].x * v.x - l[h].y * v.y;
+                acc.y += l[h].x * v.y + l[h].y * v.x;
+            }
+        acc = warp_sum(acc);
+        if (lane == 0) {
+            xq[j].x -= acc.x;
+            xq[j].y -= acc.y;
+        }
+    }
+}
+
+}  // namespace
+
+size_t ldlt_bytes(int64_t m, int64_t p, int count) {
+    const int64_t M = m + p, blocks = (m + kLd - 1) / kLd;
+    return (size_t)count * (16 * (size_t)M * kLd + 16 * (size_t)blocks * kLd * kLd + 16 * (size_t)blocks * kLd +
+                            16 * (size_t)M + 16);
+}
+
+fh_status ldlt_factor(const double *Rm, const double *Lm, int64_t m, int64_t p, const double *d_omega, int count,
+                      double *a, void *work, double *z, double *x, int *d_failed, cudaStream_t s,
+                      fh_error_info *err) {
+    const int64_t M = m + p, blocks = (m + kLd - 1) / kLd;
+    double2 *A = reinterpret_cast<double2 *>(a);
+    double2 *panel = static_cast<double2 *>(work);
+    double2 *xinv = panel + (int64_t)count * M * kLd;
+    double2 *dinv = xinv + (int64_t)count * blocks * kLd * kLd;
+    double *diag = reinterpret_cast<double *>(dinv + (int64_t)count * blocks * kLd);
+    double *growth = diag + (int64_t)count * M;
+    FHB_CUDA(cudaMemsetAsync(d_failed, 0, sizeof(int) * (size_t)count, s));
+    FHB_CUDA(cudaMemsetAsync(growth, 0, sizeof(double) * (size_t)count * M, s));
+    prof_begin(s, FH_PROF_FORM);
+    ldlt_form_kernel<<<dim3((unsigned)M, (unsigned)std::min<int64_t>((M + 255) / 256, 8)), 256, 0, s>>>(
+        Rm, Lm, M, d_omega, count, A, diag);
+    prof_end(s, FH_PROF_FORM, 16.0 * (double)M * (double)M * count / 2.0);
+    constexpr int panel_smem = 2 * 32 * kLdPad * (int)sizeof(double2);
+    constexpr int update_smem = 4 * kLdK * kLdPad * (int)sizeof(double2);
+    FHB_CUDA(cudaFuncSetAttribute(ldlt_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, panel_smem));
+    FHB_CUDA(cudaFuncSetAttribute(ldlt_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, update_smem));
+    const int64_t xs = blocks * kLd * kLd;
+    for (int64_t k0 = 0, b = 0; k0 < m; k0 += kLd, ++b) {
+        const int nb = (int)std::min<int64_t>(kLd, m - k0);
+        const int64_t rest = M - k0 - nb, tiles = (rest + kLd - 1) / kLd;
+        double2 *xb = xinv + b * kLd * kLd, *db = dinv + b * count * kLd;
+        prof_begin(s, FH_PROF_PANEL);
+        ldlt_diag_kernel<<<(unsigned)count, kDiagThreads64, 0, s>>>(A, M, k0, nb, xb, xs, db, growth, d_failed);
+        prof_end(s, FH_PROF_PANEL, 0.0);
+        if (tiles == 0) continue;
+        prof_begin(s, FH_PROF_TRSM);
+        ldlt_panel_kernel<<<dim3((unsigned)tiles, (unsigned)count), kLdThreads, panel_smem, s>>>(A, M, k0, nb, xb, xs,
+                                                                                                db, panel, growth);
+        prof_end(s, FH_PROF_TRSM, 4.0 * kLd * kLd * (double)rest * count);
+        prof_begin(s, FH_PROF_GEMM_FP64);
+        ldlt_update_kernel<<<dim3((unsigned)(tiles * (tiles + 1) / 2), (unsigned)count), kLdThreads, update_smem, s>>>(
+            A, M, k0, nb, panel);
+        prof_end(s, FH_PROF_GEMM_FP64, 4.0 * (double)rest * (double)rest * nb * count);
+        FHB_CUDA(cudaGetLastError());
+    }
+    if (m > 0) ldlt_growth_kernel<<<(unsigned)count, 256, 0, s>>>(growth, diag, M, m, d_failed);
+    if (p > 0)
+        ldlt_z_kernel<<<(unsigned)std::min<int64_t>(((int64_t)count * p * p + 255) / 256, 1024), 256, 0, s>>>(
+            A, M, m, (int)p, d_omega, count, reinterpret_cast<double2 *>(z));
+    FHB_CUDA(cudaGetLastError());
+    if (!x || m == 0 || p == 0) return FH_OK;
+    prof_begin(s, FH_PROF_SOLVE);
+    double2 *X = reinterpret_cast<double2 *>(x);
+    ldlt_rows_kernel<<<(unsigned)std::min<int64_t>(((int64_t)count * p * m + 255) / 256, 148 * 8), 256, 0, s>>>(
+        A, M, m, (int)p, count, X);
+    for (int64_t b = blocks - 1; b >= 0; --b) {
+        const int64_t k0 = b * kLd;
+        const int nb = (int)std::min<int64_t>(kLd, m - k0);
+        ldlt_back_block_kernel<<<(unsigned)(count * p), 256, 0, s>>>(xinv + b * kLd * kLd, xs, m, (int)p, k0, nb, X);
+        if (k0 > 0)
+            ldlt_back_update_kernel<<<dim3((unsigned)((k0 + 7) / 8), (unsigned)count), 256, 0, s>>>(A, M, m, (int)p,
+                                                                                                    k0, nb, X);
+    }
+    prof_end(s, FH_PROF_SOLVE, 4.0 * (double)m * (double)m * (double)p * count);
+    FHB_CUDA(cudaGetLastError());
+    return FH_OK;
+}
+
+}  // namespace fhb
+
+using namespace fhb;
+
+extern "C" fh_status fh_test_mesh_solve(const double *r, const double *l, int64_t m, int64_t p, const double *omega,
+                                        int32_t count, double *z, double *x, int32_t *failed, fh_error_info *err) {
+    clear_error(err);
+    if (!r || !l || !omega || !z || !x || !failed || m < 1 || p < 1 || count < 1)
+        return fail(err, FH_ERR_INVALID_ARGUMENT, "null argument or empty system");
+    fh_status st = ensure_device(err);
+    if (st) return st;
+    const size_t M = (size_t)(m + p), sym = 8 * M * M, zs = 16 * (size_t)(count * p * p),
+                 xs = 16 * (size_t)(count * p * m);
+    void *d[8] = {};
+    struct Release {
+        void **d;
+        ~Release() {
+            for (int k = 0; k < 8; ++k) cudaFree(d[k]);
+        }
+    } release{d};
+    const size_t bytes[8] = {sym, sym, 8 * (size_t)count, 2 * sym * (size_t)count, ldlt_bytes(m, p, count), zs, xs,
+                             4 * (size_t)count};
+    for (int k = 0; k < 8; ++k) FHB_CUDA(cudaMalloc(&d[k], bytes[k]));
+    FHB_CUDA(cudaMemcpy(d[0], r, sym, cudaMemcpyHostToDevice));
+    FHB_CUDA(cudaMemcpy(d[1], l, sym, cudaMemcpyHostToDevice));
+    FHB_CUDA(cudaMemcpy(d[2], omega, bytes[2], cudaMemcpyHostToDevice));
+    st = ldlt_factor((double *)d[0], (double *)d[1], m, p, (double *)d[2], count, (double *)d[3], d[4], (double *)d[5],
+                     (double *)d[6], (int *)d[7], nullptr, err);
+    if (st) return st;
+    FHB_CUDA(cudaMemcpy(z, d[5], zs, cudaMemcpyDeviceToHost));
+    FHB_CUDA(cudaMemcpy(x, d[6], xs, cudaMemcpyDeviceToHost));
+    FHB_CUDA(cudaMemcpy(failed, d[7], bytes[7], cudaMemcpyDeviceToHost));
+    return FH_OK;
+}

@@ -109,6 +109,17 @@ template <class T>
 fh_status panel_coop(LuBatch<T> &b, int64_t K0, int nb, const CoopScratch &cs, cudaStream_t s, fh_error_info *err);
 fh_status coop_check(const CoopScratch &cs, cudaStream_t s, fh_error_info *err);
 
+// The FP64 factorization without interchanges of `count` mesh systems
+// R + j w L (order M = m + p, port rows last, symmetric; fh_ldlt.cu): Z per
+// matrix (count x p x p) and, with x, Z_ee^-1 Z_ep (count x p columns of m).
+// a: count * M * M complex; work: ldlt_bytes.  d_failed[f] is set for a
+// matrix that elimination without pivoting does not suit; its z and x are not
+// to be used.
+constexpr int kLdltPanel = 64;
+size_t ldlt_bytes(int64_t m, int64_t p, int count);
+fh_status ldlt_factor(const double *Rm, const double *Lm, int64_t m, int64_t p, const double *d_omega, int count,
+                      double *a, void *work, double *z, double *x, int *d_failed, cudaStream_t s, fh_error_info *err);
+
 // How the trailing update A22 -= L21 U12 is computed for the FP32 form.
 enum class TrailingUpdate { Simt, TensorBf16x3 };
 

@@ -500,6 +500,13 @@ fh_status fh_system_fill_stats(const fh_system *sys, fh_fill_stats *stats);
 fh_status fh_test_trailing_update(float *a, int64_t m, int32_t count, int64_t k0, int32_t nb, int32_t mode,
                                   fh_error_info *err);
 
+/* The FP64 factorization without interchanges on its own (tests): mesh
+ * matrices r and l of order m + p (column-major, symmetric, the p port rows
+ * last), `count` angular frequencies.  z: count x p x p, x: count x p columns
+ * of m (both complex), failed[f]: 1 where the elimination was rejected. */
+fh_status fh_test_mesh_solve(const double *r, const double *l, int64_t m, int64_t p, const double *omega,
+                             int32_t count, double *z, double *x, int32_t *failed, fh_error_info *err);
+
 /* ---- device-event profiler (no reference counterpart) ------------------ */
 
 /* Kernel classes timed when profiling is on. */
