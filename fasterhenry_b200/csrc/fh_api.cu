@@ -98,7 +98,11 @@ struct fh_system {
     int32_t *d_col_loop = nullptr;
     double *d_col_sign = nullptr, *d_whr = nullptr;
     // The loop basis, its transpose over the internal loops and the branch
-    // resistances on the device: R_ee x of the refinement residuals.
+    // resistances on the device (parts of d_basis): R_ee x of the refinement
+    // residuals.
+    unsigned char *d_basis = nullptr;
+    // Frequencies per batch that the workspace has held before, by precision.
+    size_t held[3] = {0, 0, 0};
     int64_t *d_rp = nullptr, *d_toff = nullptr;
     int32_t *d_br = nullptr, *d_tloop = nullptr;
     double *d_sign = nullptr, *d_tsign = nullptr, *d_R = nullptr;
@@ -107,12 +111,11 @@ struct fh_system {
     FillStats fill{};
     float ms_congruence = 0;
     ~fh_system() {
+        if (side) cudaStreamSynchronize(side);  // an error may have left work on it
         pool.release();
         cache_free(d_Lm, stream);
         cache_free(d_Rm, stream);
-        for (void *q : {(void *)d_rp, (void *)d_toff, (void *)d_br, (void *)d_tloop, (void *)d_sign, (void *)d_tsign,
-                        (void *)d_R})
-            cache_free(q, stream);
+        cache_free(d_basis, stream);
         cache_free(d_col_ptr, stream);
         cache_free(d_first, stream);
         cache_free(d_col_loop, stream);
@@ -120,11 +123,8 @@ struct fh_system {
         cache_free(d_whr, stream);
         cache_free(d_group, stream);
         cache_free(d_coupled, stream);
-        if (side) {
-            cudaStreamSynchronize(side);
-            cudaStreamDestroy(side);
-        }
-        if (stream) cudaStreamDestroy(stream);
+        stream_release(side);
+        stream_release(stream);
     }
 };
 
@@ -154,13 +154,17 @@ fh_status ensure_device(fh_error_info *err) {
         return fail(err, FH_ERR_NO_DEVICE, "no CUDA device is available (this library has no CPU fallback)");
     int dev = 0;
     cudaGetDevice(&dev);
-    cudaDeviceProp prop;
-    if (cudaGetDeviceProperties(&prop, dev) != cudaSuccess)
+    // One attribute: the whole property struct takes milliseconds to fill.
+    int major = 0;
+    if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess)
         return fail(err, FH_ERR_NO_DEVICE, "cannot query the CUDA device");
-    if (prop.major != 10)
+    if (major != 10) {
+        cudaDeviceProp prop = {};
+        cudaGetDeviceProperties(&prop, dev);
         return fail(err, FH_ERR_NO_DEVICE,
                     std::string("this build targets sm_100a (B200); found ") + prop.name + " sm_" +
                         std::to_string(prop.major) + std::to_string(prop.minor));
+    }
     return FH_OK;
 }
 
@@ -785,8 +789,9 @@ int32_t fh_device_count(void) {
     }
     int usable = 0;
     for (int d = 0; d < count; ++d) {
-        cudaDeviceProp prop;
-        if (cudaGetDeviceProperties(&prop, d) == cudaSuccess && prop.major == 10) ++usable;
+        int major = 0;
+        if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, d) == cudaSuccess && major == 10)
+            ++usable;
     }
     return usable;
 }
@@ -800,15 +805,15 @@ fh_status fh_partial_inductance_matrix(const fh_filament *filaments, size_t n, d
     if (n == 0) return FH_OK;
     std::vector<DevFil> h(n);
     for (size_t i = 0; i < n; ++i) h[i] = make_devfil(filaments[i]);
-    DBuf<DevFil> d_fil;
-    DBuf<double> d_L;
-    DBuf<int8_t> d_m;
+    cudaStream_t s;
+    FHB_CUDA(stream_acquire(&s));
+    std::unique_ptr<CUstream_st, decltype(&stream_release)> guard(s, &stream_release);
+    DBuf<DevFil> d_fil(s);
+    DBuf<double> d_L(s);
+    DBuf<int8_t> d_m(s);
     FHB_ALLOC(d_fil, n);
     FHB_ALLOC(d_L, n * n);
     if (methods) FHB_ALLOC(d_m, n * n);
-    cudaStream_t s;
-    FHB_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    std::unique_ptr<CUstream_st, decltype(&cudaStreamDestroy)> guard(s, &cudaStreamDestroy);
     FHB_CUDA(cudaMemcpyAsync(d_fil.p, h.data(), n * sizeof(DevFil), cudaMemcpyHostToDevice, s));
     FHB_CUDA(cudaMemsetAsync(d_L.p, 0, n * n * sizeof(double), s));
     if (methods) FHB_CUDA(cudaMemsetAsync(d_m.p, 0, n * n, s));
@@ -863,9 +868,12 @@ fh_status fh_lu_solve_c64(const double *a, size_t n, const double *b, size_t nrh
     if (st) return st;
     if (n == 0) return FH_OK;
     if (n > (size_t)INT32_MAX / 2) return fail(err, FH_ERR_INVALID_ARGUMENT, "order too large");
-    DBuf<double> d_a, d_x, pv;
-    DBuf<int> piv, sing, pi;
-    DBuf<unsigned> tk;
+    cudaStream_t s;
+    FHB_CUDA(stream_acquire(&s));
+    std::unique_ptr<CUstream_st, decltype(&stream_release)> guard(s, &stream_release);
+    DBuf<double> d_a(s), d_x(s), pv(s);
+    DBuf<int> piv(s), sing(s), pi(s);
+    DBuf<unsigned> tk(s);
     FHB_ALLOC(d_a, 2 * n * n);
     FHB_ALLOC(d_x, 2 * n * nrhs);
     FHB_ALLOC(piv, n);
@@ -873,9 +881,6 @@ fh_status fh_lu_solve_c64(const double *a, size_t n, const double *b, size_t nrh
     FHB_ALLOC(pv, 16);
     FHB_ALLOC(pi, 16);
     FHB_ALLOC(tk, 1);
-    cudaStream_t s;
-    FHB_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    std::unique_ptr<CUstream_st, decltype(&cudaStreamDestroy)> guard(s, &cudaStreamDestroy);
     FHB_CUDA(cudaMemcpyAsync(d_a.p, a, 16 * n * n, cudaMemcpyHostToDevice, s));
     FHB_CUDA(cudaMemcpyAsync(d_x.p, b, 16 * n * nrhs, cudaMemcpyHostToDevice, s));
     FHB_CUDA(cudaMemsetAsync(sing.p, 0, sizeof(int), s));
@@ -951,10 +956,10 @@ fh_status fh_system_create_coupled(const fh_node *nodes, size_t n_nodes, const f
     st = ensure_device(err);
     if (st) return st;
     FHB_CUDA(cudaGetDevice(&s->device));
-    FHB_CUDA(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
+    FHB_CUDA(stream_acquire(&s->stream));
     // Default priority: the look-ahead gets its SMs by the update leaving
     // them free, not by scheduling ahead of queued update CTAs.
-    FHB_CUDA(cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking));
+    FHB_CUDA(stream_acquire(&s->side));
     cudaStream_t cs = s->stream;
     s->pool.stream = cs;
     s->nloops = s->loops.rows();
@@ -971,31 +976,39 @@ fh_status fh_system_create_coupled(const fh_node *nodes, size_t n_nodes, const f
     FHB_ALLOC(d_L, (size_t)n * n);
     TransposedLoops internal;
     transpose_loops(s->loops, n, s->m, internal);
-    {
-        auto keep = [&](void **d, size_t bytes) { return cache_alloc(d, std::max<size_t>(bytes, 16), cs); };
-        if (keep((void **)&s->d_R, 8 * (size_t)n) || keep((void **)&s->d_rp, 8 * s->loops.row_ptr.size()) ||
-            keep((void **)&s->d_br, 4 * s->loops.branch.size()) || keep((void **)&s->d_sign, 8 * s->loops.sign.size()) ||
-            keep((void **)&s->d_toff, 8 * internal.offset.size()) || keep((void **)&s->d_tloop, 4 * internal.loop.size()) ||
-            keep((void **)&s->d_tsign, 8 * internal.sign.size())) {
-            cudaGetLastError();
-            return fail(err, FH_ERR_OUT_OF_MEMORY, "device allocation of the loop basis failed");
-        }
+    // The loop basis, its transpose and R: one buffer, filled by one copy.
+    std::vector<unsigned char> staged;
+    auto stage = [&](const void *h, size_t bytes) {
+        const size_t at = (staged.size() + 255) / 256 * 256;
+        staged.resize(at + std::max<size_t>(bytes, 16), 0);
+        if (bytes) std::memcpy(staged.data() + at, h, bytes);
+        return at;
+    };
+    const size_t at_r = stage(s->resistances.data(), 8 * (size_t)n),
+                 at_rp = stage(s->loops.row_ptr.data(), 8 * s->loops.row_ptr.size()),
+                 at_br = stage(s->loops.branch.data(), 4 * s->loops.branch.size()),
+                 at_sign = stage(s->loops.sign.data(), 8 * s->loops.sign.size()),
+                 at_toff = stage(internal.offset.data(), 8 * internal.offset.size()),
+                 at_tloop = stage(internal.loop.data(), 4 * internal.loop.size()),
+                 at_tsign = stage(internal.sign.data(), 8 * internal.sign.size());
+    if (cache_alloc((void **)&s->d_basis, staged.size(), cs) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(err, FH_ERR_OUT_OF_MEMORY, "device allocation of the loop basis failed");
     }
+    s->d_R = reinterpret_cast<double *>(s->d_basis + at_r);
+    s->d_rp = reinterpret_cast<int64_t *>(s->d_basis + at_rp);
+    s->d_br = reinterpret_cast<int32_t *>(s->d_basis + at_br);
+    s->d_sign = reinterpret_cast<double *>(s->d_basis + at_sign);
+    s->d_toff = reinterpret_cast<int64_t *>(s->d_basis + at_toff);
+    s->d_tloop = reinterpret_cast<int32_t *>(s->d_basis + at_tloop);
+    s->d_tsign = reinterpret_cast<double *>(s->d_basis + at_tsign);
     if (cache_alloc((void **)&s->d_Lm, std::max<size_t>(1, (size_t)loops * loops) * 8, cs) != cudaSuccess ||
         cache_alloc((void **)&s->d_Rm, std::max<size_t>(1, (size_t)loops * loops) * 8, cs) != cudaSuccess) {
         cudaGetLastError();
         return fail(err, FH_ERR_OUT_OF_MEMORY, "device allocation of the mesh matrices failed");
     }
     FHB_CUDA(cudaMemcpyAsync(d_fil.p, h.data(), n * sizeof(DevFil), cudaMemcpyHostToDevice, cs));
-    FHB_CUDA(cudaMemcpyAsync(s->d_R, s->resistances.data(), n * 8, cudaMemcpyHostToDevice, cs));
-    FHB_CUDA(cudaMemcpyAsync(s->d_rp, s->loops.row_ptr.data(), s->loops.row_ptr.size() * 8, cudaMemcpyHostToDevice, cs));
-    FHB_CUDA(cudaMemcpyAsync(s->d_br, s->loops.branch.data(), s->loops.branch.size() * 4, cudaMemcpyHostToDevice, cs));
-    FHB_CUDA(cudaMemcpyAsync(s->d_sign, s->loops.sign.data(), s->loops.sign.size() * 8, cudaMemcpyHostToDevice, cs));
-    FHB_CUDA(cudaMemcpyAsync(s->d_toff, internal.offset.data(), internal.offset.size() * 8, cudaMemcpyHostToDevice, cs));
-    if (!internal.loop.empty()) {
-        FHB_CUDA(cudaMemcpyAsync(s->d_tloop, internal.loop.data(), internal.loop.size() * 4, cudaMemcpyHostToDevice, cs));
-        FHB_CUDA(cudaMemcpyAsync(s->d_tsign, internal.sign.data(), internal.sign.size() * 8, cudaMemcpyHostToDevice, cs));
-    }
+    FHB_CUDA(cudaMemcpyAsync(s->d_basis, staged.data(), staged.size(), cudaMemcpyHostToDevice, cs));
     FHB_CUDA(cudaMemsetAsync(d_L.p, 0, (size_t)n * n * 8, cs));
     s->total_pairs = n * (n + 1) / 2;
     s->kept_pairs = coupling_kept_pairs(s->coupling, s->disc.per_segment.data(), n_segments);
@@ -1127,12 +1140,6 @@ fh_status fh_sweep(fh_system *sys, const double *freqs, size_t nf, fh_precision 
     const double t0 = wall();
     const int64_t m = sys->m, p = sys->p;
     cudaStream_t st = sys->stream;
-    // Frequencies per batch from free device memory (the analogue of the
-    // reference's 2 GiB sweep budget, solve.rs:91 and 884).
-    size_t free_b = 0, total_b = 0;
-    FHB_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    // Own workspace is reused; memory the cache holds idle is available too.
-    free_b = (free_b + cache_idle_bytes()) / (size_t)std::max(1, sys->share) + sys->pool.held();
     if (precision < FH_PRECISION_FP64 || precision > FH_PRECISION_MIXED_FP32)
         return fail(err, FH_ERR_INVALID_ARGUMENT, "unknown precision");
     const bool mixed = precision != FH_PRECISION_FP64;
@@ -1148,7 +1155,18 @@ fh_status fh_sweep(fh_system *sys, const double *freqs, size_t nf, fh_precision 
                        (outer_for(m, update) ? 16.0 * (double)m * kOuterFp32 + 16.0 * (double)(m + kNbFp32) * kNbFp32 +
                                                    16.0 * kOuterFp32 * kOuterFp32 + 8.0 * kNbFp32 * kOuterFp32
                                              : 0.0);
-    int chunk = (int)std::max(1.0, std::min<double>((double)nf, 0.8 * (double)free_b / std::max(per, 1.0)));
+    // Frequencies per batch from free device memory (the analogue of the
+    // reference's 2 GiB sweep budget, solve.rs:91 and 884).  A batch that the
+    // workspace has held before needs no look at the free memory, a query that
+    // takes from 0.1 ms to several: its buffers are still there.
+    int chunk = (int)nf;
+    if (nf > sys->held[precision]) {
+        size_t free_b = 0, total_b = 0;
+        FHB_CUDA(cudaMemGetInfo(&free_b, &total_b));
+        // Own workspace is reused; memory the cache holds idle is available too.
+        free_b = (free_b + cache_idle_bytes()) / (size_t)std::max(1, sys->share) + sys->pool.held();
+        chunk = (int)std::max(1.0, std::min<double>((double)nf, 0.8 * (double)free_b / std::max(per, 1.0)));
+    }
     PBuf<double> d_omega, d_x, d_z;
     FHB_PALLOC(sys->pool, d_omega, kSlotOmega, (size_t)chunk);
     FHB_PALLOC(sys->pool, d_x, kSlotX, (size_t)chunk * m * p * 2);
@@ -1173,6 +1191,7 @@ fh_status fh_sweep(fh_system *sys, const double *freqs, size_t nf, fh_precision 
             e = sweep_chunk_fp64(sys, d_omega.p, count, nullptr, d_z.p, singular.data() + c0, &ms_factor, err);
         }
         if (e) return e;
+        sys->held[precision] = std::max(sys->held[precision], (size_t)count);
         FHB_CUDA(cudaMemcpyAsync(z_out + 2 * c0 * p * p, d_z.p, 16 * (size_t)count * p * p, cudaMemcpyDeviceToHost, st));
         FHB_CUDA(cudaStreamSynchronize(st));
         // Refinement that did not converge: redo those frequencies in FP64.
@@ -1816,8 +1835,8 @@ fh_status fh_test_inductance_gradient(const fh_filament *filaments, const double
     FHB_ALLOC(d_tan, n);
     FHB_ALLOC(d_D, 2 * n * n);
     cudaStream_t s;
-    FHB_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    std::unique_ptr<CUstream_st, decltype(&cudaStreamDestroy)> guard(s, &cudaStreamDestroy);
+    FHB_CUDA(stream_acquire(&s));
+    std::unique_ptr<CUstream_st, decltype(&stream_release)> guard(s, &stream_release);
     FHB_CUDA(cudaMemcpyAsync(d_fil.p, h.data(), n * sizeof(DevFil), cudaMemcpyHostToDevice, s));
     FHB_CUDA(cudaMemcpyAsync(d_tan.p, t.data(), n * sizeof(FilTan), cudaMemcpyHostToDevice, s));
     FHB_CUDA(cudaMemsetAsync(d_D.p, 0, 16 * n * n, s));
@@ -1849,8 +1868,8 @@ fh_status fh_test_coordinate_gradient(const fh_filament *filaments, const int32_
     FHB_ALLOC(d_move, n);
     FHB_ALLOC(d_D, 4 * n * n);
     cudaStream_t s;
-    FHB_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    std::unique_ptr<CUstream_st, decltype(&cudaStreamDestroy)> guard(s, &cudaStreamDestroy);
+    FHB_CUDA(stream_acquire(&s));
+    std::unique_ptr<CUstream_st, decltype(&stream_release)> guard(s, &stream_release);
     FHB_CUDA(cudaMemcpyAsync(d_fil.p, h.data(), n * sizeof(DevFil), cudaMemcpyHostToDevice, s));
     FHB_CUDA(cudaMemcpyAsync(d_seg.p, segment, n * sizeof(int32_t), cudaMemcpyHostToDevice, s));
     FHB_CUDA(cudaMemcpyAsync(d_move.p, move.data(), n, cudaMemcpyHostToDevice, s));

@@ -52,6 +52,24 @@ fh_status ensure_device(fh_error_info *err);
 // allocations from a per-device pool that keeps freed memory for reuse.
 cudaError_t cache_alloc(void **p, size_t bytes, cudaStream_t s);
 void cache_free(void *p, cudaStream_t s);
+// A non-blocking stream of the current device, from the device's idle ones or
+// new; stream_release keeps a few idle and destroys the rest.
+cudaError_t stream_acquire(cudaStream_t *s);
+void stream_release(cudaStream_t s);
+// A buffer of the memory cache that is freed in its stream's order.
+struct CacheBuf {
+    void *p = nullptr;
+    cudaStream_t s;
+    explicit CacheBuf(cudaStream_t stream) : s(stream) {}
+    CacheBuf(const CacheBuf &) = delete;
+    CacheBuf &operator=(const CacheBuf &) = delete;
+    ~CacheBuf() { cache_free(p, s); }
+    cudaError_t get(size_t bytes) { return cache_alloc(&p, bytes, s); }
+    template <class T>
+    T *as() const {
+        return static_cast<T *>(p);
+    }
+};
 // Memory held by the cache and not in use (counted as available when sizing
 // sweep batches).
 size_t cache_idle_bytes();

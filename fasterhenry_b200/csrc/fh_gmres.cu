@@ -7,6 +7,7 @@
 #include <string>
 #include <vector>
 
+#include "fh_device.cuh"
 #include "fh_gmres.cuh"
 
 namespace fhb {
@@ -251,22 +252,22 @@ struct Norm {
 
 }  // namespace
 
-GmresWork::~GmresWork() {
-    void *p[] = {V, w, r, t, u, h, red, part};
-    for (void *q : p)
-        if (q) cudaFree(q);
-}
+GmresWork::~GmresWork() { release(); }
 
-fh_status GmresWork::ensure(int64_t n_, int restart_, fh_error_info *err) {
-    if (n_ <= n && restart_ <= restart && V) return FH_OK;
+void GmresWork::release() {
     void *p[] = {V, w, r, t, u, h, red, part};
-    for (void *q : p)
-        if (q) cudaFree(q);
+    for (void *q : p) cache_free(q, stream);
     V = w = r = t = u = h = nullptr;
     red = part = nullptr;
+}
+
+fh_status GmresWork::ensure(int64_t n_, int restart_, cudaStream_t s, fh_error_info *err) {
+    if (n_ <= n && restart_ <= restart && V) return FH_OK;
+    release();
+    stream = s;
     n = n_;
     restart = restart_;
-    auto alloc = [&](void **q, size_t bytes) { return cudaMalloc(q, std::max<size_t>(bytes, 16)); };
+    auto alloc = [&](void **q, size_t bytes) { return cache_alloc(q, std::max<size_t>(bytes, 16), s); };
     if (alloc((void **)&V, sizeof(double2) * (size_t)(restart + 1) * n) != cudaSuccess ||
         alloc((void **)&w, sizeof(double2) * n) != cudaSuccess || alloc((void **)&r, sizeof(double2) * n) != cudaSuccess ||
         alloc((void **)&t, sizeof(double2) * n) != cudaSuccess || alloc((void **)&u, sizeof(double2) * n) != cudaSuccess ||
@@ -284,7 +285,7 @@ fh_status gmres_solve(int64_t n, const DeviceOp &apply, const DeviceOp &precondi
                       fh_error_info *err) {
     GmresOutcome oc;
     const int restart = (int)std::max<int64_t>(1, std::min<int64_t>(params.restart, n));
-    fh_status st = work.ensure(n, restart, err);
+    fh_status st = work.ensure(n, restart, s, err);
     if (st) return st;
     auto norm_of = [&](const double2 *v, Norm &nm) -> fh_status {
         maxabs_partial_kernel<<<kRB, kRT, 0, s>>>(v, n, work.red + kMaxPartial);

@@ -39,9 +39,11 @@ struct GmresWork {
     double2 *w = nullptr, *r = nullptr, *t = nullptr, *u = nullptr;
     double2 *h = nullptr;    // 2 x (restart + 1) projections of one Arnoldi step
     double *red = nullptr;   // reduction partials and results
-    double *part = nullptr;  // per-block partial projections, 2 x kRB x (restart + 1)
+    double *part = nullptr;  // partial projections per chunk of rows
     ~GmresWork();
-    fh_status ensure(int64_t n_, int restart_, fh_error_info *err);
+    cudaStream_t stream = nullptr;  // allocations and frees are ordered on it
+    fh_status ensure(int64_t n_, int restart_, cudaStream_t s, fh_error_info *err);
+    void release();
 };
 
 // Solves A x = b; x holds the initial guess on entry.  b, x: device.

@@ -145,7 +145,7 @@ inline unsigned grid_n(int64_t n) { return (unsigned)std::max<int64_t>(1, std::m
 
 template <class T>
 cudaError_t put(T **d, const std::vector<T> &h, cudaStream_t s) {
-    cudaError_t e = cudaMalloc((void **)d, std::max<size_t>(1, h.size()) * sizeof(T));
+    cudaError_t e = cache_alloc((void **)d, std::max<size_t>(1, h.size()) * sizeof(T), s);
     if (e != cudaSuccess || h.empty()) return e;
     return cudaMemcpyAsync(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, s);
 }
@@ -190,8 +190,7 @@ struct fh_iterative {
                         d_diag,    d_b,     d_x,      d_parts,  d_flux,  d_res,    d_cor,  d_ax,   d_col_ptr,
                         d_first,   d_segi,  d_col_loop, d_col_sign, d_whr, d_ip,   d_ib,   d_dens, d_pow,
                         d_segc,    d_segp,  d_segpk, d_long,  d_t_long};
-        for (void *q : ptrs)
-            if (q) cudaFree(q);
+        for (void *q : ptrs) cache_free(q, stream);
     }
 };
 
@@ -256,9 +255,9 @@ fh_status refined_solve(fh_iterative *s, double omega, const DeviceOp &apply, co
     const int64_t m = s->m;
     cudaStream_t cs = s->stream;
     if (!s->d_res) {
-        FHB_CUDA(cudaMalloc(&s->d_res, sizeof(double2) * m));
-        FHB_CUDA(cudaMalloc(&s->d_cor, sizeof(double2) * m));
-        FHB_CUDA(cudaMalloc(&s->d_ax, sizeof(double2) * m));
+        FHB_CUDA(cache_alloc((void **)&s->d_res, sizeof(double2) * m, cs));
+        FHB_CUDA(cache_alloc((void **)&s->d_cor, sizeof(double2) * m, cs));
+        FHB_CUDA(cache_alloc((void **)&s->d_ax, sizeof(double2) * m, cs));
     }
     std::vector<double2> hb((size_t)m), hr((size_t)m);
     FHB_CUDA(cudaMemcpyAsync(hb.data(), s->d_b, sizeof(double2) * m, cudaMemcpyDeviceToHost, cs));
@@ -364,7 +363,7 @@ fh_status prepare_currents(fh_iterative *s, fh_error_info *err) {
     FHB_CUDA(put(&s->d_col_sign, cols.sign, cs));
     FHB_CUDA(put(&s->d_whr, whr, cs));
     FHB_CUDA(put(&s->d_first, s->layout.segment_first, cs));
-    auto alloc = [&](void **q, size_t bytes) { return cudaMalloc(q, std::max<size_t>(bytes, 16)); };
+    auto alloc = [&](void **q, size_t bytes) { return cache_alloc(q, std::max<size_t>(bytes, 16), cs); };
     if (alloc((void **)&s->d_ip, 16 * (size_t)p) || alloc((void **)&s->d_ib, 16 * (size_t)n) ||
         alloc((void **)&s->d_dens, 8 * (size_t)n) || alloc((void **)&s->d_pow, 8 * (size_t)n) ||
         alloc((void **)&s->d_segc, 16 * (size_t)nseg) || alloc((void **)&s->d_segp, 8 * (size_t)nseg) ||
@@ -423,7 +422,7 @@ fh_status fh_iterative_create(const fh_node *nodes, size_t n_nodes, const fh_seg
     if (st) return st;
     st = ensure_device(err);
     if (st) return st;
-    FHB_CUDA(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
+    FHB_CUDA(stream_acquire(&s->stream));
     cudaStream_t cs = s->stream;
     const int64_t n = (int64_t)s->disc.filaments.size();
     s->n = n;
@@ -447,11 +446,10 @@ fh_status fh_iterative_create(const fh_node *nodes, size_t n_nodes, const fh_seg
     s->r_pp.assign((size_t)p * p, 0.0);
     s->l_pp.assign((size_t)p * p, 0.0);
     if (p > 0 && n > 0) {
-        double *d_cur = nullptr, *d_fl = nullptr;
-        FHB_CUDA(cudaMalloc(&d_cur, sizeof(double) * n));
-        std::unique_ptr<void, decltype(&cudaFree)> g1(d_cur, &cudaFree);
-        FHB_CUDA(cudaMalloc(&d_fl, sizeof(double) * n));
-        std::unique_ptr<void, decltype(&cudaFree)> g2(d_fl, &cudaFree);
+        CacheBuf cur(cs), fl(cs);
+        FHB_CUDA(cur.get(sizeof(double) * n));
+        FHB_CUDA(fl.get(sizeof(double) * n));
+        double *d_cur = cur.as<double>(), *d_fl = fl.as<double>();
         std::vector<double> current((size_t)n), flux((size_t)n), drop((size_t)n);
         for (int64_t q = 0; q < p; ++q) {
             std::fill(current.begin(), current.end(), 0.0);
@@ -499,15 +497,13 @@ fh_status fh_iterative_create(const fh_node *nodes, size_t n_nodes, const fh_seg
     if (!pairs.empty()) {
         std::vector<DevFil> hf((size_t)n);
         for (int64_t i = 0; i < n; ++i) hf[i] = make_devfil(s->disc.filaments[i]);
-        DevFil *d_fil = nullptr;
-        int2 *d_pairs = nullptr;
-        double *d_vals = nullptr;
-        FHB_CUDA(put(&d_fil, hf, cs));
-        std::unique_ptr<void, decltype(&cudaFree)> g1(d_fil, &cudaFree);
-        FHB_CUDA(put(&d_pairs, pairs, cs));
-        std::unique_ptr<void, decltype(&cudaFree)> g2(d_pairs, &cudaFree);
-        FHB_CUDA(cudaMalloc(&d_vals, sizeof(double) * pairs.size()));
-        std::unique_ptr<void, decltype(&cudaFree)> g3(d_vals, &cudaFree);
+        CacheBuf fil(cs), list(cs), vals(cs);
+        FHB_CUDA(put((DevFil **)&fil.p, hf, cs));
+        FHB_CUDA(put((int2 **)&list.p, pairs, cs));
+        FHB_CUDA(vals.get(sizeof(double) * pairs.size()));
+        DevFil *d_fil = fil.as<DevFil>();
+        int2 *d_pairs = list.as<int2>();
+        double *d_vals = vals.as<double>();
         st = device_fill_pairs(d_fil, n, d_pairs, (int64_t)pairs.size(), d_vals, cs, nullptr, err);
         if (st) return st;
         FHB_CUDA(cudaMemcpyAsync(values.data(), d_vals, sizeof(double) * pairs.size(), cudaMemcpyDeviceToHost, cs));
@@ -541,7 +537,7 @@ fh_status fh_iterative_create(const fh_node *nodes, size_t n_nodes, const fh_seg
     s->n_t_long = (int)t_lng.size();
     FHB_CUDA(put(&s->d_long, lng, cs));
     FHB_CUDA(put(&s->d_t_long, t_lng, cs));
-    auto alloc = [&](void **q, size_t bytes) { return cudaMalloc(q, std::max<size_t>(bytes, 16)); };
+    auto alloc = [&](void **q, size_t bytes) { return cache_alloc(q, std::max<size_t>(bytes, 16), cs); };
     if (alloc((void **)&s->d_c, sizeof(double2) * n) || alloc((void **)&s->d_drop, sizeof(double2) * n) ||
         alloc((void **)&s->d_diag, sizeof(double2) * m) || alloc((void **)&s->d_b, sizeof(double2) * m) ||
         alloc((void **)&s->d_x, sizeof(double2) * m * std::max<int64_t>(p, 1)) ||
@@ -803,7 +799,7 @@ void fh_iterative_destroy(fh_iterative *s) {
     if (!s) return;
     cudaStream_t cs = s->stream;
     delete s;
-    if (cs) cudaStreamDestroy(cs);
+    stream_release(cs);
 }
 
 fh_status fh_test_gmres_dense(const double *a, size_t n, const double *b, double *x, const double *precond,

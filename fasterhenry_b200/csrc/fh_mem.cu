@@ -17,6 +17,11 @@ namespace {
 constexpr int kMaxDevices = 64;
 std::mutex g_mu;
 cudaMemPool_t g_pool[kMaxDevices] = {};
+// Idle streams per device: creating and destroying the two of a system takes
+// 0.35 ms, a tenth of a whole call at 240 filaments.
+constexpr int kIdleStreams = 8;
+cudaStream_t g_idle[kMaxDevices][kIdleStreams] = {};
+int g_idle_count[kMaxDevices] = {};
 }  // namespace
 
 cudaError_t cache_pool(cudaMemPool_t *out) {
@@ -67,6 +72,34 @@ void cache_free(void *p, cudaStream_t s) {
     if (p) cudaFreeAsync(p, s);
 }
 
+cudaError_t stream_acquire(cudaStream_t *s) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    {
+        std::lock_guard<std::mutex> lk(g_mu);
+        if (dev >= 0 && dev < kMaxDevices && g_idle_count[dev] > 0) {
+            *s = g_idle[dev][--g_idle_count[dev]];
+            return cudaSuccess;
+        }
+    }
+    return cudaStreamCreateWithFlags(s, cudaStreamNonBlocking);
+}
+
+// Work still pending on it (frees) stays ahead of what its next owner enqueues.
+void stream_release(cudaStream_t s) {
+    if (!s) return;
+    int dev = -1;
+    if (cudaStreamGetDevice(s, &dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices) {
+        std::lock_guard<std::mutex> lk(g_mu);
+        if (g_idle_count[dev] < kIdleStreams) {
+            g_idle[dev][g_idle_count[dev]++] = s;
+            return;
+        }
+    }
+    cudaStreamDestroy(s);
+}
+
 size_t cache_idle_bytes() {
     cudaMemPool_t pool;
     if (cache_pool(&pool) != cudaSuccess) {
@@ -95,6 +128,7 @@ extern "C" fh_status fh_release_cached_memory(void) {
         cudaSetDevice(d);
         cudaDeviceSynchronize();
         cudaMemPoolTrimTo(fhb::g_pool[d], 0);
+        while (fhb::g_idle_count[d] > 0) cudaStreamDestroy(fhb::g_idle[d][--fhb::g_idle_count[d]]);
     }
     cudaSetDevice(cur);
     return FH_OK;

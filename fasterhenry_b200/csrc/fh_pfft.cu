@@ -51,7 +51,7 @@ double now_s() {
 
 template <class T>
 cudaError_t upload(T **d, const std::vector<T> &h, cudaStream_t s) {
-    cudaError_t e = cudaMalloc((void **)d, std::max<size_t>(1, h.size()) * sizeof(T));
+    cudaError_t e = cache_alloc((void **)d, std::max<size_t>(1, h.size()) * sizeof(T), s);
     if (e != cudaSuccess) return e;
     if (h.empty()) return cudaSuccess;
     return cudaMemcpyAsync(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, s);
@@ -242,12 +242,8 @@ PfftDevice::~PfftDevice() {
     if (d_work) cache_free(d_work, s);
     void *ptrs[] = {d_dir, d_proj_off, d_proj_idx, d_proj_w, d_spread_off, d_spread_fil,
                     d_spread_w, d_near_off, d_near_col, d_near_val};
-    for (void *p : ptrs)
-        if (p) cudaFree(p);
-    if (own_stream && stream) {
-        cudaStreamSynchronize(s);
-        cudaStreamDestroy(s);
-    }
+    for (void *p : ptrs) cache_free(p, s);
+    if (own_stream) stream_release(s);
 }
 
 size_t PfftDevice::memory_bytes() const {
@@ -267,7 +263,7 @@ fh_status pfft_build(const fh_filament *fil, int64_t n, const PfftConfig &cfg, v
         op.stream = stream;
     } else {
         cudaStream_t s;
-        FHB_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+        FHB_CUDA(stream_acquire(&s));
         op.stream = s;
         op.own_stream = true;
     }
@@ -294,8 +290,8 @@ fh_status pfft_build(const fh_filament *fil, int64_t n, const PfftConfig &cfg, v
         double **exact;
         NearPairs *near;
         ~Release() {
-            if (*fil) cudaFree(*fil);
-            if (*exact) cudaFree(*exact);
+            cache_free(*fil, s);
+            cache_free(*exact, s);
             near_pairs_free(*near, s);
         }
     } release{s, &d_fil, &d_exact, &near};
@@ -312,16 +308,12 @@ fh_status pfft_build(const fh_filament *fil, int64_t n, const PfftConfig &cfg, v
     op.d_spread_off = ds.spread_off;
     op.d_spread_fil = ds.spread_fil;
     op.d_spread_w = ds.spread_w;
-    struct FreeGrid {
-        double *p;
-        ~FreeGrid() {
-            if (p) cudaFree(p);
-        }
-    } free_grid{ds.pair_grid};
+    CacheBuf free_grid(s);
+    free_grid.p = ds.pair_grid;
     if (e) return e;
     op.projection_entries = ds.entries;
     const int64_t np = near.count;
-    FHB_CUDA(cudaMalloc(&d_exact, sizeof(double) * std::max<int64_t>(np, 1)));
+    FHB_CUDA(cache_alloc((void **)&d_exact, sizeof(double) * std::max<int64_t>(np, 1), s));
     if (np) {
         e = device_fill_pairs(d_fil, n, near.pairs, np, d_exact, s, nullptr, err);
         if (e) return e;

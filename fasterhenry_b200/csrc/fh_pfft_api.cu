@@ -15,8 +15,8 @@ struct fh_pfft {
     double *d_x = nullptr, *d_y = nullptr;
     size_t cap = 0;  // vectors the x / y buffers hold
     ~fh_pfft() {
-        if (d_x) cudaFree(d_x);
-        if (d_y) cudaFree(d_y);
+        cache_free(d_x, (cudaStream_t)dev.stream);
+        cache_free(d_y, (cudaStream_t)dev.stream);
     }
 };
 
@@ -79,12 +79,12 @@ fh_status fh_pfft_apply(fh_pfft *op, const double *x, double *y, size_t count, f
     if (count > 64) return fail(err, FH_ERR_INVALID_ARGUMENT, "at most 64 vectors per product");
     cudaStream_t s = (cudaStream_t)op->dev.stream;
     if (op->cap < count) {
-        if (op->d_x) cudaFree(op->d_x);
-        if (op->d_y) cudaFree(op->d_y);
+        cache_free(op->d_x, s);
+        cache_free(op->d_y, s);
         op->d_x = op->d_y = nullptr;
         op->cap = 0;
-        if (cudaMalloc(&op->d_x, sizeof(double) * n * count) != cudaSuccess ||
-            cudaMalloc(&op->d_y, sizeof(double) * n * count) != cudaSuccess) {
+        if (cache_alloc((void **)&op->d_x, sizeof(double) * n * count, s) != cudaSuccess ||
+            cache_alloc((void **)&op->d_y, sizeof(double) * n * count, s) != cudaSuccess) {
             cudaGetLastError();
             return fail(err, FH_ERR_OUT_OF_MEMORY, "device allocation of the product vectors failed");
         }

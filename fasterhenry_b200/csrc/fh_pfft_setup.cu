@@ -469,8 +469,8 @@ struct Scratch {
 };
 
 template <class T>
-cudaError_t persist(T **out, size_t count) {
-    return cudaMalloc((void **)out, std::max<size_t>(count, 1) * sizeof(T));
+cudaError_t persist(T **out, size_t count, cudaStream_t s) {
+    return cache_alloc((void **)out, std::max<size_t>(count, 1) * sizeof(T), s);
 }
 
 fh_status upload_constants(fh_error_info *err) {
@@ -551,7 +551,7 @@ fh_status pfft_device_setup(const PfftSetup &st, const fh_filament *fil, const N
                                                                d_counts, d_flag);
     FHB_CUDA(cudaGetLastError());
     // Row offsets of the projection: exclusive sum of the counts.
-    FHB_CUDA(persist(&out.proj_off, (size_t)n + 1));
+    FHB_CUDA(persist(&out.proj_off, (size_t)n + 1, s));
     size_t tb = 0;
     FHB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, d_counts, out.proj_off, (int)(n + 1), s));
     void *d_tb;
@@ -564,8 +564,8 @@ fh_status pfft_device_setup(const PfftSetup &st, const fh_filament *fil, const N
     if (flag) return fail(err, FH_ERR_PFFT, "pFFT projection left a filament's stencil box (internal error)");
     const int64_t E = out.entries;
     int32_t *d_owner, *d_lohi;
-    FHB_CUDA(persist(&out.proj_idx, (size_t)E));
-    FHB_CUDA(persist(&out.proj_w, (size_t)E));
+    FHB_CUDA(persist(&out.proj_idx, (size_t)E, s));
+    FHB_CUDA(persist(&out.proj_w, (size_t)E, s));
     FHB_CUDA(tmp.get(&d_owner, (size_t)E));
     FHB_CUDA(tmp.get(&d_lohi, (size_t)(6 * n)));
     project_emit_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(n, g, d_boxes, d_scratch, d_touched,
@@ -588,8 +588,8 @@ fh_status pfft_device_setup(const PfftSetup &st, const fh_filament *fil, const N
     FHB_CUDA(tmp.get((uint8_t **)&d_sb, sb));
     FHB_CUDA(cub::DeviceRadixSort::SortPairs(d_sb, sb, out.proj_idx, d_keys_out, d_pos, d_pos_out, (int)E, 0, end_bit,
                                              s));
-    FHB_CUDA(persist(&out.spread_fil, (size_t)E));
-    FHB_CUDA(persist(&out.spread_w, (size_t)E));
+    FHB_CUDA(persist(&out.spread_fil, (size_t)E, s));
+    FHB_CUDA(persist(&out.spread_w, (size_t)E, s));
     gather_spread_kernel<<<blocks(E, 256), 256, 0, s>>>(d_pos_out, d_owner, out.proj_w, E, out.spread_fil,
                                                         out.spread_w);
     FHB_CUDA(cudaGetLastError());
@@ -598,7 +598,7 @@ fh_status pfft_device_setup(const PfftSetup &st, const fh_filament *fil, const N
     FHB_CUDA(cudaMemsetAsync(d_gcount, 0, 8 * ((size_t)G + 1), s));
     count_keys_kernel<<<blocks(E, 256), 256, 0, s>>>(out.proj_idx, E, d_gcount);
     FHB_CUDA(cudaGetLastError());
-    FHB_CUDA(persist(&out.spread_off, (size_t)G + 1));
+    FHB_CUDA(persist(&out.spread_off, (size_t)G + 1, s));
     size_t tg = 0;
     FHB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tg, reinterpret_cast<int64_t *>(d_gcount), out.spread_off,
                                            (int)(G + 1), s));
@@ -608,7 +608,7 @@ fh_status pfft_device_setup(const PfftSetup &st, const fh_filament *fil, const N
                                            (int)(G + 1), s));
     // Grid approximations of the near pairs.
     const int64_t np = near.count;
-    FHB_CUDA(persist(&out.pair_grid, (size_t)np));
+    FHB_CUDA(persist(&out.pair_grid, (size_t)np, s));
     if (np) {
         const int2 *d_pairs = near.pairs;
         const int64_t *d_poff = near.off;
@@ -655,7 +655,7 @@ fh_status pfft_near_csr(int64_t n, int64_t np, const int2 *d_pairs, const double
                                                             d_rows);
         FHB_CUDA(cudaGetLastError());
     }
-    FHB_CUDA(persist(near_off, (size_t)n + 1));
+    FHB_CUDA(persist(near_off, (size_t)n + 1, s));
     size_t tb = 0;
     FHB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, reinterpret_cast<int64_t *>(d_rows), *near_off, (int)(n + 1),
                                            s));
@@ -673,8 +673,8 @@ fh_status pfft_near_csr(int64_t n, int64_t np, const int2 *d_pairs, const double
         FHB_CUDA(cub::DeviceRadixSort::SortPairs(d_sb, sb, d_keys, d_keys2, d_vals, d_vals2, (int)(2 * np), 0, 64, s));
     }
     FHB_CUDA(cudaStreamSynchronize(s));
-    FHB_CUDA(persist(near_col, (size_t)total));
-    FHB_CUDA(persist(near_val, (size_t)total));
+    FHB_CUDA(persist(near_col, (size_t)total, s));
+    FHB_CUDA(persist(near_val, (size_t)total, s));
     if (total) {
         near_split_kernel<<<blocks(total, 256), 256, 0, s>>>(d_keys2, d_vals2, total, n, *near_col, *near_val);
         FHB_CUDA(cudaGetLastError());
