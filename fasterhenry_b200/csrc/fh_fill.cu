@@ -520,17 +520,125 @@ __device__ __forceinline__ double point_value(const DevFil &A, const DevFil &B, 
     return kMu0Over4Pi * (total * cosv);
 }
 
+// The same sums by a whole warp (the value on every lane): the lanes share
+// B's first axis and all of A's points, or for bars of one frame the classes
+// of the first axis and A's points of the second.
+__device__ double point_value_warp(const DevFil &A, const DevFil &B, int orders, const double delta[3], int lane) {
+    const int oa0 = orders & 31, oa1 = (orders >> 5) & 31, oa2 = (orders >> 10) & 31;
+    const int ob0 = (orders >> 15) & 31, ob1 = (orders >> 20) & 31, ob2 = (orders >> 25) & 31;
+    double total = 0.0;
+    if (oa0 == ob0 && oa1 == ob1 && oa2 == ob2 && same_frame(A, B)) {
+        const double h0 = A.half[0], h1 = A.half[1], h2 = A.half[2];
+        // rows i0 = r and n - 1 - r of the triangle i0 + j0 < n side by side
+        const int rows = (oa0 + 1) / 2, work = rows * (oa0 + 1) * oa1;
+        for (int idx = lane; idx < work; idx += 32) {
+            const int rest = idx / oa1, i1 = idx - rest * oa1, r = rest / (oa0 + 1), c = rest - r * (oa0 + 1);
+            int i0 = r, j0 = c;
+            if (c >= oa0 - r) {
+                if (2 * r + 1 == oa0) continue;  // the middle row is its own partner
+                i0 = oa0 - 1 - r;
+                j0 = c - (oa0 - r);
+            }
+            const double d0 = h0 * c_quad.nodes[oa0][i0] - h0 * c_quad.nodes[oa0][j0];
+            const double w0 = (h0 * c_quad.weights[oa0][i0]) * (h0 * c_quad.weights[oa0][j0]) *
+                              (i0 + j0 == oa0 - 1 ? 1.0 : 2.0);
+            double s0 = 0.0;
+            for (int j1 = 0; i1 + j1 < oa1; ++j1) {
+                const double d1 = h1 * c_quad.nodes[oa1][i1] - h1 * c_quad.nodes[oa1][j1];
+                const double w1 = (0.5 * c_quad.weights[oa1][i1]) * (0.5 * c_quad.weights[oa1][j1]) *
+                                  (i1 + j1 == oa1 - 1 ? 1.0 : 2.0);
+                double r1[3];
+#pragma unroll
+                for (int d = 0; d < 3; ++d) r1[d] = A.axes[d] * d0 - delta[d] + A.axes[3 + d] * d1;
+                double s1 = 0.0;
+                for (int i2 = 0; i2 < oa2; ++i2)
+                    for (int j2 = 0; i2 + j2 < oa2; ++j2) {
+                        const double d2 = h2 * c_quad.nodes[oa2][i2] - h2 * c_quad.nodes[oa2][j2];
+                        const double w2 = (0.5 * c_quad.weights[oa2][i2]) * (0.5 * c_quad.weights[oa2][j2]) *
+                                          (i2 + j2 == oa2 - 1 ? 1.0 : 2.0);
+                        const double dx = r1[0] + A.axes[6] * d2, dy = r1[1] + A.axes[7] * d2,
+                                     dz = r1[2] + A.axes[8] * d2;
+                        s1 += w2 * rsqrt(dx * dx + dy * dy + dz * dz);
+                    }
+                s0 += w1 * s1;
+            }
+            total += w0 * s0;
+        }
+    } else {
+        const double ah0 = A.half[0], ah1 = 2.0 * A.half[1], ah2 = 2.0 * A.half[2];
+        const double bh0 = B.half[0], bh1 = 2.0 * B.half[1], bh2 = 2.0 * B.half[2];
+        const int work = oa0 * oa1 * oa2 * ob0;
+        for (int idx = lane; idx < work; idx += 32) {
+            int rest = idx / ob0;
+            const int lb = idx - rest * ob0;
+            const int q2 = rest / oa2, ha = rest - q2 * oa2, la = q2 / oa1, wa = q2 - la * oa1;
+            const double xl = ah0 * c_quad.nodes[oa0][la], wl = ah0 * c_quad.weights[oa0][la];
+            const double xw = ah1 * (0.5 * c_quad.nodes[oa1][wa]), ww = 0.5 * c_quad.weights[oa1][wa];
+            const double xh = ah2 * (0.5 * c_quad.nodes[oa2][ha]), wh = 0.5 * c_quad.weights[oa2][ha];
+            const double yl = bh0 * c_quad.nodes[ob0][lb], vl = bh0 * c_quad.weights[ob0][lb];
+            double p[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                p[d] = A.axes[d] * xl + A.axes[3 + d] * xw + A.axes[6 + d] * xh - (delta[d] + B.axes[d] * yl);
+            double inner = 0.0;
+            for (int wb = 0; wb < ob1; ++wb) {
+                const double yw = bh1 * (0.5 * c_quad.nodes[ob1][wb]), vw = 0.5 * c_quad.weights[ob1][wb];
+                double q[3];
+#pragma unroll
+                for (int d = 0; d < 3; ++d) q[d] = p[d] - B.axes[3 + d] * yw;
+                double s = 0.0;
+                for (int hb = 0; hb < ob2; ++hb) {
+                    const double yh = bh2 * (0.5 * c_quad.nodes[ob2][hb]), vh = 0.5 * c_quad.weights[ob2][hb];
+                    const double dx = q[0] - B.axes[6] * yh, dy = q[1] - B.axes[7] * yh, dz = q[2] - B.axes[8] * yh;
+                    s += vh * rsqrt(dx * dx + dy * dy + dz * dz);
+                }
+                inner += vw * s;
+            }
+            total += wl * ww * wh * vl * inner;
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+    return kMu0Over4Pi * (total * ndot(A.axes, B.axes));
+}
+
+// Point pairs of at least this many terms are summed by a warp, the others by
+// a thread.  Orders reach 20 per axis for bars less than a length apart, up
+// to 1e5 terms where most pairs have a few hundred, and the list ends with
+// them: alone on a thread they set the kernel's time.  1,500 bars in general
+// position (1.1 M pairs): 22.1 ms with a thread per pair, 1.5 ms so; 240
+// filaments of a spiral: 175 and 13 us.  The rule is the pair's own cost, so
+// that a pair's value does not depend on the list that it is in.
+constexpr int kHeavyBucket = 9;
+constexpr int kHeavyCost = 1 << kHeavyBucket;
+
+__device__ __forceinline__ void pair_offset(const DevFil &A, const DevFil &B, double delta[3]) {
+    long long code[3];
+    unsigned exact;
+    point_offset(A, B, delta, code, exact);
+}
+
 __global__ void __launch_bounds__(128) point_kernel(const DevFil *__restrict__ fil, const int4 *__restrict__ items,
                                                     int64_t count, double *__restrict__ L, int8_t *methods,
                                                     int64_t n, DevError *err) {
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < count;
-         t += (int64_t)gridDim.x * blockDim.x) {
-        const int4 it = items[t];
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; t0 < count; t0 += stride) {
+        const int64_t t = t0 + lane;
+        const int4 it = t < count ? items[t] : make_int4(0, 0, 0, 0);
         double delta[3];
-        long long code[3];
-        unsigned exact;
-        point_offset(fil[it.x], fil[it.y], delta, code, exact);
-        store_pair(L, methods, n, it, point_value(fil[it.x], fil[it.y], it.z, delta), kPoint, err);
+        const bool heavy = it.w >= kHeavyCost;
+        if (t < count && !heavy) {
+            pair_offset(fil[it.x], fil[it.y], delta);
+            store_pair(L, methods, n, it, point_value(fil[it.x], fil[it.y], it.z, delta), kPoint, err);
+        }
+        for (unsigned left = __ballot_sync(0xffffffffu, heavy); left; left &= left - 1) {
+            const int src = __ffs(left) - 1;
+            const int4 h = make_int4(__shfl_sync(0xffffffffu, it.x, src), __shfl_sync(0xffffffffu, it.y, src),
+                                     __shfl_sync(0xffffffffu, it.z, src), __shfl_sync(0xffffffffu, it.w, src));
+            pair_offset(fil[h.x], fil[h.y], delta);
+            const double v = point_value_warp(fil[h.x], fil[h.y], h.z, delta, lane);
+            if (lane == 0) store_pair(L, methods, n, h, v, kPoint, err);
+        }
     }
 }
 
@@ -1406,19 +1514,32 @@ __global__ void __launch_bounds__(kHeadsBlock) key_heads_kernel(const DevFil *__
 }
 
 // values[rank[h]] = the value of the pair items[heads[h]] (heads in work-list
-// order, which is cost order for the point pairs).
+// order, which is cost order for the point pairs; the items from heavy_from on
+// have at least kHeavyCost terms).  The heavy heads first and from the most
+// expensive down, a warp each, then the others, a thread each.
 __global__ void __launch_bounds__(128) point_heads_ordered_kernel(const DevFil *__restrict__ fil,
                                                                   const int4 *__restrict__ items,
                                                                   const int64_t *__restrict__ heads,
                                                                   const int64_t *__restrict__ rank, int64_t n_heads,
-                                                                  double *__restrict__ values) {
-    for (int64_t h = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; h < n_heads;
-         h += (int64_t)gridDim.x * blockDim.x) {
+                                                                  int64_t heavy_from, double *__restrict__ values) {
+    const int lane = threadIdx.x & 31;
+    const int64_t thread = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, threads = (int64_t)gridDim.x * blockDim.x;
+    int64_t lo = 0, hi = n_heads;  // the first heavy head
+    while (lo < hi) {
+        const int64_t mid = (lo + hi) / 2;
+        if (heads[mid] < heavy_from) lo = mid + 1;
+        else hi = mid;
+    }
+    double delta[3];
+    for (int64_t h = n_heads - 1 - thread / 32; h >= lo; h -= threads / 32) {
         const int4 it = items[heads[h]];
-        double delta[3];
-        long long code[3];
-        unsigned exact;
-        point_offset(fil[it.x], fil[it.y], delta, code, exact);
+        pair_offset(fil[it.x], fil[it.y], delta);
+        const double v = point_value_warp(fil[it.x], fil[it.y], it.z, delta, lane);
+        if (lane == 0) values[rank[h]] = v;
+    }
+    for (int64_t h = lo - 1 - thread; h >= 0; h -= threads) {
+        const int4 it = items[heads[h]];
+        pair_offset(fil[it.x], fil[it.y], delta);
         values[rank[h]] = point_value(fil[it.x], fil[it.y], it.z, delta);
     }
 }
@@ -2560,9 +2681,11 @@ fh_status fill_run(const DevFil *d_fil, int64_t n, const int2 *d_pairs, int64_t 
             FHB_CUDA(alloc(&d_sort_tmp, std::max<size_t>(sort_bytes, 16)));
             FHB_CUDA(cub::DeviceRadixSort::SortPairs(d_sort_tmp, sort_bytes, d_heads, d_heads_sorted, d_rank_in,
                                                      d_rank_sorted, (int)n_heads, 0, bits, stream));
-            const int hblocks = (int)std::min<int64_t>((n_heads + 127) / 128, (int64_t)sms * 64);
+            // a warp per head at most: which heads are heavy is not known here
+            const int hblocks = (int)std::min<int64_t>((n_heads + 3) / 4, (int64_t)sms * 64);
             point_heads_ordered_kernel<<<hblocks, 128, 0, stream>>>(d_fil, d_items, d_heads_sorted, d_rank_sorted,
-                                                                    n_heads, d_pvalues);
+                                                                    n_heads, (int64_t)offsets[kHeavyBucket],
+                                                                    d_pvalues);
             FHB_CUDA(cudaGetLastError());
             const int sblocks = (int)std::min<int64_t>((n_point + 255) / 256, (int64_t)sms * 16);
             point_scatter_kernel<<<sblocks, 256, 0, stream>>>(d_items, d_item_head, d_pvalues, n_point, d_L, d_methods,
