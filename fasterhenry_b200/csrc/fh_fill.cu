@@ -1048,13 +1048,32 @@ struct FarRules {
 // times the largest cross-section side, 6e-13 with m = 4 for at least four
 // times, 1.2e-13 with m = 5 for at least twice and 3.5e-13 with m = 6 for at
 // least once (random pairs of 50-400 um segments with 0.2-3 um sides).
-__device__ __forceinline__ double perp_primitive(double X, double Y, double d) {
-    const double d2 = d * d, R = sqrt(X * X + Y * Y + d2);
-    auto lg = [&](double a, double b) { return a >= 0.0 ? log(a + R) : log((b * b + d2) / (R - a)); };
+// Its four corners x0 < x1, y0 < y1 are taken together: with the log as log(n /
+// q) the two logs of a coordinate differ by one log of a ratio, and two
+// arctangents by one of the angle between (|d| R, X Y) vectors: four logs and
+// two arctangents for eight and four.
+__device__ __forceinline__ double perp_corners(double x0, double x1, double y0, double y1, double d) {
+    const double d2 = d * d, x02 = x0 * x0 + d2, x12 = x1 * x1 + d2, y02 = y0 * y0, y12 = y1 * y1;
+    const double r11 = sqrt(x12 + y12), r01 = sqrt(x02 + y12), r10 = sqrt(x12 + y02), r00 = sqrt(x02 + y02);
+    // log of (a1 over b^2 + d^2 = s, r1) minus that of (a0, s, r0)
+    auto diff = [](double a1, double r1, double a0, double r0, double s) {
+        const double n1 = a1 >= 0.0 ? a1 + r1 : s, q1 = a1 >= 0.0 ? 1.0 : r1 - a1;
+        const double n0 = a0 >= 0.0 ? a0 + r0 : s, q0 = a0 >= 0.0 ? 1.0 : r0 - a0;
+        return log((n1 * q0) / (q1 * n0));
+    };
     double f = 0.0;
-    if (X != 0.0) f += X * lg(Y, X);
-    if (Y != 0.0) f += Y * lg(X, Y);
-    if (d != 0.0) f -= d * atan(X * Y / (d * R));
+    if (x1 != 0.0) f += x1 * diff(y1, r11, y0, r10, x12);
+    if (x0 != 0.0) f -= x0 * diff(y1, r01, y0, r00, x02);
+    if (y1 != 0.0) f += y1 * diff(x1, r11, x0, r01, y12 + d2);
+    if (y0 != 0.0) f -= y0 * diff(x1, r10, x0, r00, y02 + d2);
+    if (d != 0.0) {
+        const double e = fabs(d);
+        auto turn = [e](double sa, double ra, double sb, double rb) {
+            const double ca = e * ra, cb = e * rb;
+            return atan2(sa * cb - ca * sb, ca * cb + sa * sb);
+        };
+        f -= e * (turn(x1 * y1, r11, x0 * y1, r01) - turn(x1 * y0, r10, x0 * y0, r00));
+    }
     return f;
 }
 __device__ __forceinline__ int ortho_rule_order(const OrthoBoxes &o) {
@@ -1083,32 +1102,173 @@ __device__ __forceinline__ double ortho_point(const OrthoBoxes &o, const FarRule
     const double x0 = -0.5 * o.ea[0] - xb, x1 = 0.5 * o.ea[0] - xb;
     const double y0 = o.off[kb] - 0.5 * o.eb[kb] - ap, y1 = o.off[kb] + 0.5 * o.eb[kb] - ap;
     const double d = bq - aq;
-    return w * (perp_primitive(x1, y1, d) - perp_primitive(x0, y1, d) - perp_primitive(x1, y0, d) +
-                perp_primitive(x0, y0, d));
+    return w * perp_corners(x0, x1, y0, y1, d);
 }
 
-// kMode 0: values[h] = the integral.  kMode 1: values[7 h + 0..6] = the
-// integral and its partials with respect to (width[0], width[1], offset[1],
-// height[0], height[1], offset[2]).  kMode 2: values[8 h + 0..7] = the
-// coordinate derivatives of integrand_coord (the work item's flags choose
-// the frame and the rotation axis).  The rule (panel tree, leaves, nodes) is
-// held at the pair's own geometry, except in kMode 1 and 2 for pairs whose
-// cross-sections lie at least one largest side apart (far_rule_order,
-// ortho_rule_order), which take fixed rules.  With key_counter the CTAs draw their keys
+// The work of a derivative quadrature key by the rule it takes: the panel tree
+// (a CTA), or a fixed rule over points (a warp).
+enum QuadClass { kQuadTree = 0, kQuadFar = 1, kQuadOrtho = 2, kQuadClasses = 3 };
+
+// What a key's rules need of its pair (kMode 2: the work item's flags choose
+// the frame and the rotation axis); whether it takes the orthogonal form.
+template <int kMode>
+__device__ __forceinline__ bool quad_context(const DevFil &A, const DevFil &B, int4 it, QuadCtx &ctx) {
+    bool ortho = false;
+    if (kMode == 2 && (it.w & kCoordOrtho)) {
+        int kb = 1;
+        ortho_aligned(A, B, &ctx.b, &kb);
+        ortho = kb == 1 || kb == 2;
+        if (ortho) {
+            const Aligned &q = ctx.b;
+            ctx.o = OrthoBoxes{{q.length[0], q.width[0], q.height[0]},
+                               {q.length[1], q.width[1], q.height[1]},
+                               {q.offset[0], q.offset[1], q.offset[2]},
+                               kb};
+        }
+    } else {
+        aligned_bars(A, B, &ctx.b);
+    }
+    ctx.tau = kMode == 2 ? (it.w & kCoordTauMask) : 0;
+    ctx.rot = kMode == 2 && (it.w & kCoordRot) && ctx.tau != 0;
+    ctx.sigma = (it.w & kCoordSigmaNeg) ? -1.0 : 1.0;
+    ctx.axial_start = ctx.b.offset[0] + 0.5 * (ctx.b.length[0] - ctx.b.length[1]);
+    return ortho;
+}
+
+// Sorts the keys into the lists of their classes (lists + c n_heads; the order
+// inside a list does not matter, each key writes its own values).
+template <int kMode>
+__global__ void __launch_bounds__(128) quad_classify_kernel(const DevFil *__restrict__ fil,
+                                                            const int4 *__restrict__ items,
+                                                            const int64_t *__restrict__ heads, int64_t n_heads,
+                                                            int *__restrict__ lists,
+                                                            unsigned long long *__restrict__ counts) {
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t h0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; h0 < n_heads; h0 += stride) {
+        const int64_t h = h0 + lane;
+        int cls = -1;
+        if (h < n_heads) {
+            const int4 it = items[heads[h]];
+            QuadCtx ctx;
+            const bool ortho = quad_context<kMode>(fil[it.x], fil[it.y], it, ctx);
+            cls = ortho ? (ortho_rule_order(ctx.o) ? kQuadOrtho : kQuadTree)
+                        : (far_rule_order(ctx.b) ? kQuadFar : kQuadTree);
+        }
+        for (int c = 0; c < kQuadClasses; ++c) {
+            const unsigned mask = __ballot_sync(0xffffffffu, cls == c);
+            if (!mask) continue;
+            unsigned long long at = 0;
+            if (lane == __ffs(mask) - 1) at = atomicAdd(&counts[c], (unsigned long long)__popc(mask));
+            at = __shfl_sync(0xffffffffu, at, __ffs(mask) - 1);
+            if (cls == c) lists[(int64_t)c * n_heads + (int64_t)at + __popc(mask & ((1u << lane) - 1))] = (int)h;
+        }
+    }
+}
+
+// The fixed rules, a warp per key.  kOrtho: ortho_point's product rule; else p x
+// p points on each of the overlap weights' break-point panels.  Every lane
+// forms the pair's context itself; nothing is shared between warps, so a key
+// of some hundred points costs no block barrier and no idle setup.  At 4.6 M
+// keys of a graded spiral these rules on a CTA each (128 threads, one of them
+// setting up) took most of 236 ms; here 32 ms, and the tree's keys 24 ms.
+template <int kMode, bool kOrtho>
+__global__ void __launch_bounds__(128) quad_rule_kernel(const DevFil *__restrict__ fil,
+                                                        const int4 *__restrict__ items,
+                                                        const int64_t *__restrict__ heads,
+                                                        const int *__restrict__ list, int64_t count,
+                                                        double *__restrict__ values) {
+    constexpr int kVals = kMode == 1 ? 7 : 8;
+    __shared__ FarRules rules;
+    __shared__ double s_us[4][2][5];
+    __shared__ int s_nu[4][2];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x < 24) {
+        const int m = 3 + threadIdx.x / 6, q = threadIdx.x % 6;
+        rules.n[m - 3][q] = q < m ? c_quad.nodes[m][q] : 0.0;
+        rules.w[m - 3][q] = q < m ? c_quad.weights[m][q] : 0.0;
+    }
+    __syncthreads();
+    const int64_t stride = (int64_t)gridDim.x * 4;
+    for (int64_t t = (int64_t)blockIdx.x * 4 + warp; t < count; t += stride) {
+        const int64_t h = list[t];
+        const int4 it = items[heads[h]];
+        QuadCtx ctx;
+        quad_context<kMode>(fil[it.x], fil[it.y], it, ctx);
+        if (kOrtho) {
+            const int m = ortho_rule_order(ctx.o), points = m * m * m * m;
+            double acc = 0.0;
+            for (int k = lane; k < points; k += 32) acc += ortho_point(ctx.o, rules, m, k);
+            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            if (lane < kVals) values[kVals * h + lane] = lane == 0 ? acc : 0.0;
+            continue;
+        }
+        __syncwarp();  // the previous key's break points are read
+        if (lane < 2)
+            s_nu[warp][lane] = lane == 0 ? break_points(ctx.b.width[0], ctx.b.width[1], ctx.b.offset[1], s_us[warp][0])
+                                         : break_points(ctx.b.height[0], ctx.b.height[1], ctx.b.offset[2], s_us[warp][1]);
+        __syncwarp();
+        const int m = far_rule_order(ctx.b), pp = m * m, nv = s_nu[warp][1] - 1,
+                  points = (s_nu[warp][0] - 1) * nv * pp;
+        const double *nd = rules.n[m - 3], *wt = rules.w[m - 3];
+        double v[8] = {};
+        for (int k = lane; k < points; k += 32) {
+            const int panel = k / pp, r = k - panel * pp, a = r / m, c = r - a * m;
+            const int pu = panel / nv, pv = panel - pu * nv;
+            const double u0 = s_us[warp][0][pu], u1 = s_us[warp][0][pu + 1];
+            const double v0 = s_us[warp][1][pv], v1 = s_us[warp][1][pv + 1];
+            const double hu = 0.5 * (u1 - u0), hv = 0.5 * (v1 - v0);
+            if (!(hu > 0.0 && hv > 0.0)) continue;
+            const double uu = 0.5 * (u0 + u1) + hu * nd[a], vv = 0.5 * (v0 + v1) + hv * nd[c];
+            const double wuv = (hu * wt[a]) * (hv * wt[c]);
+            double g[8];
+            if (kMode == 2) {
+                integrand_coord(ctx, uu, vv, g);
+            } else {
+                integrand_grad(ctx, uu, vv, g);
+                g[7] = 0.0;
+            }
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v[q] += wuv * g[q];
+        }
+        // each step halves the sums a lane keeps; lane 4 q ends with sum q
+#pragma unroll
+        for (int o = 16, have = 8; o > 2; o >>= 1, have >>= 1) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (q < have / 2) {
+                    const double keep = lane & o ? v[q + have / 2] : v[q];
+                    const double give = lane & o ? v[q] : v[q + have / 2];
+                    v[q] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                }
+        }
+        v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+        v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+        if (!(lane & 3) && lane / 4 < kVals) values[kVals * h + lane / 4] = v[0];
+    }
+}
+
+// The panel tree, a CTA per key.  kMode 0: values[h] = the integral.  kMode 1:
+// values[7 h + 0..6] = the integral and its partials with respect to (width[0],
+// width[1], offset[1], height[0], height[1], offset[2]).  kMode 2: values[8 h +
+// 0..7] = the coordinate derivatives of integrand_coord.  The rule (panel tree,
+// leaves, nodes) is held at the pair's own geometry.  With a list, its keys
+// alone are taken (in kMode 1 and 2, whose pairs at least one largest side
+// apart take quad_rule_kernel).  With key_counter the CTAs draw their keys
 // from it (keys differ widely in cost), else take every gridDim.x-th; in
 // kMode 2 the threads share the points of a batch of leaves evenly (a
 // direct leaf has 49 there, fewer than the CTA's threads).
 template <int kMode>
 __global__ void __launch_bounds__(kQuadThreads) aligned_quadrature_kernel(
     const DevFil *__restrict__ fil, const int4 *__restrict__ items, const int64_t *__restrict__ heads,
-    int64_t n_heads, double *__restrict__ values, unsigned long long *__restrict__ key_counter = nullptr) {
+    int64_t n_heads, double *__restrict__ values, const int *__restrict__ list = nullptr,
+    unsigned long long *__restrict__ key_counter = nullptr) {
     constexpr int kVals = kMode == 0 ? 1 : (kMode == 1 ? 7 : 8);
     __shared__ Panel stack[kStack];
     __shared__ Leaf leaves[kLeaves];
     __shared__ int s_leaf_off[kLeaves + 1];
     __shared__ long long s_key;
-    __shared__ int s_nleaves, s_done, s_far, s_npanels;
-    __shared__ FarRules far_rules;
+    __shared__ int s_nleaves, s_done;
     __shared__ QuadCtx ctx;
     __shared__ double s_red[kVals][kQuadThreads / 32];
     __shared__ double r10n[10], r10w[10], r16n[16], r16w[16], r7n[7], r7w[7];
@@ -1119,11 +1279,6 @@ __global__ void __launch_bounds__(kQuadThreads) aligned_quadrature_kernel(
             r7n[threadIdx.x] = c_quad.nodes[7][threadIdx.x];
             r7w[threadIdx.x] = c_quad.weights[7][threadIdx.x];
         }
-        if (kMode >= 1 && threadIdx.x < 6)
-            for (int m = 3; m <= 6; ++m) {
-                far_rules.n[m - 3][threadIdx.x] = threadIdx.x < m ? c_quad.nodes[m][threadIdx.x] : 0.0;
-                far_rules.w[m - 3][threadIdx.x] = threadIdx.x < m ? c_quad.weights[m][threadIdx.x] : 0.0;
-            }
     }
     if (threadIdx.x < 16) {
         r16n[threadIdx.x] = c_quad.nodes[16][threadIdx.x];
@@ -1135,33 +1290,14 @@ __global__ void __launch_bounds__(kQuadThreads) aligned_quadrature_kernel(
         __syncthreads();
         return s_key;
     };
-    for (int64_t h = draw(-1); h < n_heads; h = draw(h)) {
+    for (int64_t key = draw(-1); key < n_heads; key = draw(key)) {
+        const int64_t h = list ? list[key] : key;
         const int4 it = items[heads[h]];
         int sp = 0;
         double axial_scale = 0.0;
         if (threadIdx.x == 0) {
-            const DevFil &A = fil[it.x];
-            const DevFil &B = fil[it.y];
-            bool ortho = false;
-            if (kMode == 2 && (it.w & kCoordOrtho)) {
-                int kb = 1;
-                ortho_aligned(A, B, &ctx.b, &kb);
-                ortho = kb == 1 || kb == 2;
-                if (ortho) {
-                    const Aligned &q = ctx.b;
-                    ctx.o = OrthoBoxes{{q.length[0], q.width[0], q.height[0]},
-                                       {q.length[1], q.width[1], q.height[1]},
-                                       {q.offset[0], q.offset[1], q.offset[2]},
-                                       kb};
-                }
-            } else {
-                aligned_bars(A, B, &ctx.b);
-            }
-            ctx.tau = kMode == 2 ? (it.w & kCoordTauMask) : 0;
-            ctx.rot = kMode == 2 && (it.w & kCoordRot) && ctx.tau != 0;
-            ctx.sigma = (it.w & kCoordSigmaNeg) ? -1.0 : 1.0;
+            quad_context<kMode>(fil[it.x], fil[it.y], it, ctx);
             const Aligned &b = ctx.b;
-            ctx.axial_start = b.offset[0] + 0.5 * (b.length[0] - b.length[1]);
             double l1 = b.length[0], l2 = b.length[1], as = ctx.axial_start;
             double sep[4] = {as + l2, as, as + l2 - l1, as - l1};
             double largest = 0.0;
@@ -1175,47 +1311,11 @@ __global__ void __launch_bounds__(kQuadThreads) aligned_quadrature_kernel(
             // Push panels in reverse so that they pop in the reference's order.
             for (int a = nu - 2; a >= 0; --a)
                 for (int c = nv - 2; c >= 0; --c) stack[sp++] = Panel{us[a], us[a + 1], vs[c], vs[c + 1], 0, 0};
-            // product rules for pairs far apart: negative order for the
-            // orthogonal form
-            s_far = kMode == 0 ? 0 : (ortho ? -ortho_rule_order(ctx.o) : far_rule_order(b));
-            s_npanels = sp;  // the break-point panels, for the far rule
         }
         double acc = 0.0, gacc[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
         long long visited = 0;  // panels popped; bounded so that no input can loop without end
         bool overflow = false;
-        int far_m = 0;
-        if (kMode >= 1) {
-            __syncthreads();
-            far_m = s_far;
-            if (far_m > 0) {
-                // p x p points on each break-point panel, the panels as pushed
-                const int pp = far_m * far_m, points = s_npanels * pp;
-                const double *nd = far_rules.n[far_m - 3], *wt = far_rules.w[far_m - 3];
-                for (int k = threadIdx.x; k < points; k += kQuadThreads) {
-                    const Panel pn = stack[k / pp];
-                    const int a = (k % pp) / far_m, c = k % far_m;
-                    const double hu = 0.5 * (pn.u1 - pn.u0), hv = 0.5 * (pn.v1 - pn.v0);
-                    if (!(hu > 0.0 && hv > 0.0)) continue;
-                    const double uu = 0.5 * (pn.u0 + pn.u1) + hu * nd[a], vv = 0.5 * (pn.v0 + pn.v1) + hv * nd[c];
-                    const double wuv = (hu * wt[a]) * (hv * wt[c]);
-                    if (kMode == 2) {
-                        double g[8];
-                        integrand_coord(ctx, uu, vv, g);
-                        acc += wuv * g[0];
-                        for (int q = 0; q < 7; ++q) gacc[q] += wuv * g[1 + q];
-                    } else {
-                        double g[7];
-                        integrand_grad(ctx, uu, vv, g);
-                        acc += wuv * g[0];
-                        for (int q = 0; q < 6; ++q) gacc[q] += wuv * g[1 + q];
-                    }
-                }
-            } else if (far_m < 0) {
-                const int mo = -far_m, points = mo * mo * mo * mo;
-                for (int k = threadIdx.x; k < points; k += kQuadThreads) acc += ortho_point(ctx.o, far_rules, mo, k);
-            }
-        }
-        for (; !far_m;) {
+        for (;;) {
             if (threadIdx.x == 0) {
                 // Walk the panel tree until the leaf buffer is full or the tree is done.
                 int nl = 0;
@@ -2538,6 +2638,43 @@ fh_status distinct_keys(Key, const DevFil *d_fil, const int4 *d_list, int64_t co
     return FH_OK;
 }
 
+// The derivative quadratures of the distinct keys (kMode 1: 7 values a key,
+// kMode 2: 8): the keys sorted by the rule they take, then a kernel per rule.
+template <int kMode, class Alloc>
+fh_status derivative_quadrature(const DevFil *d_fil, const int4 *d_quad, const int64_t *d_heads, int64_t n_heads,
+                                double *d_values, Alloc &alloc, cudaStream_t stream, fh_error_info *err) {
+    if (n_heads > INT32_MAX) return fail(err, FH_ERR_INVALID_ARGUMENT, "too many distinct quadrature pairs");
+    const int64_t sms = 148;
+    int *d_lists = nullptr;
+    unsigned long long *d_counts = nullptr;  // per class, then the tree's key counter
+    FHB_CUDA(alloc((void **)&d_lists, sizeof(int) * kQuadClasses * (size_t)n_heads));
+    FHB_CUDA(alloc((void **)&d_counts, sizeof(unsigned long long) * (kQuadClasses + 1)));
+    FHB_CUDA(cudaMemsetAsync(d_counts, 0, sizeof(unsigned long long) * (kQuadClasses + 1), stream));
+    quad_classify_kernel<kMode><<<(unsigned)std::min<int64_t>((n_heads + 127) / 128, sms * 32), 128, 0, stream>>>(
+        d_fil, d_quad, d_heads, n_heads, d_lists, d_counts);
+    FHB_CUDA(cudaGetLastError());
+    unsigned long long counts[kQuadClasses];
+    FHB_CUDA(cudaMemcpyAsync(counts, d_counts, sizeof counts, cudaMemcpyDeviceToHost, stream));
+    FHB_CUDA(cudaStreamSynchronize(stream));
+    if (counts[kQuadTree]) {
+        const unsigned grid = (unsigned)std::min<int64_t>((int64_t)counts[kQuadTree], sms * 16);
+        aligned_quadrature_kernel<kMode><<<grid, kQuadThreads, 0, stream>>>(
+            d_fil, d_quad, d_heads, (int64_t)counts[kQuadTree], d_values, d_lists + kQuadTree * n_heads,
+            d_counts + kQuadClasses);
+    }
+    auto warps = [&](unsigned long long n) { return (unsigned)std::min<int64_t>(((int64_t)n + 3) / 4, sms * 64); };
+    if (counts[kQuadFar])
+        quad_rule_kernel<kMode, false><<<warps(counts[kQuadFar]), 128, 0, stream>>>(
+            d_fil, d_quad, d_heads, d_lists + kQuadFar * n_heads, (int64_t)counts[kQuadFar], d_values);
+    if constexpr (kMode == 2) {
+        if (counts[kQuadOrtho])
+            quad_rule_kernel<kMode, true><<<warps(counts[kQuadOrtho]), 128, 0, stream>>>(
+                d_fil, d_quad, d_heads, d_lists + kQuadOrtho * n_heads, (int64_t)counts[kQuadOrtho], d_values);
+    }
+    FHB_CUDA(cudaGetLastError());
+    return FH_OK;
+}
+
 // The Gauss rules and order thresholds in constant memory, once per device.
 fh_status upload_quad_tables(fh_error_info *err) {
     int dev = 0;
@@ -2729,8 +2866,8 @@ fh_status fill_run(const DevFil *d_fil, int64_t n, const int2 *d_pairs, int64_t 
         const int blocks = (int)std::min<int64_t>((n_quad + 255) / 256, (int64_t)sms * 16);
         int qblocks = (int)std::min<int64_t>(n_heads, (int64_t)sms * 16);
         if (grad) {
-            aligned_quadrature_kernel<1><<<qblocks, kQuadThreads, 0, stream>>>(d_fil, d_quad, d_heads, n_heads,
-                                                                                 d_values);
+            const fh_status qs = derivative_quadrature<1>(d_fil, d_quad, d_heads, n_heads, d_values, alloc, stream, err);
+            if (qs) return qs;
             FHB_CUDA(cudaGetLastError());
             aligned_grad_scatter_kernel<<<blocks, 256, 0, stream>>>(d_fil, d_tan, d_quad, d_item_head, d_values, n_quad,
                                                                     *grad, n, d_err);
@@ -2909,12 +3046,8 @@ fh_status device_fill_coord(const DevFil *d_fil, const int32_t *d_seg, const uin
         st.unique_aligned = n_heads;
         double *d_values = nullptr;
         FHB_CUDA(alloc((void **)&d_values, 64 * (size_t)n_heads));
-        unsigned long long *d_keys = nullptr;
-        FHB_CUDA(alloc((void **)&d_keys, sizeof(unsigned long long)));
-        FHB_CUDA(cudaMemsetAsync(d_keys, 0, sizeof(unsigned long long), stream));
-        const int qblocks = (int)std::min<int64_t>(n_heads, (int64_t)sms * 16);
-        aligned_quadrature_kernel<2><<<qblocks, kQuadThreads, 0, stream>>>(d_fil, d_quad, d_heads, n_heads, d_values,
-                                                                          d_keys);
+        const fh_status qs = derivative_quadrature<2>(d_fil, d_quad, d_heads, n_heads, d_values, alloc, stream, err);
+        if (qs) return qs;
         FHB_CUDA(cudaGetLastError());
         const int blocks = (int)std::min<int64_t>((n_quad + 255) / 256, (int64_t)sms * 16);
         coord_quad_scatter_kernel<<<blocks, 256, 0, stream>>>(d_fil, d_quad, d_item_head, d_values, n_quad, out, n,
