@@ -895,73 +895,55 @@ __device__ __forceinline__ void integrand_grad(const QuadCtx &c, double u, doubl
 struct LineTerms {
     double k, das, dl1, dl2, j1, j1b;
 };
-// line_terms evaluates the four corner distances q of the rectangle once:
-// R = sqrt(q^2 + rho^2) and L = log(|q| + R) serve the kernel (|q| L - R,
-// the terms of lines_parallel in its own operation order, so k is the same
-// double), its partials (sign(q) L) and the moments (R).
+//
+// For rho > 0 the terms with log(rho) cancel: with A = asinh(q / rho) the
+// antiderivative is q A - R, so k and its partials are sums of A and R over
+// the four corner distances q, and the moments take the same A and R.  A is
+// log((|q| + R) / rho) with q's sign: an absolute error of an ulp of 1 where q
+// is small against rho, and the sums over the corners are about l1 l2 / rho^2,
+// above 1e-2 for pairs the point rule leaves.  A log where |q| >= rho / 2 and an
+// asinh below it, both in most warps, had made this the larger part of the
+// coordinate quadrature: 40 -> 18.5 ms for 3.2 M pairs apart and 23.6 -> 20.5 ms
+// for the tree's (log1p of (|q| + q^2 / (rho + R)) / rho: 23 and 28.6).  rho = 0
+// (lines in one axis, without overlap) keeps the logs.
 __device__ bool line_terms(double l1, double l2, double as, double rho, bool moments, LineTerms *t) {
     const double r2 = rho * rho;
     const double e = as + l2;
     const double q[4] = {e, as, e - l1, as - l1};
-    double R[4], P[4], D[4];
+    t->j1 = t->j1b = 0.0;
+    if (!(r2 > 0.0)) {
+        if (rmax(rmin(l1, e) - rmax(as, 0.0), 0.0) != 0.0) return false;
+        double P[4], D[4];
+        for (int i = 0; i < 4; ++i) {
+            const double aq = fabs(q[i]), L = aq > 0.0 ? log(2.0 * aq) : 0.0;
+            P[i] = aq * L - aq;
+            D[i] = q[i] > 0.0 ? L : -L;
+        }
+        t->k = P[0] - P[1] - P[2] + P[3];
+        t->das = D[0] - D[1] - D[2] + D[3];
+        t->dl1 = D[2] - D[3];
+        t->dl2 = D[0] - D[2];
+        return true;
+    }
+    const double inv = 1.0 / rho;
+    double R[4], A[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const double aq = fabs(q[i]);
         R[i] = sqrt(aq * aq + r2);
-        if (aq == 0.0) {
-            P[i] = -R[i];
-            D[i] = 0.0;
-        } else {
-            const double L = log(aq + R[i]);
-            P[i] = aq * L - R[i];
-            D[i] = q[i] > 0.0 ? L : -L;
-        }
+        A[i] = copysign(log((aq + R[i]) * inv), q[i]);
     }
-    const double smooth = P[0] - P[1] - P[2] + P[3];
-    const double overlap = rmax(rmin(l1, e) - rmax(as, 0.0), 0.0);
-    double log_rho = 0.0;
-    if (overlap == 0.0) {
-        t->k = smooth;
-    } else if (rho > 0.0) {
-        log_rho = log(rho);
-        t->k = smooth - 2.0 * overlap * log_rho;
-    } else {
-        return false;
-    }
-    t->das = D[0] - D[1] - D[2] + D[3];
-    t->dl1 = D[2] - D[3];
-    t->dl2 = D[0] - D[2];
-    if (overlap > 0.0) {
-        const double hi = l1 < e ? 1.0 : (l1 == e ? 0.5 : 0.0);    // d min(l1, e) / d l1
-        const double lo = as > 0.0 ? 1.0 : (as == 0.0 ? 0.5 : 0.0);  // d max(as, 0) / d as
-        const double lr = 2.0 * log_rho;
-        t->dl1 -= lr * hi;
-        t->dl2 -= lr * (1.0 - hi);
-        t->das -= lr * ((1.0 - hi) - lo);
-    }
-    t->j1 = t->j1b = 0.0;
-    if (moments && r2 > 0.0) {
-        // psi(x) = x R(x) / (2 rho^2) - asinh(x / rho) / 2 at the four
-        // corners; asinh(|x| / rho) = log(|x| + R) - log(rho), taken from the
-        // log already formed where |x| >= rho / 2 (there the difference
-        // keeps all but a few ulps of a result of at least 0.48)
-        const double lr1 = log_rho != 0.0 ? log_rho : log(rho);
+    t->k = (q[0] * A[0] - R[0]) - (q[1] * A[1] - R[1]) - (q[2] * A[2] - R[2]) + (q[3] * A[3] - R[3]);
+    t->das = A[0] - A[1] - A[2] + A[3];
+    t->dl1 = A[2] - A[3];
+    t->dl2 = A[0] - A[2];
+    if (moments) {
+        const double ir2 = inv * inv;
         double psi[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const double aq = fabs(q[i]);
-            double ash;
-            if (aq >= 0.5 * rho) {
-                const double L = q[i] > 0.0 ? D[i] : -D[i];  // log(|x| + R)
-                ash = q[i] > 0.0 ? L - lr1 : lr1 - L;
-            } else {
-                ash = asinh(q[i] / rho);
-            }
-            psi[i] = q[i] * R[i] / (2.0 * r2) - 0.5 * ash;
-        }
-        const double a = as, b = e;
-        const double i00 = (R[0] - R[2] - R[1] + R[3]) / r2;
-        const double i10 = (b * (R[0] - R[2]) / r2 + psi[2] - psi[0]) - (a * (R[1] - R[3]) / r2 + psi[3] - psi[1]);
+        for (int i = 0; i < 4; ++i) psi[i] = 0.5 * (q[i] * R[i] * ir2 - A[i]);
+        const double i00 = (R[0] - R[2] - R[1] + R[3]) * ir2;
+        const double i10 = (e * (R[0] - R[2]) * ir2 + psi[2] - psi[0]) - (as * (R[1] - R[3]) * ir2 + psi[3] - psi[1]);
         const double i01 = i10 - t->das;  // int int (x' - x) / R^3 = -dk/das
         t->j1 = i10 - 0.5 * l1 * i00;
         t->j1b = i01 - (as + 0.5 * l2) * i00;
@@ -1171,7 +1153,8 @@ __global__ void __launch_bounds__(128) quad_classify_kernel(const DevFil *__rest
 // forms the pair's context itself; nothing is shared between warps, so a key
 // of some hundred points costs no block barrier and no idle setup.  At 4.6 M
 // keys of a graded spiral these rules on a CTA each (128 threads, one of them
-// setting up) took most of 236 ms; here 32 ms, and the tree's keys 24 ms.
+// setting up) took most of 236 ms; here 32 ms, and the tree's keys 24 ms
+// (the rules' points got cheaper since, line_terms).
 template <int kMode, bool kOrtho>
 __global__ void __launch_bounds__(128) quad_rule_kernel(const DevFil *__restrict__ fil,
                                                         const int4 *__restrict__ items,
@@ -2083,6 +2066,15 @@ struct CoordClass {
 
 __device__ __forceinline__ int bump_order(int o) { return o < kMaxRule - 1 ? o + 1 : o; }
 
+// Terms of a point sum per m x m points of a panel at which the panels' product
+// rule takes over for parallel pairs of two segments.  Measured on a graded
+// spiral of 3,672 filaments: 5.8 ns a key of that rule (four to nine panels of
+// 16 to 36 points) against 16 ns a pair of 5,000 terms (1.7 M of them, 8e9
+// terms, 27 to 31.5 ms): even at about 1,700 terms for nine panels of m = 4.
+// The rule is the more accurate one (1e-11 against the point orders' 1e-8
+// estimate).
+constexpr int kFarTerms = 120;
+
 __device__ CoordClass coord_classify(const DevFil &fi, const DevFil &fj, bool same) {
     CoordClass c{-1, 0, 0, 0, false};
     c.swap = canonical_greater(fi, fj);
@@ -2122,7 +2114,16 @@ __device__ CoordClass coord_classify(const DevFil &fi, const DevFil &fj, bool sa
     const double gap = separation(a, b);
     bool point = point_orders(a, gap, oa) && point_orders(b, gap, ob);
     if (point && oa[0] * oa[1] * oa[2] * ob[0] * ob[1] * ob[2] > 4096) point = false;
-    if (point) {
+    // A pair that the point rule could take goes by the panels' product rule
+    // where that is cheaper (kFarTerms) and its frame allows.
+    bool rule = false;
+    if (point && !same) {
+        const int m = far_rule_order(ab);
+        const int terms = bump_order(oa[0]) * bump_order(oa[1]) * bump_order(oa[2]) * bump_order(ob[0]) *
+                          bump_order(ob[1]) * bump_order(ob[2]);
+        rule = m > 0 && terms > kFarTerms * m * m;
+    }
+    if (point && !rule) {
         c.cat = kCoordCatPoint;
         c.orders = pack();
         c.flags = same ? kCoordSame : 0;
@@ -2147,6 +2148,11 @@ __device__ CoordClass coord_classify(const DevFil &fi, const DevFil &fj, bool sa
         if (fabs(d) < 1.0 - 1e-12 || fabs(a.axes[2]) > 1e-12 ||
             (fabs(ab.offset[1]) <= 0.5 * (ab.width[0] + ab.width[1]) &&
              fabs(ab.offset[2]) <= 0.5 * (ab.height[0] + ab.height[1]))) {
+            if (point) {
+                c.cat = kCoordCatPoint;
+                c.orders = pack();
+                return c;
+            }
             c.cat = -1;
             c.fail = FH_ERR_UNSUPPORTED;
             return c;
