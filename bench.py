@@ -410,7 +410,7 @@ def run_c3(args):
     out = {
         "metric": "batched Z(w) sweeps of 64 uneven spirals x 16 freqs: mixed+IR, s", "value": round(step, 6),
         "unit": "s", "n_gpus": 1, "steps": args.steps, "warmup": args.warmup, "ms_per_step": round(step * 1e3, 3),
-        "higher_is_better": False, "scaling": "weak", "vs_baseline": None, "dtype": "c64 (FP32 SIMT) + FP64 residual",
+        "higher_is_better": False, "scaling": "weak", "vs_baseline": None, "dtype": "c128 (FP64 tensor)",
         "data": "synthetic",
         "config": {"workload": WORKLOADS["c3"][0], "systems": len(systems),
                    "filaments_min": min(c["filaments"] for c in counts),
@@ -418,7 +418,7 @@ def run_c3(args):
                    "internal_meshes_min": min(c["internal_meshes"] for c in counts),
                    "internal_meshes_max": max(c["internal_meshes"] for c in counts),
                    "internal_meshes_total": sum(c["internal_meshes"] for c in counts),
-                   "items": sum(len(f) for f in freqs), "l2": "working sets of up to 4.3 MB per item; no flush"},
+                   "items": sum(len(f) for f in freqs), "l2": "working sets of up to 9.4 MB per item; no flush"},
         "launches_per_step": b["launches"], "kernel_ms": round(b["ms"], 3),
         "kernel_tflops": round(b["work"] / (b["ms"] * 1e-3) / 1e12, 2) if b["ms"] else None,
         "autotune": {"first_call_s": round(first_call_s, 3), "table": table},

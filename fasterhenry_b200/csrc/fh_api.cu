@@ -644,8 +644,8 @@ fh_status sweep_chunk_mixed(fh_system *s, const double *d_omega, int count, doub
 
 // fh_batch_sweep in a mixed precision: every (system, frequency) of the
 // systems with m <= FH_BATCH_MAX_ORDER in one persistent launch
-// (fh_batchsolve.cu), largest first; items whose refinement did not converge
-// are redone by the FP64 sweep.  Frequencies are checked per system first:
+// (fh_batchsolve.cu), largest first; items whose elimination without
+// interchanges was rejected are redone by the FP64 sweep.  Frequencies are checked per system first:
 // a system with an invalid frequency is left to the per-system path, which
 // reports it.  done[i] is set for the systems finished here.
 fh_status batch_sweep_persistent(fh_system *const *systems, size_t k, const double *const *freqs, const size_t *nf,
@@ -709,17 +709,23 @@ fh_status batch_sweep_persistent(fh_system *const *systems, size_t k, const doub
     std::vector<double> z((size_t)(2 * std::max<int64_t>(1, zoff.back())));
     std::vector<int32_t> status((size_t)std::max(1, nitems), 0);
     if (nitems > 0) {
-        const int ctas = std::min(batch_resident_ctas(), nitems);
+        int ctas = std::min(batch_resident_ctas(), nitems);
         const size_t slot = batch_slot_bytes(mmax, pmax);
         PBuf<unsigned char> d_items, d_z, d_status, d_counter, d_work;
         FHB_PALLOC(pool, d_items, kSlotBatchItems, sizeof(BatchItem) * items.size());
         FHB_PALLOC(pool, d_z, kSlotBatchZ, 8 * z.size());
         FHB_PALLOC(pool, d_status, kSlotBatchStatus, sizeof(int32_t) * status.size());
         FHB_PALLOC(pool, d_counter, kSlotBatchCounter, 16);
+        // a slot per CTA (18 MB at the order limit); fewer CTAs where memory is short
+        void *slots = nullptr;
+        while (ctas > 1 && pool.get(kSlotBatchWork, slot * (size_t)ctas, &slots) != cudaSuccess) {
+            cudaGetLastError();
+            ctas = (ctas + 1) / 2;
+        }
         FHB_PALLOC(pool, d_work, kSlotBatchWork, slot * (size_t)ctas);
         FHB_CUDA(cudaMemcpyAsync(d_items.p, items.data(), sizeof(BatchItem) * items.size(), cudaMemcpyHostToDevice, st));
         double work = 0.0;
-        for (const BatchItem &it : items) work += 8.0 / 3.0 * std::pow((double)sys[it.sys].m, 3.0);
+        for (const BatchItem &it : items) work += 4.0 / 3.0 * std::pow((double)(sys[it.sys].m + sys[it.sys].p), 3.0);
         prof_begin(st, FH_PROF_BATCH);
         fh_status e = batch_launch(reinterpret_cast<const BatchSys *>(d_sys.p),
                                    reinterpret_cast<const BatchItem *>(d_items.p), nitems,
@@ -733,7 +739,7 @@ fh_status batch_sweep_persistent(fh_system *const *systems, size_t k, const doub
                                  st));
         FHB_CUDA(cudaStreamSynchronize(st));
     }
-    // outputs; FP64 for the items that did not converge
+    // outputs; the FP64 sweep for the rejected items
     std::vector<size_t> item_of(items.size());
     for (size_t q = 0; q < items.size(); ++q) item_of[(size_t)items[q].index] = q;
     size_t idx = 0;

@@ -1,5 +1,5 @@
-// Batched mixed-precision sweeps of many small systems in one persistent
-// launch (fh_batchsolve.cu) and the autotuner that picks their tile shapes
+// Batched sweeps of many small systems in one persistent launch
+// (fh_batchsolve.cu) and the autotuner that picks their tile shapes
 // (fh_batchtune.cpp).
 #pragma once
 
@@ -30,18 +30,19 @@ struct BatchItem {
     int32_t pad = 0;
 };
 
-// Tile configurations: panel width NB x trailing tile TILE.
+// Tile configurations: tile edge, k per stage of the operands, stages held.
 constexpr int kBatchConfigs = 4;
-constexpr int kBatchNb[kBatchConfigs] = {16, 16, 32, 32};
-constexpr int kBatchTile[kBatchConfigs] = {32, 64, 32, 64};
+constexpr int kBatchEdge[kBatchConfigs] = {32, 32, 64, 64};
+constexpr int kBatchStage[kBatchConfigs] = {16, 32, 8, 16};
+constexpr int kBatchBuffers[kBatchConfigs] = {4, 2, 4, 2};
 
 size_t batch_smem_bytes();
 size_t batch_slot_bytes(int64_t mmax, int pmax);
 // Persistent CTAs that fit the device at once.
 int batch_resident_ctas();
 // One launch over all items (sorted by cost, largest first).  status[index]
-// receives the refinement iterations, or -1 for an item that must be redone
-// in FP64 (zero pivot, or refinement without convergence).
+// receives 0, or -1 for an item that must be redone with interchanges (zero
+// pivot, or too much growth).
 fh_status batch_launch(const BatchSys *d_systems, const BatchItem *d_items, int nitems, unsigned *d_counter,
                        void *d_work, size_t slot_bytes, int64_t mmax, int pmax, double2 *d_z, int32_t *d_status,
                        int ctas, cudaStream_t s, fh_error_info *err);

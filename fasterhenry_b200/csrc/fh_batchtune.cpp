@@ -1,13 +1,14 @@
 // The autotuner of the batched small-system solve (fh_batchsolve.cu): for
 // each order bucket (orders 128 (b - 1) < m <= 128 b) it times every tile
-// configuration (panel width NB x trailing tile TILE) on one item of the
+// configuration (tile edge and operand pipeline) on one item of the
 // first system that falls in the bucket -- one CTA, CUDA events, best of
 // two runs after a warm-up -- and keeps the fastest.  The table is kept in
 // a small JSON file per device name, so later processes skip the
 // measurement:
 //
-//   {"format": 1, "device": "<name>", "buckets": {"<b>": <config>, ...}}
+//   {"format": 1, "kernel": "ldlt", "device": "<name>", "buckets": {"<b>": <config>, ...}}
 //
+// A table of another kernel's configurations (an older file) is measured anew.
 // Path: $FH_AUTOTUNE_CACHE, else $XDG_CACHE_HOME/fasterhenry_b200/
 // batch_tiles.json, else $HOME/.cache/fasterhenry_b200/batch_tiles.json.
 // A file that cannot be read or written only costs the measurement.
@@ -45,6 +46,7 @@ std::string device_name() {
 
 // Parses this file's own format; anything else leaves the table empty.
 void parse(const std::string &text, const std::string &device, std::map<int, int> &out) {
+    if (text.find("\"kernel\": \"ldlt\"") == std::string::npos) return;
     const size_t d = text.find("\"device\"");
     if (d == std::string::npos) return;
     const size_t q0 = text.find('"', text.find(':', d) + 1);
@@ -79,7 +81,7 @@ void make_dirs(const std::string &path) {
 void save(const std::string &path) {
     make_dirs(path);
     std::ostringstream o;
-    o << "{\"format\": 1, \"device\": \"" << g_device << "\", \"buckets\": {";
+    o << "{\"format\": 1, \"kernel\": \"ldlt\", \"device\": \"" << g_device << "\", \"buckets\": {";
     bool first = true;
     for (const auto &kv : g_table) {
         o << (first ? "" : ", ") << "\"" << kv.first << "\": " << kv.second;

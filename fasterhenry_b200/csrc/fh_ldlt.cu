@@ -32,6 +32,7 @@
 #include <algorithm>
 
 #include "fh_device.cuh"
+#include "fh_ldlt.cuh"
 #include "fh_lu.cuh"
 
 namespace fhb {
@@ -42,25 +43,6 @@ constexpr int kLdPad = kLd + 2;       // row of a staged chunk: four k and two r
 constexpr int kLdK = 16;              // k per stage of the update
 constexpr int kLdThreads = 256;
 constexpr int kDiagThreads64 = 512;
-constexpr double kGrowthLimit = 128.0;  // on 1-norms of complex numbers, at most twice the moduli's product
-
-// m16n8k4: two stacked m8n8k4 fragments of A and C.
-__device__ __forceinline__ void dmma(double (&lo)[2], double (&hi)[2], double a0, double a1, double b) {
-    asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
-                 : "+d"(lo[0]), "+d"(lo[1]), "+d"(hi[0]), "+d"(hi[1])
-                 : "d"(a0), "d"(a1), "d"(b));
-}
-// base[at] to shared memory, or zeros when !live (the address is then base's).
-__device__ __forceinline__ void copy16(double2 *dst, const double2 *base, int64_t at, bool live) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(live ? base + at : base),
-                 "r"(live ? 16 : 0));
-}
-__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;"); }
-template <int N>
-__device__ __forceinline__ void copy_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N));
-}
 
 // A = R + j w L on the tiles on and below the diagonal, order M, and the
 // diagonal's 1-norms.
@@ -79,164 +61,16 @@ __global__ void __launch_bounds__(256) ldlt_form_kernel(const double *__restrict
     }
 }
 
-// y -= l t
-__device__ __forceinline__ void sub_mul(double2 &y, double2 l, double2 t) {
-    y.x -= l.x * t.x - l.y * t.y;
-    y.y -= l.x * t.y + l.y * t.x;
-}
-
-// The diagonal block [k0, k0 + nb)^2 of every matrix (one CTA each): L below
-// its diagonal and D on it, in place; L^-1 (unit lower, zeros above and
-// beyond nb) and D^-1.  Gauss-Jordan in one array: until step k place (i, k)
-// holds the Schur complement's entry, after it the entry of L^-1, which
-// starts as -l_ik; step j takes l_ij times v from row i, where v is row j of
-// L^-1 left of the pivot and column j of the complement beyond it.
-//
-// A warp owns the columns w + 16 c and its lanes the rows lane and lane + 32,
-// in registers (columns from 32 on only the lower rows); v goes through a
-// double buffer with one barrier per step, and rows at or above the pivot take
-// part with l = 0.  The steps run in four segments of 16, so that which of a
-// warp's columns lie left or right of the pivot is known at compile time.
-//
-// Bound by its chain of 64 steps of one barrier, one division and some forty
-// dependent instructions, at most one CTA per matrix: 38 us (88 us with a row
-// per thread, whose columns' cases diverge in every step).
-struct DiagBlock {
-    double2 lo[2], hi[4];  // rows lane and lane + 32 of column w + 16 c
-    double sum0, sum1;     // the rows' |l|^2 |d| over the block (warp 0)
-};
-template <int JC>
-__device__ __forceinline__ void diag_segment(DiagBlock &b, double2 (&v)[2][kLd], double2 *__restrict__ A, int64_t M,
-                                             int nb, int w, int lane, double2 *__restrict__ dinv,
-                                             int *__restrict__ failed) {
-    constexpr bool upper = JC < 2;  // pivots among the rows `lane`
-    const int r0 = lane, r1 = lane + 32;
-    for (int jw = 0; jw < 16; ++jw) {
-        const int j = 16 * JC + jw;
-        if (j >= nb) return;
-        double2 *vj = v[jw & 1];
-        // row j of L^-1 and column j of the complement
-        if (lane == (j & 31)) {
-#pragma unroll
-            for (int c = 0; c < JC; ++c) vj[w + 16 * c] = upper ? b.lo[c < 2 ? c : 0] : b.hi[c];
-            if (w < jw) vj[w + 16 * JC] = upper ? b.lo[upper ? JC : 0] : b.hi[JC];
-        }
-        if (w == jw) {
-            if (upper && r0 >= j) vj[r0] = b.lo[upper ? JC : 0];
-            if (r1 >= j) vj[r1] = b.hi[JC];
-        }
-        __syncthreads();
-        const double2 d = vj[j], q1 = vj[r1];
-        double2 q0 = make_double2(0.0, 0.0);
-        if (upper) q0 = vj[r0];
-        const double n = 1.0 / (d.x * d.x + d.y * d.y);
-        const double2 inv = make_double2(d.x * n, -d.y * n);
-        double2 l0 = make_double2(q0.x * inv.x - q0.y * inv.y, q0.x * inv.y + q0.y * inv.x);
-        double2 l1 = make_double2(q1.x * inv.x - q1.y * inv.y, q1.x * inv.y + q1.y * inv.x);
-        if (!upper || r0 <= j) l0 = make_double2(0.0, 0.0);
-        if (r1 <= j) l1 = make_double2(0.0, 0.0);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            if (c == JC && w == jw) {  // L's column, and the start of L^-1's
-                if (upper && r0 > j) {
-                    if (r0 < nb) A[r0 + (int64_t)j * M] = l0;
-                    b.lo[upper ? JC : 0] = make_double2(-l0.x, -l0.y);
-                }
-                if (r1 > j) {
-                    if (r1 < nb) A[r1 + (int64_t)j * M] = l1;
-                    b.hi[JC] = make_double2(-l1.x, -l1.y);
-                }
-            } else {
-                const double2 t = vj[w + 16 * c];
-                if (c < 2 && upper) sub_mul(b.lo[c < 2 ? c : 0], l0, t);
-                sub_mul(b.hi[c], l1, t);
-            }
-        }
-        if (w == 0) {
-            if (upper) b.sum0 += (fabs(q0.x) + fabs(q0.y)) * (fabs(l0.x) + fabs(l0.y));
-            b.sum1 += (fabs(q1.x) + fabs(q1.y)) * (fabs(l1.x) + fabs(l1.y));
-            if (r0 == j) b.sum0 += fabs(d.x) + fabs(d.y);
-            if (r1 == j) b.sum1 += fabs(d.x) + fabs(d.y);
-        }
-        if (w == 15 && lane == 0) {
-            A[j + (int64_t)j * M] = d;
-            dinv[j] = inv;
-            if (!isfinite(inv.x) || !isfinite(inv.y) || !isfinite(d.x) || !isfinite(d.y)) *failed = 1;
-        }
-    }
-}
-
+// The diagonal block [k0, k0 + nb)^2 of every matrix, one CTA each (DiagBlock).
 __global__ void __launch_bounds__(kDiagThreads64) ldlt_diag_kernel(double2 *__restrict__ a, int64_t M, int64_t k0,
                                                                    int nb, double2 *__restrict__ xinv,
                                                                    int64_t xinv_stride, double2 *__restrict__ dinv,
                                                                    double *__restrict__ growth,
                                                                    int *__restrict__ failed) {
-    static_assert(kLd == 64 && kDiagThreads64 == 512, "16 warps of four columns, two rows per lane");
-    __shared__ double2 v[2][kLd];
-    double2 *A = a + (int64_t)blockIdx.x * M * M + k0 + k0 * M;
-    double2 *X = xinv + (int64_t)blockIdx.x * xinv_stride, *D = dinv + (int64_t)blockIdx.x * kLd;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r0 = lane, r1 = lane + 32;
-    const double2 zero = make_double2(0.0, 0.0);
-    if (threadIdx.x < 2 * kLd) v[threadIdx.x / kLd][threadIdx.x % kLd] = zero;  // rows that no step publishes
-    DiagBlock b;
-    b.sum0 = b.sum1 = 0.0;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        const int k = w + 16 * c;
-        if (c < 2) b.lo[c < 2 ? c : 0] = r0 >= k && r0 < nb ? A[r0 + k * M] : zero;
-        b.hi[c] = r1 >= k && r1 < nb ? A[r1 + k * M] : zero;
-    }
-    __syncthreads();
-    diag_segment<0>(b, v, A, M, nb, w, lane, D, failed + blockIdx.x);
-    diag_segment<1>(b, v, A, M, nb, w, lane, D, failed + blockIdx.x);
-    diag_segment<2>(b, v, A, M, nb, w, lane, D, failed + blockIdx.x);
-    diag_segment<3>(b, v, A, M, nb, w, lane, D, failed + blockIdx.x);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        const int k = w + 16 * c;
-        X[r0 + k * kLd] = c < 2 && k < r0 && r0 < nb ? b.lo[c < 2 ? c : 0]
-                                                     : make_double2(r0 == k && r0 < nb ? 1.0 : 0.0, 0.0);
-        X[r1 + k * kLd] = k < r1 && r1 < nb ? b.hi[c] : make_double2(r1 == k && r1 < nb ? 1.0 : 0.0, 0.0);
-    }
-    if (w == 0) {
-        double *G = growth + (int64_t)blockIdx.x * M + k0;
-        if (r0 < nb) G[r0] += b.sum0;
-        if (r1 < nb) G[r1] += b.sum1;
-    }
-}
-
-// The fragments of one k4 step of a 64 x 64 tile: warp (wr, wc) owns rows
-// 32 wr .. +32 and columns 16 wc .. +16.  Fragment layout of m16n8k4 f64: A at
-// (rows g and g + 8, k t), B at (k t, column g), C at (rows g and g + 8,
-// columns 2 t, 2 t + 1), with g = lane / 4, t = lane % 4.  SIGN: +1 adds, -1 subtracts.
-template <int SIGN>
-__device__ __forceinline__ void tile_step(const double2 *__restrict__ l, const double2 *__restrict__ u, int wr, int wc,
-                                          int g, int t, double (&re)[4][2][2], double (&im)[4][2][2]) {
-    double2 lf[4], uf[2];
-#pragma unroll
-    for (int fm = 0; fm < 4; ++fm) {
-        lf[fm] = l[t * kLdPad + 32 * wr + 8 * fm + g];
-        if (SIGN < 0) lf[fm].x = -lf[fm].x;
-        else lf[fm].y = -lf[fm].y;
-    }
-#pragma unroll
-    for (int fn = 0; fn < 2; ++fn) uf[fn] = u[t * kLdPad + 16 * wc + 8 * fn + g];
-    // SIGN < 0: lf = (-l_re, l_im); SIGN > 0: lf = (l_re, -l_im)
-    // eight independent products between two on the same accumulator
-#pragma unroll
-    for (int fm = 0; fm < 4; fm += 2)
-#pragma unroll
-        for (int fn = 0; fn < 2; ++fn) {
-            dmma(re[fm][fn], re[fm + 1][fn], lf[fm].x, lf[fm + 1].x, uf[fn].x);
-            dmma(im[fm][fn], im[fm + 1][fn], lf[fm].x, lf[fm + 1].x, uf[fn].y);
-        }
-#pragma unroll
-    for (int fm = 0; fm < 4; fm += 2)
-#pragma unroll
-        for (int fn = 0; fn < 2; ++fn) {
-            dmma(re[fm][fn], re[fm + 1][fn], lf[fm].y, lf[fm + 1].y, uf[fn].y);
-            dmma(im[fm][fn], im[fm + 1][fn], -lf[fm].y, -lf[fm + 1].y, uf[fn].x);
-        }
+    __shared__ double2 v[2 * kLd];
+    DiagBlock<kLd, kDiagThreads64 / 32> block;
+    block.factor(v, a + (int64_t)blockIdx.x * M * M + k0 + k0 * M, M, nb, nb,
+                 xinv + (int64_t)blockIdx.x * xinv_stride, kLd, dinv + (int64_t)blockIdx.x * kLd, growth + (int64_t)blockIdx.x * M + k0, failed + blockIdx.x);
 }
 
 // Rows [c0, M) of the panel [k0, k0 + nb): B = A21 L11^-T into `panel`
@@ -271,7 +105,7 @@ __global__ void __launch_bounds__(kLdThreads, 2)
         if (kc == 0 || wc >= 2) {
 #pragma unroll 2
             for (int k4 = 0; k4 < 32; k4 += 4)
-                tile_step<1>(Ls + k4 * kLdPad, Us + k4 * kLdPad, wr, wc, g, t, re, im);
+                tile_step<1>(Ls + k4 * kLdPad, kLdPad, Us + k4 * kLdPad, kLdPad, 32 * wr, 16 * wc, g, t, re, im);
         }
     }
 #pragma unroll
@@ -360,7 +194,7 @@ __global__ void __launch_bounds__(kLdThreads, 2)
         const double2 *L = smem + (st & 1) * 2 * kLdK * kLdPad, *U = L + kLdK * kLdPad;
 #pragma unroll
         for (int k4 = 0; k4 < kLdK; k4 += 4)
-            tile_step<-1>(L + k4 * kLdPad, U + k4 * kLdPad, wr, wc, g, t, re, im);
+            tile_step<-1>(L + k4 * kLdPad, kLdPad, U + k4 * kLdPad, kLdPad, 32 * wr, 16 * wc, g, t, re, im);
         __syncthreads();  // before the stage after next overwrites this buffer
     }
 #pragma unroll

@@ -342,11 +342,11 @@ fh_status fh_sweep(fh_system *sys, const double *frequencies_hz, size_t nf, fh_p
  * frequencies freqs[i][0..nf[i]) into z_out[i] (nf[i] x p_i x p_i), as
  * fh_sweep would.  In the mixed precisions every (system, frequency) of the
  * systems with at most FH_BATCH_MAX_ORDER internal loops is solved in ONE
- * persistent launch (FP32 factors without interchanges, FP64-residual
- * refinement, work items largest first, tile shapes per order bucket from an
+ * persistent launch (FP64 factors without interchanges on the tensor
+ * instruction, work items largest first, tile shapes per order bucket from an
  * autotuner whose table is kept in a JSON file: $FH_AUTOTUNE_CACHE, else the
- * user's cache directory); an item whose refinement does not converge is
- * redone in FP64.  Larger systems, and every system in FP64, are swept as by
+ * user's cache directory); an item whose elimination grows too much is redone
+ * by fh_sweep in FP64.  Larger systems, and every system in FP64, are swept as by
  * fh_sweep, up to `concurrency` (<= 0: 4) at once on their own streams.  On
  * failure the first failing system (lowest index) is reported, its index in
  * fh_error_info.detail. */
@@ -506,6 +506,9 @@ fh_status fh_test_trailing_update(float *a, int64_t m, int32_t count, int64_t k0
  * of m (both complex), failed[f]: 1 where the elimination was rejected. */
 fh_status fh_test_mesh_solve(const double *r, const double *l, int64_t m, int64_t p, const double *omega,
                              int32_t count, double *z, double *x, int32_t *failed, fh_error_info *err);
+/* The same through the batched kernel, in one of its tile configurations. */
+fh_status fh_test_batch_solve(const double *r, const double *l, int64_t m, int64_t p, const double *omega,
+                              int32_t count, int32_t config, double *z, int32_t *failed, fh_error_info *err);
 
 /* ---- device-event profiler (no reference counterpart) ------------------ */
 
