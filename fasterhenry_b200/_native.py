@@ -250,7 +250,7 @@ def load():
     L.fh_test_mesh_solve.argtypes = [c_double_p, c_double_p, ctypes.c_int64, ctypes.c_int64, c_double_p,
                                      ctypes.c_int32, c_double_p, c_double_p, P(ctypes.c_int32), ei]
     L.fh_test_batch_solve.argtypes = [c_double_p, c_double_p, ctypes.c_int64, ctypes.c_int64, c_double_p,
-                                      ctypes.c_int32, ctypes.c_int32, c_double_p, P(ctypes.c_int32), ei]
+                                      ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, c_double_p, P(ctypes.c_int32), ei]
     L.fh_system_fill_stats.argtypes = [ctypes.c_void_p, P(FillStats)]
     L.fh_profile_enable.argtypes = [ctypes.c_int32]
     L.fh_profile_enable.restype = None

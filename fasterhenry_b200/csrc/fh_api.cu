@@ -725,10 +725,20 @@ fh_status batch_sweep_persistent(fh_system *const *systems, size_t k, const doub
         FHB_PALLOC(pool, d_work, kSlotBatchWork, slot * (size_t)ctas);
         FHB_CUDA(cudaMemcpyAsync(d_items.p, items.data(), sizeof(BatchItem) * items.size(), cudaMemcpyHostToDevice, st));
         double work = 0.0;
-        for (const BatchItem &it : items) work += 4.0 / 3.0 * std::pow((double)(sys[it.sys].m + sys[it.sys].p), 3.0);
+        auto cost = [&](const BatchItem &it) {
+            return 4.0 / 3.0 * std::pow((double)(sys[it.sys].m + sys[it.sys].p), 3.0);
+        };
+        for (const BatchItem &it : items) work += cost(it);
+        // An item of more than a CTA's even share of the work would set the
+        // time of the whole batch on its own: a group of CTAs takes it (64
+        // spirals of orders 56-736 x 16 frequencies: 3.8 ms from one share on;
+        // 3.7, 4.6 and 7.5 ms from 1.5, 2 and 3, 4.3 from half a share, 5.1
+        // with every item grouped, 7.5 with none).
+        int grouped = 0;
+        while (grouped < nitems && cost(items[(size_t)grouped]) > work / ctas) ++grouped;
         prof_begin(st, FH_PROF_BATCH);
         fh_status e = batch_launch(reinterpret_cast<const BatchSys *>(d_sys.p),
-                                   reinterpret_cast<const BatchItem *>(d_items.p), nitems,
+                                   reinterpret_cast<const BatchItem *>(d_items.p), nitems, grouped,
                                    reinterpret_cast<unsigned *>(d_counter.p), d_work.p, slot, mmax, pmax,
                                    reinterpret_cast<double2 *>(d_z.p), reinterpret_cast<int32_t *>(d_status.p), ctas,
                                    st, err);

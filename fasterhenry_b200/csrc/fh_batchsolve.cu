@@ -26,10 +26,16 @@
 // and writes a tile once; a trailing update per panel would also read and
 // write every C per panel, and the slots of all CTAs together exceed L2.
 //
-// 64 spirals of orders 56-736 x 16 frequencies on one B200: 7.8 ms, 7 of the
-// 37 TFLOP/s of the instruction, bound by the items of the largest orders,
-// which all start together and take a CTA for most of that time (the FP32
-// factors from the scalar pipes with FP64 refinement: 36 ms).
+// Items larger than a CTA's even share of the launch would set its time on
+// their own, so the leading ones are taken by clusters of CTAs: in block
+// column j the tiles go round, the first CTA starting with the diagonal block
+// while the others take the sums of theirs; one cluster barrier hands them
+// L_jj^-1, a second ends the column.
+//
+// 64 spirals of orders 56-736 x 16 frequencies on one B200: 3.8 ms, 14.5 of
+// the 37 TFLOP/s of the instruction, bound by the diagonal blocks' chains and
+// by few tiles per column (7.5 ms with a CTA for every item, 36 ms with FP32
+// factors from the scalar pipes and FP64 refinement).
 //
 // An item with a vanishing pivot or too much growth is marked; the host
 // redoes it with the FP64 sweep.  E and the depth of the operand pipeline come
@@ -56,7 +62,11 @@ struct Shared {
     BatchSys sys;
     BatchItem item;
     int next, bad;
+    int group, rank;  // CTAs on this item, and this one's place among them
 };
+
+__device__ __forceinline__ void group_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void group_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 
 // The tiling of a bordered matrix of m internal rows and p ports.
 struct Tiling {
@@ -76,8 +86,8 @@ struct Tiling {
 };
 
 template <int E, int KS, int BUFS>
-__device__ __forceinline__ void solve_item(double2 *tiles, double *growth, double2 *smem, Shared &sh, double2 *z_all,
-                                           int32_t *status) {
+__device__ __forceinline__ void solve_item(double2 *tiles, double *growth, double2 *dinv, double2 *smem, Shared &sh,
+                                           double2 *z_all, int32_t *status) {
     constexpr int kPad = E + 2;  // row of a staged chunk (bank offsets as in fh_ldlt.cu)
     constexpr int FM = E / 16, FN = E / 32;
     static_assert(BUFS * 2 * KS >= E, "the buffers also hold a whole tile");
@@ -97,13 +107,16 @@ __device__ __forceinline__ void solve_item(double2 *tiles, double *growth, doubl
         z[(int64_t)a * p + c] = v;
         z[(int64_t)c * p + a] = v;
     };
-    for (int i = tid; i < T * E; i += kBT) growth[i] = 0.0;
+    if (sh.rank == 0)
+        for (int i = tid; i < T * E; i += kBT) growth[i] = 0.0;
     if (tid == 0) sh.bad = 0;
     __syncthreads();
     for (int j = 0; j < T; ++j) {
         const int nb = min(E, max(0, mi - j * E));
         const int stages = min(j, tl.inner) * (E / KS);
-        for (int ti = j; ti < T; ++ti) {
+        bool joined = sh.group == 1 || nb == 0;  // past the wait for the diagonal block
+        if (!joined && sh.rank != 0) group_arrive();
+        for (int ti = j + sh.rank; ti < T; ti += sh.group) {
             auto load = [&](int st) {
                 if (st < stages) {
                     double2 *l = smem + (st % BUFS) * 2 * KS * kPad, *u = l + KS * kPad;
@@ -176,7 +189,7 @@ __device__ __forceinline__ void solve_item(double2 *tiles, double *growth, doubl
             __syncthreads();
             if (ti == j) {
                 DiagBlock<E, kBT / 32> block;
-                block.factor(sh.v, smem, kPad, E, nb, smem, kPad, sh.dinv, growth + j * E, &sh.bad);
+                block.factor(sh.v, smem, kPad, E, nb, smem, kPad, sh.dinv, sh.rowsum, &sh.bad);
                 __syncthreads();
                 if (nb < E) {  // the last tile ends with the ports
                     for (int idx = tid; idx < p * p; idx += kBT) {
@@ -186,8 +199,16 @@ __device__ __forceinline__ void solve_item(double2 *tiles, double *growth, doubl
                 } else {
                     double2 *x = tile(j, j);
                     for (int idx = tid; idx < E * E; idx += kBT) x[idx] = smem[idx / E * kPad + idx % E];
+                    if (tid < E) dinv[tid] = sh.dinv[tid];
                 }
+                if (!joined) group_arrive();
             } else {
+                if (!joined) {
+                    group_wait();
+                    joined = true;
+                    if (tid < E) sh.dinv[tid] = dinv[tid];
+                    __syncthreads();
+                }
                 // B = C X^T; X = L_jj^-1 is lower triangular: column c of B needs k <= c
                 const double2 *x = tile(j, j);
                 double bre[FM][FN][2] = {}, bim[FM][FN][2] = {};
@@ -216,50 +237,78 @@ __device__ __forceinline__ void solve_item(double2 *tiles, double *growth, doubl
                 }
             }
             __syncthreads();
-            if (ti > j && tid < E) growth[ti * E + tid] += sh.rowsum[tid];
+            if (tid < E) atomicAdd(&growth[ti * E + tid], sh.rowsum[tid]);
+        }
+        if (!joined) group_wait();
+        if (sh.group > 1) {  // the column is complete
+            group_arrive();
+            group_wait();
         }
     }
     __syncthreads();
+    if (sh.rank != 0) return;
     bool bad = sh.bad != 0;
     for (int i = tid; i < m; i += kBT)
-        bad = bad || !(growth[off + i] <= kGrowthLimit * (fabs(R[i + i * ld]) + fabs(w * L[i + i * ld])));
+        bad = bad || !(__ldcg(&growth[off + i]) <= kGrowthLimit * (fabs(R[i + i * ld]) + fabs(w * L[i + i * ld])));
     bad = __syncthreads_or(bad);
     if (tid == 0) status[sh.item.index] = bad ? -1 : 0;
 }
 
 template <int C>
-__device__ __forceinline__ void solve_config(double2 *tiles, double *growth, double2 *smem, Shared &sh,
-                                             double2 *z_all, int32_t *status) {
-    solve_item<kBatchEdge[C], kBatchStage[C], kBatchBuffers[C]>(tiles, growth, smem, sh, z_all, status);
+__device__ __forceinline__ void solve_config(double2 *tiles, double *growth, double2 *dinv, double2 *smem,
+                                             Shared &sh, double2 *z_all, int32_t *status) {
+    solve_item<kBatchEdge[C], kBatchStage[C], kBatchBuffers[C]>(tiles, growth, dinv, smem, sh, z_all, status);
 }
 
 __global__ void __launch_bounds__(kBT, 2)
-    batch_kernel(const BatchSys *__restrict__ systems, const BatchItem *__restrict__ items, int nitems,
-                 unsigned *counter, unsigned char *work, size_t slot_bytes, size_t tile_bytes, double2 *z_all,
-                 int32_t *status) {
+    batch_kernel(const BatchSys *__restrict__ systems, const BatchItem *__restrict__ items, int nitems, int grouped,
+                 unsigned *counter, unsigned char *work, size_t slot_bytes, size_t tile_bytes, size_t growth_bytes,
+                 int ctas, double2 *z_all, int32_t *status) {
     extern __shared__ __align__(16) unsigned char batch_smem[];
     __shared__ Shared sh;
-    unsigned char *base = work + (size_t)blockIdx.x * slot_bytes;
-    double2 *tiles = reinterpret_cast<double2 *>(base);
-    double *growth = reinterpret_cast<double *>(base + tile_bytes);
     double2 *smem = reinterpret_cast<double2 *>(batch_smem);
-    for (;;) {
+    const int rank = (int)blockIdx.x % kBatchGroup;
+    // the first `grouped` items by groups of CTAs (the clusters), then a CTA per item
+    for (int phase = grouped > 0 ? 0 : 1; phase < 2; ++phase) {
+        const int count = phase == 0 ? grouped : nitems - grouped;
+        if (phase == 1 && (int)blockIdx.x >= ctas) return;  // no slot
+        const size_t slot = blockIdx.x - (phase == 0 ? rank : 0);
+        unsigned char *base = work + slot * slot_bytes;
+        double2 *tiles = reinterpret_cast<double2 *>(base);
+        double *growth = reinterpret_cast<double *>(base + tile_bytes);
+        double2 *dinv = reinterpret_cast<double2 *>(base + tile_bytes + growth_bytes);
         if (threadIdx.x == 0) {
-            sh.next = (int)atomicAdd(counter, 1u);
-            if (sh.next < nitems) {
-                sh.item = items[sh.next];
+            sh.group = phase == 0 ? kBatchGroup : 1;
+            sh.rank = phase == 0 ? rank : 0;
+        }
+        for (;;) {
+            if (threadIdx.x == 0 && sh.rank == 0) sh.next = (int)atomicAdd(counter + phase, 1u);
+            if (phase == 0) {
+                group_arrive();
+                group_wait();
+                unsigned own = (unsigned)__cvta_generic_to_shared(&sh.next), first;
+                int next;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(first) : "r"(own));
+                asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(next) : "r"(first) : "memory");
+                group_arrive();  // the first CTA's `next` stays until all have read it
+                group_wait();
+                if (threadIdx.x == 0) sh.next = next;
+            }
+            if (threadIdx.x == 0 && sh.next < count) {
+                sh.item = items[sh.next + (phase == 0 ? 0 : grouped)];
                 sh.sys = systems[sh.item.sys];
             }
+            __syncthreads();
+            if (sh.next >= count) break;
+            switch (sh.item.cfg) {
+                case 0: solve_config<0>(tiles, growth, dinv, smem, sh, z_all, status); break;
+                case 1: solve_config<1>(tiles, growth, dinv, smem, sh, z_all, status); break;
+                case 2: solve_config<2>(tiles, growth, dinv, smem, sh, z_all, status); break;
+                default: solve_config<3>(tiles, growth, dinv, smem, sh, z_all, status); break;
+            }
+            __syncthreads();
         }
-        __syncthreads();
-        if (sh.next >= nitems) return;
-        switch (sh.item.cfg) {
-            case 0: solve_config<0>(tiles, growth, smem, sh, z_all, status); break;
-            case 1: solve_config<1>(tiles, growth, smem, sh, z_all, status); break;
-            case 2: solve_config<2>(tiles, growth, smem, sh, z_all, status); break;
-            default: solve_config<3>(tiles, growth, smem, sh, z_all, status); break;
-        }
-        __syncthreads();
+        __syncthreads();  // before the next phase's `group` and `rank`
     }
 }
 
@@ -288,30 +337,50 @@ size_t batch_smem_bytes() {
 
 size_t batch_slot_bytes(int64_t mmax, int pmax) {
     int64_t rows = 0;
-    const size_t bytes = tile_bytes(mmax, pmax, &rows) + sizeof(double) * (size_t)rows;
+    const size_t bytes = tile_bytes(mmax, pmax, &rows) + sizeof(double) * (size_t)rows + sizeof(double2) * 64;
     return (bytes + 255) / 256 * 256;
 }
 
-int batch_resident_ctas() {
-    int dev = 0, sms = 0, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)batch_smem_bytes());
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, batch_kernel, kBT, batch_smem_bytes());
-    return std::max(1, sms) * std::max(1, per);
+namespace {
+
+cudaLaunchConfig_t launch_config(int ctas, cudaLaunchAttribute *attr, cudaStream_t s) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3((unsigned)((ctas + kBatchGroup - 1) / kBatchGroup * kBatchGroup));
+    c.blockDim = dim3(kBT);
+    c.dynamicSmemBytes = batch_smem_bytes();
+    c.stream = s;
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = kBatchGroup;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    c.attrs = attr;
+    c.numAttrs = 1;
+    return c;
 }
 
-fh_status batch_launch(const BatchSys *d_systems, const BatchItem *d_items, int nitems, unsigned *d_counter,
-                       void *d_work, size_t slot_bytes, int64_t mmax, int pmax, double2 *d_z, int32_t *d_status,
-                       int ctas, cudaStream_t s, fh_error_info *err) {
+}  // namespace
+
+int batch_resident_ctas() {
+    int clusters = 0;
+    cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)batch_smem_bytes());
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t c = launch_config(kBatchGroup, &attr, nullptr);
+    if (cudaOccupancyMaxActiveClusters(&clusters, batch_kernel, &c) != cudaSuccess) cudaGetLastError();
+    return kBatchGroup * std::max(1, clusters);
+}
+
+fh_status batch_launch(const BatchSys *d_systems, const BatchItem *d_items, int nitems, int grouped,
+                       unsigned *d_counter, void *d_work, size_t slot_bytes, int64_t mmax, int pmax, double2 *d_z,
+                       int32_t *d_status, int ctas, cudaStream_t s, fh_error_info *err) {
     FHB_CUDA(cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)batch_smem_bytes()));
-    FHB_CUDA(cudaMemsetAsync(d_counter, 0, sizeof(unsigned), s));
+    FHB_CUDA(cudaMemsetAsync(d_counter, 0, 2 * sizeof(unsigned), s));
     int64_t rows = 0;
-    batch_kernel<<<ctas, kBT, batch_smem_bytes(), s>>>(d_systems, d_items, nitems, d_counter,
-                                                      static_cast<unsigned char *>(d_work), slot_bytes,
-                                                      tile_bytes(mmax, pmax, &rows), d_z, d_status);
-    FHB_CUDA(cudaGetLastError());
+    const size_t tb = tile_bytes(mmax, pmax, &rows);
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t c = launch_config(ctas, &attr, s);
+    FHB_CUDA(cudaLaunchKernelEx(&c, batch_kernel, d_systems, d_items, nitems, grouped, d_counter,
+                                static_cast<unsigned char *>(d_work), slot_bytes, tb, sizeof(double) * (size_t)rows,
+                                ctas, d_z, d_status));
     return FH_OK;
 }
 
@@ -320,10 +389,11 @@ fh_status batch_launch(const BatchSys *d_systems, const BatchItem *d_items, int 
 using namespace fhb;
 
 extern "C" fh_status fh_test_batch_solve(const double *r, const double *l, int64_t m, int64_t p, const double *omega,
-                                         int32_t count, int32_t config, double *z, int32_t *failed,
-                                         fh_error_info *err) {
+                                         int32_t count, int32_t config, int32_t grouped, double *z,
+                                         int32_t *failed, fh_error_info *err) {
     clear_error(err);
-    if (!r || !l || !omega || !z || !failed || m < 0 || p < 1 || count < 1 || config < 0 || config >= kBatchConfigs)
+    if (!r || !l || !omega || !z || !failed || m < 0 || p < 1 || count < 1 || config < 0 || config >= kBatchConfigs ||
+        grouped < 0 || grouped > count)
         return fail(err, FH_ERR_INVALID_ARGUMENT, "null argument, empty system or unknown configuration");
     fh_status st = ensure_device(err);
     if (st) return st;
@@ -337,7 +407,7 @@ extern "C" fh_status fh_test_batch_solve(const double *r, const double *l, int64
             for (int k = 0; k < 8; ++k) cudaFree(d[k]);
         }
     } release{d};
-    const size_t bytes[8] = {sym, sym, sizeof(BatchSys), sizeof(BatchItem) * (size_t)count, sizeof(unsigned),
+    const size_t bytes[8] = {sym, sym, sizeof(BatchSys), sizeof(BatchItem) * (size_t)count, 2 * sizeof(unsigned),
                              slot * (size_t)ctas, zs, 4 * (size_t)count};
     for (int k = 0; k < 8; ++k) FHB_CUDA(cudaMalloc(&d[k], bytes[k]));
     BatchSys sys;
@@ -353,7 +423,7 @@ extern "C" fh_status fh_test_batch_solve(const double *r, const double *l, int64
     FHB_CUDA(cudaMemcpy(d[1], l, sym, cudaMemcpyHostToDevice));
     FHB_CUDA(cudaMemcpy(d[2], &sys, sizeof sys, cudaMemcpyHostToDevice));
     FHB_CUDA(cudaMemcpy(d[3], items.data(), bytes[3], cudaMemcpyHostToDevice));
-    st = batch_launch((BatchSys *)d[2], (BatchItem *)d[3], count, (unsigned *)d[4], d[5], slot, m, (int)p,
+    st = batch_launch((BatchSys *)d[2], (BatchItem *)d[3], count, grouped, (unsigned *)d[4], d[5], slot, m, (int)p,
                       (double2 *)d[6], (int32_t *)d[7], ctas, nullptr, err);
     if (st) return st;
     FHB_CUDA(cudaMemcpy(z, d[6], zs, cudaMemcpyDeviceToHost));

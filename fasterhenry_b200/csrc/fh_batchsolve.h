@@ -35,17 +35,22 @@ constexpr int kBatchConfigs = 4;
 constexpr int kBatchEdge[kBatchConfigs] = {32, 32, 64, 64};
 constexpr int kBatchStage[kBatchConfigs] = {16, 32, 8, 16};
 constexpr int kBatchBuffers[kBatchConfigs] = {4, 2, 4, 2};
+// CTAs that share an item of the leading, grouped ones: a cluster (3.8 ms for
+// 64 spirals of orders 56-736 x 16 frequencies; clusters of 2 take 4.1, of 8
+// 4.8).
+constexpr int kBatchGroup = 4;
 
 size_t batch_smem_bytes();
 size_t batch_slot_bytes(int64_t mmax, int pmax);
 // Persistent CTAs that fit the device at once.
 int batch_resident_ctas();
-// One launch over all items (sorted by cost, largest first).  status[index]
+// One launch over all items (sorted by cost, largest first), the first
+// `grouped` of them by groups of CTAs; d_counter: two words.  status[index]
 // receives 0, or -1 for an item that must be redone with interchanges (zero
 // pivot, or too much growth).
-fh_status batch_launch(const BatchSys *d_systems, const BatchItem *d_items, int nitems, unsigned *d_counter,
-                       void *d_work, size_t slot_bytes, int64_t mmax, int pmax, double2 *d_z, int32_t *d_status,
-                       int ctas, cudaStream_t s, fh_error_info *err);
+fh_status batch_launch(const BatchSys *d_systems, const BatchItem *d_items, int nitems, int grouped,
+                       unsigned *d_counter, void *d_work, size_t slot_bytes, int64_t mmax, int pmax, double2 *d_z,
+                       int32_t *d_status, int ctas, cudaStream_t s, fh_error_info *err);
 
 // The autotuner's table: the best configuration per order bucket (orders
 // 128 (b - 1) < m <= 128 b), measured on this device on first use and kept

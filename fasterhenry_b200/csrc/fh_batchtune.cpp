@@ -142,7 +142,7 @@ fh_status BatchTuner::config_for(const BatchSys &sys, const BatchSys *d_sys_one,
     FHB_CUDA(cache_alloc(&items, sizeof(BatchItem), s));
     FHB_CUDA(cache_alloc(&z, sizeof(double2) * (size_t)pmax * pmax, s));
     FHB_CUDA(cache_alloc(&status, sizeof(int32_t), s));
-    FHB_CUDA(cache_alloc(&counter, sizeof(unsigned), s));
+    FHB_CUDA(cache_alloc(&counter, 2 * sizeof(unsigned), s));
     cudaEvent_t e0, e1;
     FHB_CUDA(cudaEventCreate(&e0));
     FHB_CUDA(cudaEventCreate(&e1));
@@ -164,8 +164,8 @@ fh_status BatchTuner::config_for(const BatchSys &sys, const BatchSys *d_sys_one,
         float ms = 1e30f;
         for (int rep = 0; rep < 3; ++rep) {
             FHB_CUDA(cudaEventRecord(e0, s));
-            fh_status st = batch_launch(d_sys_one, static_cast<BatchItem *>(items), 1, static_cast<unsigned *>(counter),
-                                        work, slot, mmax, pmax, static_cast<double2 *>(z),
+            fh_status st = batch_launch(d_sys_one, static_cast<BatchItem *>(items), 1, 0,
+                                        static_cast<unsigned *>(counter), work, slot, mmax, pmax, static_cast<double2 *>(z),
                                         static_cast<int32_t *>(status), 1, s, err);
             if (st) return st;
             FHB_CUDA(cudaEventRecord(e1, s));

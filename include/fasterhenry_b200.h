@@ -506,9 +506,11 @@ fh_status fh_test_trailing_update(float *a, int64_t m, int32_t count, int64_t k0
  * of m (both complex), failed[f]: 1 where the elimination was rejected. */
 fh_status fh_test_mesh_solve(const double *r, const double *l, int64_t m, int64_t p, const double *omega,
                              int32_t count, double *z, double *x, int32_t *failed, fh_error_info *err);
-/* The same through the batched kernel, in one of its tile configurations. */
+/* The same through the batched kernel, in one of its tile configurations, the
+ * first `grouped` frequencies by groups of CTAs. */
 fh_status fh_test_batch_solve(const double *r, const double *l, int64_t m, int64_t p, const double *omega,
-                              int32_t count, int32_t config, double *z, int32_t *failed, fh_error_info *err);
+                              int32_t count, int32_t config, int32_t grouped, double *z, int32_t *failed,
+                              fh_error_info *err);
 
 /* ---- device-event profiler (no reference counterpart) ------------------ */
 
