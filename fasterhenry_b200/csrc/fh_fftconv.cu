@@ -15,6 +15,21 @@
 //   4. axis 1 inverse  C[n0][m1][m2]  -> B[n0][n1][m2]
 //   5. axis 2 inverse  B[n0][n1][m2]  -> A[n0][n1][n2]   (the potentials)
 //
+// A thin grid (4 to 16 points along axis 2: a planar layout's thickness) is
+// not transformed along axis 2 at all.  With d the distance along it, the
+// kernel's two-axis spectrum K_d is real and the rest is y_i = sum_j K_|i-j|
+// x_j over n2 points, n2 products per point against two transforms of twice
+// the length:
+//
+//   1. axis 1 forward  A[n0][n1][n2]  -> C[n0][m1][n2]   (n0 n2 lines)
+//   2. axis 0 forward, the product along axis 2, axis 0 inverse, in place in C
+//      (m1 n2 lines): a tile is the n2 lines of one k1
+//   3. axis 1 inverse  C[n0][m1][n2]  -> A[n0][n1][n2]
+//
+// which transforms n2 lines where the five steps transform m2 >= 2 n2 - 1.
+// Above 16 points the tile outgrows a shared buffer of two CTAs per SM; up to
+// 3 the lines of a tile are shorter than a 32-byte sector.
+//
 // Each step is one launch.  What bounds a step is the shared-memory traffic
 // and the latency of its butterflies, not the device memory, so:
 //   * a length is cut into as few stages as possible (radices up to 16 in
@@ -35,6 +50,9 @@
 // with two buffers that came before:
 //   FP32   45 + 115 + 309 + 104 + 58 =  631   (104 + 284 + 1008 + 290 + 101)
 //   FP64  110 + 182 + 511 + 178 + 129 = 1110
+// and the thin form's three steps on the same grid:
+//   FP32   47 + 185 + 54 = 287      FP64   89 + 356 + 97 = 542
+// (300 x 300 x 16 sources, 600 x 600 x 32: 163 and 321).
 // FP32 issues instructions in 0.6 of the cycles (packed FP32 arithmetic, see
 // cadd; twiddles in rows of 16-byte loads) at 32 warps per SM; 256 and 384
 // threads per CTA measured within 5 %.
@@ -65,6 +83,7 @@ constexpr int fft_threads() {
     return sizeof(T) == 4 ? 512 : 256;
 }
 constexpr size_t kFftSmemBudget = 110 * 1024;  // two CTAs per SM
+constexpr size_t kFftSmemMost = 227 * 1024;
 constexpr int kFftTilePoints = 8192;
 constexpr double kPi = 3.14159265358979323846;
 
@@ -297,6 +316,14 @@ __device__ __forceinline__ void twiddle(double2 (&v)[R], const double2 *__restri
     for (int r = 1; r < R; ++r) v[r] = cmul(v[r], __ldg(row + r));
 }
 
+// Where a tile's element (point t, line l) lies in the shared buffer, and which
+// runs fastest over the threads.
+enum Layout {
+    kStrided,  // t 2^lg + l, lines first
+    kContig,   // l pitch + t, points first
+    kThin      // l pitch + t, lines first (any number of lines)
+};
+
 // Where a tile's lines lie in device memory.
 template <class V>
 struct Lines {
@@ -305,27 +332,31 @@ struct Lines {
     int inner;
     int count;      // lines of this tile
     int n_in, keep; // points read, points written; the rest is zero
+    unsigned magic; // of count (kThin)
 };
 
 // One stage of radix R = ax.R[st] over the tile's lines: point b R S + k + r S
-// of every block b, offset k, by one thread.  Element (point t, line l) of the
-// shared buffer is t * 2^lg + l (kContig: l * pitch + t).
+// of every block b, offset k, by one thread.
 //   DIT = false: DFT then twiddle (forward); true: twiddle then DFT (inverse).
 //   GIN / GOUT: from / to device memory instead of the buffer.
 //   MID: the forward's last stage, the spectrum and the inverse's first.
-template <int R, class T, bool CONTIG, bool DIT, bool GIN, bool GOUT, bool MID>
+template <int R, class T, int LAYOUT, bool DIT, bool GIN, bool GOUT, bool MID>
 __device__ __forceinline__ void fft_stage(typename Cplx<T>::type *buf, const FftAxis &ax, int st, int lg, int pitch,
                                           const typename Cplx<T>::type *__restrict__ tw_all,
                                           const Lines<typename Cplx<T>::type> &g, const T *__restrict__ spectrum) {
     using V = typename Cplx<T>::type;
     const int S = ax.S[st], nb = ax.m / R;
     const V *__restrict__ tw = tw_all + ax.tw[st];
-    const int total = nb << lg;
+    const int total = LAYOUT == kThin ? nb * g.count : nb << lg;
+    auto at = [&](int t, int l) { return LAYOUT == kStrided ? (t << lg) + l : l * pitch + t; };
     for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
         int l, j;
-        if (CONTIG) {
+        if (LAYOUT == kContig) {
             l = fast_div(idx, ax.magic_nb[st]);
             j = idx - l * nb;
+        } else if (LAYOUT == kThin) {
+            j = fast_div(idx, g.magic);
+            l = idx - j * g.count;
         } else {
             l = idx & ((1 << lg) - 1);
             j = idx >> lg;
@@ -334,7 +365,7 @@ __device__ __forceinline__ void fft_stage(typename Cplx<T>::type *buf, const Fft
         const int k = j - b * S;
         const int t0 = b * R * S + k;
         V v[R];
-        const bool live = CONTIG || l < g.count;
+        const bool live = LAYOUT != kStrided || l < g.count;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const int t = t0 + r * S;
@@ -343,7 +374,7 @@ __device__ __forceinline__ void fft_stage(typename Cplx<T>::type *buf, const Fft
                 if (live && t < g.n_in) v[r] = g.src[t * g.inner + l];
                 if (DIT) v[r] = cswap(v[r]);
             } else {
-                v[r] = buf[CONTIG ? l * pitch + t : (t << lg) + l];
+                v[r] = buf[at(t, l)];
             }
         }
         if (DIT && S > 1) twiddle<R>(v, tw + k * twiddle_row(R));
@@ -363,13 +394,13 @@ __device__ __forceinline__ void fft_stage(typename Cplx<T>::type *buf, const Fft
             if (GOUT) {
                 if (live && t < g.keep) g.dst[t * g.inner + l] = DIT || MID ? cswap(v[r]) : v[r];
             } else {
-                buf[CONTIG ? l * pitch + t : (t << lg) + l] = v[r];
+                buf[at(t, l)] = v[r];
             }
         }
     }
 }
 
-template <class T, bool CONTIG, bool DIT, bool GIN, bool GOUT, bool MID>
+template <class T, int LAYOUT, bool DIT, bool GIN, bool GOUT, bool MID>
 __device__ __forceinline__ void fft_stage_any(typename Cplx<T>::type *buf, const FftAxis &ax, int st, int lg,
                                               int pitch, const typename Cplx<T>::type *__restrict__ tw,
                                               const Lines<typename Cplx<T>::type> &g,
@@ -377,7 +408,7 @@ __device__ __forceinline__ void fft_stage_any(typename Cplx<T>::type *buf, const
     switch (ax.R[st]) {
 #define FHB_FFT_RADIX(r)                                                                             \
     case r:                                                                                          \
-        fft_stage<r, T, CONTIG, DIT, GIN, GOUT, MID>(buf, ax, st, lg, pitch, tw, g, spectrum);       \
+        fft_stage<r, T, LAYOUT, DIT, GIN, GOUT, MID>(buf, ax, st, lg, pitch, tw, g, spectrum);       \
         break;
         FHB_FFT_RADIX(1)
         FHB_FFT_RADIX(2)
@@ -392,15 +423,18 @@ __device__ __forceinline__ void fft_stage_any(typename Cplx<T>::type *buf, const
         default:
             if constexpr (sizeof(T) == 4) {
                 if (ax.R[st] == 15)
-                    fft_stage<15, T, CONTIG, DIT, GIN, GOUT, MID>(buf, ax, st, lg, pitch, tw, g, spectrum);
+                    fft_stage<15, T, LAYOUT, DIT, GIN, GOUT, MID>(buf, ax, st, lg, pitch, tw, g, spectrum);
                 else
-                    fft_stage<16, T, CONTIG, DIT, GIN, GOUT, MID>(buf, ax, st, lg, pitch, tw, g, spectrum);
+                    fft_stage<16, T, LAYOUT, DIT, GIN, GOUT, MID>(buf, ax, st, lg, pitch, tw, g, spectrum);
             }
 #undef FHB_FFT_RADIX
     }
 }
 
 enum FftKind { kForward, kInverse, kFused };
+
+// Axis 2 of at least kThinLeast and at most kThinMost points: the thin form.
+constexpr int kThinLeast = 4, kThinMost = 16;
 
 // One pruned axis transform over a batch of arrays.  An array holds
 // `outer` x len x `inner` complex elements (len = n_in for the input, keep
@@ -431,26 +465,26 @@ __global__ void __launch_bounds__(fft_threads<T>(), 2)
         g.dst = out + (int64_t)blockIdx.y * out_stride + o * keep * inner + c0;
         const T *spec = KIND == kFused ? spectrum + c0 : nullptr;
         if (last == 0) {
-            fft_stage_any<T, false, KIND == kInverse, true, true, KIND == kFused>(buf, ax, 0, lg, 0, tw, g, spec);
+            fft_stage_any<T, kStrided, KIND == kInverse, true, true, KIND == kFused>(buf, ax, 0, lg, 0, tw, g, spec);
             continue;
         }
         if (KIND != kInverse) {
-            fft_stage_any<T, false, false, true, false, false>(buf, ax, 0, lg, 0, tw, g, spec);
+            fft_stage_any<T, kStrided, false, true, false, false>(buf, ax, 0, lg, 0, tw, g, spec);
             for (int st = 1; st < last; ++st) {
                 __syncthreads();
-                fft_stage_any<T, false, false, false, false, false>(buf, ax, st, lg, 0, tw, g, spec);
+                fft_stage_any<T, kStrided, false, false, false, false>(buf, ax, st, lg, 0, tw, g, spec);
             }
             __syncthreads();
-            fft_stage_any<T, false, false, false, KIND == kForward, KIND == kFused>(buf, ax, last, lg, 0, tw, g, spec);
+            fft_stage_any<T, kStrided, false, false, KIND == kForward, KIND == kFused>(buf, ax, last, lg, 0, tw, g, spec);
         }
         if (KIND != kForward) {
-            if (KIND == kInverse) fft_stage_any<T, false, true, true, false, false>(buf, ax, last, lg, 0, tw, g, spec);
+            if (KIND == kInverse) fft_stage_any<T, kStrided, true, true, false, false>(buf, ax, last, lg, 0, tw, g, spec);
             for (int st = last - 1; st > 0; --st) {
                 __syncthreads();
-                fft_stage_any<T, false, true, false, false, false>(buf, ax, st, lg, 0, tw, g, spec);
+                fft_stage_any<T, kStrided, true, false, false, false>(buf, ax, st, lg, 0, tw, g, spec);
             }
             __syncthreads();
-            fft_stage_any<T, false, true, false, true, false>(buf, ax, 0, lg, 0, tw, g, spec);
+            fft_stage_any<T, kStrided, true, false, true, false>(buf, ax, 0, lg, 0, tw, g, spec);
         }
         __syncthreads();  // the next tile's first stage writes the buffer
     }
@@ -488,7 +522,7 @@ __global__ void __launch_bounds__(fft_threads<T>(), 2)
                 buf[count * pitch + idx] = cmake((T)0, (T)0);
         for (int k = 0; k < ax.nst; ++k) {
             __syncthreads();
-            fft_stage_any<T, true, KIND == kInverse, false, false, false>(
+            fft_stage_any<T, kContig, KIND == kInverse, false, false, false>(
                 buf, ax, KIND == kInverse ? ax.nst - 1 - k : k, lg, pitch, tw, none, nullptr);
         }
         __syncthreads();
@@ -498,6 +532,86 @@ __global__ void __launch_bounds__(fft_threads<T>(), 2)
             dst[idx] = KIND == kInverse ? cswap(v) : v;
         }
         __syncthreads();  // the next tile's loads write the buffer
+    }
+}
+
+// y_i = sum_j K_|i-j| x_j along axis 2 at every point of a tile of n2 <= N
+// lines, in place, swapped (the inverse begins).  K: [d][m].
+template <int N, class T>
+__device__ __forceinline__ void thin_product(typename Cplx<T>::type *buf, int pitch, int n2, int m,
+                                             const T *__restrict__ K) {
+    using V = typename Cplx<T>::type;
+    for (int t = threadIdx.x; t < m; t += blockDim.x) {
+        V x[N];
+        T k[N];
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            x[i] = i < n2 ? buf[i * pitch + t] : cmake((T)0, (T)0);
+            k[i] = i < n2 ? __ldg(K + i * m + t) : (T)0;
+        }
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            V y = cscale(k[i], x[0]);
+#pragma unroll
+            for (int j = 1; j < N; ++j) y = caxpy(k[i > j ? i - j : j - i], x[j], y);
+            if (i < n2) buf[i * pitch + t] = cswap(y);
+        }
+    }
+}
+
+// The strided steps of a thin grid: a tile is the n2 lines of one (i, j), whole
+// in the buffer.  kFused: forward along axis 0, the product along axis 2 with
+// K[k1][d][k0], and back.
+template <class T, int KIND>
+__global__ void __launch_bounds__(2 * fft_threads<T>(), 1)
+    fft_thin_kernel(const typename Cplx<T>::type *in, typename Cplx<T>::type *out, int64_t in_stride,
+                    int64_t out_stride, int64_t tiles, int64_t in_tile, int64_t out_tile, int inner, int n2,
+                    unsigned magic_n2, int n_in, int keep, FftAxis ax, int pitch,
+                    const typename Cplx<T>::type *__restrict__ tw, const T *__restrict__ K) {
+    using V = typename Cplx<T>::type;
+    extern __shared__ __align__(16) unsigned char fft_smem[];
+    V *buf = reinterpret_cast<V *>(fft_smem);
+    const int last = ax.nst - 1;
+    for (int64_t tt = blockIdx.x; tt < tiles; tt += gridDim.x) {
+        Lines<V> g;
+        g.inner = inner;
+        g.count = n2;
+        g.magic = magic_n2;
+        g.n_in = n_in;
+        g.keep = keep;
+        g.src = in + (int64_t)blockIdx.y * in_stride + tt * in_tile;
+        g.dst = out + (int64_t)blockIdx.y * out_stride + tt * out_tile;
+        if (KIND != kFused && last == 0) {
+            fft_stage_any<T, kThin, KIND == kInverse, true, true, false>(buf, ax, 0, 0, pitch, tw, g, nullptr);
+            continue;
+        }
+        if (KIND != kInverse) {
+            fft_stage_any<T, kThin, false, true, false, false>(buf, ax, 0, 0, pitch, tw, g, nullptr);
+            for (int st = 1; st < (KIND == kFused ? last + 1 : last); ++st) {
+                __syncthreads();
+                fft_stage_any<T, kThin, false, false, false, false>(buf, ax, st, 0, pitch, tw, g, nullptr);
+            }
+            __syncthreads();
+            if (KIND == kForward)
+                fft_stage_any<T, kThin, false, false, true, false>(buf, ax, last, 0, pitch, tw, g, nullptr);
+        }
+        if (KIND == kFused) {
+            const T *k = K + tt * n2 * ax.m;
+            if (n2 <= 8) thin_product<8>(buf, pitch, n2, ax.m, k);
+            else thin_product<kThinMost>(buf, pitch, n2, ax.m, k);
+            __syncthreads();
+        }
+        if (KIND != kForward) {
+            if (KIND == kInverse)
+                fft_stage_any<T, kThin, true, true, false, false>(buf, ax, last, 0, pitch, tw, g, nullptr);
+            for (int st = KIND == kFused ? last : last - 1; st > 0; --st) {
+                if (KIND == kInverse || st < last) __syncthreads();
+                fft_stage_any<T, kThin, true, false, false, false>(buf, ax, st, 0, pitch, tw, g, nullptr);
+            }
+            if (last > 0) __syncthreads();
+            fft_stage_any<T, kThin, true, false, true, false>(buf, ax, 0, 0, pitch, tw, g, nullptr);
+        }
+        __syncthreads();  // the next tile's first stage writes the buffer
     }
 }
 
@@ -543,6 +657,19 @@ __global__ void spectrum_store_kernel(const double2 *__restrict__ in, T *__restr
     }
 }
 
+// The spectrum of a thin grid, [k1][d][k0]: the kernel's distances d along
+// axis 2 as they are, in the convolution's order along axes 0 and 1.
+template <class T>
+__global__ void thin_store_kernel(const double2 *__restrict__ in, T *__restrict__ out, int64_t m0, int64_t m1,
+                                  int64_t n2, const int *__restrict__ map) {
+    const int64_t total = m0 * m1 * n2;
+    const double scale = 1.0 / (double)(m0 * m1);
+    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < total; p += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = p % m0, rest = p / m0, d = rest % n2, j = rest / n2;
+        out[p] = (T)(in[((int64_t)map[i] * m1 + map[m0 + j]) * n2 + d].x * scale);
+    }
+}
+
 unsigned blocks_of(int64_t work, int threads, int64_t cap = 148 * 16) {
     return (unsigned)std::max<int64_t>(1, std::min<int64_t>((work + threads - 1) / threads, cap));
 }
@@ -574,7 +701,7 @@ fh_status axis_step(const void *in, void *out, int64_t in_stride, int64_t out_st
     using V = typename Cplx<T>::type;
     const int lg = tile_lg<T>(ax.m, inner);
     const size_t smem = sizeof(V) * ((size_t)(ax.m | 1) << lg);
-    if (smem > 227 * 1024)
+    if (smem > kFftSmemMost)
         return fail(err, FH_ERR_PFFT, "pFFT convolution: axis length " + std::to_string(ax.m) +
                                           " does not fit the transform kernel's shared memory");
     const int64_t tiles = inner == 1 && KIND != kFused ? (outer + (1 << lg) - 1) >> lg
@@ -597,6 +724,41 @@ fh_status axis_step(const void *in, void *out, int64_t in_stride, int64_t out_st
             static_cast<const V *>(in), static_cast<V *>(out), in_stride, out_stride, outer, (int)inner, n_in, keep, ax,
             lg, static_cast<const V *>(tw), spectrum);
     }
+    FHB_CUDA(cudaGetLastError());
+    return FH_OK;
+}
+
+// Points between two lines of a thin tile: 16 lanes (8 in FP64) of a
+// shared-memory access are n2 lines times a few consecutive points, which this
+// spreads over all banks.
+template <class T>
+int thin_pitch(int m, int64_t n2) {
+    const int lanes = sizeof(T) == 4 ? 16 : 8;
+    const int step = (int)std::max<int64_t>(1, (lanes + n2 - 1) / n2);
+    return (m + lanes - 1) / lanes * lanes + step;
+}
+template <class T>
+size_t thin_smem(int m, int64_t n2) {
+    return sizeof(typename Cplx<T>::type) * (size_t)thin_pitch<T>(m, n2) * (size_t)n2;
+}
+template <class T>
+bool thin_grid(const FftConvShape &sh) {
+    return sh.n[2] >= kThinLeast && sh.n[2] <= kThinMost &&
+           thin_smem<T>((int)std::max(sh.m[0], sh.m[1]), sh.n[2]) <= kFftSmemMost;
+}
+
+template <class T, int KIND>
+fh_status thin_step(const void *in, void *out, int64_t in_stride, int64_t out_stride, int64_t tiles, int64_t in_tile,
+                    int64_t out_tile, int64_t inner, int64_t n2, int n_in, int keep, const FftAxis &ax,
+                    const void *tw, const T *K, int batch, cudaStream_t s, fh_error_info *err) {
+    using V = typename Cplx<T>::type;
+    const size_t smem = thin_smem<T>(ax.m, n2);
+    // two CTAs per SM, or one of twice the threads
+    const int threads = fft_threads<T>() * (smem > kFftSmemBudget ? 2 : 1);
+    FHB_CUDA(cudaFuncSetAttribute(fft_thin_kernel<T, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    fft_thin_kernel<T, KIND><<<dim3((unsigned)std::min<int64_t>(tiles, 148 * 8), (unsigned)batch), threads, smem, s>>>(
+        static_cast<const V *>(in), static_cast<V *>(out), in_stride, out_stride, tiles, in_tile, out_tile, (int)inner,
+        (int)n2, magic_of((int)n2), n_in, keep, ax, thin_pitch<T>(ax.m, n2), static_cast<const V *>(tw), K);
     FHB_CUDA(cudaGetLastError());
     return FH_OK;
 }
@@ -745,10 +907,32 @@ fh_status fftconv_setup(const FftConvShape &sh, double spacing, FftConvTables &t
         }
     } release{grid, tmp, d_map, s};
     FHB_CUDA(cudaMemcpyAsync(d_map, map.data(), sizeof(int) * map.size(), cudaMemcpyHostToDevice, s));
+    const int64_t m0 = sh.m[0], m1 = sh.m[1], m2 = sh.m[2], n2 = sh.n[2];
+    tab.shape = sh;
+    tab.fp32 = fp32;
+    if (thin_grid<T>(sh)) {
+        wrapped_kernel_kernel<<<blocks_of(m0 * m1 * n2, 256), 256, 0, s>>>(grid, sh.n[0], sh.n[1], n2, m0, m1, n2,
+                                                                          spacing);
+        FHB_CUDA(cudaGetLastError());
+        fh_status e = axis_step<double, kForward>(grid, tmp, 0, 0, m0, n2, (int)m1, (int)m1, ax64[1], tab.tw64[1],
+                                                  nullptr, 1, s, err);
+        if (!e)
+            e = axis_step<double, kForward>(tmp, grid, 0, 0, 1, m1 * n2, (int)m0, (int)m0, ax64[0], tab.tw64[0],
+                                            nullptr, 1, s, err);
+        if (e) return e;
+        FHB_CUDA(cache_alloc(&tab.thin, sizeof(T) * (size_t)(m0 * m1 * n2), s));
+        thin_store_kernel<T><<<blocks_of(m0 * m1 * n2, 256), 256, 0, s>>>(grid, static_cast<T *>(tab.thin), m0, m1, n2,
+                                                                          d_map);
+        FHB_CUDA(cudaGetLastError());
+        if (!fp32) {
+            FHB_CUDA(cudaStreamSynchronize(s));
+            return FH_OK;
+        }
+        // the port columns of an FP32 operator take the whole spectrum
+    }
     wrapped_kernel_kernel<<<blocks_of(P, 256), 256, 0, s>>>(grid, sh.n[0], sh.n[1], sh.n[2], sh.m[0], sh.m[1],
                                                            sh.m[2], spacing);
     FHB_CUDA(cudaGetLastError());
-    const int64_t m0 = sh.m[0], m1 = sh.m[1], m2 = sh.m[2];
     fh_status e = axis_step<double, kForward>(grid, tmp, 0, 0, m0 * m1, 1, (int)m2, (int)m2, ax64[2], tab.tw64[2],
                                               nullptr, 1, s, err);
     if (!e)
@@ -763,8 +947,6 @@ fh_status fftconv_setup(const FftConvShape &sh, double spacing, FftConvTables &t
                                                                d_map);
     FHB_CUDA(cudaGetLastError());
     FHB_CUDA(cudaStreamSynchronize(s));
-    tab.shape = sh;
-    tab.fp32 = sizeof(T) == 4;
     return FH_OK;
 }
 
@@ -777,6 +959,20 @@ fh_status fftconv_run(const FftConvTables &tab, void *work, int grids, cudaStrea
     V *A = static_cast<V *>(work);
     V *B = A + sa * grids;
     V *C = B + sb * grids;
+    if (tab.thin) {
+        const T *K = static_cast<const T *>(tab.thin);
+        C = A + sa * grids;
+        const int64_t st = n0 * m1 * n2;
+        fh_status e = thin_step<T, kForward>(A, C, sa, st, n0, n1 * n2, m1 * n2, n2, n2, (int)n1, (int)m1, tab.axis[1],
+                                             tab.tw[1], nullptr, grids, s, err);
+        if (!e)
+            e = thin_step<T, kFused>(C, C, st, st, m1, n2, n2, m1 * n2, n2, (int)n0, (int)n0, tab.axis[0], tab.tw[0],
+                                     K, grids, s, err);
+        if (!e)
+            e = thin_step<T, kInverse>(C, A, st, sa, n0, m1 * n2, n1 * n2, n2, n2, (int)m1, (int)n1, tab.axis[1],
+                                       tab.tw[1], nullptr, grids, s, err);
+        return e;
+    }
     const T *spec = static_cast<const T *>(tab.spectrum);
     fh_status e = axis_step<T, kForward>(A, B, sa, sb, n0 * n1, 1, (int)n2, (int)m2, tab.axis[2], tab.tw[2], nullptr,
                                          grids, s, err);
@@ -802,7 +998,8 @@ void fftconv_free(FftConvTables &tab, cudaStream_t s) {
         tab.tw[a] = tab.tw64[a] = nullptr;
     }
     if (tab.spectrum) cache_free(tab.spectrum, s);
-    tab.spectrum = nullptr;
+    if (tab.thin) cache_free(tab.thin, s);
+    tab.spectrum = tab.thin = nullptr;
 }
 
 template fh_status fftconv_setup<float>(const FftConvShape &, double, FftConvTables &, cudaStream_t, fh_error_info *);

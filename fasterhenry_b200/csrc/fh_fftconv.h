@@ -47,12 +47,16 @@ struct FftConvTables {
     void *tw[3] = {nullptr, nullptr, nullptr};
     void *tw64[3] = {nullptr, nullptr, nullptr};
     void *spectrum = nullptr;
+    // A thin grid's spectrum over axes 0 and 1 only (times 1 / (m0 m1)), laid
+    // out [k1][distance along axis 2][k0]; FP64 tables then have no `spectrum`.
+    void *thin = nullptr;
     bool fp32 = false;
 };
 
 // Complex elements of the work buffer per complex grid: the sources /
 // potentials A (n0 n1 n2), then B (n0 n1 m2), then C (n0 m1 m2); a batch of
-// grids keeps each part contiguous per grid (A of every grid first).
+// grids keeps each part contiguous per grid (A of every grid first).  (The thin
+// form has no B and n0 m1 n2 for C.)
 size_t fftconv_work_elems(const FftConvShape &sh);
 
 // T = float or double: the precision of the convolution.

@@ -347,7 +347,8 @@ fh_status pfft_build(const fh_filament *fil, int64_t n, const PfftConfig &cfg, v
 // each), the vectors, and per complex grid (element size E: 8 B in FP32, 16 B
 // in FP64) the pruned transform chain of fh_fftconv.cu: the sources A written
 // and read, B = n0 n1 m2 and C = n0 m1 m2 written and read twice each, the
-// spectrum (P reals), and the potentials A written and read.
+// spectrum (P reals), and the potentials A written and read.  The thin form
+// has no B, C = n0 m1 n2 and m0 m1 n2 reals of spectrum.
 double pfft_apply_bytes(const PfftDevice &op, int count, PfftProduct kind) {
     const int ncomp = (int)op.components.size();
     const double grids = (double)((count * ncomp + 1) / 2);
@@ -355,7 +356,11 @@ double pfft_apply_bytes(const PfftDevice &op, int count, PfftProduct kind) {
     const FftConvShape &sh = op.conv.shape;
     const double A = (double)sh.n[0] * sh.n[1] * sh.n[2], B = (double)sh.n[0] * sh.n[1] * sh.m[2],
                  C = (double)sh.n[0] * sh.m[1] * sh.m[2], P = (double)op.P;
-    const double conv = E * (4.0 * A + 4.0 * B + 4.0 * C) + (E / 2.0) * P;
+    const bool full = op.fft_fp32 && kind == PfftProduct::Full;
+    const bool thin = kind != PfftProduct::Ports && (full ? op.conv64 : op.conv).thin;
+    const double thinner = (double)sh.n[2] / sh.m[2];
+    const double conv = thin ? E * (4.0 * A + 4.0 * C * thinner) + (E / 2.0) * P * thinner
+                             : E * (4.0 * A + 4.0 * B + 4.0 * C) + (E / 2.0) * P;
     return 12.0 * (double)op.near_entries + 24.0 * (double)op.projection_entries + 32.0 * (double)op.n * count +
            grids * conv;
 }
