@@ -1,7 +1,9 @@
 // Device GMRES (see fh_gmres.cuh).  The Arnoldi loop, the rotations and the
 // stopping rule follow gmres.rs:91-215; every vector operation is a kernel
 // on the solver's stream, and the host reads back one Hessenberg column and
-// one norm per Arnoldi step.
+// one norm per Arnoldi step, on a second stream: the solver's own has the next
+// step's product queued by then, so the device does not wait for the host's
+// part of a step (70 us of 740 at 107,144 filaments; 15 are left).
 #include <cmath>
 #include <complex>
 #include <string>
@@ -49,9 +51,15 @@ __global__ void __launch_bounds__(kRT) maxabs_partial_kernel(const double2 *__re
     if (threadIdx.x == 0) partial[blockIdx.x] = sh[0];
 }
 
-__global__ void __launch_bounds__(kRT) max_final_kernel(const double *__restrict__ partial, double *__restrict__ out) {
+// sum |v_i / scale|^2 (gmres.rs:234-241: the scaled norm); scale is the
+// largest of the kRB maxima, which every block finds for itself.
+__global__ void __launch_bounds__(kRT) sumsq_partial_kernel(const double2 *__restrict__ v, int64_t n,
+                                                            const double *__restrict__ maxima,
+                                                            double *__restrict__ scale,
+                                                            double *__restrict__ partial) {
     __shared__ double sh[kRT];
-    sh[threadIdx.x] = partial[threadIdx.x];
+    static_assert(kRB == kRT, "one maximum per thread");
+    sh[threadIdx.x] = maxima[threadIdx.x];
     __syncthreads();
     for (int s = kRT / 2; s > 0; s >>= 1) {
         if (threadIdx.x < s) {
@@ -60,20 +68,14 @@ __global__ void __launch_bounds__(kRT) max_final_kernel(const double *__restrict
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) *out = sh[0];
-}
-
-// sum |v_i / scale|^2 (gmres.rs:234-241: the scaled norm).
-__global__ void __launch_bounds__(kRT) sumsq_partial_kernel(const double2 *__restrict__ v, int64_t n,
-                                                            const double *__restrict__ scale,
-                                                            double *__restrict__ partial) {
-    __shared__ double sh[kRT];
-    const double sc = *scale;
+    const double sc = sh[0];
+    if (blockIdx.x == 0 && threadIdx.x == 0) *scale = sc;
     double acc = 0.0;
     for (int64_t i = (int64_t)blockIdx.x * kRT + threadIdx.x; i < n; i += (int64_t)kRB * kRT) {
         const double a = v[i].x / sc, b = v[i].y / sc;
         acc += a * a + b * b;
     }
+    __syncthreads();  // sh[0] has been read
     sh[threadIdx.x] = acc;
     __syncthreads();
     for (int s = kRT / 2; s > 0; s >>= 1) {
@@ -168,7 +170,9 @@ __global__ void __launch_bounds__(kRT) multidot_final_kernel(const double *__res
     if (lane == 0) h[k] = t;
 }
 
-// w -= sum_k h[k] V_k, the terms taken in increasing k.
+// w -= sum_k h[k] V_k, the terms taken in increasing k.  Bound by reading the
+// basis: over a cycle of 400 vectors of 78,307, 43 us on average with the
+// compiler's four loads in flight per thread, 32 us with eight.
 __global__ void multi_axpy_kernel(double2 *__restrict__ w, const double2 *__restrict__ V,
                                   const double2 *__restrict__ h, int cnt, int64_t n) {
     extern __shared__ double2 hs[];
@@ -176,7 +180,19 @@ __global__ void multi_axpy_kernel(double2 *__restrict__ w, const double2 *__rest
     __syncthreads();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         double2 y = w[i];
-        for (int k = 0; k < cnt; ++k) {
+        int k = 0;
+        for (; k + 8 <= cnt; k += 8) {
+            double2 b[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) b[q] = V[(size_t)(k + q) * n + i];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const double2 a = hs[k + q];
+                y.x += -a.x * b[q].x + a.y * b[q].y;
+                y.y += -a.x * b[q].y - a.y * b[q].x;
+            }
+        }
+        for (; k < cnt; ++k) {
             const double2 a = hs[k], b = V[(size_t)k * n + i];
             y.x += -a.x * b.x + a.y * b.y;
             y.y += -a.x * b.y - a.y * b.x;
@@ -185,19 +201,27 @@ __global__ void multi_axpy_kernel(double2 *__restrict__ w, const double2 *__rest
     }
 }
 
-// y += a x (a from the host).
-__global__ void axpy_kernel(double2 *__restrict__ y, const double2 *__restrict__ x, double2 a, int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double2 b = x[i];
-        double2 v = y[i];
-        v.x += a.x * b.x - a.y * b.y;
-        v.y += a.x * b.y + a.y * b.x;
-        y[i] = v;
-    }
-}
-
 __global__ void div_real_kernel(double2 *__restrict__ out, const double2 *__restrict__ in, double s, int64_t n) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        out[i] = make_double2(in[i].x / s, in[i].y / s);
+}
+
+// out = in / |in|, the norm from its scale norm[0] and the kRB partial sums;
+// their total goes to norm[1] for the host.
+__global__ void __launch_bounds__(kRT) normalize_kernel(double2 *__restrict__ out, const double2 *__restrict__ in,
+                                                        const double *__restrict__ partial,
+                                                        double *__restrict__ norm, int64_t n) {
+    __shared__ double sh[kRT];
+    sh[threadIdx.x] = partial[threadIdx.x];
+    __syncthreads();
+    for (int s = kRT / 2; s > 0; s >>= 1) {
+        if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
+        __syncthreads();
+    }
+    const double scale = norm[0], sum = sh[0];
+    const double s = scale == 0.0 || !isfinite(scale) ? scale : scale * sqrt(sum);
+    if (blockIdx.x == 0 && threadIdx.x == 0) norm[1] = sum;
+    for (int64_t i = blockIdx.x * (int64_t)kRT + threadIdx.x; i < n; i += (int64_t)gridDim.x * kRT)
         out[i] = make_double2(in[i].x / s, in[i].y / s);
 }
 
@@ -271,7 +295,7 @@ fh_status GmresWork::ensure(int64_t n_, int restart_, cudaStream_t s, fh_error_i
     if (alloc((void **)&V, sizeof(double2) * (size_t)(restart + 1) * n) != cudaSuccess ||
         alloc((void **)&w, sizeof(double2) * n) != cudaSuccess || alloc((void **)&r, sizeof(double2) * n) != cudaSuccess ||
         alloc((void **)&t, sizeof(double2) * n) != cudaSuccess || alloc((void **)&u, sizeof(double2) * n) != cudaSuccess ||
-        alloc((void **)&h, sizeof(double2) * 2 * (restart + 1)) != cudaSuccess ||
+        alloc((void **)&h, sizeof(double2) * (2 * (restart + 1) + 1)) != cudaSuccess ||
         alloc((void **)&red, sizeof(double) * kRedLen) != cudaSuccess ||
         alloc((void **)&part, sizeof(double) * 2 * kDotChunks * (size_t)(restart + 1)) != cudaSuccess) {
         cudaGetLastError();
@@ -289,8 +313,8 @@ fh_status gmres_solve(int64_t n, const DeviceOp &apply, const DeviceOp &precondi
     if (st) return st;
     auto norm_of = [&](const double2 *v, Norm &nm) -> fh_status {
         maxabs_partial_kernel<<<kRB, kRT, 0, s>>>(v, n, work.red + kMaxPartial);
-        max_final_kernel<<<1, kRT, 0, s>>>(work.red + kMaxPartial, work.red + kScale);
-        sumsq_partial_kernel<<<kRB, kRT, 0, s>>>(v, n, work.red + kScale, work.red + kSumPartial);
+        sumsq_partial_kernel<<<kRB, kRT, 0, s>>>(v, n, work.red + kMaxPartial, work.red + kScale,
+                                                 work.red + kSumPartial);
         sum_final_kernel<<<1, kRT, 0, s>>>(work.red + kSumPartial, work.red + kSum);
         FHB_CUDA(cudaGetLastError());
         double hv[2];
@@ -326,7 +350,17 @@ fh_status gmres_solve(int64_t n, const DeviceOp &apply, const DeviceOp &precondi
     double r_norm = 0.0;
     st = residual(r_norm);
     if (st) return st;
-    std::vector<cplx> hcol_dev(2 * (size_t)(restart + 1));
+    std::vector<cplx> hcol_dev(2 * (size_t)(restart + 1) + 1);
+    struct Side {  // the stream of the readbacks, and where it may start
+        cudaStream_t s = nullptr;
+        cudaEvent_t ready = nullptr;
+        ~Side() {
+            if (ready) cudaEventDestroy(ready);
+            if (s) stream_release(s);
+        }
+    } side;
+    FHB_CUDA(stream_acquire(&side.s));
+    FHB_CUDA(cudaEventCreateWithFlags(&side.ready, cudaEventDisableTiming));
     for (;;) {
         oc.iterations = iterations;
         oc.relative_residual = r_norm / b_norm;
@@ -345,13 +379,14 @@ fh_status gmres_solve(int64_t n, const DeviceOp &apply, const DeviceOp &precondi
         std::vector<std::pair<double, cplx>> rot;
         std::vector<cplx> g((size_t)restart + 1, cplx(0.0, 0.0));
         g[0] = cplx(r_norm, 0.0);
+        auto product = [&](int j) -> fh_status {  // w = A M V_j
+            fh_status e = precondition(work.V + (size_t)j * n, work.u, err);
+            return e ? e : apply(work.u, work.w, err);
+        };
+        bool queued = false;
         while ((int)hess.size() < restart && iterations < params.max_iterations) {
             const int j = (int)hess.size();
-            double2 *vj = work.V + (size_t)j * n;
-            st = precondition(vj, work.u, err);
-            if (st) return st;
-            st = apply(work.u, work.w, err);
-            if (st) return st;
+            if (!queued && (st = product(j))) return st;
             iterations += 1;
             // Classical Gram-Schmidt twice: each pass projects w on all of
             // V_0 .. V_j in one product and removes them in one update (the
@@ -359,23 +394,36 @@ fh_status gmres_solve(int64_t n, const DeviceOp &apply, const DeviceOp &precondi
             // orthogonality; three launches per pass instead of three per
             // basis vector).
             for (int pass = 0; pass < 2; ++pass) {
-                double2 *hp = work.h + pass * (restart + 1);
+                double2 *hp = work.h + pass * (j + 1);
                 multidot_partial_kernel<<<dim3(kDotChunks, (unsigned)(j / kDotVecs + 1)), kDotThreads, 0, s>>>(
                     work.V, work.w, n, j + 1, work.part);
                 multidot_final_kernel<<<j / (kRT / 32) + 1, kRT, 0, s>>>(work.part, j + 1, hp);
                 multi_axpy_kernel<<<grid_of(n), 256, sizeof(double2) * (j + 1), s>>>(work.w, work.V, hp, j + 1, n);
             }
+            // the norm (after the columns in h), and V_j+1 from it
+            double *norm = reinterpret_cast<double *>(work.h + 2 * (j + 1));
+            maxabs_partial_kernel<<<kRB, kRT, 0, s>>>(work.w, n, work.red + kMaxPartial);
+            sumsq_partial_kernel<<<kRB, kRT, 0, s>>>(work.w, n, work.red + kMaxPartial, norm, work.red + kSumPartial);
+            normalize_kernel<<<grid_of(n), kRT, 0, s>>>(work.V + (size_t)(j + 1) * n, work.w, work.red + kSumPartial,
+                                                        norm, n);
             FHB_CUDA(cudaGetLastError());
+            FHB_CUDA(cudaEventRecord(side.ready, s));
+            // The next step's product, unless this step should be the last: the
+            // residual falls as in the step before, with a factor 2 in hand.
+            const double now = std::abs(g[(size_t)j]), rate = j > 0 ? now / std::abs(g[(size_t)j - 1]) : 1.0;
+            queued = j + 1 < restart && iterations < params.max_iterations && now * rate > 2.0 * target;
+            if (queued && (st = product(j + 1))) return st;
+            FHB_CUDA(cudaStreamWaitEvent(side.s, side.ready, 0));
+            FHB_CUDA(cudaMemcpyAsync(hcol_dev.data(), work.h, sizeof(double2) * (2 * (size_t)(j + 1) + 1),
+                                     cudaMemcpyDeviceToHost, side.s));
+            FHB_CUDA(cudaStreamSynchronize(side.s));
             Norm wn;
-            st = norm_of(work.w, wn);
-            if (st) return st;
+            wn.scale = hcol_dev[2 * (size_t)(j + 1)].real();
+            wn.sum = hcol_dev[2 * (size_t)(j + 1)].imag();
             const double next_norm = wn.value();
-            FHB_CUDA(cudaMemcpyAsync(hcol_dev.data(), work.h, sizeof(double2) * 2 * (restart + 1),
-                                     cudaMemcpyDeviceToHost, s));
-            FHB_CUDA(cudaStreamSynchronize(s));
             std::vector<cplx> column((size_t)j + 2, cplx(0.0, 0.0));
             for (int pass = 0; pass < 2; ++pass)
-                for (int k = 0; k <= j; ++k) column[k] += hcol_dev[pass * (restart + 1) + k];
+                for (int k = 0; k <= j; ++k) column[k] += hcol_dev[pass * (j + 1) + k];
             column[j + 1] = cplx(next_norm, 0.0);
             for (size_t i = 0; i < rot.size(); ++i) {
                 const double c = rot[i].first;
@@ -395,8 +443,6 @@ fh_status gmres_solve(int64_t n, const DeviceOp &apply, const DeviceOp &precondi
             g[j + 1] = -cmul_ref(std::conj(sr), gj);
             hess.push_back(column);
             if (next_norm == 0.0 || std::abs(g[j + 1]) <= target) break;
-            div_real_kernel<<<grid_of(n), 256, 0, s>>>(work.V + (size_t)(j + 1) * n, work.w, next_norm, n);
-            FHB_CUDA(cudaGetLastError());
         }
         // Back substitution, then x += M (V y).
         const int steps = (int)hess.size();
@@ -406,10 +452,10 @@ fh_status gmres_solve(int64_t n, const DeviceOp &apply, const DeviceOp &precondi
             for (int k = i + 1; k < steps; ++k) sum -= cmul_ref(hess[k][i], y[k]);
             y[i] = cdiv_ref(sum, hess[i][i]);
         }
+        for (cplx &v : y) v = -v;
+        FHB_CUDA(cudaMemcpyAsync(work.h, y.data(), sizeof(double2) * (size_t)steps, cudaMemcpyHostToDevice, s));
         FHB_CUDA(cudaMemsetAsync(work.u, 0, sizeof(double2) * n, s));
-        for (int k = 0; k < steps; ++k)
-            axpy_kernel<<<grid_of(n), 256, 0, s>>>(work.u, work.V + (size_t)k * n, make_double2(y[k].real(), y[k].imag()),
-                                                   n);
+        multi_axpy_kernel<<<grid_of(n), 256, sizeof(double2) * steps, s>>>(work.u, work.V, work.h, steps, n);
         FHB_CUDA(cudaGetLastError());
         st = precondition(work.u, work.t, err);
         if (st) return st;
