@@ -41,6 +41,9 @@ namespace {
 
 constexpr int kW = 16;         // sub-panel width
 constexpr int kNbMax = 128;    // outer panel width limit
+constexpr int kMaxCluster = 16;                // CTAs of a matrix's cluster
+constexpr int kNbResident = 64;               // of panel_resident_kernel
+constexpr size_t kResidentSmem = 180 * 1024;  // its slices' limit (44 KB are static): one CTA per SM, as the cluster form
 constexpr int kThreads = 256;
 constexpr int kBarrierStride = kGroupBarrierStride;
 
@@ -399,11 +402,207 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1) panel_coop_k
     if constexpr (kCluster) cooperative_groups::this_cluster().sync();
 }
 
+// a b, 1 / p and y -= f x in the roundings that the cluster form above takes
+// (which product of a sum is rounded by itself is the compiler's choice there).
+__device__ __forceinline__ Cx<double> mul_rn(Cx<double> a, Cx<double> b) {
+    return {__fma_rn(a.re, b.re, -__dmul_rn(a.im, b.im)), __fma_rn(a.re, b.im, __dmul_rn(a.im, b.re))};
+}
+__device__ __forceinline__ Cx<double> inverse_rn(Cx<double> p) {
+    const double ns = __fma_rn(p.re, p.re, __dmul_rn(p.im, p.im));
+    return {p.re / ns, -p.im / ns};
+}
+__device__ __forceinline__ void submul_rn(Cx<double> &y, Cx<double> f, Cx<double> x) {
+    y.re = __dsub_rn(y.re, __fma_rn(f.re, x.re, -__dmul_rn(f.im, x.im)));
+    y.im = __dsub_rn(y.im, __fma_rn(f.im, x.re, __dmul_rn(f.re, x.im)));
+}
+
+// The cluster form in FP64 for slices that fit shared memory: a CTA keeps its
+// rows of the panel there (entry (row, t) at t ld + row) from the first column
+// to the last, so a column costs shared-memory and cluster latencies instead
+// of some ten dependent trips to L2 and back.  The pivot rows of a sub-panel
+// stay with every CTA (U), which solves U12 for itself: one cluster barrier per
+// column is all that is left.  The arithmetic of every entry is that of the
+// kernel above in the same order and with the same roundings, so the factors
+// agree bit for bit (a tie between two filaments' currents falls the same way).
+//
+// Bound by the chain of a column: the arg-max, the barrier, the trip through
+// distributed shared memory and the reciprocal.  Order 900, four matrices, a
+// panel of 64 columns: 376 us from device memory, 156 us here.
+__global__ void __launch_bounds__(kThreads, 1)
+    panel_resident_kernel(Cx<double> *__restrict__ a, int64_t m, int64_t K0, int NB, int *__restrict__ pivots,
+                          int *__restrict__ singular, int per_matrix, int ld) {
+    extern __shared__ __align__(16) unsigned char panel_smem[];
+    Cx<double> *S = reinterpret_cast<Cx<double> *>(panel_smem);
+    __shared__ Cx<double> U[kW][kNbResident];
+    __shared__ double s_val[kThreads / 32];
+    __shared__ int s_idx[kThreads / 32];
+    // every CTA's candidate, written here by its CTA; this one's panel row of its
+    // candidate and, on the owner of row j, row j; double-buffered by the parity
+    // of j
+    __shared__ double c_val[2][kMaxCluster];
+    __shared__ int c_row[2][kMaxCluster];
+    __shared__ Cx<double> c_data[2][kNbResident], c_rowj[2][kNbResident];
+    auto cl = cooperative_groups::this_cluster();
+    const int f = blockIdx.x / per_matrix, slice = blockIdx.x % per_matrix;
+    Cx<double> *A = a + (int64_t)f * m * m;
+    const int rows = (int)(m - K0), chunk = (rows + per_matrix - 1) / per_matrix;
+    // rows are counted from K0 on
+    const int begin = slice * chunk, n = max(0, min(rows - begin, chunk));
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    auto better = [](double v2, int i2, double v1, int i1) { return v2 > v1 || (v2 == v1 && i2 < i1); };
+    for (int t = warp; t < NB; t += kThreads / 32)
+        for (int i = lane; i < n; i += 32) S[t * ld + i] = A[K0 + begin + i + (K0 + t) * m];
+    __syncthreads();
+    for (int s0 = 0; s0 < NB; s0 += kW) {
+        const int w = min(kW, NB - s0);
+        for (int c = 0; c < w; ++c) {
+            const int j = s0 + c, par = j & 1;
+            // 1. this CTA's candidate
+            double best = -1.0;
+            int bi = INT_MAX;
+            for (int i = tid; i < n; i += kThreads) {
+                const Cx<double> v = S[j * ld + i];
+                const double n1 = fabs(v.re) + fabs(v.im);
+                if (begin + i >= j && n1 > best) {  // rows ascend: ties keep the first
+                    best = n1;
+                    bi = begin + i;
+                }
+            }
+            for (int o = 16; o > 0; o >>= 1) {
+                const double v2 = __shfl_xor_sync(0xffffffffu, best, o);
+                const int i2 = __shfl_xor_sync(0xffffffffu, bi, o);
+                if (better(v2, i2, best, bi)) {
+                    best = v2;
+                    bi = i2;
+                }
+            }
+            if (lane == 0) {
+                s_val[warp] = best;
+                s_idx[warp] = bi;
+            }
+            __syncthreads();
+            best = s_val[lane & (kThreads / 32 - 1)];
+            bi = s_idx[lane & (kThreads / 32 - 1)];
+            for (int o = kThreads / 64; o > 0; o >>= 1) {
+                const double v2 = __shfl_xor_sync(0xffffffffu, best, o);
+                const int i2 = __shfl_xor_sync(0xffffffffu, bi, o);
+                if (better(v2, i2, best, bi)) {
+                    best = v2;
+                    bi = i2;
+                }
+            }
+            if (tid < per_matrix) {
+                *cl.map_shared_rank(&c_val[par][slice], (unsigned)tid) = best;
+                *cl.map_shared_rank(&c_row[par][slice], (unsigned)tid) = bi == INT_MAX ? -1 : bi;
+            }
+            const bool own_j = j >= begin && j < begin + n;
+            if (tid < NB) {
+                if (bi != INT_MAX) c_data[par][tid] = S[tid * ld + bi - begin];
+                if (own_j) c_rowj[par][tid] = S[tid * ld + j - begin];
+            }
+            // 2. every CTA's candidate is published
+            cl.sync();
+            // 3. the pivot (every warp for itself), and the interchange
+            double bv = -1.0;
+            int brow = INT_MAX, bslot = -1;
+            if (lane < per_matrix) {
+                const double v2 = c_val[par][lane];
+                const int r2 = c_row[par][lane];
+                if (r2 >= 0 && better(v2, r2, bv, brow)) {
+                    bv = v2;
+                    brow = r2;
+                    bslot = lane;
+                }
+            }
+            for (int o = kMaxCluster / 2; o > 0; o >>= 1) {
+                const double v2 = __shfl_xor_sync(0xffffffffu, bv, o);
+                const int r2 = __shfl_xor_sync(0xffffffffu, brow, o);
+                const int s2 = __shfl_xor_sync(0xffffffffu, bslot, o);
+                if (s2 >= 0 && better(v2, r2, bv, brow)) {
+                    bv = v2;
+                    brow = r2;
+                    bslot = s2;
+                }
+            }
+            static_assert(kMaxCluster <= 32, "a lane per CTA");
+            bv = __shfl_sync(0xffffffffu, bv, 0);
+            brow = __shfl_sync(0xffffffffu, brow, 0);
+            bslot = __shfl_sync(0xffffffffu, bslot, 0);
+            const int p = bv > 0.0 ? brow : j;  // else a zero or all-NaN column: keep the diagonal
+            if (tid == 0 && slice == 0) {
+                if (bv == 0.0) singular[f] = 1;  // exactly zero pivot (dense.rs:166-168)
+                pivots[(int64_t)f * m + K0 + j] = (int)(K0 + p);
+            }
+            if (tid < NB) {
+                const Cx<double> rj = cl.map_shared_rank(&c_rowj[par][0], (unsigned)(j / chunk))[tid];
+                const Cx<double> pr = p != j ? cl.map_shared_rank(&c_data[par][0], (unsigned)bslot)[tid] : rj;
+                U[c][tid] = pr;
+                if (p != j) {
+                    if (p >= begin && p < begin + n) S[tid * ld + p - begin] = rj;
+                    if (own_j) S[tid * ld + j - begin] = pr;
+                }
+            }
+            __syncthreads();
+            // 4. scale by the pivot's reciprocal and rank-1 update inside the
+            //    sub-panel: four lanes a row
+            const Cx<double> inv = inverse_rn(U[c][j]);
+            for (int i0 = 0; i0 < n; i0 += kThreads / 4) {
+                const int i = i0 + (tid >> 2);
+                const bool live = i < n && begin + i > j;
+                Cx<double> l{0.0, 0.0};
+                if (live) l = mul_rn(S[j * ld + i], inv);
+                __syncwarp();
+                if (live) {
+                    if ((tid & 3) == 0) S[j * ld + i] = l;
+                    for (int q = c + 1 + (tid & 3); q < w; q += 4) {
+                        Cx<double> y = S[(s0 + q) * ld + i];
+                        submul_rn(y, U[c][s0 + q], l);
+                        S[(s0 + q) * ld + i] = y;
+                    }
+                }
+            }
+            __syncthreads();
+        }
+        const int rest = NB - s0 - w;  // panel columns right of the sub-panel
+        if (rest <= 0) continue;       // (w = kW from here on)
+        // 5. U12 of the sub-panel's pivot rows
+        if (tid < rest) {
+            const int t = s0 + kW + tid;
+            Cx<double> x[kW];
+#pragma unroll
+            for (int r = 0; r < kW; ++r) x[r] = U[r][t];
+#pragma unroll
+            for (int k = 0; k < kW; ++k)
+#pragma unroll
+                for (int r = k + 1; r < kW; ++r) submul_rn(x[r], x[k], U[r][s0 + k]);
+#pragma unroll
+            for (int r = 0; r < kW; ++r) {
+                U[r][t] = x[r];
+                const int i = s0 + r - begin;
+                if (i >= 0 && i < n) S[t * ld + i] = x[r];
+            }
+        }
+        __syncthreads();
+        // 6. the rows below: A[i, rest] -= A[i, sub-panel] U12
+        const int first = max(0, s0 + kW - begin), below = n - first;
+        for (int idx = tid; idx < below * rest; idx += kThreads) {
+            const int i = first + idx % below, t = s0 + kW + idx / below;
+            Cx<double> y = S[t * ld + i];
+#pragma unroll
+            for (int r = 0; r < kW; ++r) submul_rn(y, S[(s0 + r) * ld + i], U[r][t]);
+            S[t * ld + i] = y;
+        }
+        __syncthreads();
+    }
+    for (int t = warp; t < NB; t += kThreads / 32)
+        for (int i = lane; i < n; i += 32) A[K0 + begin + i + (K0 + t) * m] = S[t * ld + i];
+    cl.sync();  // no CTA leaves while another may still read its shared memory
+}
+
 }  // namespace
 
 // Largest cluster of CTAs of the cluster form that the device can schedule
 // (0: none), for sizes up to kMaxCluster.
-constexpr int kMaxCluster = 16;
 
 template <class T>
 int cluster_fits_query(int size);
@@ -521,6 +720,10 @@ fh_status panel_coop(LuBatch<T> &b, int64_t K0, int nb, const CoopScratch &cs, c
     Cx<T> *a = reinterpret_cast<Cx<T> *>(b.a);
     int64_t m = b.m;
     if (cs.cluster) {
+        // slices in shared memory where they fit (see panel_resident_kernel)
+        const int64_t chunk = (m - K0 + cs.per_matrix - 1) / cs.per_matrix;
+        const int ld = (int)((chunk + 7) / 8 * 8 + 2);  // rows two bank groups apart: four lanes a row, two rows a pass
+        const size_t resident = sizeof(Cx<T>) * (size_t)ld * (size_t)nb;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)(cs.per_matrix * b.count));
         cfg.blockDim = dim3(kThreads);
@@ -532,6 +735,17 @@ fh_status panel_coop(LuBatch<T> &b, int64_t K0, int nb, const CoopScratch &cs, c
         attr.val.clusterDim.z = 1;
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
+        if constexpr (sizeof(T) == 8) {
+            if (nb <= kNbResident && resident <= kResidentSmem) {
+                auto kernel = panel_resident_kernel;
+                FHB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResidentSmem));
+                if (cs.per_matrix > 8)
+                    FHB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+                cfg.dynamicSmemBytes = resident;
+                FHB_CUDA(cudaLaunchKernelEx(&cfg, kernel, a, m, K0, nb, b.pivots, b.singular, cs.per_matrix, ld));
+                return FH_OK;
+            }
+        }
         FHB_CUDA(cudaLaunchKernelEx(&cfg, panel_coop_kernel<T, true>, a, m, K0, nb, b.pivots, b.singular, args));
         return FH_OK;
     }
@@ -559,3 +773,46 @@ template fh_status panel_coop<double>(LuBatch<double> &, int64_t, int, const Coo
 template fh_status panel_coop<float>(LuBatch<float> &, int64_t, int, const CoopScratch &, cudaStream_t, fh_error_info *);
 
 }  // namespace fhb
+
+using namespace fhb;
+
+extern "C" fh_status fh_test_panel(double *a, int64_t m, int32_t count, int64_t k0, int32_t nb, int32_t *pivots,
+                                   int32_t *singular, fh_error_info *err) {
+    clear_error(err);
+    if (!a || !pivots || !singular || count < 1 || nb < 1 || nb > kNbMax || k0 < 0 || k0 + nb > m)
+        return fail(err, FH_ERR_INVALID_ARGUMENT, "null argument or panel beyond the matrix");
+    fh_status st = ensure_device(err);
+    if (st) return st;
+    int per_matrix = 0;
+    size_t bytes = 0;
+    st = coop_plan<double>(count, m - k0, &per_matrix, &bytes, err, 1);
+    if (st) return st;
+    void *d[4] = {};
+    struct Release {
+        void **d;
+        ~Release() {
+            for (int k = 0; k < 4; ++k) cudaFree(d[k]);
+        }
+    } release{d};
+    const size_t size[4] = {16 * (size_t)count * m * m, 4 * (size_t)count * m, 4 * (size_t)count, bytes};
+    for (int k = 0; k < 4; ++k) {
+        FHB_CUDA(cudaMalloc(&d[k], size[k]));
+        FHB_CUDA(cudaMemset(d[k], 0, size[k]));
+    }
+    FHB_CUDA(cudaMemcpy(d[0], a, size[0], cudaMemcpyHostToDevice));
+    CoopScratch cs;
+    coop_bind<double>(d[3], count, per_matrix, cs, 1);
+    LuBatch<double> b;
+    b.a = (double *)d[0];
+    b.pivots = (int *)d[1];
+    b.singular = (int *)d[2];
+    b.m = m;
+    b.count = count;
+    st = panel_coop<double>(b, k0, nb, cs, nullptr, err);
+    if (!st) st = coop_check(cs, nullptr, err);
+    if (st) return st;
+    FHB_CUDA(cudaMemcpy(a, d[0], size[0], cudaMemcpyDeviceToHost));
+    FHB_CUDA(cudaMemcpy(pivots, d[1], size[1], cudaMemcpyDeviceToHost));
+    FHB_CUDA(cudaMemcpy(singular, d[2], size[2], cudaMemcpyDeviceToHost));
+    return FH_OK;
+}

@@ -506,7 +506,13 @@ fh_status fh_test_trailing_update(float *a, int64_t m, int32_t count, int64_t k0
  * of m (both complex), failed[f]: 1 where the elimination was rejected. */
 fh_status fh_test_mesh_solve(const double *r, const double *l, int64_t m, int64_t p, const double *omega,
                              int32_t count, double *z, double *x, int32_t *failed, fh_error_info *err);
-/* The same through the batched kernel, in one of its tile configurations, the
+/* One panel (columns k0 .. k0 + nb) of the pivoted FP64 factorization of
+ * `count` complex matrices of order m (column-major), in place; pivots: count
+ * x m rows (those of the panel's columns are set), singular: 1 where a pivot
+ * was exactly zero. */
+fh_status fh_test_panel(double *a, int64_t m, int32_t count, int64_t k0, int32_t nb, int32_t *pivots,
+                        int32_t *singular, fh_error_info *err);
+/* As fh_test_mesh_solve (Z only) through the batched kernel, in one of its tile configurations, the
  * first `grouped` frequencies by groups of CTAs. */
 fh_status fh_test_batch_solve(const double *r, const double *l, int64_t m, int64_t p, const double *omega,
                               int32_t count, int32_t config, int32_t grouped, double *z, int32_t *failed,
