@@ -79,13 +79,13 @@ __global__ void __launch_bounds__(kDiagThreads64) ldlt_diag_kernel(double2 *__re
 __global__ void __launch_bounds__(kLdThreads, 2)
     ldlt_panel_kernel(double2 *__restrict__ a, int64_t M, int64_t k0, int nb, const double2 *__restrict__ xinv,
                       int64_t xinv_stride, const double2 *__restrict__ dinv, double2 *__restrict__ panel,
-                      double *__restrict__ growth) {
+                      int64_t panel_stride, double *__restrict__ growth) {
     extern __shared__ __align__(16) unsigned char ld_smem[];
     double2 *Ls = reinterpret_cast<double2 *>(ld_smem), *Us = Ls + 32 * kLdPad;
     __shared__ double rowsum[kLd];
     double2 *A = a + (int64_t)blockIdx.y * M * M;
     const double2 *X = xinv + (int64_t)blockIdx.y * xinv_stride, *D = dinv + (int64_t)blockIdx.y * kLd;
-    double2 *P = panel + (int64_t)blockIdx.y * M * kLd;
+    double2 *P = panel + (int64_t)blockIdx.y * panel_stride;
     const int64_t r0 = k0 + nb + (int64_t)blockIdx.x * kLd;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3, wr = warp >> 2, wc = warp & 3;
@@ -132,29 +132,33 @@ __global__ void __launch_bounds__(kLdThreads, 2)
     if (tid < kLd && r0 + tid < M) growth[(int64_t)blockIdx.y * M + r0 + tid] += rowsum[tid];
 }
 
-// A22 -= L21 B^T: one 64 x 64 tile on or below the diagonal per CTA, k in
-// stages of 16 through two buffers of asynchronous copies, both operands
+// A -= L B^T over the columns [k0, k0 + nb) of L on rows and columns from base:
+// the whole lower triangle (end = M) or the columns [base, end) of one tile;
+// one 64 x 64 tile on or below the diagonal per CTA, k in stages of 16 through two buffers of asynchronous copies, both operands
 // [k][row] with re and im side by side (one 16-byte load per fragment).
 //
-// Bound by the FP64 tensor pipe: 8 x 64 operations per complex entry against
-// 32 bytes of C.  Order 2,321 x 32 matrices: 19.0 ms for the 37 panels, 29
-// TFLOP/s of the 37 that the instruction reaches alone (33.5 with the
-// kernel's memory traffic taken out; a third buffer, a fixed or random start
-// delay per CTA against lockstep, and m8n8k4 fragments measured the same or
-// slower); the full update of the pivoted form takes 38.4 ms.
+// Bound by the FP64 tensor pipe: 8 nb operations per complex entry against 32
+// bytes of C.  Order 2,321 x 32 matrices with nb = 64: 19.0 ms in all, 29
+// TFLOP/s of the 37 that the instruction reaches alone (33.5 with the kernel's
+// memory traffic taken out; a third buffer, a fixed or random start delay per
+// CTA against lockstep, and m8n8k4 fragments measured the same or slower; the
+// full update of the pivoted form takes 38.4 ms); with nb = 256 (ldlt_depth)
+// 17.5.
 __global__ void __launch_bounds__(kLdThreads, 2)
-    ldlt_update_kernel(double2 *__restrict__ a, int64_t M, int64_t k0, int nb, const double2 *__restrict__ panel) {
+    ldlt_update_kernel(double2 *__restrict__ a, int64_t M, int64_t k0, int nb, int64_t base, int64_t end,
+                       const double2 *__restrict__ panel, int64_t panel_stride) {
     extern __shared__ __align__(16) unsigned char ld_smem[];
     double2 *smem = reinterpret_cast<double2 *>(ld_smem);  // stage s: L at 2 s kLdK kLdPad, B after it
     double2 *A = a + (int64_t)blockIdx.y * M * M;
-    const double2 *P = panel + (int64_t)blockIdx.y * M * kLd;
+    const double2 *P = panel + (int64_t)blockIdx.y * panel_stride;
     // tile index to (ti >= tj)
     const int tile = blockIdx.x;
     int ti = (int)((sqrt(8.0 * (double)tile + 1.0) - 1.0) * 0.5);
     while ((int64_t)ti * (ti + 1) / 2 > tile) --ti;
     while ((int64_t)(ti + 1) * (ti + 2) / 2 <= tile) ++ti;
-    const int tj = tile - (int)((int64_t)ti * (ti + 1) / 2);
-    const int64_t base = k0 + nb, i0 = base + (int64_t)ti * kLd, j0 = base + (int64_t)tj * kLd;
+    const int tj = end < M ? 0 : tile - (int)((int64_t)ti * (ti + 1) / 2);
+    if (end < M) ti = tile;
+    const int64_t i0 = base + (int64_t)ti * kLd, j0 = base + (int64_t)tj * kLd;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3, wr = warp >> 2, wc = warp & 3;
     const int stages = (nb + kLdK - 1) / kLdK;
@@ -204,7 +208,7 @@ __global__ void __launch_bounds__(kLdThreads, 2)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 const int64_t row = i0 + 32 * wr + 8 * fm + g, col = j0 + 16 * wc + 8 * fn + 2 * t + e;
-                if (row < M && col < M) A[row + col * M] = make_double2(re[fm][fn][e], im[fm][fn][e]);
+                if (row < M && col < end) A[row + col * M] = make_double2(re[fm][fn][e], im[fm][fn][e]);
             }
 }
 
@@ -305,11 +309,23 @@ __global__ void __launch_bounds__(256) ldlt_back_update_kernel(const double2 *__
     }
 }
 
+// Panels per group: the trailing matrix is updated once per group, by all its
+// columns, and a panel within a group just before its turn, so the traffic of
+// C falls with the depth; but a panel's own update has only the panel's tiles.
+// Where these fill the chip's two CTAs per SM four panels are best, below a
+// third of that one (ms for depths 1, 2, 4: order 6,787, 32 matrices 436, 408,
+// 397; 5 matrices 74.0, 69.8, 68.7; 1 matrix 20.9, 20.3, 20.6; order 2,321,
+// 32 matrices 23.8, 22.9, 22.4; 2 matrices 3.98, 4.18, 4.36).
+int ldlt_depth(int64_t m, int64_t p, int count) {
+    const int64_t tiles = (m + p + kLd - 1) / kLd * count;
+    return tiles >= 2 * 148 ? 4 : tiles >= 96 ? 2 : 1;
+}
+
 }  // namespace
 
 size_t ldlt_bytes(int64_t m, int64_t p, int count) {
     const int64_t M = m + p, blocks = (m + kLd - 1) / kLd;
-    return (size_t)count * (16 * (size_t)M * kLd + 16 * (size_t)blocks * kLd * kLd + 16 * (size_t)blocks * kLd +
+    return (size_t)count * (16 * (size_t)M * kLd * ldlt_depth(m, p, count) + 16 * (size_t)blocks * kLd * kLd + 16 * (size_t)blocks * kLd +
                             16 * (size_t)M + 16);
 }
 
@@ -319,7 +335,7 @@ fh_status ldlt_factor(const double *Rm, const double *Lm, int64_t m, int64_t p, 
     const int64_t M = m + p, blocks = (m + kLd - 1) / kLd;
     double2 *A = reinterpret_cast<double2 *>(a);
     double2 *panel = static_cast<double2 *>(work);
-    double2 *xinv = panel + (int64_t)count * M * kLd;
+    double2 *xinv = panel + (int64_t)count * M * kLd * ldlt_depth(m, p, count);
     double2 *dinv = xinv + (int64_t)count * blocks * kLd * kLd;
     double *diag = reinterpret_cast<double *>(dinv + (int64_t)count * blocks * kLd);
     double *growth = diag + (int64_t)count * M;
@@ -334,22 +350,33 @@ fh_status ldlt_factor(const double *Rm, const double *Lm, int64_t m, int64_t p, 
     FHB_CUDA(cudaFuncSetAttribute(ldlt_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, panel_smem));
     FHB_CUDA(cudaFuncSetAttribute(ldlt_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, update_smem));
     const int64_t xs = blocks * kLd * kLd;
+    const int depth = ldlt_depth(m, p, count);
+    const int64_t ps = M * kLd * depth;
     for (int64_t k0 = 0, b = 0; k0 < m; k0 += kLd, ++b) {
         const int nb = (int)std::min<int64_t>(kLd, m - k0);
         const int64_t rest = M - k0 - nb, tiles = (rest + kLd - 1) / kLd;
+        const int g = (int)(b % depth), k = g * kLd;  // place in the group, and its columns before this panel
         double2 *xb = xinv + b * kLd * kLd, *db = dinv + b * count * kLd;
+        if (g > 0) {  // this panel's columns, from the panels of its group
+            prof_begin(s, FH_PROF_GEMM_FP64);
+            ldlt_update_kernel<<<dim3((unsigned)((M - k0 + kLd - 1) / kLd), (unsigned)count), kLdThreads, update_smem,
+                                 s>>>(A, M, k0 - k, k, k0, k0 + nb, panel, ps);
+            prof_end(s, FH_PROF_GEMM_FP64, 8.0 * kLd * (double)(M - k0) * k * count);
+        }
         prof_begin(s, FH_PROF_PANEL);
         ldlt_diag_kernel<<<(unsigned)count, kDiagThreads64, 0, s>>>(A, M, k0, nb, xb, xs, db, growth, d_failed);
         prof_end(s, FH_PROF_PANEL, 0.0);
         if (tiles == 0) continue;
         prof_begin(s, FH_PROF_TRSM);
-        ldlt_panel_kernel<<<dim3((unsigned)tiles, (unsigned)count), kLdThreads, panel_smem, s>>>(A, M, k0, nb, xb, xs,
-                                                                                                db, panel, growth);
+        ldlt_panel_kernel<<<dim3((unsigned)tiles, (unsigned)count), kLdThreads, panel_smem, s>>>(
+            A, M, k0, nb, xb, xs, db, panel + (int64_t)k * M, ps, growth);
         prof_end(s, FH_PROF_TRSM, 4.0 * kLd * kLd * (double)rest * count);
-        prof_begin(s, FH_PROF_GEMM_FP64);
-        ldlt_update_kernel<<<dim3((unsigned)(tiles * (tiles + 1) / 2), (unsigned)count), kLdThreads, update_smem, s>>>(
-            A, M, k0, nb, panel);
-        prof_end(s, FH_PROF_GEMM_FP64, 4.0 * (double)rest * (double)rest * nb * count);
+        if (g + 1 == depth || k0 + nb == m) {  // the group is complete: everything right of it
+            prof_begin(s, FH_PROF_GEMM_FP64);
+            ldlt_update_kernel<<<dim3((unsigned)(tiles * (tiles + 1) / 2), (unsigned)count), kLdThreads, update_smem,
+                                 s>>>(A, M, k0 - k, k + nb, k0 + nb, M, panel, ps);
+            prof_end(s, FH_PROF_GEMM_FP64, 4.0 * (double)rest * (double)rest * (k + nb) * count);
+        }
         FHB_CUDA(cudaGetLastError());
     }
     if (m > 0) ldlt_growth_kernel<<<(unsigned)count, 256, 0, s>>>(growth, diag, M, m, d_failed);
