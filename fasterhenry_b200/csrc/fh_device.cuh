@@ -53,8 +53,9 @@ fh_status ensure_device(fh_error_info *err);
 cudaError_t cache_alloc(void **p, size_t bytes, cudaStream_t s);
 void cache_free(void *p, cudaStream_t s);
 // A non-blocking stream of the current device, from the device's idle ones or
-// new; stream_release keeps a few idle and destroys the rest.
-cudaError_t stream_acquire(cudaStream_t *s);
+// new (urgent: of the highest priority); stream_release keeps a few idle and
+// destroys the rest.
+cudaError_t stream_acquire(cudaStream_t *s, bool urgent = false);
 void stream_release(cudaStream_t s);
 // A buffer of the memory cache that is freed in its stream's order.
 struct CacheBuf {

@@ -43,6 +43,14 @@ constexpr int kLdPad = kLd + 2;       // row of a staged chunk: four k and two r
 constexpr int kLdK = 16;              // k per stage of the update
 constexpr int kLdThreads = 256;
 constexpr int kDiagThreads64 = 512;
+// From this order on the next group's panels run beside the update of the rest
+// of the matrix, on a stream of the highest priority, whose blocks take the
+// slots that the update's leave: their chain of small launches is a fifth of
+// the time at order 2,321.  Without and with, in ms: order 6,787, 1 matrix 20.3
+// and 17.4, 4 matrices 56.5 and 52.5; order 2,321, 2 matrices 3.98 and 3.50,
+// 32 matrices 22.4 and 21.2; order 464, 32 matrices 0.89 and 0.82; 232, 1
+// matrix 0.37 and 0.37.
+constexpr int64_t kAheadOrder = 256;
 
 // A = R + j w L on the tiles on and below the diagonal, order M, and the
 // diagonal's 1-norms.
@@ -133,7 +141,7 @@ __global__ void __launch_bounds__(kLdThreads, 2)
 }
 
 // A -= L B^T over the columns [k0, k0 + nb) of L on rows and columns from base:
-// the whole lower triangle (end = M) or the columns [base, end) of one tile;
+// the whole lower triangle (end = M) or its columns [base, end);
 // one 64 x 64 tile on or below the diagonal per CTA, k in stages of 16 through two buffers of asynchronous copies, both operands
 // [k][row] with re and im side by side (one 16-byte load per fragment).
 //
@@ -143,7 +151,7 @@ __global__ void __launch_bounds__(kLdThreads, 2)
 // memory traffic taken out; a third buffer, a fixed or random start delay per
 // CTA against lockstep, and m8n8k4 fragments measured the same or slower; the
 // full update of the pivoted form takes 38.4 ms); with nb = 256 (ldlt_depth)
-// 17.5.
+// 17.5, 31.5 TFLOP/s.
 __global__ void __launch_bounds__(kLdThreads, 2)
     ldlt_update_kernel(double2 *__restrict__ a, int64_t M, int64_t k0, int nb, int64_t base, int64_t end,
                        const double2 *__restrict__ panel, int64_t panel_stride) {
@@ -153,11 +161,18 @@ __global__ void __launch_bounds__(kLdThreads, 2)
     const double2 *P = panel + (int64_t)blockIdx.y * panel_stride;
     // tile index to (ti >= tj)
     const int tile = blockIdx.x;
-    int ti = (int)((sqrt(8.0 * (double)tile + 1.0) - 1.0) * 0.5);
-    while ((int64_t)ti * (ti + 1) / 2 > tile) --ti;
-    while ((int64_t)(ti + 1) * (ti + 2) / 2 <= tile) ++ti;
-    const int tj = end < M ? 0 : tile - (int)((int64_t)ti * (ti + 1) / 2);
-    if (end < M) ti = tile;
+    int ti, tj;
+    if (end < M) {
+        const int rows = (int)((M - base + kLd - 1) / kLd);
+        tj = tile / rows;
+        ti = tile - tj * rows;
+        if (ti < tj) return;
+    } else {
+        ti = (int)((sqrt(8.0 * (double)tile + 1.0) - 1.0) * 0.5);
+        while ((int64_t)ti * (ti + 1) / 2 > tile) --ti;
+        while ((int64_t)(ti + 1) * (ti + 2) / 2 <= tile) ++ti;
+        tj = tile - (int)((int64_t)ti * (ti + 1) / 2);
+    }
     const int64_t i0 = base + (int64_t)ti * kLd, j0 = base + (int64_t)tj * kLd;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3, wr = warp >> 2, wc = warp & 3;
@@ -309,23 +324,35 @@ __global__ void __launch_bounds__(256) ldlt_back_update_kernel(const double2 *__
     }
 }
 
+// The stream of the panels and the events between it and the updates'.
+struct Ahead {
+    cudaStream_t s = nullptr;
+    cudaEvent_t e[2] = {};
+    ~Ahead() {
+        for (cudaEvent_t x : e)
+            if (x) cudaEventDestroy(x);
+        if (s) stream_release(s);
+    }
+};
+
 // Panels per group: the trailing matrix is updated once per group, by all its
 // columns, and a panel within a group just before its turn, so the traffic of
-// C falls with the depth; but a panel's own update has only the panel's tiles.
-// Where these fill the chip's two CTAs per SM four panels are best, below a
-// third of that one (ms for depths 1, 2, 4: order 6,787, 32 matrices 436, 408,
-// 397; 5 matrices 74.0, 69.8, 68.7; 1 matrix 20.9, 20.3, 20.6; order 2,321,
-// 32 matrices 23.8, 22.9, 22.4; 2 matrices 3.98, 4.18, 4.36).
+// C falls with the depth; but a panel's own update has only the panel's tiles,
+// and the first panels of a matrix wait for nothing else.  Where these fill the
+// chip's two CTAs per SM by a margin four panels are best, below a third of it
+// one (ms for depths 1, 2, 4: order 6,787, 4 matrices 57.9, 53.9, 52.5; 1
+// matrix 18.2, 17.4, 17.8; order 2,321, 32 matrices 23.1, 21.7, 21.2; 8
+// matrices 6.98, 6.74, 7.04; 2 matrices 3.50, 3.69, 4.15).
 int ldlt_depth(int64_t m, int64_t p, int count) {
     const int64_t tiles = (m + p + kLd - 1) / kLd * count;
-    return tiles >= 2 * 148 ? 4 : tiles >= 96 ? 2 : 1;
+    return tiles >= 384 ? 4 : tiles >= 96 ? 2 : 1;
 }
 
 }  // namespace
 
 size_t ldlt_bytes(int64_t m, int64_t p, int count) {
     const int64_t M = m + p, blocks = (m + kLd - 1) / kLd;
-    return (size_t)count * (16 * (size_t)M * kLd * ldlt_depth(m, p, count) + 16 * (size_t)blocks * kLd * kLd + 16 * (size_t)blocks * kLd +
+    return (size_t)count * (32 * (size_t)M * kLd * ldlt_depth(m, p, count) + 16 * (size_t)blocks * kLd * kLd + 16 * (size_t)blocks * kLd +
                             16 * (size_t)M + 16);
 }
 
@@ -335,7 +362,7 @@ fh_status ldlt_factor(const double *Rm, const double *Lm, int64_t m, int64_t p, 
     const int64_t M = m + p, blocks = (m + kLd - 1) / kLd;
     double2 *A = reinterpret_cast<double2 *>(a);
     double2 *panel = static_cast<double2 *>(work);
-    double2 *xinv = panel + (int64_t)count * M * kLd * ldlt_depth(m, p, count);
+    double2 *xinv = panel + (int64_t)count * M * kLd * ldlt_depth(m, p, count) * 2;
     double2 *dinv = xinv + (int64_t)count * blocks * kLd * kLd;
     double *diag = reinterpret_cast<double *>(dinv + (int64_t)count * blocks * kLd);
     double *growth = diag + (int64_t)count * M;
@@ -352,33 +379,74 @@ fh_status ldlt_factor(const double *Rm, const double *Lm, int64_t m, int64_t p, 
     const int64_t xs = blocks * kLd * kLd;
     const int depth = ldlt_depth(m, p, count);
     const int64_t ps = M * kLd * depth;
-    for (int64_t k0 = 0, b = 0; k0 < m; k0 += kLd, ++b) {
-        const int nb = (int)std::min<int64_t>(kLd, m - k0);
-        const int64_t rest = M - k0 - nb, tiles = (rest + kLd - 1) / kLd;
-        const int g = (int)(b % depth), k = g * kLd;  // place in the group, and its columns before this panel
-        double2 *xb = xinv + b * kLd * kLd, *db = dinv + b * count * kLd;
-        if (g > 0) {  // this panel's columns, from the panels of its group
-            prof_begin(s, FH_PROF_GEMM_FP64);
-            ldlt_update_kernel<<<dim3((unsigned)((M - k0 + kLd - 1) / kLd), (unsigned)count), kLdThreads, update_smem,
-                                 s>>>(A, M, k0 - k, k, k0, k0 + nb, panel, ps);
-            prof_end(s, FH_PROF_GEMM_FP64, 8.0 * kLd * (double)(M - k0) * k * count);
-        }
-        prof_begin(s, FH_PROF_PANEL);
-        ldlt_diag_kernel<<<(unsigned)count, kDiagThreads64, 0, s>>>(A, M, k0, nb, xb, xs, db, growth, d_failed);
-        prof_end(s, FH_PROF_PANEL, 0.0);
-        if (tiles == 0) continue;
-        prof_begin(s, FH_PROF_TRSM);
-        ldlt_panel_kernel<<<dim3((unsigned)tiles, (unsigned)count), kLdThreads, panel_smem, s>>>(
-            A, M, k0, nb, xb, xs, db, panel + (int64_t)k * M, ps, growth);
-        prof_end(s, FH_PROF_TRSM, 4.0 * kLd * kLd * (double)rest * count);
-        if (g + 1 == depth || k0 + nb == m) {  // the group is complete: everything right of it
-            prof_begin(s, FH_PROF_GEMM_FP64);
-            ldlt_update_kernel<<<dim3((unsigned)(tiles * (tiles + 1) / 2), (unsigned)count), kLdThreads, update_smem,
-                                 s>>>(A, M, k0 - k, k + nb, k0 + nb, M, panel, ps);
-            prof_end(s, FH_PROF_GEMM_FP64, 4.0 * (double)rest * (double)rest * (k + nb) * count);
-        }
+    // columns [base, end) of the trailing matrix, from the group's panels k0 ..
+    auto update = [&](int64_t k0, int64_t base, int64_t end, const double2 *P, cudaStream_t q) -> fh_status {
+        const int64_t rows = (M - base + kLd - 1) / kLd, cols = (end - base + kLd - 1) / kLd;
+        if (rows <= 0 || cols <= 0) return FH_OK;
+        const int64_t tiles = end < M ? rows * cols : rows * (rows + 1) / 2;
+        const int64_t kk = std::min({base - k0, depth * (int64_t)kLd, m - k0});
+        prof_begin(q, FH_PROF_GEMM_FP64);
+        ldlt_update_kernel<<<dim3((unsigned)tiles, (unsigned)count), kLdThreads, update_smem, q>>>(A, M, k0, (int)kk,
+                                                                                                 base, end, P, ps);
+        const double width = (double)(end - base), height = (double)(M - base);
+        prof_end(q, FH_PROF_GEMM_FP64, 8.0 * (width * height - 0.5 * width * width) * (double)kk * count);
         FHB_CUDA(cudaGetLastError());
+        return FH_OK;
+    };
+    // the panels of the group from column g0 on
+    auto panels = [&](int64_t g0, double2 *P, cudaStream_t q) -> fh_status {
+        for (int64_t k0 = g0; k0 < std::min(m, g0 + depth * kLd); k0 += kLd) {
+            const int64_t b = k0 / kLd, nb = std::min<int64_t>(kLd, m - k0), rest = M - k0 - nb;
+            double2 *xb = xinv + b * kLd * kLd, *db = dinv + b * count * kLd;
+            if (k0 > g0) {
+                const fh_status e = update(g0, k0, k0 + nb, P, q);
+                if (e) return e;
+            }
+            prof_begin(q, FH_PROF_PANEL);
+            ldlt_diag_kernel<<<(unsigned)count, kDiagThreads64, 0, q>>>(A, M, k0, (int)nb, xb, xs, db, growth,
+                                                                       d_failed);
+            prof_end(q, FH_PROF_PANEL, 0.0);
+            if (rest > 0) {
+                prof_begin(q, FH_PROF_TRSM);
+                ldlt_panel_kernel<<<dim3((unsigned)((rest + kLd - 1) / kLd), (unsigned)count), kLdThreads, panel_smem,
+                                    q>>>(A, M, k0, (int)nb, xb, xs, db, P + (k0 - g0) * M, ps, growth);
+                prof_end(q, FH_PROF_TRSM, 4.0 * kLd * kLd * (double)rest * count);
+            }
+            FHB_CUDA(cudaGetLastError());
+        }
+        return FH_OK;
+    };
+    Ahead ahead;
+    if (m >= kAheadOrder) {
+        FHB_CUDA(stream_acquire(&ahead.s, true));
+        for (cudaEvent_t &e : ahead.e) FHB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
+    const cudaStream_t q = ahead.s ? ahead.s : s;
+    auto hand_over = [&](cudaStream_t from, cudaStream_t to, cudaEvent_t e) -> fh_status {
+        if (from == to) return FH_OK;
+        FHB_CUDA(cudaEventRecord(e, from));
+        FHB_CUDA(cudaStreamWaitEvent(to, e, 0));
+        return FH_OK;
+    };
+    fh_status st = hand_over(s, q, ahead.e[0]);
+    if (!st && m > 0) st = panels(0, panel, q);
+    for (int64_t k0 = 0, group = 0; !st && k0 < m; k0 += depth * kLd, ++group) {
+        double2 *P = panel + (group & 1) * count * ps, *next = panel + ((group + 1) & 1) * count * ps;
+        const int64_t base = std::min(m, k0 + depth * kLd), end = std::min(m, base + depth * kLd);
+        if (!ahead.s) {
+            st = update(k0, base, M, P, s);
+            if (!st && base < m) st = panels(base, next, s);
+            continue;
+        }
+        st = hand_over(q, s, ahead.e[1]);
+        if (!st && base < m) {
+            st = update(k0, base, end, P, s);
+            if (!st) st = hand_over(s, q, ahead.e[0]);
+            if (!st) st = panels(base, next, q);
+        }
+        if (!st && end < M) st = update(k0, end, M, P, s);
+    }
+    if (st) return st;
     if (m > 0) ldlt_growth_kernel<<<(unsigned)count, 256, 0, s>>>(growth, diag, M, m, d_failed);
     if (p > 0)
         ldlt_z_kernel<<<(unsigned)std::min<int64_t>(((int64_t)count * p * p + 255) / 256, 1024), 256, 0, s>>>(

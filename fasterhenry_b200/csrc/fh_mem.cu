@@ -20,8 +20,8 @@ cudaMemPool_t g_pool[kMaxDevices] = {};
 // Idle streams per device: creating and destroying the two of a system takes
 // 0.35 ms, a tenth of a whole call at 240 filaments.
 constexpr int kIdleStreams = 8;
-cudaStream_t g_idle[kMaxDevices][kIdleStreams] = {};
-int g_idle_count[kMaxDevices] = {};
+cudaStream_t g_idle[2][kMaxDevices][kIdleStreams] = {};  // of the default priority, of the highest
+int g_idle_count[2][kMaxDevices] = {};
 }  // namespace
 
 cudaError_t cache_pool(cudaMemPool_t *out) {
@@ -72,28 +72,32 @@ void cache_free(void *p, cudaStream_t s) {
     if (p) cudaFreeAsync(p, s);
 }
 
-cudaError_t stream_acquire(cudaStream_t *s) {
-    int dev = 0;
+cudaError_t stream_acquire(cudaStream_t *s, bool urgent) {
+    int dev = 0, least = 0, greatest = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     {
         std::lock_guard<std::mutex> lk(g_mu);
-        if (dev >= 0 && dev < kMaxDevices && g_idle_count[dev] > 0) {
-            *s = g_idle[dev][--g_idle_count[dev]];
+        if (dev >= 0 && dev < kMaxDevices && g_idle_count[urgent][dev] > 0) {
+            *s = g_idle[urgent][dev][--g_idle_count[urgent][dev]];
             return cudaSuccess;
         }
     }
-    return cudaStreamCreateWithFlags(s, cudaStreamNonBlocking);
+    if (!urgent) return cudaStreamCreateWithFlags(s, cudaStreamNonBlocking);
+    e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
+    return e != cudaSuccess ? e : cudaStreamCreateWithPriority(s, cudaStreamNonBlocking, greatest);
 }
 
 // Work still pending on it (frees) stays ahead of what its next owner enqueues.
 void stream_release(cudaStream_t s) {
     if (!s) return;
-    int dev = -1;
-    if (cudaStreamGetDevice(s, &dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices) {
+    int dev = -1, priority = 0;
+    if (cudaStreamGetDevice(s, &dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices &&
+        cudaStreamGetPriority(s, &priority) == cudaSuccess) {
+        const int urgent = priority < 0;
         std::lock_guard<std::mutex> lk(g_mu);
-        if (g_idle_count[dev] < kIdleStreams) {
-            g_idle[dev][g_idle_count[dev]++] = s;
+        if (g_idle_count[urgent][dev] < kIdleStreams) {
+            g_idle[urgent][dev][g_idle_count[urgent][dev]++] = s;
             return;
         }
     }
@@ -128,7 +132,8 @@ extern "C" fh_status fh_release_cached_memory(void) {
         cudaSetDevice(d);
         cudaDeviceSynchronize();
         cudaMemPoolTrimTo(fhb::g_pool[d], 0);
-        while (fhb::g_idle_count[d] > 0) cudaStreamDestroy(fhb::g_idle[d][--fhb::g_idle_count[d]]);
+        for (int u = 0; u < 2; ++u)
+            while (fhb::g_idle_count[u][d] > 0) cudaStreamDestroy(fhb::g_idle[u][d][--fhb::g_idle_count[u][d]]);
     }
     cudaSetDevice(cur);
     return FH_OK;

@@ -55,6 +55,24 @@ def test_matches_numpy(fh, m, p):
         assert w != 0.0 or not z[k].imag.any()
 
 
+@pytest.mark.parametrize("m,count", [(65, 24), (130, 140), (256, 80), (257, 30), (321, 24), (577, 48), (640, 40)])
+@pytest.mark.parametrize("p", [1, 70])
+def test_groups_of_panels(fh, m, p, count):
+    """Enough matrices for groups of two and of four panels (partial ones at the
+    end, and orders on both sides of the panels' own stream)."""
+    rng = np.random.default_rng(10 * m + p)
+    r, l = spd(rng, m + p), spd(rng, m + p)
+    omega = np.linspace(0.0, 3.0, count)
+    z, x, failed = solve(r, l, m, p, omega)
+    assert not failed.any()
+    for k in [0, 1, count // 2, count - 1]:
+        a = r + 1j * omega[k] * l
+        want_x = np.linalg.solve(a[:m, :m], a[:m, m:])
+        want_z = a[m:, m:] - a[m:, :m] @ want_x
+        assert np.max(np.abs(x[k].T - want_x)) <= 1e-11 * np.max(np.abs(want_x))
+        assert np.max(np.abs(z[k] - want_z)) <= 1e-11 * np.max(np.abs(want_z))
+
+
 @pytest.mark.parametrize("m", [40, 64, 150])
 def test_rejects_what_needs_pivoting(fh, m):
     """Rows whose elimination grows: a tiny leading pivot against O(1)
