@@ -410,8 +410,8 @@ __global__ void __launch_bounds__(128) bwd_panel_kernel2(const Cx<T> *__restrict
 
 // The diagonal block of a factorization without pivoting, in one CTA per
 // matrix: the LU of the nb x nb block at (k0, k0) in place (L unit lower below
-// the diagonal, U on and above it), then L^{-1} into linv and U^{-1} into
-// uinv (matrix f at + f * mstride, column-major with leading dimension nb);
+// the diagonal, U on and above it), L^{-1} into linv and U^{-1} into uinv
+// (matrix f at + f * mstride, column-major with leading dimension nb);
 // optionally U^{-1} also into x2 (matrix f at + f * stride2, leading dimension
 // ld2) and the diagonal of U into dv (matrix f at + f * dstride).
 // For A = R + jwL with R and L symmetric positive definite (a mesh impedance
@@ -426,17 +426,20 @@ __global__ void __launch_bounds__(128) bwd_panel_kernel2(const Cx<T> *__restrict
 // and row k of the block as step k - 1 left them; the owners write those
 // entries to a shared double buffer right after their own update of step
 // k - 1 (with the reciprocal of the next pivot), so a step costs one barrier.
-// The LU is one kernel (diag_lu_kernel); the two inverses, which need only
-// the factors, run as two CTAs per matrix of a second (diag_inv_kernel).
 // The steps run in eight segments of 16 (a template per segment): inside one,
-// the row group and the column slot of k are constants, so the row groups and
-// column slots a step does not touch are left out at compile time and every
-// register index is a constant.  The inverses run in the same registers with
-// the factors kept in shared memory: X = L^{-1} by forward elimination on the
-// rows of I (row k of X is final before step k), Y = U^{-1} backward (row k
-// scaled by 1 / U_kk at step k, every thread scaling the published row).
+// the row group and the column slot of k are constants, so the row groups that
+// a step does not touch are left out at compile time and every register index
+// is a constant.
+//
+// L^{-1} comes out of the same steps (Gauss-Jordan): column k's places below the
+// diagonal take -l_rk once L has been stored, and every later step updates
+// them with the row it publishes, as it does the columns right of the pivot.
+// The matrix is symmetric, U = D L^T, so U^{-1} is the transpose of L^{-1}
+// times D^{-1} and needs no steps of its own.  Bound by the chain of nb steps:
+// 92 us for 128, where the LU took 78 and a second launch for the two
+// inverses 63.
 constexpr int kDiagThreads = 512;
-constexpr int kDiagSmemExtra = 2 * 128 + 2 * 128 + 128 + 2;  // complex entries besides the nb x nb factors
+constexpr int kDiagPitch = 129;  // of L^{-1} D^{-1} in shared memory, on its way to be transposed
 using Cf = Cx<float>;
 
 // y -= f x as four fused multiply-adds.
@@ -453,7 +456,6 @@ __device__ __forceinline__ Cf crcp(Cf p) {
 }
 
 struct DiagSmem {
-    Cf *S;     // the factors, column-major, ld nb
     Cf *colb;  // [2][128]
     Cf *rowb;  // [2][128], column c of a row at (c % 16) * 8 + c / 16 (diag_row_slot)
     Cf *dinv;  // [128]: 1 / U_kk
@@ -475,7 +477,7 @@ __device__ __forceinline__ void diag_store_row(const Cf (&v)[4][8], int warp, Cf
 
 // Column k1 (slot J, rows >= k1) and row k1 (group I) of the block into cn /
 // rn, and 1 / a(k1, k1) into *pn.  The row is written whole: its columns
-// < k1 are never read.
+// < k1 are row k1 of L^{-1}.
 template <int J, int I>
 __device__ __forceinline__ void diag_publish(const Cf (&v)[4][8], int k1, int nb, int lane, int warp, Cf *cn, Cf *rn,
                                              Cf *pn) {
@@ -492,9 +494,10 @@ __device__ __forceinline__ void diag_publish(const Cf (&v)[4][8], int k1, int nb
     }
 }
 
-// LU steps k in [16 JS, 16 JS + 16):  l_r = a_rk / a_kk,  a_rc -= l_r a_kc  (r, c > k).
+// Steps k in [16 JS, 16 JS + 16):  l_r = a_rk / a_kk,  a_rc -= l_r a_kc  (r > k, c /= k),  a_rk = -l_r.
 template <int JS>
-__device__ __forceinline__ void diag_lu_segment(Cf (&v)[4][8], int nb, int lane, int warp, const DiagSmem &sm) {
+__device__ __forceinline__ void diag_lu_segment(Cf (&v)[4][8], Cf *A, int64_t m, int nb, int lane, int warp,
+                                                const DiagSmem &sm) {
     constexpr int IS = JS / 2;  // row group of k
     const Cf zero{0.f, 0.f};
 #pragma unroll 1
@@ -503,6 +506,7 @@ __device__ __forceinline__ void diag_lu_segment(Cf (&v)[4][8], int nb, int lane,
         if (k >= nb) return;  // uniform
         const int b = k & 1, k1 = k + 1;
         const Cf inv = sm.pinv[b];
+        if (threadIdx.x == 0) sm.dinv[k] = inv;
         Cf l[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -511,17 +515,20 @@ __device__ __forceinline__ void diag_lu_segment(Cf (&v)[4][8], int nb, int lane,
             if (i >= IS && (i > IS || r > k) && r < nb) l[i] = cmul(sm.colb[b * 128 + r], inv);
         }
 #pragma unroll
-        for (int j = JS; j < 8; ++j) {
+        for (int j = 0; j < 8; ++j) {
             const int c = warp + 16 * j;
-            if (j == JS && warp <= kk) {
-                if (warp == kk) {  // column k takes the multipliers
+            if (j == JS && warp == kk) {  // column k of L, and the start of L^{-1}'s
 #pragma unroll
-                    for (int i = IS; i < 4; ++i)
-                        if (i > IS || lane + 32 * i > k) v[i][j] = l[i];
+                for (int i = IS; i < 4; ++i) {
+                    const int r = lane + 32 * i;
+                    if (i > IS || r > k) {
+                        if (r < nb) A[r + (int64_t)c * m] = l[i];
+                        v[i][j] = Cf{-l[i].re, -l[i].im};
+                    }
                 }
                 continue;
             }
-            if (c >= nb) continue;
+            if (j >= JS && c >= nb) continue;
             const Cf u = sm.rowb[b * 128 + warp * 8 + j];
 #pragma unroll
             for (int i = IS; i < 4; ++i) cfms(v[i][j], l[i], u);  // l = 0 on rows <= k
@@ -532,98 +539,6 @@ __device__ __forceinline__ void diag_lu_segment(Cf (&v)[4][8], int nb, int lane,
                 diag_publish<JS, IS>(v, k1, nb, lane, warp, cn, rn, sm.pinv + (b ^ 1));
             } else if constexpr (JS < 7) {
                 diag_publish<JS + 1, (JS + 1) / 2>(v, k1, nb, lane, warp, cn, rn, sm.pinv + (b ^ 1));
-            }
-        }
-        __syncthreads();
-    }
-}
-
-// Row k + 1 (group I) of X into rn: its owner's registers hold the whole
-// row (columns <= k as step k left them, 1 at k + 1, zeros after).
-template <int I>
-__device__ __forceinline__ void diag_publish_xrow(const Cf (&v)[4][8], int k, int lane, int warp, Cf *rn) {
-    if (lane == ((k + 1) & 31)) diag_store_row<I>(v, warp, rn);
-}
-
-// X = L^{-1} steps k in [16 JS, 16 JS + 16):  X[r][:] -= L[r][k] X[k][:]  (r > k; X[k][c] = 0 for c > k).
-template <int JS>
-__device__ __forceinline__ void diag_linv_segment(Cf (&v)[4][8], int nb, int lane, int warp, const DiagSmem &sm) {
-    constexpr int IS = JS / 2;
-    const Cf zero{0.f, 0.f};
-#pragma unroll 1
-    for (int kk = 0; kk < 16; ++kk) {
-        const int k = 16 * JS + kk;
-        if (k + 1 >= nb) return;  // uniform
-        const int b = k & 1;
-        Cf *rn = sm.rowb + (b ^ 1) * 128;
-        Cf lk[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            lk[i] = zero;
-            const int r = lane + 32 * i;
-            if (i >= IS && (i > IS || r > k) && r < nb) lk[i] = sm.S[r + k * nb];
-        }
-#pragma unroll
-        for (int j = 0; j <= JS; ++j) {
-            if (j == JS && warp > kk) continue;  // columns c <= k only
-            const Cf xk = sm.rowb[b * 128 + warp * 8 + j];
-#pragma unroll
-            for (int i = IS; i < 4; ++i) cfms(v[i][j], lk[i], xk);
-        }
-        if (kk < 15) {
-            diag_publish_xrow<IS>(v, k, lane, warp, rn);
-        } else if constexpr (JS < 7) {
-            diag_publish_xrow<(JS + 1) / 2>(v, k, lane, warp, rn);
-        }
-        __syncthreads();
-    }
-}
-
-// Row km (group I) of Y before its scaling into rn: its owner's registers
-// hold the whole row (zeros before km, 1 at km, columns >= k as step k left
-// them).
-template <int I>
-__device__ __forceinline__ void diag_publish_yrow(const Cf (&v)[4][8], int km, int lane, int warp, Cf *rn) {
-    if (lane == (km & 31)) diag_store_row<I>(v, warp, rn);
-}
-
-// Y = U^{-1} steps k = 16 JS + 15 .. 16 JS:  Y[k][:] /= U_kk;  Y[r][:] -= U[r][k] Y[k][:]  (r < k;
-// Y[k][c] = 0 for c < k).  t counts the steps taken (buffer parity).
-template <int JS>
-__device__ __forceinline__ void diag_uinv_segment(Cf (&v)[4][8], int nb, int lane, int warp, const DiagSmem &sm,
-                                                  int &t) {
-    constexpr int IS = JS / 2;
-    const Cf zero{0.f, 0.f};
-#pragma unroll 1
-    for (int kk = 15; kk >= 0; --kk) {
-        const int k = 16 * JS + kk;
-        if (k >= nb) continue;  // uniform
-        const int b = t & 1, km = k - 1;
-        ++t;
-        Cf *rn = sm.rowb + (b ^ 1) * 128;
-        const Cf inv = sm.dinv[k];
-        Cf uk[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            uk[i] = zero;
-            const int r = lane + 32 * i;
-            if (i <= IS && (i < IS || r < k)) uk[i] = sm.S[r + k * nb];
-        }
-#pragma unroll
-        for (int j = JS; j < 8; ++j) {
-            const int c = warp + 16 * j;
-            if (j == JS && warp < kk) continue;  // columns c >= k only
-            if (c >= nb) continue;
-            const Cf yk = cmul(sm.rowb[b * 128 + warp * 8 + j], inv);
-#pragma unroll
-            for (int i = 0; i <= IS; ++i) cfms(v[i][j], uk[i], yk);  // uk = 0 on rows >= k
-            if (lane == (k & 31)) v[IS][j] = yk;                       // row k, scaled
-        }
-        if (km >= 0) {
-            if (kk > 0) {
-                diag_publish_yrow<IS>(v, km, lane, warp, rn);
-            } else if constexpr (JS > 0) {
-                diag_publish_yrow<(16 * JS - 1) / 32>(v, km, lane, warp, rn);
             }
         }
         __syncthreads();
@@ -641,20 +556,23 @@ __device__ __forceinline__ Cf csqrt_principal(Cf z) {
 }
 
 // LU of the block in place (the diagonal of U into dv and its principal
-// square roots into sv, when given); one CTA per matrix.
+// square roots into sv, when given) and the inverses; one CTA per matrix.
 __global__ void __launch_bounds__(kDiagThreads, 1)
     diag_lu_kernel(Cx<float> *__restrict__ a, int64_t m, int64_t k0, int nb, Cx<float> *__restrict__ dv,
-                   Cx<float> *__restrict__ sv, int64_t dstride) {
-    __shared__ __align__(16) Cf bufs[2 * 128 + 2 * 128 + 2];
+                   Cx<float> *__restrict__ sv, int64_t dstride, Cx<float> *__restrict__ linv,
+                   Cx<float> *__restrict__ uinv, int64_t mstride, Cx<float> *__restrict__ x2, int64_t ld2,
+                   int64_t stride2) {
+    __shared__ __align__(16) Cf bufs[2 * 128 + 2 * 128 + 128 + 2];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    Cf *T = reinterpret_cast<Cf *>(smem_raw);  // (U^{-1})^T, row r at r, column c at c kDiagPitch
     DiagSmem sm;
-    sm.S = nullptr;
     sm.colb = bufs;
     sm.rowb = bufs + 256;
-    sm.dinv = nullptr;
-    sm.pinv = bufs + 512;
+    sm.dinv = bufs + 512;
+    sm.pinv = bufs + 640;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     Cf *A = a + (int64_t)blockIdx.x * m * m + k0 + k0 * m;
-    const Cf zero{0.f, 0.f};
+    const Cf zero{0.f, 0.f}, one{1.f, 0.f};
     Cf v[4][8];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -665,93 +583,37 @@ __global__ void __launch_bounds__(kDiagThreads, 1)
         }
     diag_publish<0, 0>(v, 0, nb, lane, warp, sm.colb, sm.rowb, sm.pinv);  // column 0, row 0, 1 / a_00
     __syncthreads();
-    diag_lu_segment<0>(v, nb, lane, warp, sm);
-    diag_lu_segment<1>(v, nb, lane, warp, sm);
-    diag_lu_segment<2>(v, nb, lane, warp, sm);
-    diag_lu_segment<3>(v, nb, lane, warp, sm);
-    diag_lu_segment<4>(v, nb, lane, warp, sm);
-    diag_lu_segment<5>(v, nb, lane, warp, sm);
-    diag_lu_segment<6>(v, nb, lane, warp, sm);
-    diag_lu_segment<7>(v, nb, lane, warp, sm);
+    diag_lu_segment<0>(v, A, m, nb, lane, warp, sm);
+    diag_lu_segment<1>(v, A, m, nb, lane, warp, sm);
+    diag_lu_segment<2>(v, A, m, nb, lane, warp, sm);
+    diag_lu_segment<3>(v, A, m, nb, lane, warp, sm);
+    diag_lu_segment<4>(v, A, m, nb, lane, warp, sm);
+    diag_lu_segment<5>(v, A, m, nb, lane, warp, sm);
+    diag_lu_segment<6>(v, A, m, nb, lane, warp, sm);
+    diag_lu_segment<7>(v, A, m, nb, lane, warp, sm);
+    Cf *li = linv + (int64_t)blockIdx.x * mstride, *ui = uinv + (int64_t)blockIdx.x * mstride;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const int r = lane + 32 * i, c = warp + 16 * j;
-            if (r < nb && c < nb) {
-                A[r + (int64_t)c * m] = v[i][j];
-                if (dv && r == c) {
-                    dv[(int64_t)blockIdx.x * dstride + r] = v[i][j];
-                    sv[(int64_t)blockIdx.x * dstride + r] = csqrt_principal(v[i][j]);
-                }
+            if (r >= nb || c >= nb) continue;
+            if (r <= c) A[r + (int64_t)c * m] = v[i][j];
+            if (dv && r == c) {
+                dv[(int64_t)blockIdx.x * dstride + r] = v[i][j];
+                sv[(int64_t)blockIdx.x * dstride + r] = csqrt_principal(v[i][j]);
             }
+            const Cf x = r > c ? v[i][j] : r == c ? one : zero;
+            li[r + c * nb] = x;
+            T[r + c * kDiagPitch] = r >= c ? cmul(x, sm.dinv[r]) : zero;
         }
-}
-
-// The inverses of the factored block's L (blockIdx.y == 0, into linv) and U
-// (blockIdx.y == 1, into uinv and optionally x2), in parallel: CTA (f, y).
-__global__ void __launch_bounds__(kDiagThreads, 1)
-    diag_inv_kernel(const Cx<float> *__restrict__ a, int64_t m, int64_t k0, int nb, Cx<float> *__restrict__ linv,
-                    Cx<float> *__restrict__ uinv, int64_t mstride, Cx<float> *__restrict__ x2, int64_t ld2,
-                    int64_t stride2) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    DiagSmem sm;
-    sm.colb = reinterpret_cast<Cf *>(smem_raw);  // the buffers first: 16-byte aligned for any nb
-    sm.rowb = sm.colb + 256;
-    sm.dinv = sm.rowb + 256;
-    sm.pinv = sm.dinv + 128;
-    sm.S = sm.pinv + 2;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const bool upper = blockIdx.y == 1;
-    const Cf *A = a + (int64_t)blockIdx.x * m * m + k0 + k0 * m;
-    const Cf zero{0.f, 0.f}, one{1.f, 0.f};
-    for (int idx = threadIdx.x; idx < nb * nb; idx += kDiagThreads) {
-        const int r = idx % nb, c = idx / nb;
-        sm.S[idx] = A[r + (int64_t)c * m];
-    }
     __syncthreads();
-    if (threadIdx.x < nb) sm.dinv[threadIdx.x] = crcp(sm.S[threadIdx.x + threadIdx.x * nb]);
-    // the first row the elimination reads: row 0 of I (X) or row nb - 1 of I (Y, before scaling)
-    if (threadIdx.x < 128) sm.rowb[diag_row_slot(threadIdx.x)] = (int)threadIdx.x == (upper ? nb - 1 : 0) ? one : zero;
-    Cf v[4][8];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[i][j] = (lane + 32 * i == warp + 16 * j) ? one : zero;
-    __syncthreads();
-    Cf *out;
-    if (!upper) {
-        diag_linv_segment<0>(v, nb, lane, warp, sm);
-        diag_linv_segment<1>(v, nb, lane, warp, sm);
-        diag_linv_segment<2>(v, nb, lane, warp, sm);
-        diag_linv_segment<3>(v, nb, lane, warp, sm);
-        diag_linv_segment<4>(v, nb, lane, warp, sm);
-        diag_linv_segment<5>(v, nb, lane, warp, sm);
-        diag_linv_segment<6>(v, nb, lane, warp, sm);
-        diag_linv_segment<7>(v, nb, lane, warp, sm);
-        out = linv + (int64_t)blockIdx.x * mstride;
-    } else {
-        int t = 0;
-        diag_uinv_segment<7>(v, nb, lane, warp, sm, t);
-        diag_uinv_segment<6>(v, nb, lane, warp, sm, t);
-        diag_uinv_segment<5>(v, nb, lane, warp, sm, t);
-        diag_uinv_segment<4>(v, nb, lane, warp, sm, t);
-        diag_uinv_segment<3>(v, nb, lane, warp, sm, t);
-        diag_uinv_segment<2>(v, nb, lane, warp, sm, t);
-        diag_uinv_segment<1>(v, nb, lane, warp, sm, t);
-        diag_uinv_segment<0>(v, nb, lane, warp, sm, t);
-        out = uinv + (int64_t)blockIdx.x * mstride;
-    }
-    Cf *out2 = upper && x2 ? x2 + (int64_t)blockIdx.x * stride2 : nullptr;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int r = lane + 32 * i, c = warp + 16 * j;
-            if (r < nb && c < nb) {
-                out[r + c * nb] = v[i][j];
-                if (out2) out2[r + (int64_t)c * ld2] = v[i][j];
-            }
+    Cf *u2 = x2 ? x2 + (int64_t)blockIdx.x * stride2 : nullptr;
+    for (int c = warp; c < nb; c += kDiagThreads / 32)
+        for (int r = lane; r < nb; r += 32) {
+            const Cf y = T[c + r * kDiagPitch];
+            ui[r + c * nb] = y;
+            if (u2) u2[r + (int64_t)c * ld2] = y;
         }
 }
 
@@ -1344,8 +1206,8 @@ fh_status lu_factor_deep(LuBatch<float> &b, LuWork &w, int nb, cudaStream_t s, f
     FHB_CUDA(cudaMemsetAsync(w.coop->error, 0, sizeof(int), s));
     if (nopivot) {
         if (!w.uinv) return fail(err, FH_ERR_INVALID_ARGUMENT, "the factorization without pivoting needs uinv");
-        const size_t diag_smem = sizeof(C) * ((size_t)nb * nb + kDiagSmemExtra);
-        FHB_CUDA(cudaFuncSetAttribute(diag_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)diag_smem));
+        FHB_CUDA(cudaFuncSetAttribute(diag_lu_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(sizeof(C) * 128 * kDiagPitch)));
         const int64_t total = (int64_t)count * m;
         identity_pivots_kernel<<<grid_for(total, 256, 1024), 256, 0, s>>>(b.pivots, total, m);
         FHB_CUDA(cudaGetLastError());
@@ -1423,11 +1285,9 @@ fh_status lu_factor_deep(LuBatch<float> &b, LuWork &w, int nb, cudaStream_t s, f
                 // (with the fused pass: U^-1 also into X's diagonal block, and
                 // U's diagonal into dvec).
                 const int64_t o = j0 - K0;
-                diag_lu_kernel<<<(unsigned)count, kDiagThreads, 0, sx>>>(a, m, j0, wj, below ? dvec + o : nullptr,
-                                                                        below ? svec + o : nullptr, W);
-                diag_inv_kernel<<<dim3((unsigned)count, 2), kDiagThreads, sizeof(C) * ((size_t)wj * wj + kDiagSmemExtra),
-                                  sx>>>(a, m, j0, wj, linv, slot(w.uinv, j0), mstride, below ? xinv + o + o * W : nullptr,
-                                       W, (int64_t)W * W);
+                diag_lu_kernel<<<(unsigned)count, kDiagThreads, sizeof(C) * (size_t)wj * kDiagPitch, sx>>>(
+                    a, m, j0, wj, below ? dvec + o : nullptr, below ? svec + o : nullptr, W, linv, slot(w.uinv, j0),
+                    mstride, below ? xinv + o + o * W : nullptr, W, (int64_t)W * W);
                 st = cudaGetLastError() == cudaSuccess ? FH_OK
                                                        : fail(err, FH_ERR_CUDA, "diagonal block factorization launch failed");
             } else {
