@@ -340,7 +340,7 @@ class SolverChoice(enum.IntEnum):
 
 
 class Precision(enum.IntEnum):
-    """FP64: the reference's FP64 LU.  MIXED_BF16X3: FP32 factors with
+    """FP64: factors in FP64 (interchanges only where growth asks for them).  MIXED_BF16X3: FP32 factors with
     split-BF16 x3 tensor-core trailing updates and FP64-residual refinement."""
     FP64 = 0
     MIXED_BF16X3 = 1

@@ -158,7 +158,7 @@ typedef enum fh_solver_choice {
 /* How the per-frequency complex LU is computed (no reference counterpart:
  * the reference always runs the FP64 form). */
 typedef enum fh_precision {
-    FH_PRECISION_FP64 = 0,          /* FP64 blocked LU, partial pivoting (dense.rs) */
+    FH_PRECISION_FP64 = 0,          /* FP64 L D L^T, where growth asks for it LU with partial pivoting (dense.rs) */
     FH_PRECISION_MIXED_BF16X3 = 1,  /* FP32 panels, split-BF16 x3 tensor-core trailing
                                        updates, FP64-residual iterative refinement */
     FH_PRECISION_MIXED_FP32 = 2     /* FP32 factors with FP32 SIMT trailing updates,
