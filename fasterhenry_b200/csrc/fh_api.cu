@@ -709,7 +709,22 @@ fh_status batch_sweep_persistent(fh_system *const *systems, size_t k, const doub
     std::vector<double> z((size_t)(2 * std::max<int64_t>(1, zoff.back())));
     std::vector<int32_t> status((size_t)std::max(1, nitems), 0);
     if (nitems > 0) {
-        int ctas = std::min(batch_resident_ctas(), nitems);
+        double work = 0.0;
+        auto cost = [&](const BatchItem &it) {
+            return 4.0 / 3.0 * std::pow((double)(sys[it.sys].m + sys[it.sys].p), 3.0);
+        };
+        for (const BatchItem &it : items) work += cost(it);
+        // An item well above a CTA's even share of the work would set the time
+        // of the whole batch on its own, and a batch of few items leaves CTAs
+        // without one: a group of CTAs takes such an item.  Spirals of orders
+        // 56-736 at 16 frequencies, items above 1, 1.5 and 2 shares grouped and
+        // none: 64 spirals 3.84, 3.60, 4.48 and 7.44 ms; 40 spirals 2.53, 2.23,
+        // 2.98 and 6.57; 25 spirals 1.15, 1.08, 1.08 and 2.92; 4 spirals at 2
+        // frequencies 0.72 with and 1.77 without.
+        const int resident = batch_resident_ctas();
+        int grouped = 0;
+        while (grouped < nitems && cost(items[(size_t)grouped]) > 1.5 * work / resident) ++grouped;
+        int ctas = (int)std::min<int64_t>(resident, (int64_t)kBatchGroup * grouped + (nitems - grouped));
         const size_t slot = batch_slot_bytes(mmax, pmax);
         PBuf<unsigned char> d_items, d_z, d_status, d_counter, d_work;
         FHB_PALLOC(pool, d_items, kSlotBatchItems, sizeof(BatchItem) * items.size());
@@ -724,18 +739,6 @@ fh_status batch_sweep_persistent(fh_system *const *systems, size_t k, const doub
         }
         FHB_PALLOC(pool, d_work, kSlotBatchWork, slot * (size_t)ctas);
         FHB_CUDA(cudaMemcpyAsync(d_items.p, items.data(), sizeof(BatchItem) * items.size(), cudaMemcpyHostToDevice, st));
-        double work = 0.0;
-        auto cost = [&](const BatchItem &it) {
-            return 4.0 / 3.0 * std::pow((double)(sys[it.sys].m + sys[it.sys].p), 3.0);
-        };
-        for (const BatchItem &it : items) work += cost(it);
-        // An item of more than a CTA's even share of the work would set the
-        // time of the whole batch on its own: a group of CTAs takes it (64
-        // spirals of orders 56-736 x 16 frequencies: 3.8 ms from one share on;
-        // 3.7, 4.6 and 7.5 ms from 1.5, 2 and 3, 4.3 from half a share, 5.1
-        // with every item grouped, 7.5 with none).
-        int grouped = 0;
-        while (grouped < nitems && cost(items[(size_t)grouped]) > work / ctas) ++grouped;
         prof_begin(st, FH_PROF_BATCH);
         fh_status e = batch_launch(reinterpret_cast<const BatchSys *>(d_sys.p),
                                    reinterpret_cast<const BatchItem *>(d_items.p), nitems, grouped,

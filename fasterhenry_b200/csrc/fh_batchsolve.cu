@@ -32,7 +32,7 @@
 // while the others take the sums of theirs; one cluster barrier hands them
 // L_jj^-1, a second ends the column.
 //
-// 64 spirals of orders 56-736 x 16 frequencies on one B200: 3.8 ms, 14.5 of
+// 64 spirals of orders 56-736 x 16 frequencies on one B200: 3.6 ms, 15 of
 // the 37 TFLOP/s of the instruction, bound by the diagonal blocks' chains and
 // by few tiles per column (7.5 ms with a CTA for every item, 36 ms with FP32
 // factors from the scalar pipes and FP64 refinement).

@@ -35,9 +35,9 @@ constexpr int kBatchConfigs = 4;
 constexpr int kBatchEdge[kBatchConfigs] = {32, 32, 64, 64};
 constexpr int kBatchStage[kBatchConfigs] = {16, 32, 8, 16};
 constexpr int kBatchBuffers[kBatchConfigs] = {4, 2, 4, 2};
-// CTAs that share an item of the leading, grouped ones: a cluster (3.8 ms for
-// 64 spirals of orders 56-736 x 16 frequencies; clusters of 2 take 4.1, of 8
-// 4.8).
+// CTAs that share an item of the leading, grouped ones: a cluster (3.6 ms for
+// 64 spirals of orders 56-736 x 16 frequencies; clusters of 2 take a twelfth
+// more, of 8 a fourth more).
 constexpr int kBatchGroup = 4;
 
 size_t batch_smem_bytes();
