@@ -1169,7 +1169,8 @@ fh_status fh_sweep(fh_system *sys, const double *freqs, size_t nf, fh_precision 
     // each), the inverses of the diagonal blocks of L and U, and a
     // super-panel's U^-1 in FP32 and packed.
     const double per = (mixed ? 8.0 * (double)m * (double)m
-                              : 16.0 * (double)(m + p) * (double)(m + p) + (double)ldlt_bytes(m, p, 1)) +
+                              : 16.0 * (double)(m + p) * (double)(m + p) +
+                                    (double)ldlt_bytes(m, p, (int)nf) / (double)std::max<size_t>(1, nf)) +
                        64.0 * (double)(m * p + 64) +
                        (outer_for(m, update) ? 16.0 * (double)m * kOuterFp32 + 16.0 * (double)(m + kNbFp32) * kNbFp32 +
                                                    16.0 * kOuterFp32 * kOuterFp32 + 8.0 * kNbFp32 * kOuterFp32

@@ -328,7 +328,9 @@ __global__ void __launch_bounds__(256) ldlt_back_update_kernel(const double2 *__
 struct Ahead {
     cudaStream_t s = nullptr;
     cudaEvent_t e[2] = {};
+    bool joined = false;  // the caller's stream waits for all of it
     ~Ahead() {
+        if (s && !joined) cudaStreamSynchronize(s);  // an error return: the buffers are the caller's
         for (cudaEvent_t x : e)
             if (x) cudaEventDestroy(x);
         if (s) stream_release(s);
@@ -352,8 +354,9 @@ int ldlt_depth(int64_t m, int64_t p, int count) {
 
 size_t ldlt_bytes(int64_t m, int64_t p, int count) {
     const int64_t M = m + p, blocks = (m + kLd - 1) / kLd;
-    return (size_t)count * (32 * (size_t)M * kLd * ldlt_depth(m, p, count) + 16 * (size_t)blocks * kLd * kLd + 16 * (size_t)blocks * kLd +
-                            16 * (size_t)M + 16);
+    // two groups of panels, the diagonal blocks' inverses, D^-1, the rows' growth and diagonal
+    return (size_t)count * (32 * (size_t)M * kLd * ldlt_depth(m, p, count) + 16 * (size_t)blocks * kLd * kLd +
+                            16 * (size_t)blocks * kLd + 16 * (size_t)M + 16);
 }
 
 fh_status ldlt_factor(const double *Rm, const double *Lm, int64_t m, int64_t p, const double *d_omega, int count,
@@ -447,6 +450,7 @@ fh_status ldlt_factor(const double *Rm, const double *Lm, int64_t m, int64_t p, 
         if (!st && end < M) st = update(k0, end, M, P, s);
     }
     if (st) return st;
+    ahead.joined = true;
     if (m > 0) ldlt_growth_kernel<<<(unsigned)count, 256, 0, s>>>(growth, diag, M, m, d_failed);
     if (p > 0)
         ldlt_z_kernel<<<(unsigned)std::min<int64_t>(((int64_t)count * p * p + 255) / 256, 1024), 256, 0, s>>>(
