@@ -42,8 +42,17 @@ namespace {
 constexpr int kW = 16;         // sub-panel width
 constexpr int kNbMax = 128;    // outer panel width limit
 constexpr int kMaxCluster = 16;                // CTAs of a matrix's cluster
-constexpr int kNbResident = 64;               // of panel_resident_kernel
-constexpr size_t kResidentSmem = 180 * 1024;  // its slices' limit (44 KB are static): one CTA per SM, as the cluster form
+// Of panel_resident_kernel: columns, and shared memory for a slice beside the
+// static part, so that as many CTAs fit an SM as of the cluster form (one in
+// FP64, two in FP32).
+template <class T>
+constexpr int resident_nb() {
+    return sizeof(T) == 8 ? 64 : 128;
+}
+template <class T>
+constexpr size_t resident_smem() {
+    return (sizeof(T) == 8 ? 180 : 88) * 1024;
+}
 constexpr int kThreads = 256;
 constexpr int kBarrierStride = kGroupBarrierStride;
 
@@ -416,24 +425,33 @@ __device__ __forceinline__ void submul_rn(Cx<double> &y, Cx<double> f, Cx<double
     y.im = __dsub_rn(y.im, __fma_rn(f.im, x.re, __dmul_rn(f.re, x.im)));
 }
 
-// The cluster form in FP64 for slices that fit shared memory: a CTA keeps its
+// In FP32 the factors precondition a refinement; the roundings are free.
+__device__ __forceinline__ Cx<float> mul_rn(Cx<float> a, Cx<float> b) { return cmul(a, b); }
+__device__ __forceinline__ Cx<float> inverse_rn(Cx<float> p) { return cdiv(Cx<float>{1.f, 0.f}, p); }
+__device__ __forceinline__ void submul_rn(Cx<float> &y, Cx<float> f, Cx<float> x) { csubmul(y, f, x); }
+
+// The cluster form for slices that fit shared memory: a CTA keeps its
 // rows of the panel there (entry (row, t) at t ld + row) from the first column
 // to the last, so a column costs shared-memory and cluster latencies instead
 // of some ten dependent trips to L2 and back.  The pivot rows of a sub-panel
 // stay with every CTA (U), which solves U12 for itself: one cluster barrier per
 // column is all that is left.  The arithmetic of every entry is that of the
-// kernel above in the same order and with the same roundings, so the factors
-// agree bit for bit (a tie between two filaments' currents falls the same way).
+// kernel above in the same order and, in FP64, with the same roundings, so the
+// factors agree bit for bit (a tie between two filaments' currents falls the
+// same way).
 //
 // Bound by the chain of a column: the arg-max, the barrier, the trip through
 // distributed shared memory and the reciprocal.  Order 900, four matrices, a
-// panel of 64 columns: 376 us from device memory, 156 us here.
-__global__ void __launch_bounds__(kThreads, 1)
-    panel_resident_kernel(Cx<double> *__restrict__ a, int64_t m, int64_t K0, int NB, int *__restrict__ pivots,
+// panel of 64 columns: 376 us from device memory, 156 us here.  FP32 (mixed
+// sweeps of orders up to 512): 32 matrices of order 464 5.9 ms a sweep before,
+// 3.5 here.
+template <class T>
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
+    panel_resident_kernel(Cx<T> *__restrict__ a, int64_t m, int64_t K0, int NB, int *__restrict__ pivots,
                           int *__restrict__ singular, int per_matrix, int ld) {
     extern __shared__ __align__(16) unsigned char panel_smem[];
-    Cx<double> *S = reinterpret_cast<Cx<double> *>(panel_smem);
-    __shared__ Cx<double> U[kW][kNbResident];
+    Cx<T> *S = reinterpret_cast<Cx<T> *>(panel_smem);
+    __shared__ Cx<T> U[kW][resident_nb<T>()];
     __shared__ double s_val[kThreads / 32];
     __shared__ int s_idx[kThreads / 32];
     // every CTA's candidate, written here by its CTA; this one's panel row of its
@@ -441,10 +459,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     // of j
     __shared__ double c_val[2][kMaxCluster];
     __shared__ int c_row[2][kMaxCluster];
-    __shared__ Cx<double> c_data[2][kNbResident], c_rowj[2][kNbResident];
+    __shared__ Cx<T> c_data[2][resident_nb<T>()], c_rowj[2][resident_nb<T>()];
     auto cl = cooperative_groups::this_cluster();
     const int f = blockIdx.x / per_matrix, slice = blockIdx.x % per_matrix;
-    Cx<double> *A = a + (int64_t)f * m * m;
+    Cx<T> *A = a + (int64_t)f * m * m;
     const int rows = (int)(m - K0), chunk = (rows + per_matrix - 1) / per_matrix;
     // rows are counted from K0 on
     const int begin = slice * chunk, n = max(0, min(rows - begin, chunk));
@@ -461,8 +479,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             double best = -1.0;
             int bi = INT_MAX;
             for (int i = tid; i < n; i += kThreads) {
-                const Cx<double> v = S[j * ld + i];
-                const double n1 = fabs(v.re) + fabs(v.im);
+                const Cx<T> v = S[j * ld + i];
+                const double n1 = (double)(fabs(v.re) + fabs(v.im));
                 if (begin + i >= j && n1 > best) {  // rows ascend: ties keep the first
                     best = n1;
                     bi = begin + i;
@@ -534,8 +552,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                 pivots[(int64_t)f * m + K0 + j] = (int)(K0 + p);
             }
             if (tid < NB) {
-                const Cx<double> rj = cl.map_shared_rank(&c_rowj[par][0], (unsigned)(j / chunk))[tid];
-                const Cx<double> pr = p != j ? cl.map_shared_rank(&c_data[par][0], (unsigned)bslot)[tid] : rj;
+                const Cx<T> rj = cl.map_shared_rank(&c_rowj[par][0], (unsigned)(j / chunk))[tid];
+                const Cx<T> pr = p != j ? cl.map_shared_rank(&c_data[par][0], (unsigned)bslot)[tid] : rj;
                 U[c][tid] = pr;
                 if (p != j) {
                     if (p >= begin && p < begin + n) S[tid * ld + p - begin] = rj;
@@ -545,17 +563,17 @@ __global__ void __launch_bounds__(kThreads, 1)
             __syncthreads();
             // 4. scale by the pivot's reciprocal and rank-1 update inside the
             //    sub-panel: four lanes a row
-            const Cx<double> inv = inverse_rn(U[c][j]);
+            const Cx<T> inv = inverse_rn(U[c][j]);
             for (int i0 = 0; i0 < n; i0 += kThreads / 4) {
                 const int i = i0 + (tid >> 2);
                 const bool live = i < n && begin + i > j;
-                Cx<double> l{0.0, 0.0};
+                Cx<T> l{(T)0, (T)0};
                 if (live) l = mul_rn(S[j * ld + i], inv);
                 __syncwarp();
                 if (live) {
                     if ((tid & 3) == 0) S[j * ld + i] = l;
                     for (int q = c + 1 + (tid & 3); q < w; q += 4) {
-                        Cx<double> y = S[(s0 + q) * ld + i];
+                        Cx<T> y = S[(s0 + q) * ld + i];
                         submul_rn(y, U[c][s0 + q], l);
                         S[(s0 + q) * ld + i] = y;
                     }
@@ -568,7 +586,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         // 5. U12 of the sub-panel's pivot rows
         if (tid < rest) {
             const int t = s0 + kW + tid;
-            Cx<double> x[kW];
+            Cx<T> x[kW];
 #pragma unroll
             for (int r = 0; r < kW; ++r) x[r] = U[r][t];
 #pragma unroll
@@ -587,7 +605,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int first = max(0, s0 + kW - begin), below = n - first;
         for (int idx = tid; idx < below * rest; idx += kThreads) {
             const int i = first + idx % below, t = s0 + kW + idx / below;
-            Cx<double> y = S[t * ld + i];
+            Cx<T> y = S[t * ld + i];
 #pragma unroll
             for (int r = 0; r < kW; ++r) submul_rn(y, S[(s0 + r) * ld + i], U[r][t]);
             S[t * ld + i] = y;
@@ -735,16 +753,15 @@ fh_status panel_coop(LuBatch<T> &b, int64_t K0, int nb, const CoopScratch &cs, c
         attr.val.clusterDim.z = 1;
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
-        if constexpr (sizeof(T) == 8) {
-            if (nb <= kNbResident && resident <= kResidentSmem) {
-                auto kernel = panel_resident_kernel;
-                FHB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResidentSmem));
-                if (cs.per_matrix > 8)
-                    FHB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-                cfg.dynamicSmemBytes = resident;
-                FHB_CUDA(cudaLaunchKernelEx(&cfg, kernel, a, m, K0, nb, b.pivots, b.singular, cs.per_matrix, ld));
-                return FH_OK;
-            }
+        if (nb <= resident_nb<T>() && resident <= resident_smem<T>()) {
+            auto kernel = panel_resident_kernel<T>;
+            FHB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)resident_smem<T>()));
+            if (cs.per_matrix > 8)
+                FHB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            cfg.dynamicSmemBytes = resident;
+            FHB_CUDA(cudaLaunchKernelEx(&cfg, kernel, a, m, K0, nb, b.pivots, b.singular, cs.per_matrix, ld));
+            return FH_OK;
         }
         FHB_CUDA(cudaLaunchKernelEx(&cfg, panel_coop_kernel<T, true>, a, m, K0, nb, b.pivots, b.singular, args));
         return FH_OK;
