@@ -13,7 +13,9 @@ from fasterhenry_b200 import fixtures as F
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("legs,nw,nh", [(1, 4, 1), (2, 5, 3), (4, 6, 2), (5, 4, 3), (7, 10, 2), (9, 8, 2), (11, 10, 3)])
+@pytest.mark.parametrize("legs,nw,nh", [(1, 4, 1), (2, 5, 3), (4, 6, 2), (5, 4, 3), (7, 10, 2), (9, 8, 2), (11, 10, 3),
+                                        # orders 128, 130, 132, 510, 512, 516
+                                        (8, 3, 3), (5, 7, 2), (6, 4, 3), (15, 6, 3), (8, 11, 3), (6, 11, 4)])
 def test_mixed_matches_fp64(fh, legs, nw, nh):
     deck = F.meander_legs(legs, nw=nw, nh=nh)
     freqs = [1e6, 1e8, 1e10]
