@@ -1222,8 +1222,9 @@ fh_status lu_factor_deep(LuBatch<float> &b, LuWork &w, int nb, cudaStream_t s, f
         return fail(err, FH_ERR_INVALID_ARGUMENT, "two-level factorization needs a packed B operand scratch");
     C *xinv = reinterpret_cast<C *>(w.xinv), *dvec = reinterpret_cast<C *>(w.dvec);
     C *svec = fused ? dvec + (int64_t)count * outer : nullptr;
-    // X's blocks below its diagonal are read as zeros and never written.
-    if (fused) FHB_CUDA(cudaMemsetAsync(w.xinv, 0, sizeof(C) * (size_t)count * outer * outer, s));
+    // X's blocks below its diagonal are read as zeros and never written (an order
+    // of one super-panel has no rows below it, and no X).
+    if (fused && m > outer) FHB_CUDA(cudaMemsetAsync(w.xinv, 0, sizeof(C) * (size_t)count * outer * outer, s));
     // Look-ahead (fused form, with a second stream and a tile counter): the
     // diagonal region of each super-panel, its X and the packing of X (the
     // "front", a chain of small launches of one or two CTAs per matrix) run
