@@ -138,7 +138,7 @@ EXPORTS = [
     "fh_test_grid_convolution",
     "fh_system_layout", "fh_currents", "fh_system_create_coupled", "fh_system_coupling", "fh_iterative_filaments",
     "fh_iterative_layout", "fh_iterative_currents", "fh_test_coordinate_gradient", "fh_test_mesh_solve",
-    "fh_test_batch_solve", "fh_test_panel",
+    "fh_test_batch_solve", "fh_test_panel", "fh_test_panel_form",
 ]
 
 PROFILE_CLASSES = ["gemm_fp64", "gemm_fp32", "gemm_tc", "panel", "trsm", "solve", "residual", "pack", "gemm_tc_inner",
@@ -251,6 +251,8 @@ def load():
                                      ctypes.c_int32, c_double_p, c_double_p, P(ctypes.c_int32), ei]
     L.fh_test_panel.argtypes = [c_double_p, ctypes.c_int64, ctypes.c_int32, ctypes.c_int64, ctypes.c_int32,
                                 P(ctypes.c_int32), P(ctypes.c_int32), ei]
+    L.fh_test_panel_form.argtypes = [c_double_p, ctypes.c_int64, ctypes.c_int32, ctypes.c_int64, ctypes.c_int32,
+                                     ctypes.c_int32, ctypes.c_int32, P(ctypes.c_int32), P(ctypes.c_int32), ei]
     L.fh_test_batch_solve.argtypes = [c_double_p, c_double_p, ctypes.c_int64, ctypes.c_int64, c_double_p,
                                       ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, c_double_p, P(ctypes.c_int32), ei]
     L.fh_system_fill_stats.argtypes = [ctypes.c_void_p, P(FillStats)]

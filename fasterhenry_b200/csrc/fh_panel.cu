@@ -29,8 +29,10 @@
 // factorization, and every CTA returns.
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <climits>
 #include <mutex>
+#include <vector>
 
 #include "fh_cx.cuh"
 #include "fh_lu.cuh"
@@ -469,7 +471,9 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
     auto better = [](double v2, int i2, double v1, int i1) { return v2 > v1 || (v2 == v1 && i2 < i1); };
     for (int t = warp; t < NB; t += kThreads / 32)
         for (int i = lane; i < n; i += 32) S[t * ld + i] = A[K0 + begin + i + (K0 + t) * m];
-    __syncthreads();
+    // The slices are loaded, and every CTA of the cluster runs: only then may
+    // the first column's candidates be written into the others' shared memory.
+    cl.sync();
     for (int s0 = 0; s0 < NB; s0 += kW) {
         const int w = min(kW, NB - s0);
         for (int c = 0; c < w; ++c) {
@@ -752,7 +756,7 @@ fh_status panel_coop(LuBatch<T> &b, int64_t K0, int nb, const CoopScratch &cs, c
         attr.val.clusterDim.z = 1;
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
-        if (nb <= resident_nb<T>() && resident <= resident_smem<T>()) {
+        if (cs.resident && nb <= resident_nb<T>() && resident <= resident_smem<T>()) {
             auto kernel = panel_resident_kernel<T>;
             FHB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)resident_smem<T>()));
@@ -792,16 +796,20 @@ template fh_status panel_coop<float>(LuBatch<float> &, int64_t, int, const CoopS
 
 using namespace fhb;
 
-extern "C" fh_status fh_test_panel(double *a, int64_t m, int32_t count, int64_t k0, int32_t nb, int32_t *pivots,
-                                   int32_t *singular, fh_error_info *err) {
-    clear_error(err);
+namespace {
+
+// Factors columns [k0, k0 + nb) in place with the CTAs per matrix that a batch
+// of order `planned` gets.
+template <class T>
+fh_status test_panel(double *a, int64_t m, int32_t count, int64_t k0, int32_t nb, int64_t planned, bool resident,
+                     int32_t *pivots, int32_t *singular, fh_error_info *err) {
     if (!a || !pivots || !singular || count < 1 || nb < 1 || nb > kNbMax || k0 < 0 || k0 + nb > m)
         return fail(err, FH_ERR_INVALID_ARGUMENT, "null argument or panel beyond the matrix");
     fh_status st = ensure_device(err);
     if (st) return st;
     int per_matrix = 0;
     size_t bytes = 0;
-    st = coop_plan<double>(count, m - k0, &per_matrix, &bytes, err, 1);
+    st = coop_plan<T>(count, planned, &per_matrix, &bytes, err, 1);
     if (st) return st;
     void *d[4] = {};
     struct Release {
@@ -810,25 +818,43 @@ extern "C" fh_status fh_test_panel(double *a, int64_t m, int32_t count, int64_t 
             for (int k = 0; k < 4; ++k) cudaFree(d[k]);
         }
     } release{d};
-    const size_t size[4] = {16 * (size_t)count * m * m, 4 * (size_t)count * m, 4 * (size_t)count, bytes};
+    std::vector<T> h(a, a + 2 * (size_t)count * m * m);
+    const size_t size[4] = {sizeof(T) * h.size(), 4 * (size_t)count * m, 4 * (size_t)count, bytes};
     for (int k = 0; k < 4; ++k) {
         FHB_CUDA(cudaMalloc(&d[k], size[k]));
         FHB_CUDA(cudaMemset(d[k], 0, size[k]));
     }
-    FHB_CUDA(cudaMemcpy(d[0], a, size[0], cudaMemcpyHostToDevice));
+    FHB_CUDA(cudaMemcpy(d[0], h.data(), size[0], cudaMemcpyHostToDevice));
     CoopScratch cs;
-    coop_bind<double>(d[3], count, per_matrix, cs, 1);
-    LuBatch<double> b;
-    b.a = (double *)d[0];
+    coop_bind<T>(d[3], count, per_matrix, cs, 1);
+    cs.resident = cs.resident && resident;
+    LuBatch<T> b;
+    b.a = (T *)d[0];
     b.pivots = (int *)d[1];
     b.singular = (int *)d[2];
     b.m = m;
     b.count = count;
-    st = panel_coop<double>(b, k0, nb, cs, nullptr, err);
+    st = panel_coop<T>(b, k0, nb, cs, nullptr, err);
     if (!st) st = coop_check(cs, nullptr, err);
     if (st) return st;
-    FHB_CUDA(cudaMemcpy(a, d[0], size[0], cudaMemcpyDeviceToHost));
+    FHB_CUDA(cudaMemcpy(h.data(), d[0], size[0], cudaMemcpyDeviceToHost));
     FHB_CUDA(cudaMemcpy(pivots, d[1], size[1], cudaMemcpyDeviceToHost));
     FHB_CUDA(cudaMemcpy(singular, d[2], size[2], cudaMemcpyDeviceToHost));
+    std::copy(h.begin(), h.end(), a);
     return FH_OK;
+}
+
+}  // namespace
+
+extern "C" fh_status fh_test_panel(double *a, int64_t m, int32_t count, int64_t k0, int32_t nb, int32_t *pivots,
+                                   int32_t *singular, fh_error_info *err) {
+    clear_error(err);
+    return test_panel<double>(a, m, count, k0, nb, m - k0, true, pivots, singular, err);
+}
+
+extern "C" fh_status fh_test_panel_form(double *a, int64_t m, int32_t count, int64_t k0, int32_t nb, int32_t single,
+                                        int32_t resident, int32_t *pivots, int32_t *singular, fh_error_info *err) {
+    clear_error(err);
+    return single ? test_panel<float>(a, m, count, k0, nb, m, resident != 0, pivots, singular, err)
+                  : test_panel<double>(a, m, count, k0, nb, m, resident != 0, pivots, singular, err);
 }

@@ -512,6 +512,12 @@ fh_status fh_test_mesh_solve(const double *r, const double *l, int64_t m, int64_
  * was exactly zero. */
 fh_status fh_test_panel(double *a, int64_t m, int32_t count, int64_t k0, int32_t nb, int32_t *pivots,
                         int32_t *singular, fh_error_info *err);
+/* The same with the CTAs per matrix that a factorization of order m plans (its
+ * later panels leave some without rows), in FP64 or (single: entries rounded on
+ * entry) FP32, with the slices in shared memory where they fit (resident) or in
+ * device memory. */
+fh_status fh_test_panel_form(double *a, int64_t m, int32_t count, int64_t k0, int32_t nb, int32_t single,
+                             int32_t resident, int32_t *pivots, int32_t *singular, fh_error_info *err);
 /* As fh_test_mesh_solve (Z only) through the batched kernel, in one of its tile configurations, the
  * first `grouped` frequencies by groups of CTAs. */
 fh_status fh_test_batch_solve(const double *r, const double *l, int64_t m, int64_t p, const double *omega,
