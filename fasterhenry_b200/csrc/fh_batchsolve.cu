@@ -188,7 +188,7 @@ __device__ __forceinline__ void solve_item(double2 *tiles, double *growth, doubl
             if (tid < E) sh.rowsum[tid] = 0.0;
             __syncthreads();
             if (ti == j) {
-                DiagBlock<E, kBT / 32> block;
+                DiagBlock<E, kBT / 32, false> block;
                 block.factor(sh.v, smem, kPad, E, nb, smem, kPad, sh.dinv, sh.rowsum, &sh.bad);
                 __syncthreads();
                 if (nb < E) {  // the last tile ends with the ports

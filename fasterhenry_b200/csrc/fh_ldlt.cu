@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(kDiagThreads64) ldlt_diag_kernel(double2 *__re
                                                                    double *__restrict__ growth,
                                                                    int *__restrict__ failed) {
     __shared__ double2 v[2 * kLd];
-    DiagBlock<kLd, kDiagThreads64 / 32> block;
+    DiagBlock<kLd, kDiagThreads64 / 32, true> block;
     block.factor(v, a + (int64_t)blockIdx.x * M * M + k0 + k0 * M, M, nb, nb,
                  xinv + (int64_t)blockIdx.x * xinv_stride, kLd, dinv + (int64_t)blockIdx.x * kLd, growth + (int64_t)blockIdx.x * M + k0, failed + blockIdx.x);
 }

@@ -39,11 +39,11 @@ __device__ __forceinline__ void sub_mul(double2 &y, double2 l, double2 t) {
 
 // The first nb steps on a diagonal block of `rows` rows (nb <= rows <= NB) by one
 // CTA of WARPS warps: L below its diagonal and D on it, in place in A (leading
-// dimension M); L^-1 (unit lower, zeros above) in X's first nb rows and the
-// Schur complement of the other rows in its trailing corner (leading dimension
-// ldx; X may be A); D^-1; the rows' growth added to G.  v: 2 NB entries of
-// shared memory.  Gauss-Jordan
-// in one array: until step k place (i, k) holds the Schur complement's entry,
+// dimension M) where KEEP asks for them; L^-1 (unit lower, zeros above) in X's
+// first nb rows and the Schur complement of the other rows in its trailing
+// corner (leading dimension ldx; without KEEP X may be A, whose places take no
+// other store); D^-1; the rows' growth added to G.  v: 2 NB entries of shared
+// memory.  Gauss-Jordan in one array: until step k place (i, k) holds the Schur complement's entry,
 // after it the entry of L^-1, which starts as -l_ik; step j takes l_ij times v
 // from row i, where v is row j of L^-1 left of the pivot and column j of the
 // complement beyond it.
@@ -57,7 +57,7 @@ __device__ __forceinline__ void sub_mul(double2 &y, double2 l, double2 t) {
 // Bound by its chain of NB steps of one barrier, one division and some forty
 // dependent instructions: 38 us for 64 with 16 warps (88 us with a row per
 // thread, whose columns' cases diverge in every step).
-template <int NB, int WARPS>
+template <int NB, int WARPS, bool KEEP>
 struct DiagBlock {
     static_assert((NB == 32 || NB == 64) && (WARPS == 8 || WARPS == 16), "rows lane and lane + 32");
     static constexpr int kLo = 32 / WARPS, kCols = NB / WARPS, kHi = NB == 64 ? kCols : 0;
@@ -100,11 +100,11 @@ struct DiagBlock {
                 for (int c = 0; c < kCols; ++c) {
                     if (c == JC && w == jw) {  // L's column, and the start of L^-1's
                         if (upper && r0 > j) {
-                            if (r0 < rows) A[r0 + (int64_t)j * M] = l0;
+                            if (KEEP && r0 < rows) A[r0 + (int64_t)j * M] = l0;
                             lo[jl] = make_double2(-l0.x, -l0.y);
                         }
                         if (NB == 64 && r1 > j) {
-                            if (r1 < rows) A[r1 + (int64_t)j * M] = l1;
+                            if (KEEP && r1 < rows) A[r1 + (int64_t)j * M] = l1;
                             hi[jh] = make_double2(-l1.x, -l1.y);
                         }
                     } else {
@@ -120,7 +120,7 @@ struct DiagBlock {
                     if (r1 == j) sum1 += fabs(d.x) + fabs(d.y);
                 }
                 if (w == WARPS - 1 && lane == 0) {
-                    A[j + (int64_t)j * M] = d;
+                    if (KEEP) A[j + (int64_t)j * M] = d;
                     dinv[j] = inv;
                     if (!isfinite(inv.x) || !isfinite(inv.y) || !isfinite(d.x) || !isfinite(d.y)) *failed = 1;
                 }
