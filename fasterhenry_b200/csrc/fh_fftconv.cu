@@ -69,6 +69,7 @@
 #include <algorithm>
 #include <cmath>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "fh_device.cuh"
@@ -320,6 +321,7 @@ __device__ __forceinline__ void twiddle(double2 (&v)[R], const double2 *__restri
 // runs fastest over the threads.
 enum Layout {
     kStrided,  // t 2^lg + l, lines first
+    kWide,     // the same; places in device memory beyond 32-bit indices
     kContig,   // l pitch + t, points first
     kThin      // l pitch + t, lines first (any number of lines)
 };
@@ -348,7 +350,12 @@ __device__ __forceinline__ void fft_stage(typename Cplx<T>::type *buf, const Fft
     const int S = ax.S[st], nb = ax.m / R;
     const V *__restrict__ tw = tw_all + ax.tw[st];
     const int total = LAYOUT == kThin ? nb * g.count : nb << lg;
-    auto at = [&](int t, int l) { return LAYOUT == kStrided ? (t << lg) + l : l * pitch + t; };
+    constexpr bool kLines = LAYOUT == kStrided || LAYOUT == kWide;
+    auto at = [&](int t, int l) { return kLines ? (t << lg) + l : l * pitch + t; };
+    auto place = [&](int t, int l) -> std::conditional_t<LAYOUT == kWide, int64_t, int> {
+        if constexpr (LAYOUT == kWide) return (int64_t)t * g.inner + l;
+        else return t * g.inner + l;
+    };
     for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
         int l, j;
         if (LAYOUT == kContig) {
@@ -365,13 +372,13 @@ __device__ __forceinline__ void fft_stage(typename Cplx<T>::type *buf, const Fft
         const int k = j - b * S;
         const int t0 = b * R * S + k;
         V v[R];
-        const bool live = LAYOUT != kStrided || l < g.count;
+        const bool live = !kLines || l < g.count;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const int t = t0 + r * S;
             if (GIN) {
                 v[r] = cmake((T)0, (T)0);
-                if (live && t < g.n_in) v[r] = g.src[t * g.inner + l];
+                if (live && t < g.n_in) v[r] = g.src[place(t, l)];
                 if (DIT) v[r] = cswap(v[r]);
             } else {
                 v[r] = buf[at(t, l)];
@@ -382,7 +389,7 @@ __device__ __forceinline__ void fft_stage(typename Cplx<T>::type *buf, const Fft
         if (MID) {
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                const T s = live ? spectrum[(t0 + r * S) * g.inner + l] : (T)0;
+                const T s = live ? spectrum[place(t0 + r * S, l)] : (T)0;
                 v[r] = cmake(s * v[r].y, s * v[r].x);  // swapped: the inverse begins
             }
             dft<R>(v);
@@ -392,7 +399,7 @@ __device__ __forceinline__ void fft_stage(typename Cplx<T>::type *buf, const Fft
         for (int r = 0; r < R; ++r) {
             const int t = t0 + r * S;
             if (GOUT) {
-                if (live && t < g.keep) g.dst[t * g.inner + l] = DIT || MID ? cswap(v[r]) : v[r];
+                if (live && t < g.keep) g.dst[place(t, l)] = DIT || MID ? cswap(v[r]) : v[r];
             } else {
                 buf[at(t, l)] = v[r];
             }
@@ -442,7 +449,9 @@ constexpr int kThinLeast = 4, kThinMost = 16;
 // 2^lg lines of consecutive c (tail tiles: fewer).  kFused: forward, times
 // spectrum[t inner + c] (real), and back; in and out may be the same array,
 // since a CTA reads its whole tile before it writes and tiles are disjoint.
-template <class T, int KIND>
+// LAYOUT kWide: len x inner may pass 2^31 (axis 0 of the largest tori), for a
+// sixth more time on the fused step.
+template <class T, int KIND, int LAYOUT>
 __global__ void __launch_bounds__(fft_threads<T>(), 2)
     fft_strided_kernel(const typename Cplx<T>::type *in, typename Cplx<T>::type *out, int64_t in_stride,
                        int64_t out_stride, int64_t outer, int inner, int n_in, int keep, FftAxis ax, int lg,
@@ -465,26 +474,26 @@ __global__ void __launch_bounds__(fft_threads<T>(), 2)
         g.dst = out + (int64_t)blockIdx.y * out_stride + o * keep * inner + c0;
         const T *spec = KIND == kFused ? spectrum + c0 : nullptr;
         if (last == 0) {
-            fft_stage_any<T, kStrided, KIND == kInverse, true, true, KIND == kFused>(buf, ax, 0, lg, 0, tw, g, spec);
+            fft_stage_any<T, LAYOUT, KIND == kInverse, true, true, KIND == kFused>(buf, ax, 0, lg, 0, tw, g, spec);
             continue;
         }
         if (KIND != kInverse) {
-            fft_stage_any<T, kStrided, false, true, false, false>(buf, ax, 0, lg, 0, tw, g, spec);
+            fft_stage_any<T, LAYOUT, false, true, false, false>(buf, ax, 0, lg, 0, tw, g, spec);
             for (int st = 1; st < last; ++st) {
                 __syncthreads();
-                fft_stage_any<T, kStrided, false, false, false, false>(buf, ax, st, lg, 0, tw, g, spec);
+                fft_stage_any<T, LAYOUT, false, false, false, false>(buf, ax, st, lg, 0, tw, g, spec);
             }
             __syncthreads();
-            fft_stage_any<T, kStrided, false, false, KIND == kForward, KIND == kFused>(buf, ax, last, lg, 0, tw, g, spec);
+            fft_stage_any<T, LAYOUT, false, false, KIND == kForward, KIND == kFused>(buf, ax, last, lg, 0, tw, g, spec);
         }
         if (KIND != kForward) {
-            if (KIND == kInverse) fft_stage_any<T, kStrided, true, true, false, false>(buf, ax, last, lg, 0, tw, g, spec);
+            if (KIND == kInverse) fft_stage_any<T, LAYOUT, true, true, false, false>(buf, ax, last, lg, 0, tw, g, spec);
             for (int st = last - 1; st > 0; --st) {
                 __syncthreads();
-                fft_stage_any<T, kStrided, true, false, false, false>(buf, ax, st, lg, 0, tw, g, spec);
+                fft_stage_any<T, LAYOUT, true, false, false, false>(buf, ax, st, lg, 0, tw, g, spec);
             }
             __syncthreads();
-            fft_stage_any<T, kStrided, true, false, true, false>(buf, ax, 0, lg, 0, tw, g, spec);
+            fft_stage_any<T, LAYOUT, true, false, true, false>(buf, ax, 0, lg, 0, tw, g, spec);
         }
         __syncthreads();  // the next tile's first stage writes the buffer
     }
@@ -718,11 +727,15 @@ fh_status axis_step(const void *in, void *out, int64_t in_stride, int64_t out_st
             static_cast<const V *>(in), static_cast<V *>(out), in_stride, out_stride, outer, n_in, keep, ax, lg,
             magic_of(n_in), magic_of(keep), static_cast<const V *>(tw));
     } else {
-        FHB_CUDA(cudaFuncSetAttribute(fft_strided_kernel<T, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
-        fft_strided_kernel<T, KIND><<<grid, fft_threads<T>(), smem, s>>>(
-            static_cast<const V *>(in), static_cast<V *>(out), in_stride, out_stride, outer, (int)inner, n_in, keep, ax,
-            lg, static_cast<const V *>(tw), spectrum);
+        auto kernel = fft_strided_kernel<T, KIND, kStrided>;
+        // axis 0 of more than 2^31 points; along axis 1 (inner = m2) there are
+        // never as many
+        if constexpr (KIND == kFused || (KIND == kForward && sizeof(T) == 8))
+            if ((int64_t)ax.m * inner > INT32_MAX) kernel = fft_strided_kernel<T, KIND, kWide>;
+        FHB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kernel<<<grid, fft_threads<T>(), smem, s>>>(static_cast<const V *>(in), static_cast<V *>(out), in_stride,
+                                                    out_stride, outer, (int)inner, n_in, keep, ax, lg,
+                                                    static_cast<const V *>(tw), spectrum);
     }
     FHB_CUDA(cudaGetLastError());
     return FH_OK;
