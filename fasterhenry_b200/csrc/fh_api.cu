@@ -17,44 +17,9 @@
 #include "fh_batchsolve.h"
 #include "fh_device.cuh"
 #include "fh_lu.cuh"
+#include "fh_pool.h"
 
 using namespace fhb;
-
-// Device workspace of a system's sweeps, kept between calls: one buffer per
-// role (slot), grown when a sweep needs more.  Repeated sweeps then allocate
-// nothing, and no cudaFree (which synchronizes the device) runs inside a
-// sweep after the first.
-struct DevPool {
-    std::vector<std::pair<void *, size_t>> slot;
-    cudaStream_t stream = nullptr;  // the owner's stream: allocations and frees are ordered on it
-    ~DevPool() { release(); }
-    void release() {
-        for (auto &b : slot)
-            if (b.first) cache_free(b.first, stream);
-        slot.clear();
-    }
-    size_t held() const {
-        size_t t = 0;
-        for (const auto &b : slot) t += b.second;
-        return t;
-    }
-    cudaError_t get(int id, size_t bytes, void **out) {
-        if ((int)slot.size() <= id) slot.resize((size_t)id + 1, {nullptr, 0});
-        auto &b = slot[(size_t)id];
-        if (b.second < bytes) {
-            if (b.first) cache_free(b.first, stream);
-            b = {nullptr, 0};
-            const cudaError_t e = cache_alloc(&b.first, std::max<size_t>(bytes, 1), stream);
-            if (e != cudaSuccess) {
-                b.first = nullptr;
-                return e;
-            }
-            b.second = bytes;
-        }
-        *out = b.first;
-        return cudaSuccess;
-    }
-};
 
 struct fh_system {
     DevPool pool;
@@ -101,8 +66,6 @@ struct fh_system {
     // resistances on the device (parts of d_basis): R_ee x of the refinement
     // residuals.
     unsigned char *d_basis = nullptr;
-    // Frequencies per batch that the workspace has held before, by precision.
-    size_t held[3] = {0, 0, 0};
     int64_t *d_rp = nullptr, *d_toff = nullptr;
     int32_t *d_br = nullptr, *d_tloop = nullptr;
     double *d_sign = nullptr, *d_tsign = nullptr, *d_R = nullptr;
@@ -1180,11 +1143,11 @@ fh_status fh_sweep(fh_system *sys, const double *freqs, size_t nf, fh_precision 
                                                    16.0 * kOuterFp32 * kOuterFp32 + 8.0 * kNbFp32 * kOuterFp32
                                              : 0.0);
     // Frequencies per batch from free device memory (the analogue of the
-    // reference's 2 GiB sweep budget, solve.rs:91 and 884).  A batch that the
-    // workspace has held before needs no look at the free memory, a query that
-    // takes from 0.1 ms to several: its buffers are still there.
+    // reference's 2 GiB sweep budget, solve.rs:91 and 884).  A batch whose
+    // buffers the workspace holds needs no look at the free memory, a query
+    // that takes from 0.1 ms to several.
     int chunk = (int)nf;
-    if (nf > sys->held[precision]) {
+    if (nf > sys->pool.batch[precision]) {
         size_t free_b = 0, total_b = 0;
         FHB_CUDA(cudaMemGetInfo(&free_b, &total_b));
         // Own workspace is reused; memory the cache holds idle is available too.
@@ -1215,7 +1178,7 @@ fh_status fh_sweep(fh_system *sys, const double *freqs, size_t nf, fh_precision 
             e = sweep_chunk_fp64(sys, d_omega.p, count, nullptr, d_z.p, singular.data() + c0, &ms_factor, err);
         }
         if (e) return e;
-        sys->held[precision] = std::max(sys->held[precision], (size_t)count);
+        sys->pool.batch[precision] = std::max(sys->pool.batch[precision], (size_t)count);
         FHB_CUDA(cudaMemcpyAsync(z_out + 2 * c0 * p * p, d_z.p, 16 * (size_t)count * p * p, cudaMemcpyDeviceToHost, st));
         FHB_CUDA(cudaStreamSynchronize(st));
         // Refinement that did not converge: redo those frequencies in FP64.
