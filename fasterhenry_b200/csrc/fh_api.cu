@@ -1624,6 +1624,7 @@ fh_status fh_gradient(fh_system *sys, double frequency_hz, const fh_param_spec *
     // 4. Derivative fills and the products with the branch currents.
     size_t free_b = 0, total_b = 0;
     FHB_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    free_b += cache_idle_bytes();  // its buffers come from the cache
     const size_t part = gradient_part_elems(n, (int)p);
     const double need = (want_dims ? 16.0 : 0.0) * (double)n * (double)n +
                         (want_coords ? 32.0 * (double)n * (double)n + 64.0 * (double)(n * p) : 0.0) +
