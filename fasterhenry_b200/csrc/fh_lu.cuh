@@ -30,7 +30,7 @@ struct CoopScratch {
     void *rowj = nullptr;         // row j of each matrix, count * 2 * 128 complex
     int per_matrix = 0;           // CTAs per matrix
     bool cluster = false;         // the CTAs of a matrix form one thread-block cluster
-    bool resident = true;         // which may keep its slices in shared memory
+    bool resident = false;        // which the device can launch with slices in shared memory
 };
 
 // Workspace for the factorization (pivot search partials).  With `coop`

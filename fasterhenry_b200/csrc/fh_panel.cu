@@ -620,17 +620,38 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
     cl.sync();  // no CTA leaves while another may still read its shared memory
 }
 
-}  // namespace
+// Clusters of `size` CTAs of a kernel that the device can hold at once (0:
+// none can be launched), for sizes up to kMaxCluster.
+int clusters_at_once(const void *kernel, int size, size_t dynamic_smem) {
+    if ((size > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
+        (dynamic_smem && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)dynamic_smem) != cudaSuccess)) {
+        cudaGetLastError();
+        return 0;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)size);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = dynamic_smem;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)size;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return clusters;
+}
 
-// Largest cluster of CTAs of the cluster form that the device can schedule
-// (0: none), for sizes up to kMaxCluster.
-
-template <class T>
-int cluster_fits_query(int size);
-
-// cluster_fits_query, asked once per device and size (the occupancy query
-// costs milliseconds; sweeps ask on every batch).
-template <class T>
+// Of the cluster form, or of the one with its slices in shared memory: asked
+// once per device and size (the occupancy query costs milliseconds; sweeps ask
+// on every batch).
+template <class T, bool kResident>
 int cluster_fits(int size) {
     if (size < 2 || size > kMaxCluster) return 0;
     static std::mutex mu;
@@ -643,36 +664,15 @@ int cluster_fits(int size) {
     }
     std::lock_guard<std::mutex> lk(mu);
     if (!asked[dev][size]) {
-        known[dev][size] = cluster_fits_query<T>(size);
+        known[dev][size] =
+            kResident ? clusters_at_once((const void *)panel_resident_kernel<T>, size, resident_smem<T>())
+                      : clusters_at_once((const void *)panel_coop_kernel<T, true>, size, 0);
         asked[dev][size] = true;
     }
     return known[dev][size];
 }
 
-template <class T>
-int cluster_fits_query(int size) {
-    auto kernel = panel_coop_kernel<T, true>;
-    if (size > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)size);
-    cfg.blockDim = dim3(kThreads);
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = (unsigned)size;
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, (void *)kernel, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    return clusters;
-}
+}  // namespace
 
 template <class T>
 fh_status coop_plan(int count, int64_t m, int *per_matrix, size_t *bytes, fh_error_info *err, int share) {
@@ -691,7 +691,7 @@ fh_status coop_plan(int count, int64_t m, int *per_matrix, size_t *bytes, fh_err
     // second wave of clusters would double the panel's time.
     if (pm >= 2 && pm <= kMaxCluster) {
         int size = pm;
-        while (size >= 2 && cluster_fits<T>(size) < count * std::max(1, share)) --size;
+        while (size >= 2 && cluster_fits<T, false>(size) < count * std::max(1, share)) --size;
         if (size >= 2) pm = size;
     }
     if ((int64_t)pm * count > capacity)
@@ -706,7 +706,7 @@ fh_status coop_plan(int count, int64_t m, int *per_matrix, size_t *bytes, fh_err
 template <class T>
 bool coop_cluster(int count, int per_matrix, int share) {
     return per_matrix >= 2 && per_matrix <= kMaxCluster &&
-           cluster_fits<T>(per_matrix) >= count * std::max(1, share);
+           cluster_fits<T, false>(per_matrix) >= count * std::max(1, share);
 }
 
 template <class T>
@@ -727,6 +727,7 @@ void coop_bind(void *mem, int count, int per_matrix, CoopScratch &cs, int share)
     cs.rowj = p + off;
     cs.per_matrix = per_matrix;
     cs.cluster = coop_cluster<T>(count, per_matrix, share);
+    cs.resident = cs.cluster && cluster_fits<T, true>(per_matrix) > 0;
 }
 
 template <class T>

@@ -72,3 +72,14 @@ def test_each_form_matches_numpy(fh, m, count, k0, nb, single, resident):
     got, piv = factor(a, k0, nb, single, resident)
     for f in range(min(count, 2)):
         check(a[f], got[f], piv[f], k0, nb, 1.5e-4 if single else 3e-13)
+
+
+def test_a_plan_without_a_cluster(fh):
+    """A plan of one CTA a matrix is no cluster: neither form, and the same
+    result whichever is asked for."""
+    rng = np.random.default_rng(5)
+    a = rng.standard_normal((2, 60, 60)) + 1j * rng.standard_normal((2, 60, 60))
+    want, piv = factor(a, 0, 60, 0, 0)
+    got, piv2 = factor(a, 0, 60, 0, 1)
+    assert np.array_equal(piv, piv2) and np.array_equal(got, want)
+    check(a[0], got[0], piv[0], 0, 60, 3e-13)
