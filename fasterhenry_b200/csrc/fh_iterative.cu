@@ -154,7 +154,13 @@ using cplx = std::complex<double>;
 
 }  // namespace
 
-struct fh_iterative {
+// A system's stream, given back after everything that frees on it.
+struct OwnStream {
+    cudaStream_t stream = nullptr;
+    ~OwnStream() { stream_release(stream); }
+};
+
+struct fh_iterative : OwnStream {
     Discretized disc;
     LoopBasis loops;
     std::vector<double> resistances;
@@ -163,7 +169,6 @@ struct fh_iterative {
     fh_timing timing{};
     GmresParams gp;
     PfftDevice op;
-    cudaStream_t stream = nullptr;
     // Host blocks of M R M^T and M L M^T (column-major (m x p), (p x p)).
     std::vector<double> r_ep, l_ep, r_pp, l_pp, r_diag, l_diag;
     // Device: loop basis rows and its transpose over the internal loops.
@@ -796,10 +801,7 @@ fh_status fh_iterative_currents(fh_iterative *s, const double *freqs, size_t nf,
 }
 
 void fh_iterative_destroy(fh_iterative *s) {
-    if (!s) return;
-    cudaStream_t cs = s->stream;
     delete s;
-    stream_release(cs);
 }
 
 fh_status fh_test_gmres_dense(const double *a, size_t n, const double *b, double *x, const double *precond,
