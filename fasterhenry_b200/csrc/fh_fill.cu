@@ -1000,6 +1000,14 @@ __device__ __forceinline__ void integrand_coord(const QuadCtx &c, double u, doub
     }
 }
 
+// The distance of the cross-sections of two parallel bars, and their largest side.
+__device__ __forceinline__ double cross_section_gap(const Aligned &b, double *side) {
+    const double gu = rmax(fabs(b.offset[1]) - 0.5 * (b.width[0] + b.width[1]), 0.0);
+    const double gv = rmax(fabs(b.offset[2]) - 0.5 * (b.height[0] + b.height[1]), 0.0);
+    *side = rmax(rmax(b.width[0], b.width[1]), rmax(b.height[0], b.height[1]));
+    return hypot(gu, gv);
+}
+
 // The coordinate derivatives of a pair whose cross-sections lie far apart
 // against their size, without the panel tree: a p x p Gauss rule on each of
 // the overlap weights' break-point panels (the integrand is a product of
@@ -1010,10 +1018,8 @@ __device__ __forceinline__ void integrand_coord(const QuadCtx &c, double u, doub
 // of the reference the values agreed to 2e-11, 7e-13 and 8e-12 in those
 // bands (random pairs of 50-400 um bars with 0.2-3 um sides).
 __device__ __forceinline__ int far_rule_order(const Aligned &b) {
-    const double gu = rmax(fabs(b.offset[1]) - 0.5 * (b.width[0] + b.width[1]), 0.0);
-    const double gv = rmax(fabs(b.offset[2]) - 0.5 * (b.height[0] + b.height[1]), 0.0);
-    const double g = hypot(gu, gv);
-    const double side = rmax(rmax(b.width[0], b.width[1]), rmax(b.height[0], b.height[1]));
+    double side;
+    const double g = cross_section_gap(b, &side);
     if (g >= 4.0 * side) return 4;
     if (g >= 2.0 * side) return 5;
     if (g >= side) return 6;
@@ -2073,14 +2079,28 @@ struct CoordClass {
 
 __device__ __forceinline__ int bump_order(int o) { return o < kMaxRule - 1 ? o + 1 : o; }
 
-// Terms of a point sum per m x m points of a panel at which the panels' product
-// rule takes over for parallel pairs of two segments.  Measured on a graded
-// spiral of 3,672 filaments: 5.8 ns a key of that rule (four to nine panels of
-// 16 to 36 points) against 16 ns a pair of 5,000 terms (1.7 M of them, 8e9
-// terms, 27 to 31.5 ms): even at about 1,700 terms for nine panels of m = 4.
-// The rule is the more accurate one (1e-11 against the point orders' 1e-8
-// estimate).
-constexpr int kFarTerms = 120;
+// Terms of a point sum at which the panels' product rule takes over for
+// parallel pairs of two segments.  Measured on a graded spiral of 3,672
+// filaments: 5.8 ns a key of that rule (four to nine panels of 16 points)
+// against 16 ns a pair of 5,000 terms (1.7 M of them, 8e9 terms, 27 to 31.5
+// ms): even at about 1,700 terms for nine panels.
+constexpr int kFarTerms = 1920;
+
+// Whether the rule is the more accurate one, too.  Its error falls with the
+// cross-sections' gap g against their largest side s; and since it takes the
+// sideways derivative from the weights' slope, one of a pair much further
+// apart along the bars than across them is a small difference.  2,997 pairs of
+// 50-400 um bars with 0.3-100 um sides at g >= 8 s and no further apart along
+// the bars than g: rms errors of the derivatives along, across, by stretch and
+// by rotation 6e-13, 1e-12, 2e-14 and 7e-11, where the point sums have 8e-10,
+// 6e-11, 3e-11 and 5e-9.  At 4 s <= g < 8 s the rule is off by up to 2e-9
+// across, and by 1.5e-8 for bars nearly in one line; the point sums by 5e-10
+// and 1e-10.
+__device__ __forceinline__ bool far_rule_better(const Aligned &b) {
+    double side;
+    const double g = cross_section_gap(b, &side);
+    return g >= 8.0 * side && fabs(b.offset[0]) - 0.5 * (b.length[0] + b.length[1]) <= g;
+}
 
 __device__ CoordClass coord_classify(const DevFil &fi, const DevFil &fj, bool same) {
     CoordClass c{-1, 0, 0, 0, false};
@@ -2122,14 +2142,10 @@ __device__ CoordClass coord_classify(const DevFil &fi, const DevFil &fj, bool sa
     bool point = point_orders(a, gap, oa) && point_orders(b, gap, ob);
     if (point && oa[0] * oa[1] * oa[2] * ob[0] * ob[1] * ob[2] > 4096) point = false;
     // A pair that the point rule could take goes by the panels' product rule
-    // where that is cheaper (kFarTerms) and its frame allows.
-    bool rule = false;
-    if (point && !same) {
-        const int m = far_rule_order(ab);
-        const int terms = bump_order(oa[0]) * bump_order(oa[1]) * bump_order(oa[2]) * bump_order(ob[0]) *
-                          bump_order(ob[1]) * bump_order(ob[2]);
-        rule = m > 0 && terms > kFarTerms * m * m;
-    }
+    // where that is cheaper and as accurate, and its frame allows.
+    const bool rule = point && !same && far_rule_better(ab) &&
+                      bump_order(oa[0]) * bump_order(oa[1]) * bump_order(oa[2]) * bump_order(ob[0]) *
+                              bump_order(ob[1]) * bump_order(ob[2]) > kFarTerms;
     if (point && !rule) {
         c.cat = kCoordCatPoint;
         c.orders = pack();
