@@ -228,8 +228,8 @@ int outer_for(int64_t m, TrailingUpdate mode) {
 // Factor + solve + Schur for `count` frequencies in FP64 with partial
 // pivoting.  d_x (count x m x p complex) receives the solutions; z (count x p
 // x p) the impedances.
-fh_status sweep_chunk_pivoted(fh_system *s, const double *d_omega, int count, double *d_x, double *d_z, int *h_singular,
-                           float *ms_factor, fh_error_info *err) {
+fh_status sweep_chunk_pivoted(fh_system *s, const double *d_omega, int count, double *d_x, double *d_z,
+                              int *h_singular, float *ms_factor, fh_error_info *err) {
     const int64_t m = s->m, p = s->p, ld = s->nloops;
     cudaStream_t st = s->stream;
     if (m > 0) {
@@ -291,10 +291,13 @@ fh_status sweep_chunk_pivoted(fh_system *s, const double *d_omega, int count, do
 }
 
 // The FP64 form of `count` frequencies: L D L^T without interchanges
-// (fh_ldlt.cu), and the frequencies whose matrix that does not suit (an
-// inductance matrix made indefinite, for instance by a truncated coupling, or
-// a singular system) again with partial pivoting, which decides whether they
-// are singular.  d_x may be null where only Z is wanted.
+// (fh_ldlt.cu), and the frequencies whose matrix that does not suit (one that
+// the fill's rounding makes indefinite, one whose pivots have no finite
+// reciprocal, a singular system) again with partial pivoting, which decides
+// whether they are singular.  Such a list is factored twice; a truncated
+// coupling does not cause it, since its groups are transitive and the
+// inductance matrix stays block diagonal and definite.  d_x may be null where
+// only Z is wanted.
 fh_status sweep_chunk_fp64(fh_system *s, const double *d_omega, int count, double *d_x, double *d_z, int *h_singular,
                            float *ms_factor, fh_error_info *err) {
     const int64_t m = s->m, p = s->p, M = s->nloops;
@@ -612,9 +615,10 @@ fh_status sweep_chunk_mixed(fh_system *s, const double *d_omega, int count, doub
 // fh_batch_sweep in a mixed precision: every (system, frequency) of the
 // systems with m <= FH_BATCH_MAX_ORDER in one persistent launch
 // (fh_batchsolve.cu), largest first; items whose elimination without
-// interchanges was rejected are redone by the FP64 sweep.  Frequencies are checked per system first:
-// a system with an invalid frequency is left to the per-system path, which
-// reports it.  done[i] is set for the systems finished here.
+// interchanges was rejected are redone by the FP64 sweep.  Frequencies are
+// checked per system first: a system with an invalid frequency is left to the
+// per-system path, which reports it.  done[i] is set for the systems finished
+// here.
 fh_status batch_sweep_persistent(fh_system *const *systems, size_t k, const double *const *freqs, const size_t *nf,
                                  double *const *z_out, std::vector<char> &done, fh_error_info *err) {
     std::vector<size_t> take;
@@ -1411,7 +1415,8 @@ fh_status fh_currents(fh_system *sys, const double *freqs, size_t nf, const doub
         if (!mixed || redo) {  // refinement that did not converge: the whole batch in FP64
             // With partial pivoting: the filament of largest |J| is a tie
             // wherever a bundle is symmetric, which the last bits decide, and
-            // the reference decides it by this elimination.
+            // the reference decides it by this elimination.  (The last bits
+            // of the inductances are the fill's own, so it is a tie still.)
             e = sweep_chunk_pivoted(sys, d_omega.p, count, d_x.p, d_z.p, singular.data(), &ms_factor, err);
             if (e) return e;
         }

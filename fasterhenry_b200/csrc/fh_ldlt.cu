@@ -1,6 +1,6 @@
 // Batched FP64 factorization of the mesh system without interchanges,
 // A = L D L^T with a unit lower triangular L (no conjugation), for the FP64
-// sweep, the filament currents and the gradient.
+// sweep and the gradient.
 //
 // Z_ee = R_ee + j w L_ee is complex symmetric, and with both parts positive
 // definite elimination without pivoting is stable (N. J. Higham, Math. Comp.
@@ -17,14 +17,16 @@
 //
 // Nothing is assumed of the matrix: the factors' backward error is bounded by
 // u |L| |D| |L|^T, whose diagonal sum_k |l_ik|^2 |d_k| is accumulated row by
-// row as the panels go.  A matrix with a row above kGrowthLimit |a_ii| (it is about
-// |a_ii| for the class above), or with a zero or non-finite pivot, is
+// row as the panels go.  A matrix with a row above kGrowthLimit |a_ii| (it is
+// about |a_ii| for the class above), or with a zero or non-finite pivot, is
 // reported as failed, and the caller factors it with partial pivoting.
 //
-// Per panel of 64 columns, three launches over all matrices:
+// Per panel of 64 columns, launches over all matrices:
 //   ldlt_diag_kernel    the 64 x 64 diagonal block's L and D, and L^-1;
 //   ldlt_panel_kernel   B = A21 L11^-T, L21 = B D^-1 for the rows below;
-//   ldlt_update_kernel  A22 -= L21 B^T on the tiles on and below the diagonal.
+// and A22 -= L21 B^T by ldlt_update_kernel on the tiles on and below the
+// diagonal: of the next panel's columns alone within a group of up to four
+// panels (ldlt_depth), of the rest of the matrix once per group.
 // The products run on the FP64 tensor cores (mma.sync f64: tcgen05 has no FP64
 // kind), as four real products of split real and imaginary parts.
 #include <cuda_runtime.h>
@@ -78,7 +80,8 @@ __global__ void __launch_bounds__(kDiagThreads64) ldlt_diag_kernel(double2 *__re
     __shared__ double2 v[2 * kLd];
     DiagBlock<kLd, kDiagThreads64 / 32, true> block;
     block.factor(v, a + (int64_t)blockIdx.x * M * M + k0 + k0 * M, M, nb, nb,
-                 xinv + (int64_t)blockIdx.x * xinv_stride, kLd, dinv + (int64_t)blockIdx.x * kLd, growth + (int64_t)blockIdx.x * M + k0, failed + blockIdx.x);
+                 xinv + (int64_t)blockIdx.x * xinv_stride, kLd, dinv + (int64_t)blockIdx.x * kLd,
+                 growth + (int64_t)blockIdx.x * M + k0, failed + blockIdx.x);
 }
 
 // Rows [c0, M) of the panel [k0, k0 + nb): B = A21 L11^-T into `panel`
@@ -141,9 +144,10 @@ __global__ void __launch_bounds__(kLdThreads, 2)
 }
 
 // A -= L B^T over the columns [k0, k0 + nb) of L on rows and columns from base:
-// the whole lower triangle (end = M) or its columns [base, end);
-// one 64 x 64 tile on or below the diagonal per CTA, k in stages of 16 through two buffers of asynchronous copies, both operands
-// [k][row] with re and im side by side (one 16-byte load per fragment).
+// the whole lower triangle (end = M) or its columns [base, end); one 64 x 64
+// tile on or below the diagonal per CTA, k in stages of 16 through two buffers
+// of asynchronous copies, both operands [k][row] with re and im side by side
+// (one 16-byte load per fragment).
 //
 // Bound by the FP64 tensor pipe: 8 nb operations per complex entry against 32
 // bytes of C.  Order 2,321 x 32 matrices with nb = 64: 19.0 ms in all, 29

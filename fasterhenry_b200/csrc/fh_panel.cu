@@ -43,7 +43,7 @@ namespace {
 
 constexpr int kW = 16;         // sub-panel width
 constexpr int kNbMax = 128;    // outer panel width limit
-constexpr int kMaxCluster = 16;                // CTAs of a matrix's cluster
+constexpr int kMaxCluster = 16;  // CTAs of a matrix's cluster
 // Of panel_resident_kernel: columns, and shared memory for a slice beside the
 // static part, so that as many CTAs fit an SM as of the cluster form (one in
 // FP64, two in FP32).
@@ -74,9 +74,9 @@ struct CoopArgs {
 // the cluster's hardware barrier.  Otherwise the CTAs of a cooperative launch
 // exchange them through global memory and meet at a bounded counter barrier.
 template <class T, bool kCluster>
-__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1) panel_coop_kernel(Cx<T> *__restrict__ a, int64_t m, int64_t K0, int NB,
-                                                              int *__restrict__ pivots, int *__restrict__ singular,
-                                                              CoopArgs args) {
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
+    panel_coop_kernel(Cx<T> *__restrict__ a, int64_t m, int64_t K0, int NB, int *__restrict__ pivots,
+                      int *__restrict__ singular, CoopArgs args) {
     const int per_matrix = args.per_matrix;
     const int f = blockIdx.x / per_matrix, slice = blockIdx.x % per_matrix;
     Cx<T> *A = a + (int64_t)f * m * m;
@@ -444,8 +444,10 @@ __device__ __forceinline__ void submul_rn(Cx<float> &y, Cx<float> f, Cx<float> x
 //
 // Bound by the chain of a column: the arg-max, the barrier, the trip through
 // distributed shared memory and the reciprocal.  Order 900, four matrices, a
-// panel of 64 columns: 376 us from device memory, 156 us here.  FP32: 32
-// matrices of order 464 in panels of 128 columns 5.4 ms before, 3.0 here.
+// panel of 64 columns: 376 us from device memory, 156 us here.  FP32 (panels of
+// 128 columns; the mixed form up to order 128, the form without tensor cores at
+// any): 40 matrices of order 128 0.89 and 0.28 ms; of order 504, whose first
+// panel's slices do not fit, 3.82 and 1.92 for the four.
 template <class T>
 __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
     panel_resident_kernel(Cx<T> *__restrict__ a, int64_t m, int64_t K0, int NB, int *__restrict__ pivots,

@@ -547,8 +547,8 @@ fh_status pfft_device_setup(const PfftSetup &st, const fh_filament *fil, const N
     FHB_CUDA(cudaMemsetAsync(d_touched, 0, scratch_cells, s));
     FHB_CUDA(cudaMemsetAsync(d_flag, 0, 16, s));
     FHB_CUDA(cudaMemsetAsync(d_counts + n, 0, 8, s));
-    project_kernel<<<(unsigned)((n + kProjWarps - 1) / kProjWarps), 32 * kProjWarps, 0, s>>>(d_fil, n, g, st.radius, d_boxes, d_scratch, d_touched,
-                                                               d_counts, d_flag);
+    project_kernel<<<(unsigned)((n + kProjWarps - 1) / kProjWarps), 32 * kProjWarps, 0, s>>>(
+        d_fil, n, g, st.radius, d_boxes, d_scratch, d_touched, d_counts, d_flag);
     FHB_CUDA(cudaGetLastError());
     // Row offsets of the projection: exclusive sum of the counts.
     FHB_CUDA(persist(&out.proj_off, (size_t)n + 1, s));
